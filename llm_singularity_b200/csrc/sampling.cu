@@ -1,4 +1,4 @@
-// Next-token sampling on the device, one thread block per row of logits.
+// Next-token sampling on the device, one thread-block cluster per row of logits.
 //
 // Order of operations is the reference sampler's (core/src/sampling.cpp:11-118):
 //   repetition penalty on previously generated tokens (positive logit / penalty, else
@@ -6,50 +6,48 @@
 //   top-k (others dropped) -> top-p (smallest set of most probable tokens whose mass
 //   exceeds p) -> softmax over what is left -> the first index whose cumulative
 //   probability reaches the uniform draw u.
-// The reference sorts on the host; here the k-th largest value and the top-p cut are found
-// by bisection on the order-preserving integer image of the floats (32 passes over the
-// row at most), so nothing is sorted and nothing leaves the device.  Ties at the k-th
-// value are all kept.  The uniform draw comes from the caller (a counter-based generator
+// The reference sorts on the host.  Here nothing is sorted and nothing leaves the device.  Ties at the
+// k-th value are all kept.  The uniform draw comes from the caller (a counter-based generator
 // keyed by the request's seed and its count of generated tokens), which makes a request's
-// tokens independent of what else is in the batch.  All arithmetic is 32-bit.
+// tokens independent of what else is in the batch.
 //
-// `work` is scratch of the same shape as the logits, used only by rows that apply a
-// repetition penalty.
+// What bounds it is the number of times a row is walked and the blocks that walk it.  A row's logits are
+// read once: each block of the cluster keeps its contiguous slice (already divided by the
+// temperature) in shared memory.  The k-th largest value and the top-p cut are found with one histogram over
+// the values, linear from the row's maximum to its minimum, whose counts and masses the blocks add up through
+// distributed shared memory; the bucket the cut falls into is then collected (a few values) and the
+// cut picked among them exactly, by counting.  A bucket with more than kList values (rows whose values are all
+// but equal, or with outliers that stretch the range) is bisected instead, on the order-preserving integer image of the
+// floats, as many as 32 passes over the slices.  128 rows of 128,256 logits (greedy, temperature, top-k,
+// top-p and both in turn): 1,430 us with one block a row and bisection throughout, MEASURED_US us so.
+//
+// Probabilities are exp(x - max) in 32-bit; their sums are taken on 64-bit integers (exp * 2^44, so that even a
+// tail of values below 1e-9 counts), which makes every sum exact and the same whatever order the blocks add in.
+//
+// `work` is scratch of the same shape as the logits, used only where a slice does not fit shared memory
+// (lsb_sample_needs_work).
 #include "common.cuh"
 
+#include <cooperative_groups.h>
 #include <float.h>
+
+namespace cg = cooperative_groups;
 
 LSB_DEFINE_STATUS()
 
-constexpr int kSampleThreads = 1024;
+typedef unsigned long long u64;
+
+constexpr int kThreads = 512;
+constexpr int kWarps = kThreads / 32;
+constexpr int kMaxBlocks = 8;                 // blocks of a row's cluster (the portable size)
+constexpr int kSliceTarget = 8192;            // logits a block takes before another one joins the cluster
+constexpr int kBuckets = 1024;                // of the histogram, two a thread
+constexpr int kList = 1024;                   // values of one bucket that are picked among directly
+constexpr int kSliceBytes = 184 * 1024;       // most shared memory for a slice
 
 __device__ __forceinline__ unsigned int ordered(float f) {
     const unsigned int u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-struct BlockScratch {
-    float f[33];
-    int i[33];
-};
-
-__device__ __forceinline__ float block_sum_f(float v, BlockScratch& s) { return lsb_block_sum(v, s.f); }
-
-__device__ __forceinline__ int block_sum_i(int v, BlockScratch& s) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) s.i[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        int t = lane < nwarps ? s.i[lane] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) s.i[32] = t;
-    }
-    __syncthreads();
-    return s.i[32];
 }
 
 // (value, index) maximum with the lowest index winning ties
@@ -57,247 +55,459 @@ __device__ __forceinline__ void argmax_merge(float& v, int& i, float ov, int oi)
     if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
 
-__device__ __forceinline__ void block_argmax(float& v, int& idx, BlockScratch& s) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+struct Part {                                 // what a block has found in its slice
+    float mx, mn;
+    int mi;
+};
+
+struct Shared {
+    Part part;
+    u64 slot[2];                              // a block's count or mass, by turns (bisection)
+    u64 seg[kWarps];                          // kept mass of each warp's stretch of the slice
+    u64 all_seg[kMaxBlocks * kWarps];         // ... of the whole row
+    u64 scratch[kWarps];
+    float scratch_f[2 * kWarps];
+    int scratch_i[kWarps];
+    unsigned int cnt[kBuckets];               // this block's histogram
+    u64 mass[kBuckets];
+    unsigned int tot_cnt[kBuckets];           // the row's, the same in every block
+    u64 tot_mass[kBuckets];
+    float list[kList];                        // (of the cluster's first block) values of one bucket
+    u64 list_mass[kList];
+    unsigned int list_n;
+    unsigned int thr_k, thr_p;                // the two cuts, broadcast by the first block
+    u64 kept;                                 // ... and the mass of the k-th value's bucket that is kept
+    int found;                                // bucket picked by find_bucket, and what stands before it
+    u64 before;
+};
+
+__device__ __forceinline__ u64 warp_sum(u64 v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        argmax_merge(v, idx, ov, oi);
-    }
-    __syncthreads();
-    if (lane == 0) { s.f[warp] = v; s.i[warp] = idx; }
-    __syncthreads();
-    if (warp == 0) {
-        float tv = lane < nwarps ? s.f[lane] : -FLT_MAX;
-        int ti = lane < nwarps ? s.i[lane] : 0x7fffffff;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, tv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, ti, o);
-            argmax_merge(tv, ti, ov, oi);
-        }
-        if (lane == 0) { s.f[32] = tv; s.i[32] = ti; }
-    }
-    __syncthreads();
-    v = s.f[32];
-    idx = s.i[32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
-// A greedy row without a repetition penalty is scanned by kGreedyParts blocks (blockIdx.y), each its
-// slice; the partial maxima meet in device memory and the block that arrives last picks the first
-// maximum among them (the order of arrival does not matter: ties go to the lowest index).  One block
-// reading a row of 128,256 logits took 12 - 14 us, as long as a layer of the decode step.  Every other
-// row is the work of its first block alone.
-constexpr int kGreedyParts = 16;
-constexpr int kGreedyRows = 1024;                 // rows beyond this are scanned by one block each
-__device__ float greedy_part_v[kGreedyRows * kGreedyParts];
-__device__ int greedy_part_i[kGreedyRows * kGreedyParts];
-__device__ unsigned int greedy_arrived[kGreedyRows];
+__device__ __forceinline__ u64 block_sum(u64 v, Shared& s) {
+    v = warp_sum(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s.scratch[threadIdx.x >> 5] = v;
+    __syncthreads();
+    u64 t = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) t += s.scratch[w];
+    return t;
+}
+
+// The first bucket at which the running sum of val(b) passes ok(before, inclusive); every thread gets it
+// (kBuckets: none) together with the sum before it.
+template <typename Val, typename Ok>
+__device__ __forceinline__ int find_bucket(Shared& s, u64& before, Val val, Ok ok) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const u64 a = val(2 * tid), b = val(2 * tid + 1);
+    u64 run = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 up = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += up;
+    }
+    __syncthreads();
+    if (lane == 31) s.scratch[warp] = run;
+    if (tid == 0) { s.found = kBuckets; s.before = 0; }
+    __syncthreads();
+    u64 base = run - (a + b);
+    for (int w = 0; w < warp; ++w) base += s.scratch[w];
+    // (the condition turns true once along the buckets: exactly one thread finds the turn)
+    if (!ok(base, 0) && ok(base + a, 1)) { s.found = 2 * tid; s.before = base; }
+    else if (!ok(base + a, 0) && ok(base + a + b, 1)) { s.found = 2 * tid + 1; s.before = base + a; }
+    __syncthreads();
+    before = s.before;
+    return s.found;
+}
 
 // params per row: {temperature, top_p, repetition_penalty, u}
-__global__ void __launch_bounds__(kSampleThreads)
-sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vocab,
-              const float* __restrict__ params, const int* __restrict__ top_ks,
-              const int* __restrict__ prev_start, const int* __restrict__ prev_tokens,
-              int* __restrict__ out) {
-    __shared__ BlockScratch sc;
-    __shared__ float chunk_sum[kSampleThreads];
+__global__ void __launch_bounds__(kThreads, 2)
+sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vocab, int slice, int slice_in_smem,
+              float mass_scale, const float* __restrict__ params, const int* __restrict__ top_ks,
+              const int* __restrict__ prev_start, const int* __restrict__ prev_tokens, int* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ Shared s;
+    cg::cluster_group cluster = cg::this_cluster();
     lsb_pdl_launch_dependents();
     lsb_pdl_wait();
-    const int row = blockIdx.x, tid = threadIdx.x;
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int blocks = (int)gridDim.z, rank = (int)blockIdx.z;
     const float temperature = params[row * 4 + 0], top_p = params[row * 4 + 1];
     const float penalty = params[row * 4 + 2], u = params[row * 4 + 3];
     const int top_k = top_ks[row];
-    const float* src = logits + (size_t)row * vocab;
-
+    const int i0 = min(vocab, rank * slice), n = min(vocab, i0 + slice) - i0;      // this block's slice
+    const float* src = logits + (size_t)row * vocab + i0;
+    float* xs = slice_in_smem ? reinterpret_cast<float*>(dyn) : work + (size_t)row * vocab + i0;
     const int pb = prev_start ? prev_start[row] : 0, pe = prev_start ? prev_start[row + 1] : 0;
-    const int parts = (int)gridDim.y;
-    const bool shared_scan = parts > 1 && temperature == 0.0f && !(penalty != 1.0f && pe > pb);
-    if (blockIdx.y > 0 && !shared_scan) return;
-    if (penalty != 1.0f && pe > pb) {
-        float* w = work + (size_t)row * vocab;
-        for (int i = tid; i < vocab; i += kSampleThreads) w[i] = src[i];
-        __syncthreads();
-        if (tid == 0) {
-            for (int j = pb; j < pe; ++j) {
-                const int t = prev_tokens[j];
-                if (t >= 0 && t < vocab) w[t] = w[t] > 0.f ? w[t] / penalty : w[t] * penalty;
-            }
-        }
-        __syncthreads();
-        src = w;
-    }
+    const bool penalised = penalty != 1.0f && pe > pb;
+    const bool greedy = temperature == 0.0f;
+    const bool cut_k = !greedy && top_k > 0 && top_k < vocab, cut_p = !greedy && top_p < 1.0f;
 
-    if (temperature == 0.0f) {
-        float bv = -FLT_MAX;
-        int bi = 0x7fffffff;
-        // (one block reads the whole row: four 16-byte loads in flight per thread; with one 4-byte
-        // load at a time a row of 128,256 took 14 us, the length of a layer of the decode step)
-        if ((vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-            const float4* s4 = reinterpret_cast<const float4*>(src);
-            int n4 = vocab >> 2, first4 = 0;
-            if (shared_scan) {                      // this block's slice of the row
-                const int per = (n4 + parts - 1) / parts;
-                first4 = min(n4, (int)blockIdx.y * per);
-                n4 = min(n4, first4 + per);
-            }
-            for (int i0 = first4 + tid; i0 < n4; i0 += 4 * kSampleThreads) {
-                float4 v[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int i = i0 + q * kSampleThreads;
-                    v[q] = i < n4 ? s4[i] : make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int i = 4 * (i0 + q * kSampleThreads);
-                    if (i < 4 * n4) {
-                        argmax_merge(bv, bi, v[q].x, i);
-                        argmax_merge(bv, bi, v[q].y, i + 1);
-                        argmax_merge(bv, bi, v[q].z, i + 2);
-                        argmax_merge(bv, bi, v[q].w, i + 3);
-                    }
-                }
-            }
-        } else {
-            int b = 0, e = vocab;
-            if (shared_scan) {
-                const int per = (vocab + parts - 1) / parts;
-                b = min(vocab, (int)blockIdx.y * per);
-                e = min(vocab, b + per);
-            }
-            for (int i = b + tid; i < e; i += kSampleThreads) argmax_merge(bv, bi, src[i], i);
-        }
-        block_argmax(bv, bi, sc);
-        if (!shared_scan) {
-            if (tid == 0) out[row] = bi;
-            return;
-        }
-        __shared__ bool last;
-        if (tid == 0) {
-            greedy_part_v[row * kGreedyParts + blockIdx.y] = bv;
-            greedy_part_i[row * kGreedyParts + blockIdx.y] = bi;
-            __threadfence();
-            last = atomicAdd(&greedy_arrived[row], 1u) == (unsigned int)parts - 1u;
-        }
-        __syncthreads();
-        if (!last) return;
-        if (tid < 32) {
-            __threadfence();
-            float v = -FLT_MAX;
-            int idx = 0x7fffffff;
-            if (tid < parts) {
-                v = __ldcg(&greedy_part_v[row * kGreedyParts + tid]);
-                idx = __ldcg(&greedy_part_i[row * kGreedyParts + tid]);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                argmax_merge(v, idx, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, idx, o));
-            if (tid == 0) {
-                out[row] = idx;
-                greedy_arrived[row] = 0u;           // for the next launch
-            }
-        }
-        return;
-    }
-    // x_i = src[i] / temperature, recomputed in every pass (division as the reference does)
-#define X(i) (src[i] / temperature)
-
-    float mx = -FLT_MAX;
+    // ---- the slice into place (a greedy row without a penalty is only looked at), its extremes
+    float mx = -FLT_MAX, mn = FLT_MAX;
     int mi = 0x7fffffff;
-    for (int i = tid; i < vocab; i += kSampleThreads) argmax_merge(mx, mi, X(i), i);
-    block_argmax(mx, mi, sc);
-
-    unsigned int thr = 0u;                       // keep x with ordered(x) >= thr
-    if (top_k > 0 && top_k < vocab) {
-        unsigned int lo = 0u, hi = 0xffffffffu;  // count(>= lo) >= k always holds
-        while (lo < hi) {
-            const unsigned int mid = lo + (hi - lo) / 2u + ((hi - lo) & 1u);
-            int c = 0;
-            for (int i = tid; i < vocab; i += kSampleThreads) c += ordered(X(i)) >= mid;
-            c = block_sum_i(c, sc);
-            if (c >= top_k) lo = mid; else hi = mid - 1u;
+    auto see = [&](float x, int i) {
+        argmax_merge(mx, mi, x, i0 + i);
+        if (x > -INFINITY) mn = fminf(mn, x);
+    };
+    const bool keep = !greedy || penalised;
+    if (penalised) {
+        for (int i = tid; i < n; i += kThreads) xs[i] = src[i];
+        __syncthreads();
+        for (int j = pb; j < pe; ++j) {                       // in order; a token is one thread's alone
+            const int t = prev_tokens[j] - i0;
+            if (t >= 0 && t < n && t % kThreads == tid) xs[t] = xs[t] > 0.f ? xs[t] / penalty : xs[t] * penalty;
         }
-        thr = lo;
-    }
-    if (top_p < 1.0f) {
-        float tot = 0.f;
-        for (int i = tid; i < vocab; i += kSampleThreads) {
-            const float x = X(i);
-            if (ordered(x) >= thr) tot += expf(x - mx);
+        __syncthreads();
+        for (int i = tid; i < n; i += kThreads) {
+            const float x = greedy ? xs[i] : xs[i] / temperature;
+            if (!greedy) xs[i] = x;
+            see(x, i);
         }
-        tot = block_sum_f(tot, sc);
-        // smallest v with mass(x > v) <= top_p * tot; everything >= v is kept
-        unsigned int lo = thr, hi = ordered(mx);
-        while (lo < hi) {
-            const unsigned int mid = lo + (hi - lo) / 2u;
-            float mass = 0.f;
-            for (int i = tid; i < vocab; i += kSampleThreads) {
-                const float x = X(i);
-                if (ordered(x) > mid) mass += expf(x - mx);
+    } else if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(xs) & 15) == 0) {
+        const float4* s4 = reinterpret_cast<const float4*>(src);
+        const int n4 = n >> 2;
+        for (int q0 = tid; q0 < n4; q0 += 4 * kThreads) {     // four 16-byte loads in flight
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (q0 + k * kThreads < n4) v[k] = s4[q0 + k * kThreads];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int q = q0 + k * kThreads;
+                if (q < n4) {
+                    if (keep) {
+                        v[k].x /= temperature; v[k].y /= temperature; v[k].z /= temperature; v[k].w /= temperature;
+                        reinterpret_cast<float4*>(xs)[q] = v[k];
+                    }
+                    see(v[k].x, 4 * q); see(v[k].y, 4 * q + 1); see(v[k].z, 4 * q + 2); see(v[k].w, 4 * q + 3);
+                }
             }
-            mass = block_sum_f(mass, sc);
-            if (mass <= top_p * tot) hi = mid; else lo = mid + 1u;
         }
-        thr = lo;
+        for (int i = 4 * n4 + tid; i < n; i += kThreads) {
+            const float x = keep ? src[i] / temperature : src[i];
+            if (keep) xs[i] = x;
+            see(x, i);
+        }
+    } else {
+        for (int i = tid; i < n; i += kThreads) {
+            const float x = keep ? src[i] / temperature : src[i];
+            if (keep) xs[i] = x;
+            see(x, i);
+        }
     }
-
-    // inverse CDF in index order: thread t owns the contiguous chunk [t*per, (t+1)*per)
-    const int per = (vocab + kSampleThreads - 1) / kSampleThreads;
-    const int b = min(vocab, tid * per), e = min(vocab, b + per);
-    float mine = 0.f;
-    for (int i = b; i < e; ++i) {
-        const float x = X(i);
-        if (ordered(x) >= thr) mine += expf(x - mx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        argmax_merge(mx, mi, __shfl_xor_sync(0xffffffffu, mx, o), __shfl_xor_sync(0xffffffffu, mi, o));
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
     }
-    chunk_sum[tid] = mine;
+    if (lane == 0) { s.scratch_f[warp] = mx; s.scratch_i[warp] = mi; s.scratch_f[kWarps + warp] = mn; }
+    if (cut_k || cut_p)
+        for (int b = tid; b < kBuckets; b += kThreads) { s.cnt[b] = 0u; s.mass[b] = 0ull; }
     __syncthreads();
     if (tid == 0) {
-        float total = 0.f;
-        for (int t = 0; t < kSampleThreads; ++t) total += chunk_sum[t];
-        const float target = u * total;
-        // the first chunk at which the running sum reaches the target; chunks without a kept token
-        // are passed over, so that if rounding leaves the sum short of the target at the very end,
-        // the scan below ends on the last kept token (the reference's fallback, sampling.cpp:113-116)
-        float run = 0.f, before = 0.f;
-        int t = -1, last_full = 0;
-        for (int c = 0; c < kSampleThreads; ++c) {
-            if (!(chunk_sum[c] > 0.f)) continue;
-            last_full = c;
-            before = run;
-            if (run + chunk_sum[c] >= target) { t = c; break; }
-            run += chunk_sum[c];
+        for (int w = 1; w < kWarps; ++w) {
+            argmax_merge(mx, mi, s.scratch_f[w], s.scratch_i[w]);
+            mn = fminf(mn, s.scratch_f[kWarps + w]);
         }
-        if (t < 0) t = last_full;
-        run = before;
-        const int tb = min(vocab, t * per), te = min(vocab, tb + per);
-        int pick = -1, last_kept = -1;
-        for (int i = tb; i < te; ++i) {
-            const float x = X(i);
-            if (ordered(x) >= thr) {
-                run += expf(x - mx);
-                last_kept = i;
-                if (run >= target) { pick = i; break; }
+        s.part = Part{mx, mn, mi};
+        s.list_n = 0u;
+    }
+    cluster.sync();
+    {
+        mx = -FLT_MAX; mn = FLT_MAX; mi = 0x7fffffff;
+        for (int r = 0; r < blocks; ++r) {
+            const Part p = *cluster.map_shared_rank(&s.part, r);
+            argmax_merge(mx, mi, p.mx, p.mi);
+            mn = fminf(mn, p.mn);
+        }
+    }
+    if (greedy) {
+        if (rank == 0 && tid == 0) out[row] = mi;
+        cluster.sync();                                       // (a peer may still read this block's part)
+        return;
+    }
+
+    // exp(x - max) as an integer; a value that is not a number counts nothing
+    auto mass_of = [&](float x) -> u64 {
+        const float e = expf(x - mx);
+        return e > 0.f ? __float2ull_rn(e * mass_scale) : 0ull;
+    };
+    unsigned int thr = 0u;                                    // keep x with ordered(x) >= thr
+    if (cut_k || cut_p) {
+        // ---- the histogram: bucket 0 holds the maximum; a larger value never has a later bucket
+        const float inv = mx > mn ? (float)(kBuckets - 1) / (mx - mn) : 0.f;
+        auto bucket = [&](float x) { return max(0, (int)fminf((mx - x) * inv, (float)(kBuckets - 1))); };
+        for (int i = tid; i < n; i += kThreads) {
+            const float x = xs[i];
+            const int b = bucket(x);
+            atomicAdd(&s.cnt[b], 1u);
+            if (cut_p) {
+                const u64 m = mass_of(x);
+                if (m) atomicAdd(&s.mass[b], m);
             }
         }
-        if (pick < 0) pick = last_kept >= 0 ? last_kept : mi;   // rounding at the very end
-        out[row] = pick;
+        cluster.sync();
+        const int share = kBuckets / blocks;                  // (blocks is a power of two)
+        for (int j = tid; j < share; j += kThreads) {
+            const int b = rank * share + j;
+            unsigned int c = 0u;
+            u64 m = 0ull;
+            for (int r = 0; r < blocks; ++r) {
+                c += *cluster.map_shared_rank(&s.cnt[b], r);
+                m += *cluster.map_shared_rank(&s.mass[b], r);
+            }
+            for (int r = 0; r < blocks; ++r) {
+                *cluster.map_shared_rank(&s.tot_cnt[b], r) = c;
+                *cluster.map_shared_rank(&s.tot_mass[b], r) = m;
+            }
+        }
+        cluster.sync();
+        // the row's sum of val(x) over all slices (bisection only)
+        int turn = 0;
+        auto row_sum = [&](auto val) -> u64 {
+            u64 c = 0ull;
+            for (int i = tid; i < n; i += kThreads) c += val(xs[i]);
+            c = block_sum(c, s);
+            if (tid == 0) s.slot[turn] = c;
+            cluster.sync();
+            u64 t = 0ull;
+            for (int r = 0; r < blocks; ++r) t += *cluster.map_shared_rank(&s.slot[turn], r);
+            turn ^= 1;
+            return t;
+        };
+        // the values of one bucket that are >= thr, in the first block's list
+        auto collect = [&](int b) {
+            unsigned int* count = cluster.map_shared_rank(&s.list_n, 0);
+            float* list = cluster.map_shared_rank(&s.list[0], 0);
+            for (int i = tid; i < n; i += kThreads) {
+                const float x = xs[i];
+                if (bucket(x) == b && ordered(x) >= thr) {
+                    const unsigned int at = atomicAdd(count, 1u);
+                    if (at < (unsigned int)kList) list[at] = x;
+                }
+            }
+            cluster.sync();
+        };
+        int k_bucket = kBuckets;                               // the bucket of the k-th value
+        u64 k_mass = 0ull;                                     // mass of its values that are kept
+        bool listed = false;                                   // the first block's list holds it
+        if (cut_k) {
+            u64 before;
+            const u64 k = (u64)top_k;
+            k_bucket = find_bucket(s, before, [&](int b) { return (u64)s.tot_cnt[b]; },
+                                   [&](u64 sum, int) { return sum >= k; });
+            if (k_bucket < kBuckets && s.tot_cnt[k_bucket] <= (unsigned int)kList) {
+                collect(k_bucket);
+                listed = true;
+                if (rank == 0) {
+                    const int m = (int)min(s.list_n, (unsigned int)kList);
+                    const u64 r = k - before;                  // the r-th largest of the list
+                    if (tid == 0) s.thr_k = 0u;
+                    __syncthreads();
+                    for (int i = tid; i < m; i += kThreads) {
+                        const unsigned int o = ordered(s.list[i]);
+                        u64 above = 0ull, same = 0ull;
+                        for (int j = 0; j < m; ++j) {
+                            const unsigned int oj = ordered(s.list[j]);
+                            above += oj > o;
+                            same += oj == o;
+                        }
+                        if (above < r && r <= above + same) s.thr_k = o;    // (equal values write the same)
+                    }
+                    __syncthreads();
+                    const unsigned int t = s.thr_k;
+                    u64 kept = 0ull;
+                    if (cut_p)
+                        for (int i = tid; i < m; i += kThreads)
+                            if (ordered(s.list[i]) >= t) kept += mass_of(s.list[i]);
+                    kept = block_sum(kept, s);
+                    if (tid == 0)
+                        for (int o = 0; o < blocks; ++o) {
+                            *cluster.map_shared_rank(&s.thr_k, o) = t;
+                            *cluster.map_shared_rank(&s.kept, o) = kept;
+                        }
+                }
+                cluster.sync();
+                thr = s.thr_k;
+                k_mass = s.kept;
+            } else {
+                unsigned int lo = 0u, hi = 0xffffffffu;        // count(>= lo) >= k always holds
+                while (lo < hi) {
+                    const unsigned int mid = lo + (hi - lo) / 2u + ((hi - lo) & 1u);
+                    if (row_sum([&](float x) { return (u64)(ordered(x) >= mid); }) >= k) lo = mid;
+                    else hi = mid - 1u;
+                }
+                thr = lo;
+                if (cut_p && k_bucket < kBuckets)
+                    k_mass = row_sum([&](float x) { return bucket(x) == k_bucket && ordered(x) >= thr ? mass_of(x) : 0ull; });
+            }
+        }
+        if (cut_p) {
+            // mass of bucket b that is kept so far: all of it before the k-th value's bucket, none behind
+            auto kept_mass = [&](int b) { return b < k_bucket ? s.tot_mass[b] : b == k_bucket ? k_mass : 0ull; };
+            const u64 tot = block_sum(kept_mass(2 * tid) + kept_mass(2 * tid + 1), s);
+            const double most = (double)top_p * (double)tot;
+            // the smallest v with mass(x > v) <= top_p * tot; everything >= v is kept
+            u64 before;
+            const int b = find_bucket(s, before, kept_mass, [&](u64 sum, int) { return (double)sum > most; });
+            if (b == kBuckets) {
+                // nothing exceeds it: no mass at all (thr stays), or a negative top_p (the maximum alone)
+                if (most < 0.0) thr = ordered(mx);
+            } else if (s.tot_cnt[b] <= (unsigned int)kList) {
+                if (!(listed && b == k_bucket)) {
+                    if (rank == 0 && tid == 0) s.list_n = 0u;
+                    cluster.sync();
+                    collect(b);
+                }
+                if (rank == 0) {
+                    const int m = (int)min(s.list_n, (unsigned int)kList);
+                    if (tid == 0) s.thr_p = ordered(mx);
+                    for (int i = tid; i < m; i += kThreads) s.list_mass[i] = mass_of(s.list[i]);
+                    __syncthreads();
+                    for (int i = tid; i < m; i += kThreads) {
+                        const unsigned int o = ordered(s.list[i]);
+                        if (o < thr) continue;
+                        u64 above = before;
+                        for (int j = 0; j < m; ++j)
+                            if (ordered(s.list[j]) > o) above += s.list_mass[j];
+                        if ((double)above <= most) atomicMin(&s.thr_p, o);
+                    }
+                    __syncthreads();
+                    if (tid == 0)
+                        for (int o = 0; o < blocks; ++o) *cluster.map_shared_rank(&s.thr_p, o) = s.thr_p;
+                }
+                cluster.sync();
+                thr = s.thr_p;
+            } else {
+                unsigned int lo = thr, hi = ordered(mx);
+                while (lo < hi) {
+                    const unsigned int mid = lo + (hi - lo) / 2u;
+                    const u64 above = row_sum([&](float x) { return ordered(x) > mid ? mass_of(x) : 0ull; });
+                    if ((double)above <= most) hi = mid; else lo = mid + 1u;
+                }
+                thr = lo;
+            }
+        }
     }
-#undef X
+
+    // ---- inverse CDF in index order: every warp owns a stretch of the slice, its kept mass meets the others'
+    const int stretch = (slice + kThreads - 1) / kThreads * 32;
+    const int b0 = min(n, warp * stretch), b1 = min(n, b0 + stretch);
+    auto kept_of = [&](int i) -> u64 {
+        const float x = xs[i];
+        return ordered(x) >= thr ? mass_of(x) : 0ull;
+    };
+    u64 mine = 0ull;
+    for (int i = b0 + lane; i < b1; i += 32) mine += kept_of(i);
+    mine = warp_sum(mine);
+    if (lane == 0) s.seg[warp] = mine;
+    cluster.sync();
+    const int segs = blocks * kWarps;
+    if (tid < segs) s.all_seg[tid] = *cluster.map_shared_rank(&s.seg[tid % kWarps], tid / kWarps);
+    __syncthreads();
+    // (every warp works the answer out for itself; the one whose stretch holds it writes it)
+    u64 part[kMaxBlocks * kWarps / 32], sum = 0ull;
+#pragma unroll
+    for (int j = 0; j < kMaxBlocks * kWarps / 32; ++j) {
+        const int at = lane * (kMaxBlocks * kWarps / 32) + j;
+        part[j] = at < segs ? s.all_seg[at] : 0ull;
+        sum += part[j];
+    }
+    u64 run = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 up = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += up;
+    }
+    const u64 total = __shfl_sync(0xffffffffu, run, 31);
+    const double target = (double)u * (double)total;
+    // the first stretch with mass at whose end the sum reaches the target; if none does (a draw of
+    // one or more), the last stretch with mass, and in it the last kept value (the reference's
+    // fallback, sampling.cpp:113-116)
+    int first = 0x7fffffff, last = -1;
+    u64 first_before = 0ull, at_end = run - sum;
+#pragma unroll
+    for (int j = 0; j < kMaxBlocks * kWarps / 32; ++j) {
+        const int at = lane * (kMaxBlocks * kWarps / 32) + j;
+        if (part[j]) {
+            last = at;
+            if (first == 0x7fffffff && (double)(at_end + part[j]) >= target) { first = at; first_before = at_end; }
+        }
+        at_end += part[j];
+    }
+    const int pick = __reduce_min_sync(0xffffffffu, first), pick_last = __reduce_max_sync(0xffffffffu, last);
+    if (pick == rank * kWarps + warp) {
+        const int owner = pick / (kMaxBlocks * kWarps / 32);
+        u64 before = __shfl_sync(0xffffffffu, first_before, owner);
+        for (int i = b0; i < b1; i += 32) {
+            const u64 m = i + lane < b1 ? kept_of(i + lane) : 0ull;
+            u64 up = m;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u64 t = __shfl_up_sync(0xffffffffu, up, o);
+                if (lane >= o) up += t;
+            }
+            const unsigned int hit = __ballot_sync(0xffffffffu, m && (double)(before + up) >= target);
+            if (hit) {
+                if (lane == 0) out[row] = i0 + i + __ffs(hit) - 1;
+                break;
+            }
+            before += __shfl_sync(0xffffffffu, up, 31);
+        }
+    } else if (pick == 0x7fffffff && pick_last == rank * kWarps + warp) {
+        int best = -1;
+        for (int i = b0 + lane; i < b1; i += 32)
+            if (kept_of(i)) best = i;
+        best = __reduce_max_sync(0xffffffffu, best);
+        if (lane == 0) out[row] = i0 + best;
+    } else if (pick_last < 0 && rank == 0 && tid == 0) {
+        out[row] = mi < vocab ? mi : 0;                       // no value has any mass
+    }
+    cluster.sync();                                           // (a peer may still read this block's sums)
 }
 
-// logits: float [rows, vocab]; work: float [rows, vocab] scratch; params: float [rows, 4]
-// = {temperature, top_p, repetition_penalty, u}; top_k: int [rows] (0 = off);
+// Blocks of a row's cluster, logits of a block's slice and its shared memory (0: the slice lives in `work`).
+static void plan(int vocab, int* blocks, int* slice, size_t* smem) {
+    int b = 1;
+    while (b < kMaxBlocks && (long long)b * kSliceTarget < vocab) b *= 2;
+    const int per = ((vocab + b - 1) / b + 3) / 4 * 4;
+    *blocks = b;
+    *slice = per;
+    *smem = (size_t)per * 4 <= kSliceBytes ? (size_t)per * 4 : 0;
+}
+
+LSB_API int lsb_sample_needs_work(int vocab) {
+    int blocks, slice;
+    size_t smem;
+    plan(vocab, &blocks, &slice, &smem);
+    return smem == 0;
+}
+
+// logits: float [rows, vocab]; work: float [rows, vocab] scratch where lsb_sample_needs_work says so, else
+// unused; params: float [rows, 4] = {temperature, top_p, repetition_penalty, u}; top_k: int [rows] (0 = off);
 // prev_start: int [rows + 1] offsets into prev_tokens, or null; out: int [rows].
 LSB_API int lsb_sample(const float* logits, float* work, int rows, int vocab, const float* params,
                        const int* top_k, const int* prev_start, const int* prev_tokens, int* out,
                        cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0) return (int)cudaErrorInvalidValue;
-    // (few rows: their greedy scans are shared out over more blocks; many rows fill the SMs by themselves)
-    const int parts = rows <= 64 && vocab >= 16384 ? kGreedyParts : 1;
-    static_assert(kGreedyParts <= 32, "the last block merges the parts with one warp");
-    return lsb_launch(sample_kernel, dim3(rows, parts), dim3(kSampleThreads), 0, stream, 1, logits, work, vocab,
-                      params, top_k, prev_start, prev_tokens, out);
+    static int configured = -1;
+    if (configured < 0)
+        configured = (int)cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSliceBytes);
+    if (configured) return configured;
+    int blocks, slice;
+    size_t smem;
+    plan(vocab, &blocks, &slice, &smem);
+    if (!smem && !work) return (int)cudaErrorInvalidValue;
+    // a value's mass is at most 2^44, and never so large that a row's sum leaves 63 bits
+    int log2 = 0;
+    while (log2 < 31 && (1ll << log2) < vocab) ++log2;
+    const float mass_scale = (float)(1ull << (63 - log2 < 44 ? 63 - log2 : 44));
+    return lsb_launch(sample_kernel, dim3(rows, 1, blocks), dim3(kThreads), smem, stream, blocks, logits, work, vocab,
+                      slice, smem ? 1 : 0, mass_scale, params, top_k, prev_start, prev_tokens, out);
 }
