@@ -9,152 +9,529 @@
 // maximum and sum, weighted sum of values, division by the sum at the end.
 //
 // Two score modifiers that other architectures use are taken here (the reference has neither;
-// the tensor-core kernels do not take them, so a mixer that asks for one runs this kernel):
+// the tensor-core kernels do not take them, so a mixer that asks for one runs these kernels):
 // a soft cap, s <- cap * tanh(s / cap), and a linear position bias per head,
 // s <- s - slope[h] * (p - key position), applied in that order before the softmax.
 //
 // Replaces paged_attention_kernel of the reference (kernels/src/attention.cu:27-172:
 // 32 threads per (head, row), per-thread v_acc[128] in registers, shared-memory tree
 // merge, one launch per request during prefill, models/llama/llama_model.cpp:603-614).
-// Here one warp owns a (row, head): lanes split the keys of a 32-key chunk for the
-// scores and split the head dims for the weighted sum; one launch covers all requests.
+//
+// Two kernels, both with keys and values in tiles of shared memory (as 32-bit, the next tile on its way in registers):
+//
+// * Single tokens are cache traffic: a block takes a kv head's group of query heads over one of up to eight
+//   stretches of the request's keys, and the stretches' sums meet through distributed shared memory.  8 requests
+//   of 300 to 1,500 tokens, 32 / 8 heads of 64 in 32-bit (29 MB): 24 us; one warp for each (request, head)
+//   walking all of its keys took 1,548 us.
+// * Portions are arithmetic: 64 rows (16 queries of 4 heads that share their keys) against a tile, 4 rows by 2 or 4
+//   keys a thread for the scores and the same 4 rows for the weighted sum, so that a row's maximum, its sum and its
+//   probabilities stay within half a warp; two multiply-adds to an instruction.  500 tokens, the same heads:
+//   88 us (1.0 GFLOP); a warp for each (row, head) took 650 us.
 #include "common.cuh"
 
+#include <cooperative_groups.h>
 #include <float.h>
+
+namespace cg = cooperative_groups;
 
 LSB_DEFINE_STATUS()
 
-constexpr int kAttnWarps = 4;
+constexpr int kThreads = 256;
 constexpr int kMaxHeadDim = 256;
+constexpr int kMaxSplits = 8;                   // stretches of a request's keys (a cluster of portable size)
 
-// dot of q (shared, float) with one key row (global, 16-byte vector loads)
-template <typename T>
-__device__ __forceinline__ float dot_row(const float* __restrict__ q, const T* __restrict__ k, int hd);
+struct AttnParams {
+    const void* qkv;                            // q of token t at qkv + t * qkv_stride
+    int qkv_stride;
+    const void* k_pages;
+    const void* v_pages;
+    const int* q_start;
+    const int* kv_len;
+    const int* table_rows;
+    const int* block_table;
+    int table_stride;
+    void* out;                                  // [tokens, nh * hd]
+    int nh, nkv, hd, page_size, num_pages;
+    float scale;
+    int window;
+    float softcap;
+    const float* slopes;
+    int heads;                                  // query heads of a block
+    int head_blocks;                            // blocks of a kv head's group
+};
 
-template <>
-__device__ __forceinline__ float dot_row<float>(const float* __restrict__ q,
-                                                const float* __restrict__ k, int hd) {
-    float s = 0.f;
-    for (int d = 0; d < hd; d += 4) {
-        const float4 kv = *reinterpret_cast<const float4*>(k + d);
-        s += q[d] * kv.x + q[d + 1] * kv.y + q[d + 2] * kv.z + q[d + 3] * kv.w;
-    }
-    return s;
+typedef unsigned long long pair32;              // two 32-bit values
+__device__ __forceinline__ pair32 twice(float a) {
+    pair32 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
 }
+__device__ __forceinline__ void fma2(pair32& acc, pair32 a, pair32 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ pair32 mul2(pair32 a, pair32 b) {
+    pair32 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void apart(pair32 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 
-template <>
-__device__ __forceinline__ float dot_row<__nv_bfloat16>(const float* __restrict__ q,
-                                                        const __nv_bfloat16* __restrict__ k, int hd) {
-    float s = 0.f;
-    for (int d = 0; d < hd; d += 8) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(k + d);
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+// four elements as they lie in memory, and as 32-bit
+__device__ __forceinline__ uint4 load_raw(const float* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ uint2 load_raw(const __nv_bfloat16* p) { return *reinterpret_cast<const uint2*>(p); }
+__device__ __forceinline__ float4 widen(uint4 v) {
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+__device__ __forceinline__ float4 widen(uint2 v) {
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+}
+template <typename T> struct Raw { typedef uint4 type; };
+template <> struct Raw<__nv_bfloat16> { typedef uint2 type; };
+
+// The keys of a tile: at most HDC / 4 pieces of four elements a row, KT rows.
+template <typename T, int KT, int HDC>
+struct Tile {
+    static constexpr int kPieces = KT * HDC / 4 / kThreads;
+    typename Raw<T>::type k[kPieces], v[kPieces];
+
+    // off: element offset of each key's row in the page pools, -1 for none
+    __device__ __forceinline__ void fetch(const AttnParams& p, const long long* off, int tid) {
+        const int per = p.hd >> 2;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(p[j]);
-            s += q[d + 2 * j] * f.x + q[d + 2 * j + 1] * f.y;
+        for (int j = 0; j < kPieces; ++j) {
+            const int idx = j * kThreads + tid, row = idx / per;
+            k[j] = typename Raw<T>::type{};
+            v[j] = typename Raw<T>::type{};
+            if (row < KT) {
+                const long long o = off[row];
+                if (o >= 0) {
+                    const long long at = o + (idx - row * per) * 4;
+                    k[j] = load_raw(reinterpret_cast<const T*>(p.k_pages) + at);
+                    v[j] = load_raw(reinterpret_cast<const T*>(p.v_pages) + at);
+                }
+            }
         }
     }
-    return s;
+    __device__ __forceinline__ void park(const AttnParams& p, float* ks, float* vs, int ldk, int tid) const {
+        const int per = p.hd >> 2;
+#pragma unroll
+        for (int j = 0; j < kPieces; ++j) {
+            const int idx = j * kThreads + tid, row = idx / per, d = (idx - row * per) * 4;
+            if (row < KT) {
+                *reinterpret_cast<float4*>(ks + row * ldk + d) = widen(k[j]);
+                *reinterpret_cast<float4*>(vs + row * p.hd + d) = widen(v[j]);
+            }
+        }
+    }
+};
+
+// Where the row of key `pos` of kv head g lies in the page pools (elements); -1 and a recorded status if its page
+// is not one of the pool's.
+__device__ __forceinline__ long long key_offset(const AttnParams& p, const int* table, int g, int pos) {
+    const int page = table[pos / p.page_size];
+    if (page < 0 || page >= p.num_pages) {
+        lsb_set_status(LSB_BAD_PAGE);
+        return -1;
+    }
+    return (((long long)page * p.nkv + g) * p.page_size + pos % p.page_size) * p.hd;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kAttnWarps * 32)
-paged_attention_generic_kernel(
-    const T* __restrict__ qkv, int qkv_stride,              // q of token t at qkv + t*stride
-    const T* __restrict__ k_pages, const T* __restrict__ v_pages,
-    const int* __restrict__ q_start, const int* __restrict__ kv_len_arr,
-    const int* __restrict__ table_rows, const int* __restrict__ block_table, int table_stride,
-    T* __restrict__ out,                                    // [tokens, nh*hd]
-    int nh, int nkv, int hd, int page_size, int num_pages, float scale, int window,
-    float softcap, const float* __restrict__ slopes) {
-    __shared__ float q_sh[kAttnWarps][kMaxHeadDim];
+__device__ __forceinline__ float modified(const AttnParams& p, float s, float slope, int distance) {
+    if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
+    return s - slope * (float)distance;
+}
+
+// ------------------------------------------------------------------ single tokens
+// Most query heads of a block: their sums are kAccs a thread.
+constexpr int kAccs = 4;
+
+template <int KT>
+static size_t single_smem(int hd, int heads) {
+    return ((size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)heads * hd * 2 + (size_t)heads * (KT + 4) + heads * 4) * 4;
+}
+
+template <typename T, int KT, int HDC>
+__global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const AttnParams p) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ long long off[2][KT];
+    cg::cluster_group cluster = cg::this_cluster();
     lsb_pdl_launch_dependents();
     lsb_pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.z, h = blockIdx.y;
-    const int qs = q_start[r];
-    const int q_len = q_start[r + 1] - qs;
-    const int i = blockIdx.x * kAttnWarps + warp;            // row within the request
-    if (i >= q_len) return;                                  // whole warp leaves together
-    const int kv_len = kv_len_arr[r];
-    const int p = kv_len - q_len + i;
-    const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
-    const int g = h / (nh / nkv);
-    const int t = qs + i;
-    const int* bt = block_table + (size_t)table_rows[r] * table_stride;
-    const float slope = slopes ? slopes[h] : 0.f;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int splits = (int)gridDim.x, split = (int)blockIdx.x, r = blockIdx.z;
+    const int g = blockIdx.y / p.head_blocks, group = p.nh / p.nkv;
+    const int h0 = g * group + (int)(blockIdx.y % p.head_blocks) * p.heads;
+    const int H = min(p.heads, (g + 1) * group - h0);
+    const int t = p.q_start[r];
+    if (p.q_start[r + 1] - t != 1) return;                     // (all blocks of the cluster alike)
+    const int hd = p.hd, ldk = hd + 4, lds = KT + 4;
+    float* ks = sm;
+    float* vs = ks + KT * ldk;
+    float* qs = vs + KT * hd;                                  // [heads][hd], scaled
+    float* os = qs + p.heads * hd;                             // [heads][hd], the stretch's sums
+    float* ps = os + p.heads * hd;                             // [heads][KT + 4]
+    float* ml = ps + p.heads * lds;                            // running maximum, sum, factor of the last tile; m and l stay
+    const int pos = p.kv_len[r] - 1;
+    const int lo = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
+    // this block's stretch: whole sixteens of keys
+    const int per = ((pos - lo + 1 + splits - 1) / splits + 15) / 16 * 16;
+    const int first = lo + split * per, last = min(pos + 1, first + per);     // [first, last), maybe empty
+    const int* table = p.block_table + (size_t)p.table_rows[r] * p.table_stride;
 
-    const T* q = qkv + (size_t)t * qkv_stride + (size_t)h * hd;
-    for (int d = lane; d < hd; d += 32) q_sh[warp][d] = lsb_to_float(q[d]) * scale;
-    __syncwarp();
-
-    constexpr int kAccs = kMaxHeadDim / 32;
+    const T* q = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.qkv_stride + (size_t)h0 * hd;
+    for (int i = tid; i < H * hd; i += kThreads) qs[i] = lsb_to_float(q[i]) * p.scale;
+    if (tid < H) { ml[4 * tid] = -FLT_MAX; ml[4 * tid + 1] = 0.f; }
+    if (tid < KT) off[0][tid] = first + tid < last ? key_offset(p, table, g, first + tid) : -1;
     float acc[kAccs];
 #pragma unroll
-    for (int c = 0; c < kAccs; ++c) acc[c] = 0.f;
-    float m = -FLT_MAX, l = 0.f;
-
-    for (int base = lo; base <= p; base += 32) {
-        const int kj = base + lane;
-        float s = -FLT_MAX;
-        long long off = -1;                                  // element offset of the key/value row
-        if (kj <= p) {
-            const int page = bt[kj / page_size];
-            if (page < 0 || page >= num_pages) {
-                lsb_set_status(LSB_BAD_PAGE);
-            } else {
-                off = (((long long)page * nkv + g) * page_size + (kj % page_size)) * hd;
-                s = dot_row<T>(q_sh[warp], k_pages + off, hd);
-                if (softcap > 0.f) s = softcap * tanhf(s / softcap);
-                s -= slope * (float)(p - kj);
+    for (int a = 0; a < kAccs; ++a) acc[a] = 0.f;
+    __syncthreads();
+    Tile<T, KT, HDC> tile;
+    tile.fetch(p, off[0], tid);
+    for (int base = first, turn = 0; base < last; base += KT, turn ^= 1) {
+        tile.park(p, ks, vs, ldk, tid);
+        const int next = base + KT;
+        if (tid < KT) off[turn ^ 1][tid] = next + tid < last ? key_offset(p, table, g, next + tid) : -1;
+        __syncthreads();
+        if (next < last) tile.fetch(p, off[turn ^ 1], tid);
+        for (int i = tid; i < H * KT; i += kThreads) {         // a (head, key) each: whole warps share a head
+            const int h = i / KT, k = i % KT;
+            float s = -FLT_MAX;
+            if (off[turn][k] >= 0) {
+                const ulonglong2* a = reinterpret_cast<const ulonglong2*>(qs + h * hd);
+                const ulonglong2* b = reinterpret_cast<const ulonglong2*>(ks + k * ldk);
+                pair32 s0 = 0ull, s1 = 0ull;
+                for (int d = 0; d < hd / 4; d += 4) {          // (hd is a multiple of 16)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const ulonglong2 x = a[d + e], y = b[d + e];
+                        fma2(s0, x.x, y.x);
+                        fma2(s1, x.y, y.y);
+                    }
+                }
+                float s00, s01, s10, s11;
+                apart(s0, s00, s01);
+                apart(s1, s10, s11);
+                s = modified(p, (s00 + s01) + (s10 + s11), p.slopes ? p.slopes[h0 + h] : 0.f, pos - (base + k));
+            }
+            ps[h * lds + k] = s;
+        }
+        __syncthreads();
+        for (int h = warp; h < H; h += kThreads / 32) {
+            float* row = ps + h * lds;
+            float s[KT / 32], mx = -FLT_MAX;
+#pragma unroll
+            for (int j = 0; j < KT / 32; ++j) { s[j] = row[lane + 32 * j]; mx = fmaxf(mx, s[j]); }
+            const float m = ml[4 * h], m_new = fmaxf(m, lsb_warp_max(mx));
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < KT / 32; ++j) {
+                const float e = off[turn][lane + 32 * j] >= 0 ? expf(s[j] - m_new) : 0.f;
+                row[lane + 32 * j] = e;
+                sum += e;
+            }
+            sum = lsb_warp_sum(sum);
+            __syncwarp();
+            if (lane == 0) {
+                const float corr = expf(m - m_new);            // m == -FLT_MAX first: exp(-huge) = 0
+                ml[4 * h] = m_new;
+                ml[4 * h + 1] = ml[4 * h + 1] * corr + sum;
+                ml[4 * h + 2] = corr;
             }
         }
-        const float m_new = fmaxf(m, lsb_warp_max(s));
-        const float corr = expf(m - m_new);                // m == -FLT_MAX first: exp(-huge) = 0
-        const float pj = (off >= 0) ? expf(s - m_new) : 0.f;
-        l = l * corr + lsb_warp_sum(pj);
+        __syncthreads();
 #pragma unroll
-        for (int c = 0; c < kAccs; ++c) acc[c] *= corr;
-        const int n_valid = min(32, p - base + 1);
-        for (int j = 0; j < n_valid; ++j) {
-            const float w = __shfl_sync(0xffffffffu, pj, j);
-            const long long voff = __shfl_sync(0xffffffffu, off, j);
-            if (voff < 0) continue;
-            const T* v = v_pages + voff;
-#pragma unroll
-            for (int c = 0; c < kAccs; ++c) {
-                const int d = lane + 32 * c;
-                if (d < hd) acc[c] += w * lsb_to_float(v[d]);
+        for (int a = 0; a < kAccs; ++a) {
+            const int i = a * kThreads + tid;
+            if (i < H * hd) {
+                const int h = i / hd, d = i - h * hd;
+                const float4* w = reinterpret_cast<const float4*>(ps + h * lds);
+                float o = acc[a] * ml[4 * h + 2];
+#pragma unroll 4
+                for (int k = 0; k < KT / 4; ++k) {
+                    const float4 e = w[k];
+                    const float* v = vs + 4 * k * hd + d;
+                    o = fmaf(e.x, v[0], o);
+                    o = fmaf(e.y, v[hd], o);
+                    o = fmaf(e.z, v[2 * hd], o);
+                    o = fmaf(e.w, v[3 * hd], o);
+                }
+                acc[a] = o;
             }
         }
-        m = m_new;
+        __syncthreads();
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    T* o = out + (size_t)t * nh * hd + (size_t)h * hd;
 #pragma unroll
-    for (int c = 0; c < kAccs; ++c) {
-        const int d = lane + 32 * c;
-        if (d < hd) o[d] = lsb_from_float<T>(acc[c] * inv);
+    for (int a = 0; a < kAccs; ++a)
+        if (a * kThreads + tid < H * hd) os[a * kThreads + tid] = acc[a];
+    cluster.sync();
+    // every block brings its share of the outputs together, stretches in order
+    T* out = reinterpret_cast<T*>(p.out) + (size_t)t * p.nh * hd + (size_t)h0 * hd;
+    for (int i = split * kThreads + tid; i < H * hd; i += splits * kThreads) {
+        const int h = i / hd;
+        float m = -FLT_MAX;
+        for (int s = 0; s < splits; ++s) m = fmaxf(m, *cluster.map_shared_rank(ml + 4 * h, s));
+        float l = 0.f, o = 0.f;
+        for (int s = 0; s < splits; ++s) {
+            const float f = expf(*cluster.map_shared_rank(ml + 4 * h, s) - m);
+            l += f * *cluster.map_shared_rank(ml + 4 * h + 1, s);
+            o += f * *cluster.map_shared_rank(os + i, s);
+        }
+        out[i] = lsb_from_float<T>(l > 0.f ? o * (1.f / l) : 0.f);
+    }
+    cluster.sync();                                            // (a peer may still read this block's sums)
+}
+
+// ------------------------------------------------------------------ portions
+constexpr int kRows = 64;                       // (query, head) rows of a block
+constexpr int kPortionHeads = 4;                // most query heads of a block
+
+template <int KT>
+static size_t portion_smem(int hd) {
+    return ((size_t)kRows * (hd + 4) + (size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)kRows * (KT + 4)) * 4;
+}
+
+template <typename T, int KT, int HDC>
+__global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portion_kernel(const AttnParams p) {
+    constexpr int KPT = KT / 16;                // keys of a thread's scores
+    constexpr int CPT = HDC / 64;               // groups of four columns of a thread's sums
+    extern __shared__ __align__(16) float sm[];
+    __shared__ long long off[2][KT];
+    lsb_pdl_launch_dependents();
+    lsb_pdl_wait();
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, r = blockIdx.z;
+    const int g = blockIdx.y / p.head_blocks, group = p.nh / p.nkv;
+    const int h0 = g * group + (int)(blockIdx.y % p.head_blocks) * p.heads;
+    const int H = min(p.heads, (g + 1) * group - h0);
+    const int qs0 = p.q_start[r], q_len = p.q_start[r + 1] - qs0;
+    const int queries = kRows / p.heads;
+    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * queries;          // the longest rows first
+    if (q_len <= 1 || i0 >= q_len) return;
+    const int hd = p.hd, ldk = hd + 4, ldp = KT + 4;
+    float* qs = sm;
+    float* ks = qs + kRows * ldk;
+    float* vs = ks + KT * ldk;
+    float* ps = vs + KT * hd;
+    const int pos0 = p.kv_len[r] - q_len + i0;                 // of the block's first query
+    const int pos_last = min(pos0 + queries, p.kv_len[r]) - 1;
+    const int lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+    const int* table = p.block_table + (size_t)p.table_rows[r] * p.table_stride;
+
+    // row x: query i0 + x / heads, head h0 + x % heads (rows beyond the portion or the group stay zero)
+    for (int i = tid; i < kRows * hd; i += kThreads) {
+        const int x = i / hd, d = i - x * hd, qi = i0 + x / p.heads, h = x % p.heads;
+        qs[x * ldk + d] = qi < q_len && h < H && x / p.heads < queries
+            ? lsb_to_float(reinterpret_cast<const T*>(p.qkv)[(size_t)(qs0 + qi) * p.qkv_stride + (size_t)(h0 + h) * hd + d]) * p.scale
+            : 0.f;
+    }
+    if (tid < KT) off[0][tid] = lo + tid <= pos_last ? key_offset(p, table, g, lo + tid) : -1;
+    int pos[4], row_lo[4];
+    float slope[4], m[4], l[4];
+    pair32 acc[4][2 * CPT];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int x = ty * 4 + i;
+        pos[i] = min(pos0 + x / p.heads, pos_last);
+        row_lo[i] = p.window > 0 ? pos[i] - p.window + 1 : 0;
+        slope[i] = p.slopes && x % p.heads < H ? p.slopes[h0 + x % p.heads] : 0.f;
+        m[i] = -FLT_MAX;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 2 * CPT; ++c) acc[i][c] = 0ull;
+    }
+    __syncthreads();
+    Tile<T, KT, HDC> tile;
+    tile.fetch(p, off[0], tid);
+    for (int base = lo, turn = 0; base <= pos_last; base += KT, turn ^= 1) {
+        tile.park(p, ks, vs, ldk, tid);
+        const int next = base + KT;
+        if (tid < KT) off[turn ^ 1][tid] = next + tid <= pos_last ? key_offset(p, table, g, next + tid) : -1;
+        __syncthreads();
+        if (next <= pos_last) tile.fetch(p, off[turn ^ 1], tid);
+        // scores: rows 4 ty + i, keys tx + 16 j
+        pair32 s2[4][KPT];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) s2[i][j] = 0ull;
+#pragma unroll 2
+        for (int d = 0; d < hd; d += 4) {
+            ulonglong2 a[4], b[KPT];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(qs + (ty * 4 + i) * ldk + d);
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ks + (tx + 16 * j) * ldk + d);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < KPT; ++j) {
+                    fma2(s2[i][j], a[i].x, b[j].x);
+                    fma2(s2[i][j], a[i].y, b[j].y);
+                }
+        }
+        // a row's 16 threads are half a warp
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float s[KPT], mx = m[i];
+            bool seen[KPT];
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) {
+                const int key = base + tx + 16 * j;
+                float u, v;
+                apart(s2[i][j], u, v);
+                seen[j] = key <= pos[i] && key >= row_lo[i] && off[turn][tx + 16 * j] >= 0;
+                s[j] = seen[j] ? modified(p, u + v, slope[i], pos[i] - key) : -FLT_MAX;
+                mx = fmaxf(mx, s[j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float corr = expf(m[i] - mx);                // m == -FLT_MAX first: exp(-huge) = 0
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < KPT; ++j) {
+                const float e = seen[j] ? expf(s[j] - mx) : 0.f;
+                ps[(ty * 4 + i) * ldp + tx + 16 * j] = e;
+                sum += e;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            m[i] = mx;
+            l[i] = l[i] * corr + sum;
+            const pair32 c2 = twice(corr);
+#pragma unroll
+            for (int c = 0; c < 2 * CPT; ++c) acc[i][c] = mul2(acc[i][c], c2);
+        }
+        __syncwarp();                                          // the row's probabilities were written by this warp
+        // the weighted sum: columns 4 tx + 64 c
+#pragma unroll 2
+        for (int k = 0; k < KT; k += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (ty * 4 + i) * ldp + k);
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                const int d = tx * 4 + 64 * c;
+                if (d < hd) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vs + (k + e) * hd + d);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const pair32 we = twice(e == 0 ? w[i].x : e == 1 ? w[i].y : e == 2 ? w[i].z : w[i].w);
+                            fma2(acc[i][2 * c], we, v.x);
+                            fma2(acc[i][2 * c + 1], we, v.y);
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int x = ty * 4 + i, qi = i0 + x / p.heads, h = x % p.heads;
+        if (qi >= q_len || h >= H || x / p.heads >= queries) continue;
+        const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+        T* o = reinterpret_cast<T*>(p.out) + (size_t)(qs0 + qi) * p.nh * hd + (size_t)(h0 + h) * hd;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+            const int d = tx * 4 + 64 * c;
+            if (d < hd) {
+                float v[4];
+                apart(acc[i][2 * c], v[0], v[1]);
+                apart(acc[i][2 * c + 1], v[2], v[3]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[d + e] = lsb_from_float<T>(v[e] * inv);
+            }
+        }
     }
 }
 
-// qkv: [tokens, qkv_stride] with the nh*hd query values first in each row.  softcap: 0 for none;
-// slopes: float [nh] or null.
+// ------------------------------------------------------------------ host side
+static int num_sms() {
+    static int cached[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    if (cached[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
+        cached[dev] = n;
+    }
+    return cached[dev];
+}
+
+template <typename T, int KT, int HDC>
+static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int max_keys, cudaStream_t stream) {
+    static int configured = -1;
+    const int group = p.nh / p.nkv;
+    if (configured < 0) {
+        // (the largest either kernel asks for: heads of HDC, as many as a block takes of the smallest, 16)
+        configured = (int)cudaFuncSetAttribute(attention_single_kernel<T, KT, HDC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        if (!configured)
+            configured = (int)cudaFuncSetAttribute(attention_portion_kernel<T, KT, HDC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    }
+    if (configured) return configured;
+    if (n_single > 0) {
+        AttnParams s = p;
+        s.heads = kAccs * kThreads / p.hd;
+        if (s.heads > group) s.heads = group;
+        s.head_blocks = (group + s.heads - 1) / s.heads;
+        // two blocks an SM, as many stretches as that takes; no stretch shorter than a tile where the longest
+        // context is known (a captured launch has to serve any)
+        const long long blocks = (long long)n_single * p.nkv * s.head_blocks;
+        long long splits = (2ll * num_sms() + blocks / 2) / blocks;
+        if (max_keys > 0 && splits > (max_keys + KT - 1) / KT) splits = (max_keys + KT - 1) / KT;
+        splits = splits < 1 ? 1 : splits > kMaxSplits ? kMaxSplits : splits;
+        if ((long long)p.nkv * s.head_blocks > 65535) return (int)cudaErrorInvalidValue;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)splits, p.nkv * s.head_blocks, n_requests);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = single_smem<KT>(p.hd, s.heads);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        int n = 0;
+        if (lsb_pdl_enabled()) {
+            attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[n++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)splits;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = n;
+        const int rc = (int)cudaLaunchKernelEx(&cfg, attention_single_kernel<T, KT, HDC>, s);
+        if (rc) return rc;
+    }
+    if (max_q_len > 1) {
+        p.heads = group < kPortionHeads ? group : kPortionHeads;
+        p.head_blocks = (group + p.heads - 1) / p.heads;
+        const int queries = kRows / p.heads;
+        if ((long long)p.nkv * p.head_blocks > 65535) return (int)cudaErrorInvalidValue;
+        const dim3 grid((max_q_len + queries - 1) / queries, p.nkv * p.head_blocks, n_requests);
+        return lsb_launch(attention_portion_kernel<T, KT, HDC>, grid, dim3(kThreads), portion_smem<KT>(p.hd), stream, 1, p);
+    }
+    return 0;
+}
+
+// qkv: [tokens, qkv_stride] with the nh*hd query values first in each row.  softcap: 0 for none; slopes: float [nh] or
+// null.  n_single: requests that bring one token; max_keys: the longest context (0: not known, the launch is captured).
 LSB_API int lsb_paged_attention_generic(
     const void* qkv, int qkv_stride, const void* k_pages, const void* v_pages,
     const int* q_start, const int* kv_len, const int* table_rows, const int* block_table,
-    int table_stride, void* out, int dtype, int n_requests, int max_q_len,
+    int table_stride, void* out, int dtype, int n_requests, int max_q_len, int n_single, int max_keys,
     int nh, int nkv, int hd, int page_size, int num_pages, float scale, int window,
     float softcap, const float* slopes, cudaStream_t stream) {
     if (n_requests <= 0 || max_q_len <= 0) return 0;
     if (hd % 16 || hd <= 0 || hd > kMaxHeadDim || nkv <= 0 || nh % nkv) return (int)cudaErrorInvalidValue;
     if (n_requests > 65535 || nh > 65535) return (int)cudaErrorInvalidValue;
-    dim3 grid((max_q_len + kAttnWarps - 1) / kAttnWarps, nh, n_requests);
-    LSB_DISPATCH_DTYPE(dtype, return lsb_launch(
-        paged_attention_generic_kernel<T>, grid, dim3(kAttnWarps * 32), 0, stream, 1,
-        (const T*)qkv, qkv_stride, (const T*)k_pages, (const T*)v_pages, q_start, kv_len,
-        table_rows, block_table, table_stride, (T*)out, nh, nkv, hd, page_size, num_pages,
-        scale, window, softcap, slopes));
+    const AttnParams p{qkv, qkv_stride, k_pages, v_pages, q_start, kv_len, table_rows, block_table, table_stride, out,
+                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0};
+    LSB_DISPATCH_DTYPE(dtype, {
+        if (hd <= 64) return launch<T, 64, 64>(p, n_requests, max_q_len, n_single, max_keys, stream);
+        if (hd <= 128) return launch<T, 32, 128>(p, n_requests, max_q_len, n_single, max_keys, stream);
+        return launch<T, 32, 256>(p, n_requests, max_q_len, n_single, max_keys, stream);
+    });
     return 0;
 }

@@ -837,8 +837,10 @@ def paged_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache, s
     if modified or not tensor_core_attention_ok(qkv.dtype, hd, nh, nkv):
         if decode_rope is not None:
             raise KernelError("attention: only the tensor-core decode kernel rotates by itself")
-        _call("attention", "lsb_paged_attention_generic", *common, _i(_dt(qkv)),
-              _i(ctx.n_requests), _i(ctx.max_q_len), *tail, _f(softcap), _p(slopes), _stream(out))
+        # (a captured launch has to serve contexts of any length)
+        longest = 0 if getattr(ctx, "fixed_launch", False) else ctx.max_kv_len
+        _call("attention", "lsb_paged_attention_generic", *common, _i(_dt(qkv)), _i(ctx.n_requests), _i(ctx.max_q_len),
+              _i(_batch_shape(ctx)[0]), _i(longest), *tail, _f(softcap), _p(slopes), _stream(out))
         return
     R = ctx.n_requests
     n_decode, first, last = _batch_shape(ctx)
