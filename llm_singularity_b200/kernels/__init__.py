@@ -1132,11 +1132,15 @@ def _chunk_scratch(name: str, numel: int, device, dtype) -> torch.Tensor:
 def chunk_scan(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: int, key_heads: int, key_dim: int, value_dim: int,
                state: torch.Tensor, ctx, out: torch.Tensor, first: int, *, q_lo: int = -1, k_lo: int = -1,
                log_keep: Optional[torch.Tensor] = None, write: Optional[torch.Tensor] = None,
-               log_decay: Optional[torch.Tensor] = None, q_scale: float = 1.0) -> None:
+               log_decay: Optional[torch.Tensor] = None, q_scale: float = 1.0, acts=("none", "none", "none")) -> None:
     """What ``linear_scan`` does for a memory that fades by one number per head and token, for the requests from
     ``first`` on, in chunks on the tensor cores.  ``rows`` bfloat16: q, k and v at their offsets, with ``q_lo`` / ``k_lo``
     the rounded rests of q and k.  ``log_keep`` and ``write`` (32-bit [T, heads]): the logarithm of the fade and the
-    factor of a write; or ``log_decay`` [heads], the same for every token, with writes as they are."""
+    factor of a write; or ``log_decay`` [heads], the same for every token, with writes as they are.  ``acts``: what q, k and v
+    pass on the way in ("silu" or "none"; not where they come with rests), in 32-bit."""
+    silu = sum(1 << i for i, name in enumerate(acts) if _SCAN_ACTS[name])
+    if silu and q_lo >= 0:
+        raise KernelError("chunk_scan: operands with rests have passed their activations")
     _req(rows, "rows", torch.bfloat16, 2)
     _req(state, "state", torch.float32, 4)
     _req(out, "out", torch.float32, 2)
@@ -1158,8 +1162,8 @@ def chunk_scan(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: in
     starts = _chunk_scratch("starts", n * heads * 2 * value_dim * key_dim, rows.device, torch.bfloat16)
     fade = _chunk_scratch("fade", n * heads, rows.device, torch.float32)
     _call("chunk_scan", "lsb_chunk_scan", _p(rows), _ll(ld), _i(q_off), _i(k_off), _i(v_off), _i(q_lo), _i(k_lo), _i(heads),
-          _i(key_heads), _i(key_dim), _i(value_dim), _p(log_keep), _p(write), _p(log_decay), _f(q_scale), _p(state),
-          _i(state.shape[0]), ctypes.c_void_p(ctx.q_start.data_ptr() + 4 * first),
+          _i(key_heads), _i(key_dim), _i(value_dim), _p(log_keep), _p(write), _p(log_decay), _f(q_scale), _i(silu),
+          _p(state), _i(state.shape[0]), ctypes.c_void_p(ctx.q_start.data_ptr() + 4 * first),
           ctypes.c_void_p(ctx.table_rows.data_ptr() + 4 * first), _i(n_req), _i(ctx.max_q_len), _p(out), _p(gain), _p(starts),
           _p(fade), _stream(out))
 

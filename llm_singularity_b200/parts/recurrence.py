@@ -11,8 +11,8 @@ b = 1 - a; no key, no other scale).  The outputs are RMS-normed (all heads toget
 over the row, or each head by itself with one weight of head size or none), optionally multiplied by
 sigmoid or silu of W_g x, and projected by W_o.  With a fixed decay q and k may be rotated by the tokens'
 positions and k scaled (retention): the projections leave their product in 32-bit, walked tokens are rotated
-there, and prompt portions run in chunks on the tensor cores (``csrc/chunk_scan.cu``) with rotated queries and
-keys as sums of two bfloat16 numbers.
+there, and queries and keys are rotated into sums of two bfloat16 numbers.  Prompt portions of a memory with a fixed decay
+run in chunks on the tensor cores (``csrc/chunk_scan.cu``), everything else token by token.
 
 The state starts at zero when a request takes a slot, is 32-bit, and is carried from step to
 step in the slot's row of a ``StateSpec`` cache.  One product makes all projections of a step
@@ -55,7 +55,7 @@ class LinearRecurrence(Part):
         self.k_scale = float(getattr(s, "k_scale", 1.0))
         if self.k_scale != 1.0 and s.gate != "fixed_decay":
             raise ValueError("a factor on k goes with a fixed decay")
-        if self.position is not None and rt.dtype == torch.bfloat16:
+        if s.gate == "fixed_decay" and rt.dtype == torch.bfloat16:
             self.kernels = self.kernels + ("chunk_scan",)
         # the output kernel that knows heads without a weight and the silu gate
         self.plain_output = s.out_norm != "unit" and self.gate_act == "sigmoid"
@@ -67,10 +67,12 @@ class LinearRecurrence(Part):
         self.qk = s.num_heads * s.key_dim
         self.vv = s.num_heads * s.value_dim
         self.decay = self.log_decay = None
+        self.fades = False                          # every head's decay is at most one (the chunked form's powers stay bounded)
         if s.gate == "fixed_decay":
             decay = torch.tensor([float(d) for d in s.decay], dtype=torch.float64)
             self.decay = decay.to(dtype=torch.float32, device=rt.device)
             if bool((decay >= 0).all()):
+                self.fades = bool((decay <= 1).all())
                 self.log_decay = torch.log(decay).to(dtype=torch.float32, device=rt.device)
 
     @classmethod
@@ -118,11 +120,19 @@ class LinearRecurrence(Part):
         o = self.rt.empty(x.shape[0], self.vv, dtype=torch.float32)
         # [T, q | k or f | v | g]
         proj = ops.linear(x, self.w_in) if self.position is None else ops.linear(x, self.w_in, out_dtype=torch.float32)
+        # prompt portions in chunks on the tensor cores where they can be, the rest walked
+        first = ops.chunk_scan_first(ctx, self.rt.dtype, s.key_dim, s.value_dim) \
+            if self.log_decay is not None and hasattr(ops, "chunk_scan_first") else None
         if self.position is None:
-            self._walk(proj, ctx, cache, o)
+            if first is None or not self.fades:
+                self._walk(proj, ctx, cache, o)
+            else:
+                if first:                           # single tokens in front of the portions
+                    self._walk(proj, ctx, cache, o, requests=first)
+                ops.chunk_scan(proj, 0, self.qk, 2 * self.qk, s.num_heads, s.num_heads, s.key_dim, s.value_dim, cache.state, ctx, o,
+                               first, log_decay=self.log_decay, q_scale=self.k_scale,
+                               acts=(s.q_activation, s.k_activation, s.v_activation))
         else:
-            # prompt portions in chunks on the tensor cores where they can be, the rest walked
-            first = ops.chunk_scan_first(ctx, self.rt.dtype, s.key_dim, s.value_dim) if self.log_decay is not None else None
             if first is None:
                 ops.turn_heads(proj, 0, self.qk, s.num_heads, s.key_dim, self.table[0], ctx)
                 self._walk(proj, ctx, cache, o)
