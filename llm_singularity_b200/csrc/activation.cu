@@ -9,10 +9,9 @@
 // the same formulas in its epilogue; this kernel serves the 32-bit path and shapes that product
 // does not take.
 #include "common.cuh"
+#include "gate_act.cuh"
 
 LSB_DEFINE_STATUS()
-
-enum : int { LSB_ACT_SILU = 1, LSB_ACT_GELU_TANH = 2, LSB_ACT_NONE = 3, LSB_ACT_CAPPED_GLU = 5 };
 
 template <typename T>
 __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ out,
@@ -23,18 +22,7 @@ __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ 
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (; idx < total; idx += stride) {
         // out is [tokens, inter] and gate_up [tokens, 2 * inter]: element idx reads 2 idx, 2 idx + 1
-        const float g = lsb_to_float(gate_up[2 * idx]);
-        float u = lsb_to_float(gate_up[2 * idx + 1]);
-        float a;
-        if (act == LSB_ACT_CAPPED_GLU) {
-            const float gc = fminf(g, limit);
-            u = fminf(fmaxf(u, -limit), limit) + 1.f;
-            a = gc / (1.f + expf(-1.702f * gc));
-        } else if (act == LSB_ACT_SILU) a = g / (1.f + expf(-g));
-        else if (act == LSB_ACT_GELU_TANH)
-            a = 0.5f * g * (1.f + tanhf(0.7978845608f * (g + 0.044715f * g * g * g)));
-        else a = g;
-        out[idx] = lsb_from_float<T>(a * u);
+        out[idx] = lsb_from_float<T>(lsb_gated(lsb_to_float(gate_up[2 * idx]), lsb_to_float(gate_up[2 * idx + 1]), act, limit));
     }
 }
 

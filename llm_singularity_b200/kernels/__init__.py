@@ -534,6 +534,12 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
         _call("gemm_tc", "lsb_gemm_tc", _p(x), _p(w), _p(out), _i(1 if out_dtype == torch.float32 else 0),
               _i(M), _i(N), _i(K), _i(act), _f(0.0), _stream(out))
         return out
+    if x.dtype == torch.float32 and _lib("gemm_f32").lsb_gemm_f32_supported(_p(x), _p(w), _i(M), _i(N), _i(K)):
+        out = torch.empty((M, N // 2 if gated else N), dtype=out_dtype, device=x.device)
+        _call("gemm_f32", "lsb_gemm_f32", _p(x), _p(w), _p(out), _i(M), _i(N), _i(K), _i(act if gated else 0), _stream(out))
+        if plain_act is not None:
+            plain_activation(out, out, plain_act)
+        return out
     out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     _call("gemm", "lsb_gemm_nt", _p(x), _p(w), _p(out), _i(_dt(x)), _i(_dt(out)), _i(M), _i(N), _i(K),
           _ll(K), _ll(K), _ll(N), _stream(out))

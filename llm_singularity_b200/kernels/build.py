@@ -37,6 +37,7 @@ SOURCES: Dict[str, object] = {          # library -> its source file (or files)
     "attention_tc": "attention_tc.cu",
     "attention_tc5": "attention_tc5.cu",
     "gemm": "gemm.cu",
+    "gemm_f32": "gemm_f32.cu",
     "gemm_tc": "gemm_tc.cu",
     "gemm_small": "gemm_small.cu",
     "gemm_stream": "gemm_stream.cu",
@@ -61,7 +62,7 @@ SOURCES: Dict[str, object] = {          # library -> its source file (or files)
     # host code only: pools, block tables, prefix tree; scheduler
     "host_runtime": ("host_memory.cpp", "host_scheduler.cpp", "host_step.cpp"),
 }
-HEADERS = ["common.cuh", "attention_tc_noalloc.h", "attention_dv.cuh", "attention_tc5.cuh", "stream_warm.cuh"]     # of the CUDA libraries
+HEADERS = ["common.cuh", "attention_tc_noalloc.h", "attention_dv.cuh", "attention_tc5.cuh", "stream_warm.cuh", "gate_act.cuh"]     # of the CUDA libraries
 HOST_HEADERS = ["host_memory.h"]                          # of the host runtime
 
 

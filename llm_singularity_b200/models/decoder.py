@@ -125,6 +125,8 @@ class DecoderModel:
                     names.append(k)
         if self.rt.dtype == torch.bfloat16 and "gemm" in names:
             names += ["gemm_tc", "gemm_small", "gemm_stream"]    # bfloat16 products run on the tensor cores
+        elif "gemm" in names:
+            names.append("gemm_f32")
         return names
 
     # ------------------------------------------------------------------ forward
