@@ -12,8 +12,8 @@
 //                  accumulating in TMEM (HD columns) over all tiles; the softmax warps rescale O only
 //                  when a row's maximum has outgrown its reference by 2^8, and read it once at the end
 // Warp 0 issues the TMA loads (one lane per page of the tile), warp 1 issues the MMAs and owns the
-// TMEM allocation, warps 2-5 do the softmax and the final store.  Three blocks fit per SM (head 64),
-// so one block's softmax overlaps the others' matrix products.  All mbarrier waits are bounded.
+// TMEM allocation, warps 2-5 do the softmax and the final store.  Two blocks share an SM, so one
+// block's softmax overlaps the other's matrix products.  All mbarrier waits are bounded.
 //
 // Query row i of a request with q_len new tokens and kv_len cached tokens sits at position
 // p = kv_len - q_len + i and sees keys [max(0, p - window + 1), p].  This kernel takes what the
@@ -28,8 +28,7 @@ LSB_DEFINE_STATUS()
 #include "attention_tc5.cuh"
 
 constexpr int kThreads = 224;        // warps: TMA, MMA for S, four softmax warps, MMA for P V
-constexpr int kKvStages = 4;          // K/V tiles in flight
-constexpr int kBlocksPerSm64 = 2;     // blocks of head size 64 that share an SM (head 128: one)
+constexpr int kBlocksPerSm = 2;       // blocks that share an SM: one's softmax beside the other's products
 constexpr int kBtCache = 512;         // block-table entries of this block's key range kept in smem
 
 struct AttnParams {
@@ -56,30 +55,46 @@ struct Smem {
     static constexpr int kKB = HD / 64;                     // 64-dim blocks of a head
     static constexpr int kQBytes = kRows * HD * 2;
     static constexpr int kKVBytes = kKeys * HD * 2;         // one of K or V, one stage
-    static constexpr size_t kTotal = 1024 + kQBytes + 2 * kKvStages * kKVBytes +
-                                     kBtCache * 4 + 20 * 8 + 16;
+    // Tiles in flight.  Two blocks of head size 128 have room for two; a K tile is handed back as soon as its scores
+    // are formed there, a V tile when its share of O is, each through a barrier of its own.  At head size 64 there is
+    // room for four, and K and V of a tile come and go together (a barrier less to wait on: 2 us of 42 at 2,048 tokens).
+    static constexpr int kStages = HD == 64 ? 4 : 2;
+    // Tensor memory: half an SM's 512 columns for each block.  S twice (kKeys columns of 32-bit scores each: even and
+    // odd tiles) and O (HD columns); P (kKeys / 2 columns a tile: two bfloat16 per column) beside them at head size 64.
+    // At 128 P takes the place of its own tile's S: a row's scores are in its thread's registers by then, and S of the
+    // tile after the next waits for the P V product instead of for the registers.  With columns of their own for P
+    // a block took all 512 and had the SM to itself: 2,011 queries over 4,096 keys and their own, 32 / 8 heads, 297 us
+    // then, 211 us (800 TFLOP/s) now.
+    static constexpr bool kShareS = HD == 128;
+    static constexpr uint32_t kPCol = kShareS ? 0 : 2 * kKeys, kPStep = kShareS ? kKeys : kKeys / 2;
+    static constexpr uint32_t kOCol = kShareS ? 2 * kKeys : 3 * kKeys;
+    static constexpr uint32_t kTmemCols = 256;
+    static_assert(kOCol + HD <= kTmemCols, "two blocks share the SM's tensor memory");
+    static constexpr int kBars = 1 + 4 * kStages + 8;
+    static constexpr size_t kTotal = 1024 + kQBytes + 2 * kStages * kKVBytes + kBtCache * 4 + kBars * 8 + 16;
 };
 
 template <int HD>
-__global__ void __launch_bounds__(kThreads, HD == 64 ? kBlocksPerSm64 : 1)
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                              const __grid_constant__ CUtensorMap map_v, const AttnParams prm) {
     using L = Smem<HD>;
     constexpr int KB = L::kKB;
-    // tensor memory: S twice (kKeys columns of 32-bit scores each: even and odd tiles), P twice
-    // (kKeys / 2 columns each: two bfloat16 per column), the O tile (HD columns)
-    constexpr uint32_t kTmemCols = (3 * kKeys + HD) <= 128 ? 128 : (3 * kKeys + HD) <= 256 ? 256 : 512;
+    constexpr uint32_t kTmemCols = L::kTmemCols;
+    constexpr int ST = L::kStages;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sQ = base;                                // [KB][128 rows][128 B]
     unsigned char* sK = sQ + L::kQBytes;                     // [stages][KB][128 keys][128 B]
-    unsigned char* sV = sK + kKvStages * L::kKVBytes;        // [stages][KB][128 keys][128 B]
-    int* sBT = reinterpret_cast<int*>(sV + kKvStages * L::kKVBytes);
+    unsigned char* sV = sK + ST * L::kKVBytes;               // [stages][KB][128 keys][128 B]
+    int* sBT = reinterpret_cast<int*>(sV + ST * L::kKVBytes);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sBT + kBtCache);
     uint64_t* q_full = bars;                                 // TMA -> MMA
-    uint64_t* kv_full = bars + 1;                            // [stages] TMA -> MMA
-    uint64_t* kv_empty = kv_full + kKvStages;                // [stages] MMA -> TMA
-    uint64_t* s_full = kv_empty + kKvStages;                 // [2] MMA -> softmax: S of an even / odd tile
+    uint64_t* k_full = bars + 1;                             // [stages] TMA -> MMA
+    uint64_t* k_empty = k_full + ST;                         // [stages] MMA -> TMA
+    uint64_t* v_full = k_empty + ST;                         // the same for V
+    uint64_t* v_empty = v_full + ST;
+    uint64_t* s_full = v_empty + ST;                         // [2] MMA -> softmax: S of an even / odd tile
     // P of even and of odd tiles has a barrier each: a softmax warp may be a whole tile ahead of
     // another (S of the next tile comes early), and its arrival for tile t + 1 must not count
     // towards tile t, whose P a slower warp has yet to write.  Two tiles ahead it cannot be: P of
@@ -116,7 +131,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
     if (threadIdx.x == 0) {
         abort_flag = 0;
         mbar_init(q_full, 1);
-        for (int s = 0; s < kKvStages; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+        for (int s = 0; s < 4 * ST; ++s) mbar_init(&k_full[s], 1);     // (k_full, k_empty, v_full, v_empty)
         mbar_init(&s_full[0], 1);
         mbar_init(&s_full[1], 1);
         mbar_init(&p_full[0], 4);
@@ -146,8 +161,8 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_s = *tmem_slot;                      // S of even tiles, then of odd tiles
-    const uint32_t tmem_p = tmem_s + 2 * kKeys;              // P of even tiles, then of odd tiles
-    const uint32_t tmem_o = tmem_s + 3 * kKeys;              // O tile
+    const uint32_t tmem_p = tmem_s + L::kPCol;               // P of even tiles, then of odd tiles
+    const uint32_t tmem_o = tmem_s + L::kOCol;               // O tile
     const int n_tiles = t1 - t0;
 
     if (warp == 0) {
@@ -160,15 +175,13 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
             for (int kb = 0; kb < KB; ++kb)
                 tma_load_2d(sQ + kb * (kRows * 128), &map_q, q_full, h * HD + kb * 64, qs + i0);
         }
-        bool ok = true;
-        for (int t = 0; t < n_tiles && ok; ++t) {
-            const int s = t % kKvStages;
-            if (t >= kKvStages) {
-                if (lane == 0) ok = mbar_wait(&kv_empty[s], (uint32_t)((t / kKvStages) - 1) & 1, &abort_flag);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                if (!ok) break;
-            }
-            if (lane == 0) mbar_expect_tx(&kv_full[s], 2 * L::kKVBytes);
+        // one tile of K or V into its stage, page by page, once the stage is free
+        auto load = [&](int t, const CUtensorMap* map, unsigned char* stages, uint64_t* full, uint64_t* empty) -> bool {
+            const int s = t % ST;
+            int free = 1;
+            if (t >= ST && lane == 0) free = mbar_wait(&empty[s], (uint32_t)((t / ST) - 1) & 1, &abort_flag) ? 1 : 0;
+            if (!__shfl_sync(0xffffffffu, free, 0)) return false;
+            if (lane == 0) mbar_expect_tx(&full[s], (L::kShareS ? 1 : 2) * L::kKVBytes);
             __syncwarp();
             if (lane < pages_per_tile) {
                 // pages past the last needed one repeat it: their keys are masked, their bytes finite
@@ -184,19 +197,31 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
                         page = 0;
                     }
                 }
-                const int row_off = lane * prm.page_size * 128;    // bytes into a 64-dim block
-                for (int kb = 0; kb < KB; ++kb) {
-                    tma_load_4d(sK + s * L::kKVBytes + kb * (kKeys * 128) + row_off, &map_k, &kv_full[s], kb * 64, 0, g, page);
-                    tma_load_4d(sV + s * L::kKVBytes + kb * (kKeys * 128) + row_off, &map_v, &kv_full[s], kb * 64, 0, g, page);
-                }
+                unsigned char* dst = stages + s * L::kKVBytes + lane * prm.page_size * 128;    // rows of a 64-dim block
+                for (int kb = 0; kb < KB; ++kb) tma_load_4d(dst + kb * (kKeys * 128), map, &full[s], kb * 64, 0, g, page);
+                if (!L::kShareS) tma_load_4d(dst + (sV - sK), &map_v, &full[s], 0, 0, g, page);
             }
+            return true;
+        };
+        if (L::kShareS) {
+            // K runs a tile ahead of V: its stage is free that much earlier
+            bool ok = load(0, &map_k, sK, k_full, k_empty);
+            for (int t = 0; t < n_tiles && ok; ++t) {
+                if (t + 1 < n_tiles) ok = load(t + 1, &map_k, sK, k_full, k_empty);
+                if (ok) ok = load(t, &map_v, sV, v_full, v_empty);
+            }
+        } else {
+            bool ok = true;
+            for (int t = 0; t < n_tiles && ok; ++t) ok = load(t, &map_k, sK, k_full, k_empty);
         }
         // copies in flight must land before the block may exit
         if (lane == 0) {
             int dummy = 0;
             mbar_wait(q_full, 0, &dummy);
-            for (int t = max(0, n_tiles - kKvStages); t < n_tiles; ++t)
-                mbar_wait(&kv_full[t % kKvStages], (uint32_t)(t / kKvStages) & 1, &dummy);
+            for (int t = max(0, n_tiles - ST); t < n_tiles; ++t) {
+                mbar_wait(&k_full[t % ST], (uint32_t)(t / ST) & 1, &dummy);
+                if (L::kShareS) mbar_wait(&v_full[t % ST], (uint32_t)(t / ST) & 1, &dummy);
+            }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
@@ -215,7 +240,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
                 db_k0[kb] = desc_kmajor(sK + kb * (kKeys * 128));
             }
             auto issue_s = [&](int t) {
-                const uint64_t stage = (uint64_t)((t % kKvStages) * (L::kKVBytes >> 4));    // address field: bytes / 16
+                const uint64_t stage = (uint64_t)((t % ST) * (L::kKVBytes >> 4));    // address field: bytes / 16
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) {
 #pragma unroll
@@ -224,12 +249,13 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
                                   idesc_qk, (kb | k) ? 1u : 0u);
                 }
                 umma_commit(&s_full[t & 1]);
+                if (L::kShareS) umma_commit(&k_empty[t % ST]);
             };
             for (int t = 0; t < n_tiles && ok; ++t) {
-                ok = mbar_wait(&kv_full[t % kKvStages], (uint32_t)(t / kKvStages) & 1, &abort_flag);
+                ok = mbar_wait(&k_full[t % ST], (uint32_t)(t / ST) & 1, &abort_flag);
                 if (!ok) break;
-                if (t >= 2) {                                  // this buffer's last S is in registers
-                    ok = mbar_wait(&s_free[t & 1], (uint32_t)((t >> 1) - 1) & 1, &abort_flag);
+                if (t >= 2) {                                  // this buffer's last S is in registers; its P is used up
+                    ok = mbar_wait(L::kShareS ? &o_full[t & 1] : &s_free[t & 1], (uint32_t)((t >> 1) - 1) & 1, &abort_flag);
                     if (!ok) break;
                 }
                 tc_fence_after();
@@ -245,19 +271,20 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
             const uint64_t db_v0 = desc_mnmajor(sV, kKeys * 128);
             bool ok = true;
             for (int t = 0; t < n_tiles && ok; ++t) {
-                const int s = t % kKvStages;
+                const int s = t % ST;
+                if (L::kShareS && !mbar_wait(&v_full[s], (uint32_t)(t / ST) & 1, &abort_flag)) break;
                 // P of this tile (and O rescaled where a row's reference maximum moved)
                 ok = mbar_wait(&p_full[t & 1], (uint32_t)(t >> 1) & 1, &abort_flag);
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t db = db_v0 + (uint64_t)(s * (L::kKVBytes >> 4));
-                const uint32_t pa = tmem_p + (uint32_t)((t & 1) * (kKeys / 2));
+                const uint32_t pa = tmem_p + (uint32_t)(t & 1) * L::kPStep;
 #pragma unroll
                 for (int j = 0; j < kKeys / 16; ++j)           // 16 keys per MMA: eight columns of P, 16 rows of V
                     umma_bf16_ts(tmem_o, pa + j * 8, db + (uint64_t)(j * ((16 * 128) >> 4)), idesc_pv, (t | j) ? 1u : 0u);
                 umma_commit(&o_full[t & 1]);
-                // K of this stage was read by the S product that this P descends from
-                umma_commit(&kv_empty[s]);
+                // (K of this stage was read by the S product that this P descends from)
+                umma_commit(L::kShareS ? &v_empty[s] : &k_empty[s]);
             }
         }
     } else {
@@ -307,13 +334,14 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
             const bool full = key0 + kKeys - 1 <= p0 && rows == kRows &&
                               (prm.window <= 0 || key0 > p_last - prm.window);
             // this tile's P buffer was read by the P V of the tile before the previous one
+            // (where P shares S's columns, S of this tile was not formed before that)
             uint32_t p_free = 1;
-            if (t > 1 && lane == 0) p_free = mbar_test(&o_full[t & 1], (uint32_t)((t >> 1) - 1) & 1);
+            if (!L::kShareS && t > 1 && lane == 0) p_free = mbar_test(&o_full[t & 1], (uint32_t)((t >> 1) - 1) & 1);
             // S of this row: kKeys values, read from TMEM once.  Tiles wholly below the diagonal (the
             // common case) skip the key tests; partial maxima / sums are independent so that a warp
             // with a scheduler to itself still finds instructions to issue.
             tmem_ld_wait();
-            warp_arrive(&s_free[t & 1], lane);                 // S of the tile after the next may overwrite this one
+            if (!L::kShareS) warp_arrive(&s_free[t & 1], lane);    // S of the tile after the next may overwrite this one
             // columns of this tile the row may see: [c_lo, c_hi]
             if (modified) {
                 // cap tanh(z) = cap - 2 cap / (1 + e^(2 z)); the distance to key x of the tile is dist0 - x
@@ -402,7 +430,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
             // P stays in tensor memory: the P V product takes it from there as its A operand
 #pragma unroll
             for (int c0 = 0; c0 < kKeys / 2; c0 += 32)
-                tmem_st_32x32(tmem_p + lane_sel + (uint32_t)((t & 1) * (kKeys / 2) + c0),
+                tmem_st_32x32(tmem_p + lane_sel + (uint32_t)(t & 1) * L::kPStep + (uint32_t)c0,
                               *reinterpret_cast<uint32_t(*)[32]>(&pw[c0]));
             loaded = __shfl_sync(0xffffffffu, s_next, 0) != 0;
             if (loaded) {
