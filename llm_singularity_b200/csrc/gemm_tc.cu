@@ -162,6 +162,8 @@ struct GemmParams {
     // earlier in the stream, so a block reads it only after the wait on that kernel.
     const int* tile_group;
     int group_rows;
+    // persistent form: columns of a tile (a multiple of 16 up to 256) and stages of the ring
+    int bn, stages;
     // Swapped: P stacks the groups' matrices and tile_group[j0 / BN] names the group of a BN-row tile of Q.
     int group_swap;
 };
@@ -315,8 +317,8 @@ template <int BN, bool GATED>
 __device__ __forceinline__ void epilogue_staged(const GemmParams& prm, unsigned char* stage_base, uint32_t tmem_base,
                                                 int q, int lane, int i0, int j0) {
     constexpr int OUT_COLS = GATED ? BN / 2 : BN;
-    constexpr int CPROW = OUT_COLS / 8;                       // 16-byte chunks per output row
-    static_assert(CPROW >= 8, "the swizzle needs at least eight chunks per row");
+    constexpr int CPROW = OUT_COLS / 8;                       // 16-byte chunks per output row (a power of two)
+    constexpr int SW = CPROW >= 8 ? 7 : CPROW - 1;            // which of a row's chunks change places
     uint4* mine = reinterpret_cast<uint4*>(stage_base) + (size_t)q * 32 * CPROW;
 #pragma unroll
     for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -336,7 +338,7 @@ __device__ __forceinline__ void epilogue_staged(const GemmParams& prm, unsigned 
                     w[y] = *reinterpret_cast<uint32_t*>(&h);
                 }
                 const int cc = (c0 / 32) * 2 + k;
-                mine[lane * CPROW + (cc ^ (lane & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
+                mine[lane * CPROW + (cc ^ (lane & SW))] = make_uint4(w[0], w[1], w[2], w[3]);
             }
         } else {
             if (prm.plain) plain_act_all(r, prm.plain);
@@ -350,7 +352,7 @@ __device__ __forceinline__ void epilogue_staged(const GemmParams& prm, unsigned 
                     w[y] = *reinterpret_cast<uint32_t*>(&h);
                 }
                 const int cc = (c0 / 32) * 4 + k;
-                mine[lane * CPROW + (cc ^ (lane & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
+                mine[lane * CPROW + (cc ^ (lane & SW))] = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
     }
@@ -363,7 +365,7 @@ __device__ __forceinline__ void epilogue_staged(const GemmParams& prm, unsigned 
         const int row = idx / CPROW, c = idx % CPROW;
         const int i = i0 + q * 32 + row;
         if (i < prm.rows_p)
-            *reinterpret_cast<uint4*>(out + (long long)i * prm.ldc_i + jo + c * 8) = mine[row * CPROW + (c ^ (row & 7))];
+            *reinterpret_cast<uint4*>(out + (long long)i * prm.ldc_i + jo + c * 8) = mine[row * CPROW + (c ^ (row & SW))];
     }
     __syncwarp();                                              // the buffer may be refilled right away
 }
@@ -671,33 +673,47 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-constexpr int kEpiCols = 128;                                 // columns drained per pass
-constexpr int kEpiBytes = 4 * 32 * kEpiCols * 2;             // 4 warps x 32 rows x 128 bf16
+constexpr int kEpiBytes = 4 * 32 * 128;                      // 4 warps x 32 rows x 128 bytes of a row at a time
+constexpr int kMaxStages = 8;
+constexpr int kPersistentMin = 128;                          // columns of a product from which on tiles of 128 and wider pay
+constexpr int kPersistentSmem = 226 * 1024;                  // what a block may ask for
 
-template <int BN, int STAGES>
-struct PersistentLayout {
-    static constexpr int kPBytes = kBM * kBK * 2;
-    static constexpr int kQBytes = BN * kBK * 2;
-    static constexpr int kStageBytes = kPBytes + kQBytes;
-    static constexpr int kBars = 2 * STAGES + 4;
-    static constexpr size_t kTotal = 1024 + (size_t)STAGES * kStageBytes + kEpiBytes + kBars * 8 + 16;
-};
+static constexpr int stage_bytes(int bn) { return (kBM + bn) * kBK * 2; }
+static constexpr size_t persistent_smem(int bn, int stages) {
+    return 1024 + (size_t)stages * stage_bytes(bn) + kEpiBytes + (2 * kMaxStages + 4) * 8 + 16;
+}
 
-template <int BN, int STAGES>
+// The row-major, whole-tile epilogues of one accumulator, in passes whose rows are 128 bytes, the rest narrower.  A warp
+// keeps to its own 4 KB of the staging buffer whatever the width of a pass (epilogue_staged gives it 32 rows of the
+// pass's width): a warp that is a pass behind would find its rows overwritten otherwise.
+template <bool GATED>
+__device__ __forceinline__ void drain_staged(const GemmParams& prm, unsigned char* epi, uint32_t tmem_acc, int q, int lane,
+                                             int i0, int j0) {
+    constexpr int PASS = GATED ? 128 : 64;
+    int h = 0;
+#pragma unroll 1
+    for (; h + PASS <= prm.bn; h += PASS) epilogue_staged<PASS, GATED>(prm, epi, tmem_acc + h, q, lane, i0, j0 + h);
+    if (GATED && (prm.bn & 64)) {
+        epilogue_staged<64, GATED>(prm, epi + q * 2048, tmem_acc + h, q, lane, i0, j0 + h);
+        h += 64;
+    }
+    if (prm.bn & 32) epilogue_staged<32, GATED>(prm, epi + q * (GATED ? 3072 : 2048), tmem_acc + h, q, lane, i0, j0 + h);
+}
+
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                           const GemmParams prm, int tiles_m, int tiles_n) {
-    using L = PersistentLayout<BN, STAGES>;
-    static_assert(BN == 16 || BN == 32 || BN == 64 || BN == 128 || BN == 256,
-                  "two accumulators of BN columns: a power of two of TMEM columns, at most 512");
-    constexpr uint32_t kTmemCols = 2 * BN;
+    const int BN = prm.bn, STAGES = prm.stages;
+    const uint32_t kPBytes = kBM * kBK * 2, kStageBytes = kPBytes + (uint32_t)BN * (kBK * 2);
+    // two accumulators, each a power of two of TMEM columns
+    const uint32_t acc_cols = BN <= 16 ? 16 : BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* stages = base;
-    unsigned char* epi = base + (size_t)STAGES * L::kStageBytes;
+    unsigned char* epi = base + (size_t)STAGES * kStageBytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(epi + kEpiBytes);
-    uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;                      // [2]
+    uint64_t* empty = full + kMaxStages;
+    uint64_t* acc_full = empty + kMaxStages;                  // [2]
     uint64_t* acc_empty = acc_full + 2;                       // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     __shared__ int abort_flag;
@@ -725,14 +741,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
         for (int t = blockIdx.x; t < n_tiles && pre < STAGES && !groups; t += gridDim.x) {
             const int i0 = (t % tiles_m) * kBM, j0 = (t / tiles_m) * BN;
             for (int kb = 0; kb < nkb && pre < STAGES; ++kb, ++pre) {
-                unsigned char* st = stages + (size_t)pre * L::kStageBytes;
-                mbar_expect_tx(&full[pre], L::kStageBytes);
+                unsigned char* st = stages + (size_t)pre * kStageBytes;
+                mbar_expect_tx(&full[pre], kStageBytes);
                 if (weights_p) tma_load_2d(st, &map_p, &full[pre], kb * kBK, i0);
-                else tma_load_2d(st + L::kPBytes, &map_q, &full[pre], kb * kBK, j0);
+                else tma_load_2d(st + kPBytes, &map_q, &full[pre], kb * kBK, j0);
             }
         }
     }
-    if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+    if (warp == 1) tmem_alloc(tmem_slot, 2 * acc_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -742,7 +758,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
     if (warp == 0) {
         if (lane == 0) {
             lsb_pdl_wait();
-            long long it = 0;                                  // K blocks issued so far, over all tiles
+            int issued = 0;                                    // K blocks issued so far, over all tiles (as far as it matters)
+            int s = 0;
+            uint32_t round = 0;                                // how often the ring has been gone round
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
                 const int i0 = row_of(t) * kBM;
@@ -752,30 +770,34 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
                     if (g < 0) continue;
                     j0 += g * prm.group_rows;
                 }
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = (int)(it % STAGES);
-                    unsigned char* st = stages + (size_t)s * L::kStageBytes;
-                    if (it < pre) {                            // the other half of a box requested above
-                        if (weights_p) tma_load_2d(st + L::kPBytes, &map_q, &full[s], kb * kBK, j0);
+                for (int kb = 0; kb < nkb; ++kb) {
+                    unsigned char* st = stages + (size_t)s * kStageBytes;
+                    if (round == 0 && s < pre) {               // the other half of a box requested above
+                        if (weights_p) tma_load_2d(st + kPBytes, &map_q, &full[s], kb * kBK, j0);
                         else tma_load_2d(st, &map_p, &full[s], kb * kBK, i0);
-                        continue;
+                    } else {
+                        if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, &abort_flag)) { ok = false; break; }
+                        mbar_expect_tx(&full[s], kStageBytes);
+                        tma_load_2d(st, &map_p, &full[s], kb * kBK, i0);
+                        tma_load_2d(st + kPBytes, &map_q, &full[s], kb * kBK, j0);
                     }
-                    if (it >= STAGES && !mbar_wait(&empty[s], (uint32_t)((it / STAGES) - 1) & 1, &abort_flag)) { ok = false; break; }
-                    mbar_expect_tx(&full[s], L::kStageBytes);
-                    tma_load_2d(st, &map_p, &full[s], kb * kBK, i0);
-                    tma_load_2d(st + L::kPBytes, &map_q, &full[s], kb * kBK, j0);
+                    issued = min(issued + 1, STAGES);
+                    if (++s == STAGES) { s = 0; ++round; }
                 }
             }
             // copies still in flight must land before the block may exit
-            for (long long k = it > STAGES ? it - STAGES : 0; k < it; ++k) {
+            for (int k = 0; k < issued; ++k) {
                 int dummy = 0;
-                mbar_wait(&full[k % STAGES], (uint32_t)(k / STAGES) & 1, &dummy);
+                if (s == 0) { s = STAGES; --round; }
+                --s;
+                mbar_wait(&full[s], round & 1, &dummy);
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BN);
-            long long it = 0;
+            const uint32_t idesc = make_idesc(BN);
+            int s = 0;
+            uint32_t parity = 0;
             int local = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
@@ -785,18 +807,18 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
                 ok = mbar_wait(&acc_empty[a], (uint32_t)((local >> 1) & 1) ^ 1u, &abort_flag);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)(a * BN);
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = (int)(it % STAGES);
-                    ok = mbar_wait(&full[s], (uint32_t)(it / STAGES) & 1, &abort_flag);
+                const uint32_t tmem_d = tmem_base + (uint32_t)a * acc_cols;
+                for (int kb = 0; kb < nkb; ++kb) {
+                    ok = mbar_wait(&full[s], parity, &abort_flag);
                     if (!ok) break;
                     tc_fence_after();
-                    unsigned char* st = stages + (size_t)s * L::kStageBytes;
-                    const uint64_t dp = make_smem_desc(st), dq = make_smem_desc(st + L::kPBytes);
+                    unsigned char* st = stages + (size_t)s * kStageBytes;
+                    const uint64_t dp = make_smem_desc(st), dq = make_smem_desc(st + kPBytes);
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k)
                         umma_bf16(tmem_d, dp + 2 * k, dq + 2 * k, idesc, (kb | k) ? 1u : 0u);
                     umma_commit(&empty[s]);
+                    if (++s == STAGES) { s = 0; parity ^= 1u; }
                 }
                 umma_commit(&acc_full[a]);
                 ++local;
@@ -806,8 +828,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
         const int q = warp & 3;
         const int il = q * 32 + lane;
         const int n_out = prm.swiglu == 1 ? prm.rows_q / 2 : prm.rows_q;
-        const bool aligned = !prm.out_f32 && (n_out % 8) == 0 && (((uintptr_t)prm.out) & 15) == 0;
-        const bool aligned32 = prm.out_f32 && !prm.swiglu && (n_out % 4) == 0 && prm.ldc_j == 1 && (((uintptr_t)prm.out) & 15) == 0;
+        // (whole tiles leave through shared memory; a tile's columns are a multiple of 32 then)
+        const bool staged = prm.ldc_j == 1 && (BN & 31) == 0 && (((uintptr_t)prm.out) & 15) == 0;
+        const bool aligned = staged && !prm.out_f32 && prm.swiglu != 2 && (n_out % 8) == 0;
+        const bool aligned32 = staged && prm.out_f32 && !prm.swiglu && (n_out % 4) == 0;
         int local = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
@@ -818,25 +842,22 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
             tc_fence_after();
             ok = ok && !abort_flag;
             if (!ok) break;
-            const uint32_t tmem_acc = tmem_base + (uint32_t)(a * BN);
-            if (BN >= kEpiCols && aligned && j0 + BN <= prm.rows_q) {
-#pragma unroll
-                for (int h = 0; h < BN / kEpiCols; ++h) {
-                    if (prm.swiglu == 1)
-                        epilogue_staged<kEpiCols, true>(prm, epi, tmem_acc + h * kEpiCols, q, lane, i0, j0 + h * kEpiCols);
-                    else
-                        epilogue_staged<kEpiCols, false>(prm, epi, tmem_acc + h * kEpiCols, q, lane, i0, j0 + h * kEpiCols);
-                }
-            } else if (BN >= kEpiCols && aligned32 && j0 + BN <= prm.rows_q) {
+            const uint32_t tmem_acc = tmem_base + (uint32_t)a * acc_cols;
+            if (aligned && j0 + BN <= prm.rows_q) {
+                if (prm.swiglu == 1) drain_staged<true>(prm, epi, tmem_acc, q, lane, i0, j0);
+                else drain_staged<false>(prm, epi, tmem_acc, q, lane, i0, j0);
+            } else if (aligned32 && j0 + BN <= prm.rows_q) {
 #pragma unroll 1
-                for (int h = 0; h < BN / (kEpiCols / 2); ++h)
-                    epilogue_staged_f32<kEpiCols / 2>(prm, epi, tmem_acc + h * (kEpiCols / 2), q, lane, i0, j0 + h * (kEpiCols / 2));
+                for (int h = 0; h < BN; h += 32)
+                    epilogue_staged_f32<32>(prm, epi, tmem_acc + h, q, lane, i0, j0 + h);
             } else {
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 32) {
                     uint32_t r[32];
-                    load_acc<BN>(tmem_acc, q, c0, true, r);
-                    store_chunk<BN>(prm, r, i0 + il, j0 + c0, 32, lane);
+                    const bool whole = BN - c0 >= 32;
+                    if (whole) load_acc<32>(tmem_acc + c0, q, 0, true, r);
+                    else load_acc<16>(tmem_acc + c0, q, 0, true, r);
+                    store_chunk<256>(prm, r, i0 + il, j0 + c0, whole ? 32 : 16, lane);
                 }
             }
             tc_fence_before();
@@ -848,7 +869,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, 2 * acc_cols);
     }
 }
 
@@ -898,23 +919,25 @@ static int launch(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams
     return lsb_launch(gemm_tc_kernel<BN, STAGES>, grid, dim3(kGemmThreads), smem, stream, prm.splits, mp, mq, prm);
 }
 
-template <int BN, int STAGES>
-static int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& prm, int tiles_m,
+// bn columns a tile; as deep a ring as fits
+static int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, GemmParams prm, int bn, int tiles_m,
                              int tiles_n, cudaStream_t stream) {
     static int configured = -1;
     static int sms = 0;
-    constexpr size_t smem = PersistentLayout<BN, STAGES>::kTotal;
     if (configured < 0) {
-        configured = (int)cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, STAGES>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        configured = (int)cudaFuncSetAttribute(gemm_tc_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kPersistentSmem);
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
     if (configured) return configured;
+    prm.bn = bn;
+    prm.stages = kMaxStages;
+    while (persistent_smem(bn, prm.stages) > kPersistentSmem) --prm.stages;
     const int tiles = tiles_m * tiles_n;
     const int blocks = tiles < sms ? tiles : sms;
-    return lsb_launch(gemm_tc_persistent_kernel<BN, STAGES>, dim3(blocks), dim3(kGemmThreads), smem, stream, 1,
+    return lsb_launch(gemm_tc_persistent_kernel, dim3(blocks), dim3(kGemmThreads), persistent_smem(bn, prm.stages), stream, 1,
                       mp, mq, prm, tiles_m, tiles_n);
 }
 
@@ -986,22 +1009,24 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
         *splits = s;
     } else {
         *swap = 0;
-        // the widest tile that still fills the machine reasonably
+        // Persistent blocks walk the tile list.  What a tile costs is its stream of operands, (128 + bn) rows of
+        // K (128 x 256 x 64 takes the tensor core 512 cycles and its 48 KB about as long from L2), so the width is the
+        // one whose rounds over the SMs bring the fewest rows; the widest of equal ones.  2,048 tokens times
+        // 3,072 x 2,048: 192 tiles of 256 columns are two rounds, one of them a third full; 256 of 192 are two
+        // rounds of five sixths the length.
         const int mt = (M + kBM - 1) / kBM;
         int best = 64;
-        double best_eff = -1.0;
-        const int cands[3] = {256, 128, 64};
-        for (int c = 0; c < 3; ++c) {
-            const int t = mt * ((N + cands[c] - 1) / cands[c]);
-            const int waves = (t + sms - 1) / sms;
-            double eff = (double)t / ((double)waves * sms);
-            if (cands[c] == 64) eff *= 0.8;      // narrower tiles reuse P less
-            else if (cands[c] == 128) eff *= 0.93;
-            if (eff > best_eff + 1e-9) { best_eff = eff; best = cands[c]; }
+        if (N >= kPersistentMin) {
+            long long least = 0x7fffffffffffffffLL;
+            for (int c = 256; c >= 128; c -= 32) {
+                const long long t = (long long)mt * ((N + c - 1) / c);
+                long long rows = (t + sms - 1) / sms * (kBM + c);
+                if (c == 256) rows = rows * 15 / 16;          // (a narrower one has to be worth its traffic)
+                if (rows < least) { least = rows; best = c; }
+            }
+        } else if (N > 64) {
+            best = 128;
         }
-        // persistent blocks walk the tile list, so whole waves no longer matter: take the widest
-        // tile unless that leaves SMs without any
-        if (mt * ((N + 255) / 256) >= most || N >= 2048) best = 256;
         *bn = best;
         *splits = 1;
         // A few hundred tokens make too few 128 x 256 tiles for the SMs.  Where the walk through K
@@ -1009,7 +1034,7 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
         // wave; summing the partial tiles costs about as much as 2048 of K, so shorter walks stay
         // whole.  (The gated epilogue needs whole sums: gated products stay unsplit too.)
         const int tiles = mt * ((N + 255) / 256);
-        if (best == 256 && tiles < most && !swiglu) {
+        if (N >= 256 && tiles < most && !swiglu) {
             int s = sms / tiles;
             if (s > 8) s = 8;
             if (s > num_kb / 32) s = num_kb / 32;
@@ -1018,9 +1043,7 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
                 *splits = (num_kb + per - 1) / per;
             }
         }
-        // Unsplit and at most half the SMs busy: tiles half as wide bring the rest in (each
-        // block's stream of operands, which is what a lone tile waits for, gets shorter).
-        if (*splits == 1 && best == 256 && tiles <= sms / 2 && N > 128) *bn = 128;
+        if (*splits > 1) *bn = 256;
     }
     return 0;
 }
@@ -1042,6 +1065,7 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
     if (!known_act(swiglu) || (plain && !known_plain(plain))) return (int)cudaErrorInvalidValue;
     int swap, bn, splits;
     lsb_gemm_tc_plan(M, N, K, swiglu, &swap, &bn, &splits);
+    if (!swap && out_f32 && swiglu && bn > 128) bn = 256;      // (not a persistent product: widths that are compiled)
     const int n_out = swiglu ? N / 2 : N;
     GemmParams prm;
     prm.K = K;
@@ -1085,8 +1109,7 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
     if (!swap && !(out_f32 && swiglu) && bn >= 128) {
         // prompts: persistent blocks, double-buffered accumulator
         const int tm = (M + kBM - 1) / kBM, tn = (N + bn - 1) / bn;
-        return bn == 256 ? launch_persistent<256, 4>(mp, mq, prm, tm, tn, stream)
-                         : launch_persistent<128, 6>(mp, mq, prm, tm, tn, stream);
+        return launch_persistent(mp, mq, prm, bn, tm, tn, stream);
     }
     if (splits > 1) {
         switch (bn) {
@@ -1100,13 +1123,7 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
         // Many more weight slabs than SMs (the output head): persistent blocks walk the slabs, the
         // loads of the next slab run under the epilogue of this one and no SM idles between waves.
         const int tm = (int)grid.x;
-        switch (bn) {
-            case 16: rc = launch_persistent<16, 8>(mp, mq, prm, tm, 1, stream); break;
-            case 32: rc = launch_persistent<32, 8>(mp, mq, prm, tm, 1, stream); break;
-            case 64: rc = launch_persistent<64, 6>(mp, mq, prm, tm, 1, stream); break;
-            case 128: rc = launch_persistent<128, 5>(mp, mq, prm, tm, 1, stream); break;
-            default: return (int)cudaErrorInvalidValue;
-        }
+        rc = launch_persistent(mp, mq, prm, bn, tm, 1, stream);
     } else if (swap && (int)grid.x > sms && bn <= 64) {
         // More weight slabs than SMs, fewer than two rounds of them (a wide gated product): with
         // the deep ring one block fits an SM and the second round would run half empty; four
@@ -1197,7 +1214,7 @@ LSB_API int lsb_gemm_tc_grouped(const void* x, const void* w, void* out, int out
         case 128: return launch<128, 6>(mp, mq, prm, grid, stream);
         default:
             // (persistent blocks: the tile list is a few times as long as the chip is wide)
-            if (!(out_f32 && swiglu)) return launch_persistent<256, 4>(mp, mq, prm, (int)grid.x, (int)grid.y, stream);
+            if (!(out_f32 && swiglu)) return launch_persistent(mp, mq, prm, 256, (int)grid.x, (int)grid.y, stream);
             return launch<256, 4>(mp, mq, prm, grid, stream);
     }
 }
