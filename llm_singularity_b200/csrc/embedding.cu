@@ -24,6 +24,32 @@ __global__ void embedding_kernel(const T* __restrict__ table, const int* __restr
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = lsb_to_float(row[i]) * scale;
 }
 
+// Sixteen bytes of the row a thread and turn, all of them in flight: 2,048 tokens of 2,048 bfloat16 (25 MB)
+// 6.9 us, one element a thread and turn 11.8 us (eight dependent turns of 2-byte loads and 4-byte stores).
+template <typename T>
+__global__ void embedding_vec_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ out,
+                                     int hidden, int vocab, float scale) {
+    constexpr int VEC = 16 / sizeof(T);
+    lsb_pdl_launch_dependents();
+    lsb_pdl_wait();
+    const int t = blockIdx.x;
+    const int id = ids[t];
+    const bool known = id >= 0 && id < vocab;
+    if (!known && threadIdx.x == 0) lsb_set_status(LSB_BAD_TOKEN);
+    const T* row = table + (size_t)(known ? id : 0) * hidden;
+    float* o = out + (size_t)t * hidden;
+    for (int i = threadIdx.x * VEC; i < hidden; i += blockDim.x * VEC) {
+        T v[VEC];
+        *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(row + i);
+#pragma unroll
+        for (int e = 0; e < VEC; e += 4)
+            *reinterpret_cast<float4*>(o + i + e) =
+                known ? make_float4(lsb_to_float(v[e]) * scale, lsb_to_float(v[e + 1]) * scale, lsb_to_float(v[e + 2]) * scale,
+                                    lsb_to_float(v[e + 3]) * scale)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
 // The same with a second table added, whose row is a hash of the token and the one before it in its
 // sequence: row (prev * mul_prev + token * mul_cur) mod buckets, and row `buckets` (the table's last)
 // for a sequence's first token.  The token before the first of a step's portion is the request's state,
@@ -83,6 +109,13 @@ LSB_API int lsb_embedding_pair(const void* table, const void* pair_table, int dt
 LSB_API int lsb_embedding(const void* table, int dtype, const int* ids, float* out,
                           int tokens, int hidden, int vocab, float scale, cudaStream_t stream) {
     if (tokens <= 0) return 0;
+    const int vec = dtype == LSB_F32 ? 4 : 8;
+    if (hidden % vec == 0 && ((uintptr_t)table % 16) == 0 && ((uintptr_t)out % 16) == 0) {
+        int threads = (hidden / vec + 31) / 32 * 32;
+        if (threads > 512) threads = 512;
+        LSB_DISPATCH_DTYPE(dtype, return lsb_launch(embedding_vec_kernel<T>, dim3(tokens), dim3(threads), 0, stream, 1,
+                                                    (const T*)table, ids, out, hidden, vocab, scale));
+    }
     int threads = hidden < 256 ? ((hidden + 31) / 32) * 32 : 256;
     LSB_DISPATCH_DTYPE(dtype, return lsb_launch(embedding_kernel<T>, dim3(tokens), dim3(threads), 0, stream, 1,
                                                 (const T*)table, ids, out, hidden, vocab, scale));
