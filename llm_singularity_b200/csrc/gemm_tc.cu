@@ -1010,13 +1010,18 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
     } else {
         *swap = 0;
         // Persistent blocks walk the tile list.  What a tile costs is its stream of operands, (128 + bn) rows of
-        // K (128 x 256 x 64 takes the tensor core 512 cycles and its 48 KB about as long from L2), so the width is the
-        // one whose rounds over the SMs bring the fewest rows; the widest of equal ones.  2,048 tokens times
-        // 3,072 x 2,048: 192 tiles of 256 columns are two rounds, one of them a third full; 256 of 192 are two
-        // rounds of five sixths the length.
+        // K (128 x 256 x 64 takes the tensor core 512 cycles and its 48 KB about as long from L2), so where 256 columns
+        // take several rounds over the SMs, the width is the one whose rounds bring the fewest rows.  2,048 tokens times
+        // 3,072 x 2,048: 192 tiles of 256 columns are two rounds, one of them a third full (26.0 us); 256 of 192 are two
+        // rounds of five sixths the length (24.8 us).  543 times 16,384 x 3,072: 67.5 -> 63.2 us.  Within one round
+        // narrower tiles only bring more of x, and take SMs that the next kernel could begin on (543 times
+        // 5,120 x 3,072: 26.3 us with 256 columns, 28.3 with 192), unless half the SMs would stay idle.
         const int mt = (M + kBM - 1) / kBM;
+        const long long wide = (long long)mt * ((N + 255) / 256);
         int best = 64;
-        if (N >= kPersistentMin) {
+        if (N >= kPersistentMin && wide <= sms) {
+            best = wide <= sms / 2 ? 128 : 256;
+        } else if (N >= kPersistentMin) {
             long long least = 0x7fffffffffffffffLL;
             for (int c = 256; c >= 128; c -= 32) {
                 const long long t = (long long)mt * ((N + c - 1) / c);
