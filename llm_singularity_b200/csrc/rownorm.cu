@@ -201,6 +201,64 @@ rows_norm_gate_kernel(const float* __restrict__ x, const float* __restrict__ w, 
     }
 }
 
+// The same with four values a thread and turn (16-byte accesses), the row kept in shared memory between its sum and its
+// use, a warp a group where there are several: 1,503 rows of 2,048 (25 MB) 9.7 us, one value a thread
+// and turn 19.9 us (eight dependent turns, a division each for the group and the weight's place).
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads)
+rows_norm_gate_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, int w_len,
+                          const T* __restrict__ gate, long long gate_stride, T* __restrict__ out,
+                          int n, int groups, float eps) {
+    extern __shared__ __align__(16) float sh[];
+    float* row = sh;
+    float* factor = sh + n;
+    float* scratch = factor + groups;
+    lsb_pdl_launch_dependents();
+    lsb_pdl_wait();
+    const size_t t = blockIdx.x;
+    const int gs = n / groups;
+    float ss = 0.f;
+    for (int i = threadIdx.x * 4; i < n; i += blockDim.x * 4) {
+        float v[4];
+        load4(x + t * n + i, v);
+        store4(row + i, v);
+        ss += v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+    }
+    if (groups == 1) {
+        ss = lsb_block_sum(ss, scratch);
+        if (threadIdx.x == 0) factor[0] = 1.f / sqrtf(ss / (float)gs + eps);
+    } else {
+        __syncthreads();
+        const int lane = threadIdx.x & 31;
+        for (int g = threadIdx.x >> 5; g < groups; g += blockDim.x >> 5) {
+            float sum = 0.f;
+            for (int i = lane * 4; i < gs; i += 128) {
+                float v[4];
+                load4(row + g * gs + i, v);
+                sum += v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+            }
+            sum = lsb_warp_sum(sum);
+            if (lane == 0) factor[g] = 1.f / sqrtf(sum / (float)gs + eps);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x * 4; i < n; i += blockDim.x * 4) {
+        float v[4], k[4];
+        load4(row + i, v);
+        load4(w + i % w_len, k);
+        const float f = factor[i / gs];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = v[e] * f * k[e];
+        if (gate) {
+            float z[4];
+            load4(gate + t * gate_stride + i, z);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] *= lsb_sigmoid(z[e]);
+        }
+        store4(out + t * n + i, v);
+    }
+}
+
 template <typename T>
 __global__ void cast_rows_kernel(const float* __restrict__ x, T* __restrict__ out, long long count) {
     lsb_pdl_launch_dependents();
@@ -305,6 +363,14 @@ LSB_API int lsb_rows_norm_gate(const float* x, const float* w, int w_len, const 
         return (int)cudaErrorInvalidValue;
     const size_t smem = row_smem(n, groups);
     LSB_DISPATCH_DTYPE(dtype, {
+        const size_t es = sizeof(T) * 4;
+        if (n % 4 == 0 && (n / groups) % 4 == 0 && w_len % 4 == 0 && gate_stride % 4 == 0 && (uintptr_t)x % 16 == 0 &&
+            (uintptr_t)w % 16 == 0 && (uintptr_t)gate % es == 0 && (uintptr_t)out % es == 0) {
+            int vrc = allow_smem(rows_norm_gate_vec_kernel<T>, smem);
+            if (vrc) return vrc;
+            return lsb_launch(rows_norm_gate_vec_kernel<T>, dim3(rows), dim3(kRowThreads), smem, stream, 1, x, w, w_len,
+                              (const T*)gate, gate_stride, (T*)out, n, groups, eps);
+        }
         int rc = allow_smem(rows_norm_gate_kernel<T>, smem);
         if (rc) return rc;
         return lsb_launch(rows_norm_gate_kernel<T>, dim3(rows), dim3(kRowThreads), smem, stream, 1,
