@@ -13,16 +13,19 @@
 //
 // What bounds it is the number of times a row is walked and the blocks that walk it.  A row's logits are
 // read once: each block of the cluster keeps its contiguous slice (already divided by the
-// temperature) in shared memory.  The k-th largest value and the top-p cut are found with one histogram over
-// the values, linear from the row's maximum to its minimum, whose counts and masses the blocks add up through
-// distributed shared memory; the bucket the cut falls into is then collected (a few values) and the
-// cut picked among them exactly, by counting.  A bucket with more than kList values (rows whose values are all
-// but equal, or with outliers that stretch the range) is bisected instead, on the order-preserving integer image of the
-// floats, as many as 32 passes over the slices.  128 rows of 128,256 logits (greedy, temperature, top-k,
-// top-p and both in turn): 1,430 us with one block a row and bisection throughout, MEASURED_US us so.
+// temperature) in shared memory.  The cuts are found with histograms over the values, linear in the distance to the
+// row's maximum, that the blocks add up through distributed shared memory.  Counts give the bucket of the k-th value; where
+// only a few values reach that far, they are collected and both cuts picked among them exactly, by counting.  A cut
+// by mass alone takes a histogram of masses, near the maximum first (adding 64-bit masses in shared memory is slow
+// where all values of a row take part: 183 us for 128 rows with top-p alone), and the values of the one bucket the cut
+// falls into.  A bucket with more than kList values (rows whose values are all but equal, or with outliers that
+// stretch the range) is bisected instead, on the order-preserving integer image of the floats, as many as 32 passes
+// over the slices.  128 rows of 128,256 logits (greedy, temperature, top-k, top-p and both in turn): 1,425 us
+// with one block a row and bisection throughout, 100 us so.
 //
-// Probabilities are exp(x - max) in 32-bit; their sums are taken on 64-bit integers (exp * 2^44, so that even a
-// tail of values below 1e-9 counts), which makes every sum exact and the same whatever order the blocks add in.
+// Probabilities are exp(x - max) in 32-bit.  A thread adds its few dozen in 32-bit, everything beyond is added in 64-bit in
+// a fixed order; the histogram's masses, which arrive in any order, are 64-bit integers (exp * 2^44, so that even a tail
+// of values below 1e-9 counts): the same token every time.
 //
 // `work` is scratch of the same shape as the logits, used only where a slice does not fit shared memory
 // (lsb_sample_needs_work).
@@ -43,6 +46,7 @@ constexpr int kMaxBlocks = 8;                 // blocks of a row's cluster (the 
 constexpr int kSliceTarget = 8192;            // logits a block takes before another one joins the cluster
 constexpr int kBuckets = 1024;                // of the histogram, two a thread
 constexpr int kList = 1024;                   // values of one bucket that are picked among directly
+constexpr int kWhole = 512;                   // values up to the k-th that are, all of them
 constexpr int kSliceBytes = 184 * 1024;       // most shared memory for a slice
 
 __device__ __forceinline__ unsigned int ordered(float f) {
@@ -62,10 +66,11 @@ struct Part {                                 // what a block has found in its s
 
 struct Shared {
     Part part;
-    u64 slot[2];                              // a block's count or mass, by turns (bisection)
-    u64 seg[kWarps];                          // kept mass of each warp's stretch of the slice
-    u64 all_seg[kMaxBlocks * kWarps];         // ... of the whole row
+    double slot[2];                           // a block's count or mass, by turns
+    double seg[kWarps];                       // kept mass of each warp's stretch of the slice
+    double all_seg[kMaxBlocks * kWarps];      // ... of the whole row
     u64 scratch[kWarps];
+    double scratch_d[kWarps];
     float scratch_f[2 * kWarps];
     int scratch_i[kWarps];
     unsigned int cnt[kBuckets];               // this block's histogram
@@ -75,8 +80,8 @@ struct Shared {
     float list[kList];                        // (of the cluster's first block) values of one bucket
     u64 list_mass[kList];
     unsigned int list_n;
-    unsigned int thr_k, thr_p;                // the two cuts, broadcast by the first block
-    u64 kept;                                 // ... and the mass of the k-th value's bucket that is kept
+    unsigned int thr_k, thr_p;                // the first block's work on the two cuts
+    unsigned int cut, cut_mass;               // ... and what it tells the others
     int found;                                // bucket picked by find_bucket, and what stands before it
     u64 before;
 };
@@ -95,6 +100,23 @@ __device__ __forceinline__ u64 block_sum(u64 v, Shared& s) {
     u64 t = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) t += s.scratch[w];
+    return t;
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ double block_sum(double v, Shared& s) {
+    v = warp_sum(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s.scratch_d[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) t += s.scratch_d[w];
     return t;
 }
 
@@ -206,8 +228,6 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
         mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
     }
     if (lane == 0) { s.scratch_f[warp] = mx; s.scratch_i[warp] = mi; s.scratch_f[kWarps + warp] = mn; }
-    if (cut_k || cut_p)
-        for (int b = tid; b < kBuckets; b += kThreads) { s.cnt[b] = 0u; s.mass[b] = 0ull; }
     __syncthreads();
     if (tid == 0) {
         for (int w = 1; w < kWarps; ++w) {
@@ -232,240 +252,302 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
         return;
     }
 
-    // exp(x - max) as an integer; a value that is not a number counts nothing
-    auto mass_of = [&](float x) -> u64 {
+    // exp(x - max), as a number and as an integer; a value that is not a number counts nothing
+    auto weight_of = [&](float x) -> float {
         const float e = expf(x - mx);
-        return e > 0.f ? __float2ull_rn(e * mass_scale) : 0ull;
+        return e > 0.f ? e : 0.f;
+    };
+    auto mass_of = [&](float x) -> u64 { return __float2ull_rn(weight_of(x) * mass_scale); };
+    // f(value) for every value of the slice, four a thread and turn
+    const int n4 = (reinterpret_cast<uintptr_t>(xs) & 15) == 0 ? n >> 2 : 0;
+    auto each = [&](auto f) {
+#pragma unroll 2
+        for (int i = tid; i < n4; i += kThreads) {
+            const float4 v = reinterpret_cast<const float4*>(xs)[i];
+            f(v.x); f(v.y); f(v.z); f(v.w);
+        }
+        for (int i = 4 * n4 + tid; i < n; i += kThreads) f(xs[i]);
     };
     unsigned int thr = 0u;                                    // keep x with ordered(x) >= thr
     if (cut_k || cut_p) {
-        // ---- the histogram: bucket 0 holds the maximum; a larger value never has a later bucket
-        const float inv = mx > mn ? (float)(kBuckets - 1) / (mx - mn) : 0.f;
-        auto bucket = [&](float x) { return max(0, (int)fminf((mx - x) * inv, (float)(kBuckets - 1))); };
-        for (int i = tid; i < n; i += kThreads) {
-            const float x = xs[i];
-            const int b = bucket(x);
-            atomicAdd(&s.cnt[b], 1u);
-            if (cut_p) {
-                const u64 m = mass_of(x);
-                if (m) atomicAdd(&s.mass[b], m);
+        // The histogram's buckets are linear in the distance to the maximum, as far as `span`: a larger value never has
+        // a later bucket (kBuckets: none).
+        float span = INFINITY, inv = mx > mn ? (float)(kBuckets - 1) / (mx - mn) : 0.f;
+        auto bucket = [&](float x) {
+            const float d = mx - x;
+            return d <= span ? min(kBuckets - 1, max(0, (int)(d * inv))) : kBuckets;
+        };
+        // counts (and masses) of the values that are kept so far, over the whole row
+        auto histogram = [&](bool masses) {
+            for (int b = tid; b < kBuckets; b += kThreads) { s.cnt[b] = 0u; s.mass[b] = 0ull; }
+            __syncthreads();
+            each([&](float x) {
+                const int b = ordered(x) >= thr ? bucket(x) : kBuckets;
+                if (b < kBuckets) {
+                    atomicAdd(&s.cnt[b], 1u);
+                    if (masses) {
+                        const u64 m = mass_of(x);
+                        if (m) atomicAdd(&s.mass[b], m);
+                    }
+                }
+            });
+            cluster.sync();
+            const int share = kBuckets / blocks;              // (blocks is a power of two)
+            for (int j = tid; j < share; j += kThreads) {
+                const int b = rank * share + j;
+                unsigned int c = 0u;
+                u64 m = 0ull;
+                for (int r = 0; r < blocks; ++r) {
+                    c += *cluster.map_shared_rank(&s.cnt[b], r);
+                    if (masses) m += *cluster.map_shared_rank(&s.mass[b], r);
+                }
+                for (int r = 0; r < blocks; ++r) {
+                    *cluster.map_shared_rank(&s.tot_cnt[b], r) = c;
+                    if (masses) *cluster.map_shared_rank(&s.tot_mass[b], r) = m;
+                }
             }
-        }
-        cluster.sync();
-        const int share = kBuckets / blocks;                  // (blocks is a power of two)
-        for (int j = tid; j < share; j += kThreads) {
-            const int b = rank * share + j;
-            unsigned int c = 0u;
-            u64 m = 0ull;
-            for (int r = 0; r < blocks; ++r) {
-                c += *cluster.map_shared_rank(&s.cnt[b], r);
-                m += *cluster.map_shared_rank(&s.mass[b], r);
-            }
-            for (int r = 0; r < blocks; ++r) {
-                *cluster.map_shared_rank(&s.tot_cnt[b], r) = c;
-                *cluster.map_shared_rank(&s.tot_mass[b], r) = m;
-            }
-        }
-        cluster.sync();
-        // the row's sum of val(x) over all slices (bisection only)
+            cluster.sync();
+        };
+        // the row's sum of val(x) over all slices
         int turn = 0;
-        auto row_sum = [&](auto val) -> u64 {
-            u64 c = 0ull;
-            for (int i = tid; i < n; i += kThreads) c += val(xs[i]);
-            c = block_sum(c, s);
+        auto row_sum = [&](auto val) -> double {              // (a thread's few values in 32-bit, sums of those in 64-bit)
+            float part = 0.f;
+            each([&](float x) { part += val(x); });
+            const double c = block_sum((double)part, s);
             if (tid == 0) s.slot[turn] = c;
             cluster.sync();
-            u64 t = 0ull;
+            double t = 0.0;
             for (int r = 0; r < blocks; ++r) t += *cluster.map_shared_rank(&s.slot[turn], r);
             turn ^= 1;
             return t;
         };
-        // the values of one bucket that are >= thr, in the first block's list
-        auto collect = [&](int b) {
+        // the values of buckets b0 .. b1 that are kept so far, in the first block's list
+        auto collect = [&](int b0, int b1) {
             unsigned int* count = cluster.map_shared_rank(&s.list_n, 0);
             float* list = cluster.map_shared_rank(&s.list[0], 0);
-            for (int i = tid; i < n; i += kThreads) {
-                const float x = xs[i];
-                if (bucket(x) == b && ordered(x) >= thr) {
+            each([&](float x) {
+                const int b = bucket(x);
+                if (b >= b0 && b <= b1 && ordered(x) >= thr) {
                     const unsigned int at = atomicAdd(count, 1u);
                     if (at < (unsigned int)kList) list[at] = x;
                 }
-            }
+            });
             cluster.sync();
         };
-        int k_bucket = kBuckets;                               // the bucket of the k-th value
-        u64 k_mass = 0ull;                                     // mass of its values that are kept
-        bool listed = false;                                   // the first block's list holds it
+        // (first block) the r-th largest of the list's m values
+        auto pick_kth = [&](int m, u64 r) -> unsigned int {
+            if (tid == 0) s.thr_k = 0u;
+            __syncthreads();
+            for (int i = tid; i < m; i += kThreads) {
+                const unsigned int o = ordered(s.list[i]);
+                u64 above = 0ull, same = 0ull;
+                for (int j = 0; j < m; ++j) {
+                    const unsigned int oj = ordered(s.list[j]);
+                    above += oj > o;
+                    same += oj == o;
+                }
+                if (above < r && r <= above + same) s.thr_k = o;      // (equal values write the same)
+            }
+            __syncthreads();
+            return s.thr_k;
+        };
+        // (first block) the smallest of the list's values >= least before which there is no more mass than `most`;
+        // list_mass is there, `before` is the mass of larger values that are not in the list
+        auto pick_mass = [&](int m, unsigned int least, u64 before, double most) -> unsigned int {
+            if (tid == 0) s.thr_p = ordered(mx);
+            __syncthreads();
+            for (int i = tid; i < m; i += kThreads) {
+                const unsigned int o = ordered(s.list[i]);
+                if (o < least) continue;
+                u64 above = before;
+                for (int j = 0; j < m; ++j)
+                    if (ordered(s.list[j]) > o) above += s.list_mass[j];
+                if ((double)above <= most) atomicMin(&s.thr_p, o);
+            }
+            __syncthreads();
+            return s.thr_p;
+        };
+        auto share_out = [&](unsigned int* slot, unsigned int v) {     // (first block, thread 0)
+            for (int r = 0; r < blocks; ++r) *cluster.map_shared_rank(slot, r) = v;
+        };
+        bool done = !cut_p;                                    // nothing is left to be cut behind the k-th value
+        bool listed = false;                                   // the list has been used
         if (cut_k) {
             u64 before;
             const u64 k = (u64)top_k;
-            k_bucket = find_bucket(s, before, [&](int b) { return (u64)s.tot_cnt[b]; },
-                                   [&](u64 sum, int) { return sum >= k; });
-            if (k_bucket < kBuckets && s.tot_cnt[k_bucket] <= (unsigned int)kList) {
-                collect(k_bucket);
-                listed = true;
+            histogram(false);
+            const int kb = find_bucket(s, before, [&](int b) { return (u64)s.tot_cnt[b]; }, [&](u64 sum, int) { return sum >= k; });
+            if (kb < kBuckets && before + s.tot_cnt[kb] <= (u64)kWhole) {
+                // a few values up to the k-th: both cuts among them
+                collect(0, kb);
                 if (rank == 0) {
                     const int m = (int)min(s.list_n, (unsigned int)kList);
-                    const u64 r = k - before;                  // the r-th largest of the list
-                    if (tid == 0) s.thr_k = 0u;
-                    __syncthreads();
-                    for (int i = tid; i < m; i += kThreads) {
-                        const unsigned int o = ordered(s.list[i]);
-                        u64 above = 0ull, same = 0ull;
-                        for (int j = 0; j < m; ++j) {
-                            const unsigned int oj = ordered(s.list[j]);
-                            above += oj > o;
-                            same += oj == o;
+                    unsigned int t = pick_kth(m, k);
+                    if (cut_p) {
+                        u64 tot = 0ull;
+                        for (int i = tid; i < m; i += kThreads) {
+                            s.list_mass[i] = ordered(s.list[i]) >= t ? mass_of(s.list[i]) : 0ull;
+                            tot += s.list_mass[i];
                         }
-                        if (above < r && r <= above + same) s.thr_k = o;    // (equal values write the same)
+                        tot = block_sum(tot, s);
+                        t = pick_mass(m, t, 0ull, (double)top_p * (double)tot);
                     }
-                    __syncthreads();
-                    const unsigned int t = s.thr_k;
-                    u64 kept = 0ull;
-                    if (cut_p)
-                        for (int i = tid; i < m; i += kThreads)
-                            if (ordered(s.list[i]) >= t) kept += mass_of(s.list[i]);
-                    kept = block_sum(kept, s);
-                    if (tid == 0)
-                        for (int o = 0; o < blocks; ++o) {
-                            *cluster.map_shared_rank(&s.thr_k, o) = t;
-                            *cluster.map_shared_rank(&s.kept, o) = kept;
-                        }
+                    if (tid == 0) share_out(&s.cut, t);
                 }
                 cluster.sync();
-                thr = s.thr_k;
-                k_mass = s.kept;
+                thr = s.cut;
+                done = true;
+            } else if (kb < kBuckets && s.tot_cnt[kb] <= (unsigned int)kList) {
+                collect(kb, kb);
+                listed = true;
+                if (rank == 0) {
+                    const unsigned int t = pick_kth((int)min(s.list_n, (unsigned int)kList), k - before);
+                    if (tid == 0) share_out(&s.cut, t);
+                }
+                cluster.sync();
+                thr = s.cut;
             } else {
                 unsigned int lo = 0u, hi = 0xffffffffu;        // count(>= lo) >= k always holds
                 while (lo < hi) {
                     const unsigned int mid = lo + (hi - lo) / 2u + ((hi - lo) & 1u);
-                    if (row_sum([&](float x) { return (u64)(ordered(x) >= mid); }) >= k) lo = mid;
+                    if (row_sum([&](float x) { return ordered(x) >= mid ? 1.f : 0.f; }) >= (double)k) lo = mid;
                     else hi = mid - 1u;
                 }
                 thr = lo;
-                if (cut_p && k_bucket < kBuckets)
-                    k_mass = row_sum([&](float x) { return bucket(x) == k_bucket && ordered(x) >= thr ? mass_of(x) : 0ull; });
             }
         }
-        if (cut_p) {
-            // mass of bucket b that is kept so far: all of it before the k-th value's bucket, none behind
-            auto kept_mass = [&](int b) { return b < k_bucket ? s.tot_mass[b] : b == k_bucket ? k_mass : 0ull; };
-            const u64 tot = block_sum(kept_mass(2 * tid) + kept_mass(2 * tid + 1), s);
-            const double most = (double)top_p * (double)tot;
-            // the smallest v with mass(x > v) <= top_p * tot; everything >= v is kept
-            u64 before;
-            const int b = find_bucket(s, before, kept_mass, [&](u64 sum, int) { return (double)sum > most; });
-            if (b == kBuckets) {
-                // nothing exceeds it: no mass at all (thr stays), or a negative top_p (the maximum alone)
-                if (most < 0.0) thr = ordered(mx);
-            } else if (s.tot_cnt[b] <= (unsigned int)kList) {
-                if (!(listed && b == k_bucket)) {
-                    if (rank == 0 && tid == 0) s.list_n = 0u;
-                    cluster.sync();
-                    collect(b);
+        if (!done) {
+            // the smallest v with mass(x > v) <= top_p * (mass kept so far); everything >= v is kept
+            const double tot = row_sum([&](float x) { return ordered(x) >= thr ? weight_of(x) : 0.f; });
+            const double most = (double)top_p * tot;
+            if (most < 0.0) {
+                thr = ordered(mx);                             // (a negative top_p: the maximum alone)
+            } else if (tot > 0.0) {
+                // Most of the mass lies near the maximum and most of the values do not: the histogram goes 10 down
+                // (e^-10 of the maximum's weight) first, all the way if the cut lies further.
+                const double most_mass = most * (double)mass_scale;
+                u64 before = 0ull;
+                int b = kBuckets;
+                for (int reach = 0; reach < 2 && b == kBuckets; ++reach) {
+                    span = reach == 0 ? 10.f : INFINITY;
+                    inv = reach == 0 ? (float)(kBuckets - 1) / span : mx > mn ? (float)(kBuckets - 1) / (mx - mn) : 0.f;
+                    histogram(true);
+                    b = find_bucket(s, before, [&](int i) { return s.tot_mass[i]; }, [&](u64 sum, int) { return (double)sum > most_mass; });
                 }
-                if (rank == 0) {
-                    const int m = (int)min(s.list_n, (unsigned int)kList);
-                    if (tid == 0) s.thr_p = ordered(mx);
-                    for (int i = tid; i < m; i += kThreads) s.list_mass[i] = mass_of(s.list[i]);
-                    __syncthreads();
-                    for (int i = tid; i < m; i += kThreads) {
-                        const unsigned int o = ordered(s.list[i]);
-                        if (o < thr) continue;
-                        u64 above = before;
-                        for (int j = 0; j < m; ++j)
-                            if (ordered(s.list[j]) > o) above += s.list_mass[j];
-                        if ((double)above <= most) atomicMin(&s.thr_p, o);
+                if (b < kBuckets && s.tot_cnt[b] <= (unsigned int)kList) {
+                    if (listed) {
+                        if (rank == 0 && tid == 0) s.list_n = 0u;
+                        cluster.sync();
                     }
-                    __syncthreads();
-                    if (tid == 0)
-                        for (int o = 0; o < blocks; ++o) *cluster.map_shared_rank(&s.thr_p, o) = s.thr_p;
+                    collect(b, b);
+                    if (rank == 0) {
+                        const int m = (int)min(s.list_n, (unsigned int)kList);
+                        for (int i = tid; i < m; i += kThreads) s.list_mass[i] = mass_of(s.list[i]);
+                        const unsigned int t = pick_mass(m, thr, before, most_mass);
+                        if (tid == 0) share_out(&s.cut_mass, t);
+                    }
+                    cluster.sync();
+                    thr = s.cut_mass;
+                } else {
+                    unsigned int lo = thr, hi = ordered(mx);
+                    while (lo < hi) {
+                        const unsigned int mid = lo + (hi - lo) / 2u;
+                        const double above = row_sum([&](float x) { return ordered(x) > mid ? weight_of(x) : 0.f; });
+                        if (above <= most) hi = mid; else lo = mid + 1u;
+                    }
+                    thr = lo;
                 }
-                cluster.sync();
-                thr = s.thr_p;
-            } else {
-                unsigned int lo = thr, hi = ordered(mx);
-                while (lo < hi) {
-                    const unsigned int mid = lo + (hi - lo) / 2u;
-                    const u64 above = row_sum([&](float x) { return ordered(x) > mid ? mass_of(x) : 0ull; });
-                    if ((double)above <= most) hi = mid; else lo = mid + 1u;
-                }
-                thr = lo;
             }
         }
     }
 
     // ---- inverse CDF in index order: every warp owns a stretch of the slice, its kept mass meets the others'
-    const int stretch = (slice + kThreads - 1) / kThreads * 32;
+    constexpr int kPer = kMaxBlocks * kWarps / 32;
+    const int stretch = (slice + 4 * kThreads - 1) / (4 * kThreads) * 128;
     const int b0 = min(n, warp * stretch), b1 = min(n, b0 + stretch);
-    auto kept_of = [&](int i) -> u64 {
-        const float x = xs[i];
-        return ordered(x) >= thr ? mass_of(x) : 0ull;
+    auto kept_of = [&](float x) -> float { return ordered(x) >= thr ? weight_of(x) : 0.f; };
+    // the lane's four values from i on (zeros past the stretch)
+    auto four = [&](int i, float (&v)[4]) {
+        if (i + 3 < b1 && (reinterpret_cast<uintptr_t>(xs + i) & 15) == 0) {
+            const float4 x = *reinterpret_cast<const float4*>(xs + i);
+            v[0] = kept_of(x.x); v[1] = kept_of(x.y); v[2] = kept_of(x.z); v[3] = kept_of(x.w);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = i + e < b1 ? kept_of(xs[i + e]) : 0.f;
+        }
     };
-    u64 mine = 0ull;
-    for (int i = b0 + lane; i < b1; i += 32) mine += kept_of(i);
-    mine = warp_sum(mine);
-    if (lane == 0) s.seg[warp] = mine;
+    float mine = 0.f;
+    for (int i = b0 + 4 * lane; i < b1; i += 128) {
+        float v[4];
+        four(i, v);
+        mine += (v[0] + v[1]) + (v[2] + v[3]);
+    }
+    const double stretch_sum = warp_sum((double)mine);
+    if (lane == 0) s.seg[warp] = stretch_sum;
     cluster.sync();
     const int segs = blocks * kWarps;
     if (tid < segs) s.all_seg[tid] = *cluster.map_shared_rank(&s.seg[tid % kWarps], tid / kWarps);
     __syncthreads();
     // (every warp works the answer out for itself; the one whose stretch holds it writes it)
-    u64 part[kMaxBlocks * kWarps / 32], sum = 0ull;
+    double part[kPer], sum = 0.0;
 #pragma unroll
-    for (int j = 0; j < kMaxBlocks * kWarps / 32; ++j) {
-        const int at = lane * (kMaxBlocks * kWarps / 32) + j;
-        part[j] = at < segs ? s.all_seg[at] : 0ull;
+    for (int j = 0; j < kPer; ++j) {
+        part[j] = lane * kPer + j < segs ? s.all_seg[lane * kPer + j] : 0.0;
         sum += part[j];
     }
-    u64 run = sum;
+    double run = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const u64 up = __shfl_up_sync(0xffffffffu, run, o);
+        const double up = __shfl_up_sync(0xffffffffu, run, o);
         if (lane >= o) run += up;
     }
-    const u64 total = __shfl_sync(0xffffffffu, run, 31);
-    const double target = (double)u * (double)total;
+    const double target = (double)u * __shfl_sync(0xffffffffu, run, 31);
     // the first stretch with mass at whose end the sum reaches the target; if none does (a draw of
     // one or more), the last stretch with mass, and in it the last kept value (the reference's
     // fallback, sampling.cpp:113-116)
     int first = 0x7fffffff, last = -1;
-    u64 first_before = 0ull, at_end = run - sum;
+    double first_before = 0.0, at_end = run - sum;
 #pragma unroll
-    for (int j = 0; j < kMaxBlocks * kWarps / 32; ++j) {
-        const int at = lane * (kMaxBlocks * kWarps / 32) + j;
-        if (part[j]) {
-            last = at;
-            if (first == 0x7fffffff && (double)(at_end + part[j]) >= target) { first = at; first_before = at_end; }
+    for (int j = 0; j < kPer; ++j) {
+        if (part[j] > 0.0) {
+            last = lane * kPer + j;
+            if (first == 0x7fffffff && at_end + part[j] >= target) { first = last; first_before = at_end; }
         }
         at_end += part[j];
     }
-    const int pick = __reduce_min_sync(0xffffffffu, first), pick_last = __reduce_max_sync(0xffffffffu, last);
+    const int last_stretch = __reduce_max_sync(0xffffffffu, last);
+    const int found = __reduce_min_sync(0xffffffffu, first), pick = found == 0x7fffffff ? last_stretch : found;
     if (pick == rank * kWarps + warp) {
-        const int owner = pick / (kMaxBlocks * kWarps / 32);
-        u64 before = __shfl_sync(0xffffffffu, first_before, owner);
-        for (int i = b0; i < b1; i += 32) {
-            const u64 m = i + lane < b1 ? kept_of(i + lane) : 0ull;
-            u64 up = m;
+        double before = __shfl_sync(0xffffffffu, first_before, pick / kPer);
+        int token = -1, kept_last = -1;
+        for (int i = b0; i < b1 && token < 0; i += 128) {
+            float v[4];
+            four(i + 4 * lane, v);
+            const double own = ((double)v[0] + (double)v[1]) + ((double)v[2] + (double)v[3]);
+            double up = own;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const u64 t = __shfl_up_sync(0xffffffffu, up, o);
+                const double t = __shfl_up_sync(0xffffffffu, up, o);
                 if (lane >= o) up += t;
             }
-            const unsigned int hit = __ballot_sync(0xffffffffu, m && (double)(before + up) >= target);
-            if (hit) {
-                if (lane == 0) out[row] = i0 + i + __ffs(hit) - 1;
-                break;
+            double reach = before + up - own;                  // the sum in front of the lane's values
+            int at = 0x7fffffff, kept = -1;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                reach += (double)v[e];
+                if (v[e] > 0.f) {
+                    kept = i + 4 * lane + e;
+                    if (found != 0x7fffffff && at == 0x7fffffff && reach >= target) at = kept;
+                }
             }
+            kept_last = max(kept_last, __reduce_max_sync(0xffffffffu, kept));
+            at = __reduce_min_sync(0xffffffffu, at);
+            if (at != 0x7fffffff) token = at;
             before += __shfl_sync(0xffffffffu, up, 31);
         }
-    } else if (pick == 0x7fffffff && pick_last == rank * kWarps + warp) {
-        int best = -1;
-        for (int i = b0 + lane; i < b1; i += 32)
-            if (kept_of(i)) best = i;
-        best = __reduce_max_sync(0xffffffffu, best);
-        if (lane == 0) out[row] = i0 + best;
-    } else if (pick_last < 0 && rank == 0 && tid == 0) {
+        // (where rounding leaves the sum short of the target at the stretch's end: its last kept value)
+        if (lane == 0) out[row] = i0 + (token >= 0 ? token : kept_last);
+    } else if (last_stretch < 0 && rank == 0 && tid == 0) {
         out[row] = mi < vocab ? mi : 0;                       // no value has any mass
     }
     cluster.sync();                                           // (a peer may still read this block's sums)
