@@ -69,3 +69,36 @@ LSB_API long long lsbh_pack_step(int R, const int32_t* q_len, const int32_t* sta
     summary[3] = max_kv;
     return n;
 }
+
+// A request's sampling settings as SamplingParams.packed lays them out.
+struct SamplingRecord {
+    double temperature, top_p, penalty;
+    int64_t top_k;
+    uint64_t seed;
+};
+static_assert(sizeof(SamplingRecord) == 40, "no padding");
+
+// Per-row parameters of the sampling kernel: params[r] = {temperature, top_p, penalty, u}, top_k[r].  u is the request's
+// draw number draws[r]: one splitmix64 scramble of seed + (draw + 1) * golden, its top 24 bits centred in their cell
+// (0.5 for a greedy row).  Returns 1 if a row is not greedy, + 2 if one has a penalty; -(r + 1) if row r's top_k does
+// not fit 32 bits.
+LSB_API int lsbh_pack_sampling(int R, const void* records, const int64_t* draws, float* params, int32_t* top_k) {
+    const SamplingRecord* rec = static_cast<const SamplingRecord*>(records);
+    int flags = 0;
+    for (int r = 0; r < R; ++r) {
+        const SamplingRecord& p = rec[r];
+        if (p.top_k != (int32_t)p.top_k) return -(r + 1);
+        const bool greedy = p.temperature == 0.0;
+        flags |= (greedy ? 0 : 1) | (p.penalty != 1.0 ? 2 : 0);
+        uint64_t z = p.seed + ((uint64_t)draws[r] + 1u) * 0x9E3779B97F4A7C15ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        z ^= z >> 31;
+        params[4 * r] = (float)p.temperature;
+        params[4 * r + 1] = (float)p.top_p;
+        params[4 * r + 2] = (float)p.penalty;
+        params[4 * r + 3] = greedy ? 0.5f : (float)(((double)(z >> 40) + 0.5) / (double)(1 << 24));
+        top_k[r] = (int32_t)p.top_k;
+    }
+    return flags;
+}

@@ -7,7 +7,9 @@ here it keys the request's own stream of uniform draws.
 """
 from __future__ import annotations
 
+import struct
 from dataclasses import dataclass
+from functools import cached_property
 
 
 @dataclass(frozen=True)
@@ -31,6 +33,12 @@ class SamplingParams:
     @property
     def greedy(self) -> bool:
         return self.temperature == 0.0
+
+    @cached_property
+    def packed(self) -> bytes:
+        """The settings as the host library reads them (``csrc/host_step.cpp``), formed once."""
+        return struct.pack("<dddqQ", self.temperature, self.top_p, self.repetition_penalty, int(self.top_k),
+                           int(self.seed) & ((1 << 64) - 1))
 
 
 GREEDY = SamplingParams(temperature=0.0)

@@ -8,13 +8,34 @@ its penalty without effect; here the request's generated tokens are passed.
 """
 from __future__ import annotations
 
-from typing import List, Optional, Sequence
+from array import array
+from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
 
+from ..cache import native
 from .params import SamplingParams
-from .rng import uniform
+
+
+def _pack(params: Sequence[SamplingParams], draw_index: Sequence[int]) -> Tuple[np.ndarray, bool, bool]:
+    """(float32 [5 R]: the rows of (temperature, top_p, penalty, u), then the rows' top_k as int32 bits; whether all rows
+    are greedy; whether one has a repetition penalty).  ``rng.uniform`` states the draws."""
+    R = len(params)
+    if len(draw_index) != R:
+        raise ValueError("one draw index per SamplingParams")
+    host = np.empty(5 * R, dtype=np.float32)
+    draws = array("q", draw_index)
+    flags = native.lib().lsbh_pack_sampling(R, b"".join([p.packed for p in params]), draws.buffer_info()[0],
+                                            host.ctypes.data, host.ctypes.data + 16 * R)
+    if flags < 0:
+        raise OverflowError(f"top_k {params[-flags - 1].top_k} does not fit 32 bits")
+    return host, not flags & 1, bool(flags & 2)
+
+
+def _rows(buf: torch.Tensor, R: int) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(params [R, 4], top_k [R]) in a device copy of such an array."""
+    return buf[:4 * R].view(R, 4), buf[4 * R:].view(torch.int32)
 
 
 class StagedSampling:
@@ -22,8 +43,9 @@ class StagedSampling:
     step to step (one set per number of rows), and the launch that uses them.  Calling it is the
     same work every time, so a decode step captured in a CUDA graph can hold it."""
 
-    def __init__(self, ops, params: torch.Tensor, top_k: torch.Tensor, out: torch.Tensor):
-        self.ops, self.params, self.top_k, self.out = ops, params, top_k, out
+    def __init__(self, ops, buf: torch.Tensor, out: torch.Tensor):
+        self.ops, self.buf, self.out = ops, buf, out
+        self.params, self.top_k = _rows(buf, out.shape[0])
         self.key = ("sample", out.shape[0])
 
     def __call__(self, logits: torch.Tensor) -> torch.Tensor:
@@ -45,31 +67,24 @@ class Sampler:
         of their batch size and return the launch that samples with them; None where a repetition
         penalty is in use (it needs the generated tokens, packed per step by :meth:`sample`)."""
         R = len(params)
-        if R == 0 or any(p.repetition_penalty != 1.0 for p in params):
+        if R == 0:
+            return None
+        host, greedy, penal = _pack(params, draw_index)
+        if penal:
             return None
         st = self._staged.get(R)
-        dev = self.rt.device
         if st is None:
-            st = self._staged[R] = StagedSampling(
-                self.rt.ops, torch.tensor([[0.0, 1.0, 1.0, 0.5]] * R, dtype=torch.float32, device=dev),
-                torch.zeros(R, dtype=torch.int32, device=dev), torch.empty(R, dtype=torch.int32, device=dev))
-            st.greedy = True
-        if all(p.greedy for p in params):
-            if not st.greedy:                        # back to the constant rows of an all-greedy batch
-                st.params.copy_(torch.tensor([[0.0, 1.0, 1.0, 0.5]] * R, dtype=torch.float32))
-                st.top_k.zero_()
-                st.greedy = True
+            dev = self.rt.device
+            st = self._staged[R] = StagedSampling(self.rt.ops, torch.from_numpy(host).to(dev),
+                                                  torch.empty(R, dtype=torch.int32, device=dev))
+            st.greedy = greedy
             return st
-        fl = np.empty((R, 4), dtype=np.float32)
-        tk = np.empty(R, dtype=np.int32)
-        for r, (p, n) in enumerate(zip(params, draw_index)):
-            fl[r] = (p.temperature, p.top_p, 1.0, 0.5 if p.greedy else uniform(p.seed, n))
-            tk[r] = p.top_k
-        # (pageable host arrays: the copies have left them when these calls return; on the device
-        # they run in stream order, after the sampling of the step before)
-        st.params.copy_(torch.from_numpy(fl), non_blocking=True)
-        st.top_k.copy_(torch.from_numpy(tk), non_blocking=True)
-        st.greedy = False
+        if greedy and st.greedy:                         # nothing has changed since the last all-greedy step
+            return st
+        # (a pageable host array: the copy has left it when this call returns; on the device it runs in stream
+        # order, after the sampling of the step before)
+        st.buf.copy_(torch.from_numpy(host), non_blocking=True)
+        st.greedy = greedy
         return st
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams],
@@ -82,26 +97,17 @@ class Sampler:
         if len(params) != R or len(draw_index) != R:
             raise ValueError("one SamplingParams and one draw index per row of logits")
         dev = self.rt.device
-        if all(p.greedy and p.repetition_penalty == 1.0 for p in params):
+        host, greedy, penal = _pack(params, draw_index)
+        if greedy and not penal:
             # nothing varies from step to step: keep the per-row arrays on the device
             cached = self._greedy.get(R)
             if cached is None:
-                fl = torch.tensor([[0.0, 1.0, 1.0, 0.5]] * R, dtype=torch.float32, device=dev)
-                cached = self._greedy[R] = (fl, torch.zeros(R, dtype=torch.int32, device=dev),
-                                            torch.empty(R, dtype=torch.int32, device=dev))
+                cached = self._greedy[R] = _rows(torch.from_numpy(host).to(dev), R) \
+                    + (torch.empty(R, dtype=torch.int32, device=dev),)
             d_fl, d_tk, out = cached
             self.rt.ops.sample(logits, d_fl, d_tk, None, None, out)
             return out
-        fl = np.empty((R, 4), dtype=np.float32)
-        tk = np.empty(R, dtype=np.int32)
-        penal = False
-        for r, (p, n) in enumerate(zip(params, draw_index)):
-            fl[r] = (p.temperature, p.top_p, p.repetition_penalty,
-                     0.5 if p.greedy else uniform(p.seed, n))
-            tk[r] = p.top_k
-            penal |= p.repetition_penalty != 1.0
-        d_fl = torch.from_numpy(fl).to(dev, non_blocking=True)
-        d_tk = torch.from_numpy(tk).to(dev, non_blocking=True)
+        d_fl, d_tk = _rows(torch.from_numpy(host).to(dev, non_blocking=True), R)
         d_start = d_prev = None
         if penal and previous is not None:
             start = np.zeros(R + 1, dtype=np.int32)
