@@ -225,7 +225,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_qk = make_idesc(kKeys, 0);
             bool ok = mbar_wait(q_full, 0, &abort_flag);
             // S has two buffers: S of tile t + 2 is issued as soon as the softmax warps hold S of
@@ -266,7 +266,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
         // ---------------------------------------------------------------- MMA issuer for O += P V
         // A thread of its own: issuing one of these small MMAs takes the better part of a hundred
         // cycles, and behind the S products of the other issuer every tile would wait for both.
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_pv = make_idesc(HD, 1);
             const uint64_t db_v0 = desc_mnmajor(sV, kKeys * 128);
             bool ok = true;

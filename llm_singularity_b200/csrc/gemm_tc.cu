@@ -123,6 +123,15 @@ __device__ __forceinline__ float4 ld_peer_f4(const void* own_smem, uint32_t rank
     return v;
 }
 
+// One lane of a converged warp, chosen so that the compiler knows it is one: operands of tcgen05.mma live in uniform
+// registers, and a product issued by "lane 0" of a branch costs its thread more than the tensor core needs for a narrow
+// one (256 rows times 3,072 x 2,048: 14.5 us that way, 11.4 us; the head for 64 rows: 98 and 93 us).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 // Shared-memory matrix descriptor of a K-major tile written by TMA with the 128-byte swizzle:
 // rows of 128 bytes, groups of 8 rows 1024 bytes apart (stride byte offset), tile base aligned to
 // 1024 bytes.  Fields: start address >> 4 [0,14), leading byte offset >> 4 [16,30) (unused for
@@ -531,7 +540,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(BN);
             bool ok = true;
             for (int kb = 0; kb < nkb && ok; ++kb) {
@@ -794,7 +803,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(BN);
             int s = 0;
             uint32_t parity = 0;
