@@ -183,6 +183,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
             if (!__shfl_sync(0xffffffffu, free, 0)) return false;
             if (lane == 0) mbar_expect_tx(&full[s], (L::kShareS ? 1 : 2) * L::kKVBytes);
             __syncwarp();
+            // (each lane issues its page's copies: one elected lane for all of them was 10 % slower)
             if (lane < pages_per_tile) {
                 // pages past the last needed one repeat it: their keys are masked, their bytes finite
                 int pi = (((t0 + t) * kKeys) >> prm.page_shift) + lane;
@@ -225,7 +226,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (elect_one()) {
+        if (lsb_elect_one()) {
             constexpr uint32_t idesc_qk = make_idesc(kKeys, 0);
             bool ok = mbar_wait(q_full, 0, &abort_flag);
             // S has two buffers: S of tile t + 2 is issued as soon as the softmax warps hold S of
@@ -266,7 +267,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __
         // ---------------------------------------------------------------- MMA issuer for O += P V
         // A thread of its own: issuing one of these small MMAs takes the better part of a hundred
         // cycles, and behind the S products of the other issuer every tile would wait for both.
-        if (elect_one()) {
+        if (lsb_elect_one()) {
             constexpr uint32_t idesc_pv = make_idesc(HD, 1);
             const uint64_t db_v0 = desc_mnmajor(sV, kKeys * 128);
             bool ok = true;

@@ -161,15 +161,6 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     return r;
 }
 
-// One lane of a converged warp, chosen so that the compiler knows it is one: operands of tcgen05.mma live in uniform
-// registers, and a product issued by "lane 0" of a branch costs its thread more than the tensor core needs for a narrow
-// one (256 rows times 3,072 x 2,048: 14.5 us that way, 11.4 us; the head for 64 rows: 98 and 93 us).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
-
 // K-major operand tile, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
 __device__ __forceinline__ uint64_t desc_kmajor(const void* tile) {
     uint64_t d = (uint64_t)((smem_addr(tile) >> 4) & 0x3FFFu);

@@ -47,6 +47,16 @@ __device__ __forceinline__ float lsb_warp_max(float v) {
     return v;
 }
 
+// One lane of a converged warp, always the same one, chosen so that the compiler knows it is one: operands of
+// tcgen05.mma and of tensor copies live in uniform registers, and what "lane 0" of a branch issues costs its thread more
+// than the tensor core needs for a narrow product (256 rows times 3,072 x 2,048: 14.5 us that way, 11.4 us; the head
+// for 64 rows: 98 and 93 us).
+__device__ __forceinline__ bool lsb_elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 // Sum over a thread block (every thread gets the result). `scratch` holds 33 floats.
 __device__ __forceinline__ float lsb_block_sum(float v, float* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -123,15 +123,6 @@ __device__ __forceinline__ float4 ld_peer_f4(const void* own_smem, uint32_t rank
     return v;
 }
 
-// One lane of a converged warp, chosen so that the compiler knows it is one: operands of tcgen05.mma live in uniform
-// registers, and a product issued by "lane 0" of a branch costs its thread more than the tensor core needs for a narrow
-// one (256 rows times 3,072 x 2,048: 14.5 us that way, 11.4 us; the head for 64 rows: 98 and 93 us).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
-
 // Shared-memory matrix descriptor of a K-major tile written by TMA with the 128-byte swizzle:
 // rows of 128 bytes, groups of 8 rows 1024 bytes apart (stride byte offset), tile base aligned to
 // 1024 bytes.  Fields: start address >> 4 [0,14), leading byte offset >> 4 [16,30) (unused for
@@ -540,7 +531,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (elect_one()) {
+        if (lsb_elect_one()) {
             constexpr uint32_t idesc = make_idesc(BN);
             bool ok = true;
             for (int kb = 0; kb < nkb && ok; ++kb) {
@@ -738,7 +729,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
     auto row_of = [&](int t) { return groups ? t / tiles_n : t % tiles_m; };
     auto col_of = [&](int t) { return groups ? t % tiles_n : t / tiles_m; };
     int pre = 0;
-    if (threadIdx.x == 0) {
+    const bool producer = warp == 0 && lsb_elect_one();
+    if (producer) {
         abort_flag = 0;
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 128); }
@@ -762,10 +754,13 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (threadIdx.x != 0) lsb_pdl_wait();      // thread 0 (the TMA producer) waits after its first weight boxes
+    if (!producer) lsb_pdl_wait();             // (the TMA producer waits after its first weight boxes)
 
     if (warp == 0) {
-        if (lane == 0) {
+        // (elected like the issuer of the products: 2,048 rows times 3,072 x 2,048 23.6 -> 19.8 us.  The kernel for a tile
+        // a block, above, was no faster for it: its copies are few and asked for ahead.)
+        __syncwarp();
+        if (lsb_elect_one()) {
             lsb_pdl_wait();
             int issued = 0;                                    // K blocks issued so far, over all tiles (as far as it matters)
             int s = 0;
@@ -803,7 +798,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
             }
         }
     } else if (warp == 1) {
-        if (elect_one()) {
+        if (lsb_elect_one()) {
             const uint32_t idesc = make_idesc(BN);
             int s = 0;
             uint32_t parity = 0;
