@@ -693,11 +693,7 @@ __device__ __forceinline__ void drain_staged(const GemmParams& prm, unsigned cha
     int h = 0;
 #pragma unroll 1
     for (; h + PASS <= prm.bn; h += PASS) epilogue_staged<PASS, GATED>(prm, epi, tmem_acc + h, q, lane, i0, j0 + h);
-    if (GATED && (prm.bn & 64)) {
-        epilogue_staged<64, GATED>(prm, epi + q * 2048, tmem_acc + h, q, lane, i0, j0 + h);
-        h += 64;
-    }
-    if (prm.bn & 32) epilogue_staged<32, GATED>(prm, epi + q * (GATED ? 3072 : 2048), tmem_acc + h, q, lane, i0, j0 + h);
+    if (GATED && (prm.bn & 64)) epilogue_staged<64, GATED>(prm, epi + q * 2048, tmem_acc + h, q, lane, i0, j0 + h);
 }
 
 __global__ void __launch_bounds__(kGemmThreads)
@@ -877,6 +873,214 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
     }
 }
 
+// ------------------------------------------------------------------ pairs of blocks (long prompts)
+// The same walk with two blocks on one tile of 256 rows x bn columns (tcgen05 cta_group::2): each block brings its own
+// 128 rows of P and half of the tile's rows of Q, the tensor cores of both SMs read both halves, and each block's tensor
+// memory holds its own 128 rows of the result.  A step of 64 along K so brings a block 32 KB instead of 48 from L2, and
+// one lane issues the products of both: 2,048 x 16,384 x 2,048 gated takes 89.3 us instead of 94.6 (1,539 TFLOP/s, where
+// the power limit holds the clock).  A stage is full when both blocks' copies have landed (all four count on the first
+// block's barrier); it and the accumulators are handed back to both by commits that arrive in both.
+__device__ __forceinline__ uint32_t rank0_addr(const void* own_smem) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(own_smem)), "r"(0));
+    return a;
+}
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(smem_addr(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrives on the barrier at this offset in both blocks once all products issued so far have finished
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_addr(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// (a wait for what the other block does)
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    for (uint32_t it = 0; it < kSpinLimit; ++it) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((it & 255u) == 255u) {
+            if (*abort_flag) return false;
+            __nanosleep(128);
+        }
+    }
+    *abort_flag = 1;
+    lsb_set_status(LSB_WAIT_TIMEOUT);
+    return false;
+}
+
+static constexpr int pair_stage_bytes(int bn) { return (kBM + bn / 2) * kBK * 2; }
+static constexpr size_t pair_smem(int bn, int stages) {
+    return 1024 + (size_t)stages * pair_stage_bytes(bn) + kEpiBytes + (2 * kMaxStages + 4) * 8 + 16;
+}
+
+__global__ void __launch_bounds__(kGemmThreads)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
+                    const GemmParams prm, int tiles_m, int tiles_n) {
+    const int BN = prm.bn, STAGES = prm.stages;
+    const uint32_t kPBytes = kBM * kBK * 2, kStageBytes = kPBytes + (uint32_t)(BN / 2) * (kBK * 2);
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);   // (the same offset in both blocks)
+    unsigned char* stages = base;
+    unsigned char* epi = base + (size_t)STAGES * kStageBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(epi + kEpiBytes);
+    uint64_t* empty = full + kMaxStages;
+    uint64_t* acc_full = empty + kMaxStages;                  // [2]
+    uint64_t* acc_empty = acc_full + 2;                       // [2], the first block's counts
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    __shared__ int abort_flag;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_rank(), pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int n_tiles = tiles_m * tiles_n;
+    const int nkb = prm.num_kb;
+    auto row_of = [&](int t) { return t % tiles_m; };
+    auto col_of = [&](int t) { return t / tiles_m; };
+
+    lsb_pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_barrier();                                        // both blocks' barriers and tensor memory are there
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lsb_elect_one()) {
+            // the weights (half a tile's columns) of the first ring before the wait on the kernel before, the rest after it
+            int pre = 0;
+            for (int t = pair; t < n_tiles && pre < STAGES; t += pairs)
+                for (int kb = 0; kb < nkb && pre < STAGES; ++kb, ++pre) {
+                    if (rank == 0) mbar_expect_tx(&full[pre], 2 * kStageBytes);
+                    tma_load_2d_pair(stages + (size_t)pre * kStageBytes + kPBytes, &map_q, rank0_addr(&full[pre]), kb * kBK,
+                                     col_of(t) * BN + rank * (BN / 2));
+                }
+            lsb_pdl_wait();
+            int s = 0;
+            uint32_t round = 0;
+            bool ok = true;
+            for (int t = pair; t < n_tiles && ok; t += pairs) {
+                const int i0 = row_of(t) * (2 * kBM) + rank * kBM, j0 = col_of(t) * BN + rank * (BN / 2);
+                for (int kb = 0; kb < nkb; ++kb) {
+                    unsigned char* st = stages + (size_t)s * kStageBytes;
+                    const uint32_t bar = rank0_addr(&full[s]);
+                    if (round == 0 && s < pre) {
+                        tma_load_2d_pair(st, &map_p, bar, kb * kBK, i0);
+                    } else {
+                        if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, &abort_flag)) { ok = false; break; }
+                        if (rank == 0) mbar_expect_tx(&full[s], 2 * kStageBytes);
+                        tma_load_2d_pair(st, &map_p, bar, kb * kBK, i0);
+                        tma_load_2d_pair(st + kPBytes, &map_q, bar, kb * kBK, j0);
+                    }
+                    if (++s == STAGES) { s = 0; ++round; }
+                }
+            }
+            // Every copy has landed before a block leaves: each stage's products, which waited for its copies, hand
+            // it back once more to both blocks.
+            const long long total = (long long)((n_tiles - pair + pairs - 1) / pairs) * nkb;
+            for (long long k = total > STAGES ? total - STAGES : 0; k < total; ++k) {
+                int dummy = 0;
+                mbar_wait(&empty[k % STAGES], (uint32_t)(k / STAGES) & 1, &dummy);
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0 && lsb_elect_one()) {
+            // M = 256: twice the rows of make_idesc's field
+            const uint32_t idesc = make_idesc(BN) + ((uint32_t)(kBM >> 4) << 24);
+            int s = 0;
+            uint32_t parity = 0;
+            int local = 0;
+            bool ok = true;
+            for (int t = pair; t < n_tiles && ok; t += pairs, ++local) {
+                const int a = local & 1;
+                ok = mbar_wait_cluster(&acc_empty[a], (uint32_t)((local >> 1) & 1) ^ 1u, &abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t tmem_d = tmem_base + (uint32_t)a * 256u;
+                for (int kb = 0; kb < nkb; ++kb) {
+                    ok = mbar_wait_cluster(&full[s], parity, &abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    unsigned char* st = stages + (size_t)s * kStageBytes;
+                    const uint64_t dp = make_smem_desc(st), dq = make_smem_desc(st + kPBytes);
+#pragma unroll
+                    for (int k = 0; k < kBK / kUmmaK; ++k)
+                        umma_bf16_pair(tmem_d, dp + 2 * k, dq + 2 * k, idesc, (kb | k) ? 1u : 0u);
+                    umma_commit_pair(&empty[s]);
+                    if (++s == STAGES) { s = 0; parity ^= 1u; }
+                }
+                umma_commit_pair(&acc_full[a]);
+            }
+        }
+    } else {
+        lsb_pdl_wait();                                        // (the output may still be read by the kernel before)
+        const int q = warp & 3;
+        const int il = q * 32 + lane;
+        const int n_out = prm.swiglu == 1 ? prm.rows_q / 2 : prm.rows_q;
+        const bool staged = (((uintptr_t)prm.out) & 15) == 0;
+        const bool aligned = staged && !prm.out_f32 && (n_out % 8) == 0;
+        const bool aligned32 = staged && prm.out_f32 && !prm.swiglu && (n_out % 4) == 0;
+        int local = 0;
+        for (int t = pair; t < n_tiles; t += pairs, ++local) {
+            const int a = local & 1;
+            const int i0 = row_of(t) * (2 * kBM) + rank * kBM, j0 = col_of(t) * BN;
+            const bool ok = mbar_wait(&acc_full[a], (uint32_t)(local >> 1) & 1, &abort_flag);
+            tc_fence_after();
+            if (!ok || abort_flag) break;
+            const uint32_t tmem_acc = tmem_base + (uint32_t)a * 256u;
+            if (i0 >= prm.rows_p) {
+                // (the second block's rows lie past the matrix)
+            } else if (aligned && j0 + BN <= prm.rows_q) {
+                if (prm.swiglu == 1) drain_staged<true>(prm, epi, tmem_acc, q, lane, i0, j0);
+                else drain_staged<false>(prm, epi, tmem_acc, q, lane, i0, j0);
+            } else if (aligned32 && j0 + BN <= prm.rows_q) {
+#pragma unroll 1
+                for (int h = 0; h < BN; h += 32)
+                    epilogue_staged_f32<32>(prm, epi, tmem_acc + h, q, lane, i0, j0 + h);
+            } else {
+#pragma unroll 1
+                for (int c0 = 0; c0 < BN; c0 += 32) {
+                    uint32_t r[32];
+                    load_acc<32>(tmem_acc + c0, q, 0, true, r);
+                    store_chunk<256>(prm, r, i0 + il, j0 + c0, 32, lane);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(rank0_addr(&acc_empty[a]));    // four warps of each block
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_barrier();                                        // no block leaves, or frees tensor memory, beside a peer at work
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
+    }
+}
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -945,6 +1149,42 @@ static int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, GemmP
                       mp, mq, prm, tiles_m, tiles_n);
 }
 
+static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, GemmParams prm, int bn, int tiles_m, int tiles_n,
+                       cudaStream_t stream) {
+    static int configured = -1;
+    static int sms = 0;
+    if (configured < 0) {
+        configured = (int)cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistentSmem);
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    if (configured) return configured;
+    prm.bn = bn;
+    prm.stages = kMaxStages;
+    while (pair_smem(bn, prm.stages) > kPersistentSmem) --prm.stages;
+    const int tiles = tiles_m * tiles_n;
+    const int pairs = tiles < sms / 2 ? tiles : sms / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = pair_smem(bn, prm.stages);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (lsb_pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = 2;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel, mp, mq, prm, tiles_m, tiles_n);
+}
+
 // What happens when a wait runs out, shown without a fault: one block, a barrier that nothing
 // arrives at.  Thread 0 waits on it with a limit of `limit` polls, gives up, raises the block's
 // abort flag and records LSB_WAIT_TIMEOUT in the status word; thread 32 waits with the kernels'
@@ -991,6 +1231,27 @@ LSB_API int lsb_gemm_tc_supported(const void* x, const void* w, int M, int N, in
 // splits.  With more than one split the blocks of a tile form a thread-block cluster and sum their
 // partial tiles through distributed shared memory, so there is no scratch in global memory; the
 // portable cluster size limits the splits to 8.
+// The width of a prompt product's tiles, and whether pairs of blocks walk them.  What a 64-deep step of a tile costs is
+// about its (128 + bn) rows of operands; a pair of blocks reads half of w per block, which makes a step 1/16 shorter,
+// against a start and an end across two blocks of some four steps, and an odd number of 128-row tiles is padded to an
+// even one.  The cheapest of six is within 1 % of the best measured (30 shapes, 256 to 8,192 rows) but for one
+// at 3 %.  One block / pairs, us: 2,011 x 28,672 x 4,096 gated 323 / 306; 2,011 x 4,096 x 14,336 177 / 166;
+// 8,192 x 16,384 x 2,048 gated 361 / 342; 2,048 x 2,048 x 2,048 15.6 / 16.7; 543 (five tiles of rows) x 16,384 x 3,072
+// gated 49.3 / 52.4.  Columns 256 / 192 / 128: 700 x 4,096 x 4,096 (96, 132 and 192 tiles) 27.3 / 22.4 / 30.0;
+// 1,024 x 2,048 x 8,192 44.0 / 37.4 / 31.6; 2,048 x 3,072 x 2,048 26.5 / 21.6 / 25.2.  Widths between gained
+// nothing on these: a step does not get shorter in proportion.
+static void prompt_tiles(int M, int N, int num_kb, int sms, int* bn, bool* pair) {
+    const long long tm = (M + kBM - 1) / kBM;
+    long long least = 0x7fffffffffffffffLL;
+    for (int c = 256; c >= 128; c -= 64) {
+        const long long tn = (N + c - 1) / c;
+        const long long one = (tm * tn + sms - 1) / sms * num_kb * (kBM + c) * 16;
+        const long long two = ((tm + 1) / 2 * tn + sms / 2 - 1) / (sms / 2) * num_kb * (kBM + c) * 15 + 4 * (kBM + 256) * 16;
+        if (one < least) { least = one; *bn = c; *pair = false; }
+        if (two < least) { least = two; *bn = c; *pair = true; }
+    }
+}
+
 LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn, int* splits) {
     const int num_kb = (K + kBK - 1) / kBK;
     const int sms = num_sms();
@@ -1013,41 +1274,23 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
         *splits = s;
     } else {
         *swap = 0;
-        // Persistent blocks walk the tile list.  What a tile costs is its stream of operands, (128 + bn) rows of
-        // K (128 x 256 x 64 takes the tensor core 512 cycles and its 48 KB about as long from L2), so where 256 columns
-        // take several rounds over the SMs, the width is the one whose rounds bring the fewest rows.  2,048 tokens times
-        // 3,072 x 2,048: 192 tiles of 256 columns are two rounds, one of them a third full (26.0 us); 256 of 192 are two
-        // rounds of five sixths the length (24.8 us).  543 times 16,384 x 3,072: 67.5 -> 63.2 us.  Within one round
-        // narrower tiles only bring more of x, and take SMs that the next kernel could begin on (543 times
-        // 5,120 x 3,072: 26.3 us with 256 columns, 28.3 with 192), unless half the SMs would stay idle.
-        const int mt = (M + kBM - 1) / kBM;
-        const long long wide = (long long)mt * ((N + 255) / 256);
-        int best = 64;
-        if (N >= kPersistentMin && wide <= sms) {
-            best = wide <= sms / 2 ? 128 : 256;
-        } else if (N >= kPersistentMin) {
-            long long least = 0x7fffffffffffffffLL;
-            for (int c = 256; c >= 128; c -= 32) {
-                const long long t = (long long)mt * ((N + c - 1) / c);
-                long long rows = (t + sms - 1) / sms * (kBM + c);
-                if (c == 256) rows = rows * 15 / 16;          // (a narrower one has to be worth its traffic)
-                if (rows < least) { least = rows; best = c; }
-            }
-        } else if (N > 64) {
-            best = 128;
-        }
-        *bn = best;
+        bool pair;
+        if (N >= kPersistentMin) prompt_tiles(M, N, num_kb, sms, bn, &pair);
+        else *bn = N > 64 ? 128 : 64;
         *splits = 1;
         // A few hundred tokens make too few 128 x 256 tiles for the SMs.  Where the walk through K
         // is long (the down projection), K is split over a cluster, as many ways as fit in one
         // wave; summing the partial tiles costs about as much as 2048 of K, so shorter walks stay
-        // whole.  (The gated epilogue needs whole sums: gated products stay unsplit too.)
-        const int tiles = mt * ((N + 255) / 256);
+        // whole, and so do those with room for two or three parts only, which narrower tiles serve better
+        // (four parts, 256 x 2,048 x 8,192: 21.8 us, with 128 columns whole 28.8; three, 300 x 4,096 x 14,336: 73.6 and
+        // 52.2; two, 543 x 3,072 x 8,192: 37.5 and 31.8).  (The gated epilogue needs whole sums: gated products stay
+        // unsplit too.)
+        const int tiles = (M + kBM - 1) / kBM * ((N + 255) / 256);
         if (N >= 256 && tiles < most && !swiglu) {
             int s = sms / tiles;
             if (s > 8) s = 8;
             if (s > num_kb / 32) s = num_kb / 32;
-            if (s > 1) {
+            if (s >= 4) {
                 const int per = (num_kb + s - 1) / s;
                 *splits = (num_kb + per - 1) / per;
             }
@@ -1118,6 +1361,12 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
     if (!swap && !(out_f32 && swiglu) && bn >= 128) {
         // prompts: persistent blocks, double-buffered accumulator
         const int tm = (M + kBM - 1) / kBM, tn = (N + bn - 1) / bn;
+        bool pair = false;
+        if (N >= kPersistentMin) prompt_tiles(M, N, prm.num_kb, sms, &bn, &pair);
+        if (pair) {
+            if ((rc = make_map(&mq, w, N, K, bn / 2))) return rc;
+            return launch_pair(mp, mq, prm, bn, (tm + 1) / 2, tn, stream);
+        }
         return launch_persistent(mp, mq, prm, bn, tm, tn, stream);
     }
     if (splits > 1) {

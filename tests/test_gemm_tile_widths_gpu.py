@@ -29,3 +29,26 @@ def test_widths(M, N, K, gated, out_dtype):
     for _ in range(5):
         assert torch.equal(ops.linear(x, w, out_dtype=out_dtype, gated=gated), y)
     ops.check_status()
+
+
+@pytest.mark.parametrize("M, N, K", [(4200, 8192, 2112), (2900, 4100, 2112), (1290, 8192, 4104), (385, 28672, 2112), (200, 16384, 4104), (2048, 3072, 4104),
+                                     (3000, 2222, 4104), (1400, 4098, 4104), (1000, 2048, 8200), (1000, 1900, 8200)])
+@pytest.mark.parametrize("gated, out_dtype", [(False, torch.bfloat16), (False, torch.float32), (True, torch.bfloat16)])
+def test_pairs_of_blocks(M, N, K, gated, out_dtype):
+    """Long products, whose tiles pairs of blocks share: odd numbers of row tiles, and last tiles and K blocks cut short."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, w = (torch.randn(n, K, device="cuda", generator=g).to(torch.bfloat16) for n in (M, N))
+    y = ops.linear(x, w, out_dtype=out_dtype, gated=gated)
+    want = x.double() @ w.double().T
+    tol = 2.0 ** -25 * K * K ** 0.5            # each 16 products a cut to 2^-23 of sums that stay below 4 sqrt(K)
+    if gated:
+        gate, up = want[:, 0::2], want[:, 1::2]
+        want = gate * torch.sigmoid(gate) * up
+        tol = tol * (1.1 * up.abs() + gate.abs() + tol) + 2.0 ** -23 * (8 + 1.2 * gate.abs()) * want.abs()
+    if out_dtype == torch.bfloat16:
+        tol = tol + 2.0 ** -8 * want.abs()
+    assert y.shape == want.shape and bool(((y.double() - want).abs() <= tol).all())
+    for _ in range(5):
+        assert torch.equal(ops.linear(x, w, out_dtype=out_dtype, gated=gated), y)
+    ops.check_status()
