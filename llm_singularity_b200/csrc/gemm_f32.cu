@@ -1,8 +1,8 @@
-// out[M, N] = x[M, K] * w[N, K]^T in true 32-bit: every product a 32-bit multiply-add, no reduced-precision
-// matrix mode.  Two kernels, by the number of rows; K a multiple of 4 and 16-byte aligned bases (anything else is
-// csrc/gemm.cu's).  An activation of a gated product (w's rows alternate gate_i, up_i, out is [M, N / 2]) is
-// applied where the sums meet.  The reference hands such products to cublasSgemm
-// (kernels/src/cublas_provider.cpp:36-51) and launches silu(g) * u by itself (kernels/src/activations.cu:11-21).
+// out[M, N] = x[M, K] * w[N, K]^T of 32-bit values with 32-bit sums, no bit of an operand dropped.  Three kernels, by the
+// number of rows and K; K a multiple of 4 and 16-byte aligned bases (anything else is csrc/gemm.cu's).  An activation of
+// a gated product (w's rows alternate gate_i, up_i, out is [M, N / 2]) is applied where the sums meet.  The reference
+// hands such products to cublasSgemm (kernels/src/cublas_provider.cpp:36-51) and launches silu(g) * u by itself
+// (kernels/src/activations.cu:11-21).
 //
 // * Up to 16 rows (a decode step) the product is weight traffic.  Weight rows are dealt out over one
 //   block per SM, sixteen at most at a time: four to a warp, each row's K in two parts.  A warp copies the weights it
@@ -13,16 +13,31 @@
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
 //   four times the exchanges at the end of a group: 89 us.)
 //
-// * More rows (a prompt): arithmetic on the 32-bit pipes.  Eight warps of 64 x 64 outputs (8 x 16 a thread), arranged as a tile of 128 x 256, 128 x 128, 64 x 128 or 64 x 64;
-//   in the smaller tiles the warps that are left share out each slice of K and their sums meet at the end, so that
-//   a few hundred rows against 2,048 columns still give every SM eight busy warps.  Slices come by asynchronous copies,
-//   three to five in flight.  The same four products at 500 rows (61 GFLOP): 1,502 us, 41 TFLOP/s of the 70 that a
-//   loop of nothing but multiply-adds reaches here; 64 x 64 tiles of 4 x 4 a thread: 2,104 us.  (Slices fetched through
-//   registers, however arranged, exposed their latency: 2,400 us.)
+// * More rows (a prompt), K from 512: the tensor cores.  A 32-bit value is exactly the sum of three bfloat16 values (8
+//   bits each of its 24), so a product is nine products of parts; the six that reach 2^-23 of it are taken, the other three
+//   are not.  Blocks of 128 x 128 outputs (x 64 where those fit the SMs at once) take x and w as they are by
+//   TMA; sixteen warps, two groups by turns, split a stage of 32 along K, x's parts into tensor memory, w's into
+//   shared memory.  The tensor core cuts its sums rather than rounding them, so the leading products stay there for
+//   128 of K only and are then added up in registers; the five small ones have their own sums, 2^-8 as large.
+//   Error against 64 bits, 500 x 2,048 x 2,048: 1.5e-7 of the norm, 4.1e-7 by multiply-adds; K = 512 1.3e-7 and 1.6e-7;
+//   K = 8,192 2.2e-7 and 8.1e-7 (at K of 100 and 256 the two are alike, which is where the line comes from).  The four
+//   products of a layer at 1B sizes, 500 rows (61 GFLOP): 1,491 -> 470 us.  What bounds it is the traffic of
+//   shared memory and the chain of a stage: 0.66 us where its products take 0.4 (both operands in shared
+//   memory: 0.9; one group of eight warps besides: 1.05).  Values that bfloat16 cannot split (infinities, NaN, a row
+//   that lies below 2^-95 as a whole) and sums that leave the range are done over by multiply-adds at the end, so
+//   that they come out as there.
+//
+// * More rows, smaller K: multiply-adds on the 32-bit pipes.  Eight warps of 64 x 64 outputs (8 x 16 a thread), arranged
+//   as a tile of 128 x 256, 128 x 128, 64 x 128 or 64 x 64; in the smaller tiles the warps that are left share out each
+//   slice of K and their sums meet at the end, so that few tiles still give an SM eight busy warps.  Slices come by
+//   asynchronous copies, three to five in flight.  500 x 16,384 x 2,048: 764 us, 44 TFLOP/s of the 70 that a loop of
+//   nothing but multiply-adds reaches here.
 //
 // A row's sum is taken in an order that K and the kernel fix, the same from run to run.
 #include "common.cuh"
 #include "gate_act.cuh"
+
+#include <cuda.h>
 
 LSB_DEFINE_STATUS()
 
@@ -188,6 +203,37 @@ struct TileParams {
     int M, N, K, act;
 };
 
+// outputs (m, n .. n + 3), as far as n goes, or what the gated product makes of them (N is even then)
+__device__ __forceinline__ void store_four(const TileParams& p, long long m, long long n, float4 v) {
+    const bool wide = (p.N & 3) == 0;
+    if (p.act) {
+        float* d = p.out + m * (p.N / 2) + n / 2;
+        const float first = lsb_gated(v.x, v.y, p.act, 0.f);
+        if (wide) *reinterpret_cast<float2*>(d) = make_float2(first, lsb_gated(v.z, v.w, p.act, 0.f));
+        else {
+            d[0] = first;
+            if (n + 2 < p.N) d[1] = lsb_gated(v.z, v.w, p.act, 0.f);
+        }
+        return;
+    }
+    float* d = p.out + m * p.N + n;
+    if (wide) *reinterpret_cast<float4*>(d) = v;
+    else {
+        d[0] = v.x;
+        if (n + 1 < p.N) d[1] = v.y;
+        if (n + 2 < p.N) d[2] = v.z;
+        if (n + 3 < p.N) d[3] = v.w;
+    }
+}
+__device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s); s = fmaf(a.w, b.w, s);
+    }
+    return s;
+}
+
 constexpr int kTileThreads = 256;
 
 // WM x WN warps of 64 x 64 outputs, WK of them on the same outputs with a part of each slice of BK; ST slices in flight
@@ -279,7 +325,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_f32_kernel(const Ti
 #pragma unroll
         for (int j = 0; j < 16; ++j) tile[8 * i * LDT + 4 * j] = acc[i][j];
     __syncthreads();
-    const bool wide = (p.N & 3) == 0;
     for (int q = tid; q < BM * BN / 4; q += kTileThreads) {
         const int row = q / (BN / 4), col = q % (BN / 4) * 4;
         float4 v = *reinterpret_cast<const float4*>(smem + row * LDT + col);
@@ -290,24 +335,315 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_f32_kernel(const Ti
         }
         const long long m = m0 + row, n = n0 + col;
         if (m >= p.M || n >= p.N) continue;
-        if (p.act) {                                                   // (N is even)
-            float* d = p.out + m * (p.N / 2) + n / 2;
-            const float first = lsb_gated(v.x, v.y, p.act, 0.f);
-            if (wide) *reinterpret_cast<float2*>(d) = make_float2(first, lsb_gated(v.z, v.w, p.act, 0.f));
-            else {
-                d[0] = first;
-                if (n + 2 < p.N) d[1] = lsb_gated(v.z, v.w, p.act, 0.f);
+        store_four(p, m, n, v);
+    }
+}
+
+// ------------------------------------------------------------------ many rows, on the tensor cores
+constexpr int kSplitK = 512;                   // K from which on the split sums are the more exact ones
+constexpr int kSM = 128;                       // rows of x of a tile (tensor memory lanes)
+constexpr int kSK = 32;                        // K of a stage: 128 bytes of a 32-bit row, 64 of a plane's
+constexpr int kSPlanes = 3;
+constexpr int kSGroup = 256;                   // eight warps: a row of x or w each thread of a stage
+constexpr int kSWorkers = 2 * kSGroup;         // ... and as many for the stage after it
+constexpr int kSThreads = kSWorkers + 64;      // ... one warp for the copies, one for the products
+constexpr int kSChunk = 4;                     // stages (K = 128) whose leading products meet in tensor memory
+constexpr uint32_t kSpinLimit = 1u << 22;
+
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// false if the limit ran out or another role gave up
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    for (uint32_t it = 0; it < kSpinLimit; ++it) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((it & 255u) == 255u) {
+            if (*abort_flag) return false;
+            __nanosleep(128);
+        }
+    }
+    *abort_flag = 1;
+    lsb_set_status(LSB_WAIT_TIMEOUT);
+    return false;
+}
+__device__ __forceinline__ void tma_rows(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int k, int row) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(smem_u32(bar)), "r"(k), "r"(row) : "memory");
+}
+// (the operand of x lies in tensor memory too)
+__device__ __forceinline__ void umma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// sums += N columns of tensor memory, one row a lane
+template <int N>
+__device__ __forceinline__ void tmem_add(uint32_t addr, float (&sums)[N]) {
+    static_assert(N == 16 || N == 32, "one load");
+    uint32_t r[N];
+    if constexpr (N == 32)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                     "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                     "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                       "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                       "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                       "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                     : "r"(addr));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                     "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                       "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                     : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < N; ++i) sums[i] += __uint_as_float(r[i]);
+}
+// eight columns of tensor memory, one row a lane
+__device__ __forceinline__ void tmem_put(uint32_t addr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+// A plane of w: rows of 64 bytes with the 64-byte swizzle (16-byte piece j of row r at j ^ (r / 2 & 3)), groups of
+// eight rows 512 bytes apart; layout type 4.
+__device__ __forceinline__ uint64_t plane_desc(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
+// Two values as sums of three bfloat16 values: what a rounding leaves is exact, and the third is all that 24 bits leave.
+__device__ __forceinline__ void split3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
+    a -= __uint_as_float(h << 16);
+    b -= __uint_as_float(h & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m) : "f"(b), "f"(a));
+    a -= __uint_as_float(m << 16);
+    b -= __uint_as_float(m & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(b), "f"(a));
+}
+
+template <int BN>
+struct SplitLayout {
+    static constexpr int kRows = kSM + BN;
+    static constexpr int kRaw = kRows * kSK * 4, kPlane = BN * kSK * 2, kSplit = kSPlanes * kPlane;
+    static constexpr int kRing = BN == 128 ? 5 : 6;
+    // columns of tensor memory: two chunks' leading sums, the small products', and x's planes of two stages
+    static constexpr int kSmall = 2 * BN, kX = 3 * BN, kXPlane = kSK / 2, kXSplit = kSPlanes * kXPlane;
+    static_assert(kX + 2 * kXSplit <= 512, "tensor memory");
+    static constexpr int LDT = BN + 4;
+    static constexpr size_t kTotal = 1024 + (size_t)kRing * kRaw + 2 * kSplit;
+    static_assert(kSM * LDT * 4 <= kRing * kRaw, "the sums leave through the ring");
+};
+
+template <int BN>
+__global__ void __launch_bounds__(kSThreads, 1)
+gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const TileParams p) {
+    using L = SplitLayout<BN>;
+    constexpr int R = L::kRing;
+    extern __shared__ unsigned char raw_smem[];
+    unsigned char* ring = (unsigned char*)(((uintptr_t)raw_smem + 1023) & ~(uintptr_t)1023);
+    unsigned char* planes = ring + (size_t)R * L::kRaw;
+    __shared__ uint64_t raw_full[R], raw_empty[R], split_full[2], split_empty[2], acc_full[2], acc_empty[2], done;
+    __shared__ uint32_t tmem_slot, seen[L::kRows];
+    __shared__ int abort_flag;
+    lsb_pdl_launch_dependents();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = (int)blockIdx.y * kSM, n0 = (int)blockIdx.x * BN;
+    const int steps = (p.K + kSK - 1) / kSK;
+    if (tid < L::kRows) seen[tid] = 0;
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < R; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kSGroup / 32); }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&split_full[s], kSGroup / 32);
+            mbar_init(&split_empty[s], 1);
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], kSWorkers / 32);
+        }
+        mbar_init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    constexpr uint32_t kColumns = 512;                                  // (one block an SM)
+    if (warp == kSWorkers / 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kColumns));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == kSWorkers / 32) {
+        if (lsb_elect_one()) {
+            const uint32_t base = smem_u32(ring);
+            lsb_pdl_wait();
+            int it = 0;
+            for (; it < steps; ++it) {
+                const int s = it % R;
+                if (it >= R && !mbar_wait(&raw_empty[s], (uint32_t)(it / R - 1) & 1, &abort_flag)) break;
+                mbar_expect(&raw_full[s], L::kRaw);
+                tma_rows(base + s * L::kRaw, &map_x, &raw_full[s], it * kSK, m0);
+                tma_rows(base + s * L::kRaw + kSM * kSK * 4, &map_w, &raw_full[s], it * kSK, n0);
             }
-            continue;
+            for (int k = it > R ? it - R : 0; k < it; ++k) {            // (no copy is in flight when the block leaves)
+                int ignore = 0;
+                mbar_wait(&raw_full[k % R], (uint32_t)(k / R) & 1, &ignore);
+            }
         }
-        float* d = p.out + m * p.N + n;
-        if (wide) *reinterpret_cast<float4*>(d) = v;
-        else {
-            d[0] = v.x;
-            if (n + 1 < p.N) d[1] = v.y;
-            if (n + 2 < p.N) d[2] = v.z;
-            if (n + 3 < p.N) d[3] = v.w;
+    } else if (warp == kSWorkers / 32 + 1) {
+        if (lsb_elect_one()) {
+            // D 32-bit, A and B bfloat16, both K-major
+            constexpr uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(BN >> 3) << 17 | (uint32_t)(kSM >> 4) << 24;
+            const uint32_t small = tmem + L::kSmall;
+            for (int it = 0; it < steps; ++it) {
+                const int s = it & 1, c = it / kSChunk;
+                if (it % kSChunk == 0 && c >= 2 && !mbar_wait(&acc_empty[c & 1], (uint32_t)(c / 2 - 1) & 1, &abort_flag)) break;
+                if (!mbar_wait(&split_full[s], (uint32_t)(it >> 1) & 1, &abort_flag)) break;
+                tmem_fence_after();
+                const uint32_t at = smem_u32(planes) + s * L::kSplit;
+                const uint32_t lead = tmem + (c & 1) * BN;
+#pragma unroll
+                for (int k = 0; k < kSK / 16; ++k) {                    // 32 bytes along K: +2 in 16-byte units
+                    uint32_t a[3];
+                    uint64_t b[3];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        a[i] = tmem + L::kX + s * L::kXSplit + i * L::kXPlane + 8 * k;
+                        b[i] = plane_desc(at + i * L::kPlane) + 2 * k;
+                    }
+                    umma(small, a[0], b[2], idesc, it || k);
+                    umma(small, a[2], b[0], idesc, true);
+                    umma(small, a[1], b[1], idesc, true);
+                    umma(small, a[0], b[1], idesc, true);
+                    umma(small, a[1], b[0], idesc, true);
+                    umma(lead, a[0], b[0], idesc, it % kSChunk || k);
+                }
+                umma_commit(&split_empty[s]);
+                if (it % kSChunk == kSChunk - 1 || it == steps - 1) umma_commit(&acc_full[c & 1]);
+            }
+            umma_commit(&done);
+            int ignore = 0;
+            mbar_wait(&done, 0, &ignore);
         }
+    } else {
+        lsb_pdl_wait();                                                 // (the output may still be read by the kernel before)
+        constexpr int kMine = BN / 4;                                   // columns of a warp, of 32 rows
+        float sums[kMine];
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) sums[i] = 0.f;
+        const int q = warp & 3, part = warp >> 2;
+        const uint32_t mine = tmem + ((uint32_t)(q * 32) << 16) + part * kMine;
+        bool ok = true;
+        int taken = 0;
+        auto take = [&]() {
+            const int c = taken++;
+            ok = mbar_wait(&acc_full[c & 1], (uint32_t)(c >> 1) & 1, &abort_flag);
+            if (!ok) return;
+            tmem_fence_after();
+            tmem_add(mine + (c & 1) * BN, sums);
+            tmem_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[c & 1]);
+        };
+        const int group = warp / (kSGroup / 32), r = tid % kSGroup;     // stages it % 2 == group
+        const bool has_row = r < L::kRows;
+        uint32_t bits = 0;
+        for (int it = group; it < steps && ok; it += 2) {
+            const int s = it % R;
+            if (!mbar_wait(&raw_full[s], (uint32_t)(it / R) & 1, &abort_flag)) { ok = false; break; }
+            if (it >= 2 && !mbar_wait(&split_empty[group], (uint32_t)(it / 2 - 1) & 1, &abort_flag)) { ok = false; break; }
+            tmem_fence_after();
+            if (has_row) {
+                const unsigned char* from = ring + (size_t)s * L::kRaw + r * (kSK * 4);
+                unsigned char* to = planes + (size_t)group * L::kSplit + (r - kSM) * (kSK * 2);
+                const uint32_t to_x = tmem + ((uint32_t)(q * 32) << 16) + L::kX + group * L::kXSplit;
+#pragma unroll
+                for (int j = 0; j < kSK / 16; ++j) {                    // sixteen values
+                    uint32_t h[8], m[8], l[8];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 a = *reinterpret_cast<const float4*>(from + (((4 * j + i) ^ (r & 7)) << 4));
+                        bits |= __float_as_uint(a.x) | __float_as_uint(a.y);
+                        bits |= __float_as_uint(a.z) | __float_as_uint(a.w);
+                        split3(a.x, a.y, h[2 * i], m[2 * i], l[2 * i]);
+                        split3(a.z, a.w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1]);
+                    }
+                    if (r < kSM) {                                      // (whole warps)
+                        tmem_put(to_x + 8 * j, h);
+                        tmem_put(to_x + L::kXPlane + 8 * j, m);
+                        tmem_put(to_x + 2 * L::kXPlane + 8 * j, l);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            unsigned char* put = to + (((2 * j + i) ^ ((r >> 1) & 3)) << 4);
+                            *reinterpret_cast<uint4*>(put) = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+                            *reinterpret_cast<uint4*>(put + L::kPlane) = make_uint4(m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]);
+                            *reinterpret_cast<uint4*>(put + 2 * L::kPlane) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
+                        }
+                    }
+                }
+                if (r < kSM) {
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tmem_fence_before();
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(&split_full[group]); mbar_arrive(&raw_empty[s]); }
+            // (the chunk before this one: its products have ended by now, and those of the next need its place)
+            if (it % kSChunk >= kSChunk - 2 && it >= kSChunk) take();
+        }
+        const int chunks = (steps + kSChunk - 1) / kSChunk;
+        while (taken < chunks && ok) take();
+        if (ok) {
+            tmem_add(mine + L::kSmall, sums);
+            // every product has been issued and waited for, so that the ring is free
+            float* row = reinterpret_cast<float*>(ring) + (q * 32 + lane) * L::LDT + part * kMine;
+#pragma unroll
+            for (int j = 0; j < kMine; j += 4)
+                *reinterpret_cast<float4*>(row + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
+        }
+        if (has_row) atomicOr(&seen[r], bits);
+        tmem_fence_before();
+        asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
+        if (!abort_flag) {
+            const float* tile = reinterpret_cast<const float*>(ring);
+            // A row with nothing from 2^-95 up (but not all zeros) has values whose third part bfloat16 cannot hold.
+            auto faint = [&](int r) { return (seen[r] & 0x70000000u) == 0 && (seen[r] & 0x7fffffffu) != 0; };
+            for (int e = tid; e < kSM * BN / 4; e += kSWorkers) {
+                const int row = e / (BN / 4), col = e % (BN / 4) * 4;
+                if (m0 + row >= p.M || n0 + col >= p.N) continue;
+                __align__(16) float v[4];
+                *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(tile + row * L::LDT + col);
+                const bool row_faint = faint(row);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (!(fabsf(v[i]) <= 3.402823466e38f) || row_faint || faint(kSM + col + i))
+                        if (n0 + col + i < p.N) v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
+                store_four(p, m0 + row, n0 + col, *reinterpret_cast<float4*>(v));
+            }
+        }
+    }
+    __syncwarp();
+    __syncthreads();
+    if (warp == kSWorkers / 32) {
+        tmem_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kColumns));
     }
 }
 
@@ -354,6 +690,45 @@ static int launch_tile(const TileParams& p, cudaStream_t stream) {
     return lsb_launch(gemm_tile_f32_kernel<WM, WN, WK, BK, ST>, grid, dim3(kTileThreads), L::kTotal, stream, 1, p);
 }
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                  CUtensorMapFloatOOBfill);
+
+// [rows, K] 32-bit, boxes of [box_rows x 32], 128-byte swizzle, zeros outside
+static int map_rows(CUtensorMap* map, const float* ptr, int rows, int K, int box_rows) {
+    static EncodeTiledFn encode = nullptr;
+    if (!encode) {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            return (int)cudaErrorNotSupported;
+        encode = (EncodeTiledFn)f;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)K * 4};
+    const cuuint32_t box[2] = {(cuuint32_t)kSK, (cuuint32_t)box_rows}, unit[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), dims, strides, box, unit,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+template <int BN>
+static int launch_split(const TileParams& p, cudaStream_t stream) {
+    using L = SplitLayout<BN>;
+    static int configured = -1;
+    if (configured < 0)
+        configured = (int)cudaFuncSetAttribute(gemm_split_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
+    if (configured) return configured;
+    const dim3 grid((p.N + BN - 1) / BN, (p.M + kSM - 1) / kSM);
+    if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+    CUtensorMap mx, mw;
+    int rc;
+    if ((rc = map_rows(&mx, p.x, p.M, p.K, kSM))) return rc;
+    if ((rc = map_rows(&mw, p.w, p.N, p.K, BN))) return rc;
+    return lsb_launch(gemm_split_f32_kernel<BN>, grid, dim3(kSThreads), L::kTotal, stream, 1, mx, mw, p);
+}
+
 LSB_API int lsb_gemm_f32_supported(const void* x, const void* w, int M, int N, int K) {
     return M > 0 && N > 0 && K > 0 && K % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0 && M <= 32 * 65535;
 }
@@ -374,6 +749,12 @@ LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int 
     // multiply-add and pays its end more often, so it has to win by a few per cent.
     const TileParams p{x, w, out, M, N, K, act};
     const long long sms = num_sms();
+    if (K >= kSplitK) {
+        // 64 columns a block take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so only where one round
+        // does (500 x 3,072 x 2,048: 87.4 and 54.9)
+        if ((long long)((M + kSM - 1) / kSM) * ((N + 63) / 64) <= sms) return launch_split<64>(p, stream);
+        return launch_split<128>(p, stream);
+    }
     const int bm[4] = {128, 128, 64, 64}, bn[4] = {256, 128, 128, 64};
     const double cost[4] = {1.0, 1.0, 1.03, 1.08};
     int best = 0;

@@ -43,3 +43,36 @@ def test_more_rows(M, N, K):
 @pytest.mark.parametrize("M, N, K", [(1, 2, 4), (3, 302, 64), (8, 16384, 256), (16, 4742, 132), (17, 66, 36), (70, 640, 128), (300, 3002, 132)])
 def test_gated(M, N, K, activation):
     _check(M, N, K, activation)
+
+
+@pytest.mark.parametrize("M, N, K", [(17, 64, 4100), (129, 66, 4096), (130, 2050, 516), (300, 3002, 540), (257, 9000, 512), (500, 2048, 2052), (1000, 130, 8192), (200, 20002, 544)])
+@pytest.mark.parametrize("activation", [None, "silu", "gelu_tanh"])
+def test_split_products(M, N, K, activation):
+    """K from 512: whole, short and barely filled tiles, last stages cut short, odd numbers of chunks."""
+    _check(M, N, K, activation)
+
+
+@pytest.mark.parametrize("N", [700, 20000])
+def test_split_products_out_of_range(N):
+    """Values that the parts cannot hold: infinities, NaN, rows near and below the smallest normal number, the largest numbers."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x, w = (torch.randn(n, 520, device="cuda", generator=g) for n in (200, N))
+    x[3, 5], x[10, 7], w[9, 1], w[11, 2] = float("inf"), float("nan"), -float("inf"), 0.0
+    x[20] *= 1e-38
+    x[21] *= 1e-42
+    x[22] = 0.0
+    x[40] *= 1e-30
+    x[41, ::2] *= 1e-37
+    w[7] *= 2.0 ** -100
+    w[8] *= 1e-39
+    w[12] *= 1e10                                                    # (with x's 1e-38: 24 bits of it)
+    x[31], w[33] = 1e25, -1e25           # sums of one sign beyond the range (of both signs 32-bit sums make NaN, 64-bit ones don't)
+    y = ops.linear(x, w)
+    want = x.double() @ w.double().T
+    assert torch.equal(y.isnan(), want.isnan())
+    bound = 2.0 ** -24 * (x.abs().double() @ w.abs().double().T) * (2 + 520 ** 0.5) + 520 * 2.0 ** -149    # (and subnormal sums' own steps)
+    sure = want.abs() + bound < 3.4028234e38
+    assert bool(((y.double() - want).abs() <= bound)[sure].all()) and bool(sure.float().mean() > 0.95)
+    beyond = (want.abs() - bound > 3.4028236e38) & ~want.isnan()
+    assert torch.equal(y[beyond].double(), want[beyond].sign() * float("inf"))
