@@ -17,7 +17,9 @@
 // queries, keys and values; so nothing of the recurrence is rounded to bfloat16's 8 digits.
 //
 // kActed reads the projection itself (bfloat16) and applies silu in 32-bit while a tile is laid down, once in the first
-// kernel and once in the third: no pass of its own over memory.
+// kernel and once in the third: no pass of its own over memory.  A prompt of 1,500 tokens with
+// fades fixed by head (16 heads of 128 x 128): 83 us (output 50, gain 28, chain 5) where the walk took 528 in three; what bounds the two large ones is
+// the shared memory that mma.sync's operands pass through.
 // Sums of logarithms are formed in 64-bit and kept as pairs of floats: the difference of two of them is good
 // to 32-bit however far the memory has faded.  Different chunks and heads are different blocks; the sums
 // form in another order than in the walk: equal beyond rounding.

@@ -1,6 +1,6 @@
 // C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores, 32-bit accumulation, no reduced-precision
-// matrix mode: the product of the true 32-bit path, and of any shape the tensor-core
-// kernel does not take.  A and W are row-major with K contiguous, the layout checkpoints
+// matrix mode: the 32-bit products that csrc/gemm_f32.cu does not take (K not a multiple of 4,
+// unaligned bases), and the bfloat16 ones that the tensor-core kernel does not.  A and W are row-major with K contiguous, the layout checkpoints
 // store ([out, in]) and the reference hands to cublasSgemm
 // (kernels/src/cublas_provider.cpp:36-51).  Inputs 32-bit or bfloat16; output 32-bit or
 // the input type.  64x64 output tile per block, 16-deep slices of K staged through shared

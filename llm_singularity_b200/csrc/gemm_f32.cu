@@ -634,7 +634,8 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     if (!(fabsf(v[i]) <= 3.402823466e38f) || row_faint || faint(kSM + col + i))
-                        if (n0 + col + i < p.N) v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
+                        if (n0 + col + i < p.N)
+                            v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
                 store_four(p, m0 + row, n0 + col, *reinterpret_cast<float4*>(v));
             }
         }

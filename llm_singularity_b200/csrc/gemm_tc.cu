@@ -1279,18 +1279,19 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
         else *bn = N > 64 ? 128 : 64;
         *splits = 1;
         // A few hundred tokens make too few 128 x 256 tiles for the SMs.  Where the walk through K
-        // is long (the down projection), K is split over a cluster, as many ways as fit in one
-        // wave; summing the partial tiles costs about as much as 2048 of K, so shorter walks stay
-        // whole, and so do those with room for two or three parts only, which narrower tiles serve better
-        // (four parts, 256 x 2,048 x 8,192: 21.8 us, with 128 columns whole 28.8; three, 300 x 4,096 x 14,336: 73.6 and
-        // 52.2; two, 543 x 3,072 x 8,192: 37.5 and 31.8).  (The gated epilogue needs whole sums: gated products stay
+        // is long (the down projection), K is split over a cluster, as many ways as are sure to fit at once: clusters
+        // don't straddle the chip's groups of SMs, and 128 blocks in fours do, 144 in threes or fours don't (300 x 3,072 x 8,192 in
+        // four: 41 us, as long as two rounds).  Summing the partial tiles costs about as much as 2048 of K, so
+        // shorter walks stay whole, and so do those with room for two parts only, which narrower tiles serve better (four
+        // parts, 256 x 2,048 x 8,192: 21.8 us, with 128 columns whole 28.8; three, 543 x 2,048 x 8,192: 26.4 and 29.0;
+        // two, 543 x 3,072 x 8,192: 37.5 and 31.8).  (The gated epilogue needs whole sums: gated products stay
         // unsplit too.)
         const int tiles = (M + kBM - 1) / kBM * ((N + 255) / 256);
         if (N >= 256 && tiles < most && !swiglu) {
-            int s = sms / tiles;
+            int s = sms * 7 / 8 / tiles;
             if (s > 8) s = 8;
             if (s > num_kb / 32) s = num_kb / 32;
-            if (s >= 4) {
+            if (s >= 3) {
                 const int per = (num_kb + s - 1) / s;
                 *splits = (num_kb + per - 1) / per;
             }

@@ -420,7 +420,8 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
     ``into = (residual, norm_weight, eps)``: the product is added to ``residual`` ([M, N] 32-bit, in
     place) and what comes back is a ``NormOut``: what follows the RMS norm with that weight.
 
-    float32 operands run on the CUDA cores in true 32-bit.  bfloat16 operands run on the
+    float32 operands lose no bit and have 32-bit sums: on the CUDA cores, or with many rows and K from 512 on the
+    tensor cores as exact splits into bfloat16 parts (``csrc/gemm_f32.cu``).  bfloat16 operands run on the
     tensor cores (tcgen05, accumulators in TMEM) when K is a multiple of 8, else on the CUDA
     cores as well.
 
