@@ -6,8 +6,8 @@
 //
 // * Up to 16 rows (a decode step) the product is weight traffic.  Weight rows are dealt out over one
 //   block per SM, sixteen at most at a time: four to a warp, each row's K in two parts.  A warp copies the weights it
-//   needs into a ring of shared memory itself (asynchronously, some 140 KB in flight an SM, the first of them before
-//   the wait on the kernel before) and shares the rows of x with the three others of its part.  The sums of a
+//   needs into a ring of shared memory itself (asynchronously, some 140 KB in flight an SM, the first of them asked for
+//   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three others of its part.  The sums of a
 //   group meet once, over lanes by halving exchanges and over the two parts in shared memory, in a fixed order.
 //   The four products of a layer at 1B sizes, 8 rows (243 MB): 71 us (3.4 TB/s); as 64 x 64 tiles, 56 of their 64 rows
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
@@ -102,6 +102,14 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
             }
         }
     };
+    auto warm_w = [&](int it) {                // (a lane's 16 bytes are an eighth of a line)
+        const int g = (int)blockIdx.x + (it / chunks) * (int)gridDim.x, k0 = it % chunks * kKS + at;
+        const int n0 = g * p.per, rows = min(p.per, p.N - n0);
+        if (lane & 7) return;
+        for (int r = rg * kRW; r < min(rows, rg * kRW + kRW); ++r)
+            for (int k = k0; k < min(p.K, k0 + kKS); k += 256)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (size_t)(n0 + r) * p.K + k));
+    };
     auto copy_x = [&](int it) {
         const int k0 = it % chunks * kKS + at;
         const uint32_t st = base + ((uint32_t)(it % ST) * (kRB + MT) + kRB) * kKS * 4u;
@@ -114,10 +122,12 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
                 copy16(st + (uint32_t)(m * kKS + 256 * j) * 4u, have ? x + (size_t)m * p.K + k : p.x, have);
             }
     };
-    for (int it = 0; it < ST - 1 && it < total; ++it) copy_w(it);
+    // w may be what the kernel before has yet to write: ahead of the wait its first lines are only asked for (L2, where
+    // writes go too), and read behind it
+    for (int it = 0; it < ST - 1 && it < total; ++it) warm_w(it);
     lsb_pdl_wait();
     for (int it = 0; it < ST - 1; ++it) {
-        if (it < total) copy_x(it);
+        if (it < total) { copy_w(it); copy_x(it); }
         copies_commit();
     }
     float acc[V];

@@ -76,3 +76,20 @@ def test_split_products_out_of_range(N):
     assert bool(((y.double() - want).abs() <= bound)[sure].all()) and bool(sure.float().mean() > 0.95)
     beyond = (want.abs() - bound > 3.4028236e38) & ~want.isnan()
     assert torch.equal(y[beyond].double(), want[beyond].sign() * float("inf"))
+
+
+@pytest.mark.parametrize("M, N, K", [(1, 64, 64), (8, 2048, 512), (16, 300, 2048), (100, 128, 512)])
+def test_weights_that_the_kernel_in_front_makes(M, N, K):
+    """A product's weights may be another product's result: not read before that kernel has ended."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, a, b = (torch.randn(n, k, device="cuda", generator=g) for n, k in ((M, K), (N, 256), (K, 256)))
+    w = ops.linear(a, b)
+    want = x.double() @ w.double().T
+    bound = 2.0 ** -24 * (x.abs().double() @ w.abs().double().T) * (2 + K ** 0.5)
+    for _ in range(20):
+        made = ops.linear(a, b)
+        y = ops.linear(x, made)
+        assert torch.equal(made, w) and bool(((y.double() - want).abs() <= bound).all())
+        made.zero_()                             # (its memory goes to the next turn's weights)
+        del made
