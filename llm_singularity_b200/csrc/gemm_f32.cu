@@ -520,6 +520,7 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             // D 32-bit, A and B bfloat16, both K-major
             constexpr uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(BN >> 3) << 17 | (uint32_t)(kSM >> 4) << 24;
             const uint32_t small = tmem + L::kSmall;
+            lsb_pdl_wait();                                             // (a wait's limit is for this kernel's own copies)
             for (int it = 0; it < steps; ++it) {
                 const int s = it & 1, c = it / kSChunk;
                 if (it % kSChunk == 0 && c >= 2 && !mbar_wait(&acc_empty[c & 1], (uint32_t)(c / 2 - 1) & 1, &abort_flag)) break;

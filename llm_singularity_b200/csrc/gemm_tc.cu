@@ -1007,6 +1007,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         }
     } else if (warp == 1) {
         if (rank == 0 && lsb_elect_one()) {
+            lsb_pdl_wait();                                   // (a wait's limit is for this kernel's own copies)
             // M = 256: twice the rows of make_idesc's field
             const uint32_t idesc = make_idesc(BN) + ((uint32_t)(kBM >> 4) << 24);
             int s = 0;

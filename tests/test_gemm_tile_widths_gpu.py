@@ -52,3 +52,18 @@ def test_pairs_of_blocks(M, N, K, gated, out_dtype):
     for _ in range(5):
         assert torch.equal(ops.linear(x, w, out_dtype=out_dtype, gated=gated), y)
     ops.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_behind_a_long_kernel(dtype):
+    """A product that is launched beside a long kernel: its waits' limits do not count that kernel's time."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    # one block, some 25,000 slices one behind the other
+    a, b = (torch.randn(64, 400001, device="cuda", generator=g) for _ in range(2))
+    x, w = (torch.randn(n, 2112, device="cuda", generator=g).to(dtype) for n in (700, 4096))
+    want = ops.linear(x, w)
+    for _ in range(3):
+        ops.linear(a, b)
+        assert torch.equal(ops.linear(x, w), want)
+    ops.check_status()
