@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const Att
             l += f * *cluster.map_shared_rank(ml + 4 * h + 1, s);
             o += f * *cluster.map_shared_rank(os + i, s);
         }
-        out[i] = lsb_from_float<T>(l > 0.f ? o * (1.f / l) : 0.f);
+        out[i] = lsb_from_float<T>(o * (l > 0.f ? 1.f / l : 0.f));       // (a sum that is not a number stays none)
     }
     cluster.sync();                                            // (a peer may still read this block's sums)
 }

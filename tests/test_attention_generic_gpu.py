@@ -64,3 +64,55 @@ def test_edges(dtype, nh, nkv, hd, window, softcap, bias, captured):
 
 def test_many_requests_leave_the_keys_whole():
     _run(torch.float32, 4, 4, 32, [1] * 60 + [3] * 4, [5 + 37 * i % 300 for i in range(64)], 0, 0.0, False, False)
+
+
+def _poisoned(what, dtype, nh, nkv, hd, q_lens, kv_lens, window, spots):
+    """Attention over a cache in which request r's key or value at each of spots[r] holds numbers that are none, and what
+    64-bit sums over each row's own keys alone make of it."""
+    from llm_singularity_b200 import kernels as ops
+    from llm_singularity_b200.engine.batch import ContextBuilder
+    from llm_singularity_b200.parts.base import KVCacheView
+    g = torch.Generator(device="cuda").manual_seed(sum(kv_lens) + hd)
+    R, T, group = len(q_lens), sum(q_lens), nh // nkv
+    ctx, _ = ContextBuilder("cuda", 4096, 64).build([[0] * n for n in q_lens], [k - q for k, q in zip(kv_lens, q_lens)],
+                                                    list(range(R)), [[] for _ in range(R)])
+    per = -(-max(kv_lens) // PAGE)
+    table = torch.arange(R * per, dtype=torch.int32).view(R, per).cuda()
+    kp, vp = (torch.randn(R * per, nkv, PAGE, hd, device="cuda", generator=g).to(dtype) for _ in range(2))
+    bad = [float("nan"), float("inf"), -float("inf")]
+    for r, at in enumerate(spots):
+        for i, key in enumerate(at):
+            (kp if what == "keys" else vp)[r * per + key // PAGE, i % nkv, key % PAGE, (5 * i) % hd] = bad[i % 3]
+    qkv = torch.randn(T, (nh + 2 * nkv) * hd, device="cuda", generator=g).to(dtype)
+    out, scale = torch.zeros(T, nh * hd, dtype=dtype, device="cuda"), 1.0 / math.sqrt(hd)
+    ops.paged_attention(qkv, nh, nkv, hd, ctx, KVCacheView(kp, vp, table, PAGE, window or None, 0), scale, window, out)
+    ops.check_status()
+    t, same = 0, 0
+    for r in range(R):
+        n, L = q_lens[r], kv_lens[r]
+        K, V = (p[r * per:(r + 1) * per].transpose(1, 2).reshape(-1, nkv, hd).double().repeat_interleave(group, 1) for p in (kp, vp))
+        for i in range(n):
+            pos = L - n + i
+            seen = slice(max(0, pos - window + 1) if window else 0, pos + 1)
+            s = torch.einsum("hd,jhd->hj", qkv[t + i, :nh * hd].double().view(nh, hd), K[seen]) * scale
+            w = torch.softmax(s, -1)
+            want = torch.einsum("hj,jhd->hd", w, V[seen]).reshape(-1)
+            y = out[t + i].double()
+            assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf()), (r, i)
+            fine = want.isfinite()
+            same += int(fine.sum())
+            size = 6.0 * (1 + s[s.isfinite()].abs().max().item())
+            tol = size * 2.0 ** -20 + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
+            assert bool(((y - want).abs() <= tol)[fine].all()) and torch.equal(y[want.isinf()], want[want.isinf()]), (r, i)
+        t += n
+    assert same > 0 and same < out.numel()
+
+
+SIZES = [(torch.float32, 8, 2, 64), (torch.float32, 4, 4, 128), (torch.float32, 6, 2, 256), (torch.bfloat16, 6, 1, 80)]
+
+
+@pytest.mark.parametrize("what", ["keys", "values"])
+@pytest.mark.parametrize("dtype, nh, nkv, hd", SIZES)
+def test_single_tokens_that_see_no_number(what, dtype, nh, nkv, hd):
+    _poisoned(what, dtype, nh, nkv, hd, [1, 1, 1, 1], [1, 40, 700, 300], 0, [[], [3], [0, 500, 699], []])
+    _poisoned(what, dtype, nh, nkv, hd, [1, 1], [300, 300], 50, [[100, 249], [250]])
