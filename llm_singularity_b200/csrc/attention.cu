@@ -113,16 +113,21 @@ struct Tile {
             }
         }
     }
-    __device__ __forceinline__ void park(const AttnParams& p, float* ks, float* vs, int ldk, int tid) const {
+    // (returns whether every value of this thread's is a number and finite)
+    __device__ __forceinline__ bool park(const AttnParams& p, float* ks, float* vs, int ldk, int tid) const {
         const int per = p.hd >> 2;
+        float zero = 0.f;                                      // times a number 0, times anything else NaN
 #pragma unroll
         for (int j = 0; j < kPieces; ++j) {
             const int idx = j * kThreads + tid, row = idx / per, d = (idx - row * per) * 4;
             if (row < KT) {
                 *reinterpret_cast<float4*>(ks + row * ldk + d) = widen(k[j]);
-                *reinterpret_cast<float4*>(vs + row * p.hd + d) = widen(v[j]);
+                const float4 w = widen(v[j]);
+                *reinterpret_cast<float4*>(vs + row * p.hd + d) = w;
+                zero = fmaf(w.x, zero, fmaf(w.y, zero, fmaf(w.z, zero, w.w * zero)));
             }
         }
+        return zero == 0.f;
     }
 };
 
@@ -344,10 +349,10 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
     Tile<T, KT, HDC> tile;
     tile.fetch(p, off[0], tid);
     for (int base = lo, turn = 0; base <= pos_last; base += KT, turn ^= 1) {
-        tile.park(p, ks, vs, ldk, tid);
+        const bool finite = tile.park(p, ks, vs, ldk, tid);
         const int next = base + KT;
         if (tid < KT) off[turn ^ 1][tid] = next + tid <= pos_last ? key_offset(p, table, g, next + tid) : -1;
-        __syncthreads();
+        const bool by_row = __syncthreads_or(!finite);
         if (next <= pos_last) tile.fetch(p, off[turn ^ 1], tid);
         // scores: rows 4 ty + i, keys tx + 16 j
         pair32 s2[4][KPT];
@@ -404,6 +409,26 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
         }
         __syncwarp();                                          // the row's probabilities were written by this warp
         // the weighted sum: columns 4 tx + 64 c
+        if (by_row) {
+            // an infinity or NaN among the values: a row takes in only the keys it sees (0 times such a value is none)
+            for (int k = 0; k < KT; ++k) {
+                if (off[turn][k] < 0) continue;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (base + k > pos[i] || base + k < row_lo[i]) continue;
+                    const pair32 we = twice(ps[(ty * 4 + i) * ldp + k]);
+#pragma unroll
+                    for (int c = 0; c < CPT; ++c) {
+                        const int d = tx * 4 + 64 * c;
+                        if (d < hd) {
+                            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vs + k * hd + d);
+                            fma2(acc[i][2 * c], we, v.x);
+                            fma2(acc[i][2 * c + 1], we, v.y);
+                        }
+                    }
+                }
+            }
+        } else
 #pragma unroll 2
         for (int k = 0; k < KT; k += 4) {
             float4 w[4];

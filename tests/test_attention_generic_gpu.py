@@ -116,3 +116,11 @@ SIZES = [(torch.float32, 8, 2, 64), (torch.float32, 4, 4, 128), (torch.float32, 
 def test_single_tokens_that_see_no_number(what, dtype, nh, nkv, hd):
     _poisoned(what, dtype, nh, nkv, hd, [1, 1, 1, 1], [1, 40, 700, 300], 0, [[], [3], [0, 500, 699], []])
     _poisoned(what, dtype, nh, nkv, hd, [1, 1], [300, 300], 50, [[100, 249], [250]])
+
+
+@pytest.mark.parametrize("window", [0, 20])
+@pytest.mark.parametrize("what", ["keys", "values"])
+@pytest.mark.parametrize("dtype, nh, nkv, hd", SIZES)
+def test_portions_beside_what_is_no_number(what, dtype, nh, nkv, hd, window):
+    """Only the rows that see such a key or value are affected: not those before it, nor those whose window has passed it."""
+    _poisoned(what, dtype, nh, nkv, hd, [100, 2, 33], [100, 90, 140], window, [[50, 71, 99], [], [20, 110, 130]])
