@@ -36,9 +36,10 @@ class SamplingParams:
 
     @cached_property
     def packed(self) -> bytes:
-        """The settings as the host library reads them (``csrc/host_step.cpp``), formed once."""
-        return struct.pack("<dddqQ", self.temperature, self.top_p, self.repetition_penalty, int(self.top_k),
-                           int(self.seed) & ((1 << 64) - 1))
+        """The settings as the host library reads them (``csrc/host_step.cpp``), formed once.  (Greedy rows have no use
+        for top_k, whatever it is; one beyond 64 bits is refused like any beyond 32.)"""
+        return struct.pack("<dddqQ", self.temperature, self.top_p, self.repetition_penalty,
+                           0 if self.greedy else min(int(self.top_k), (1 << 63) - 1), int(self.seed) & ((1 << 64) - 1))
 
 
 GREEDY = SamplingParams(temperature=0.0)

@@ -9,6 +9,7 @@ its penalty without effect; here the request's generated tokens are passed.
 from __future__ import annotations
 
 from array import array
+from operator import index
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -22,10 +23,15 @@ def _pack(params: Sequence[SamplingParams], draw_index: Sequence[int]) -> Tuple[
     """(float32 [5 R]: the rows of (temperature, top_p, penalty, u), then the rows' top_k as int32 bits; whether all rows
     are greedy; whether one has a repetition penalty).  ``rng.uniform`` states the draws."""
     R = len(params)
-    if len(draw_index) != R:
-        raise ValueError("one draw index per SamplingParams")
+    try:
+        draws = array("q", draw_index)
+    except (TypeError, OverflowError):               # (a greedy row's draw is not looked at; others are whole numbers, modulo 2^64)
+        draws = array("Q", [0 if p.greedy else index(n) & (1 << 64) - 1 for p, n in zip(params, draw_index)])
+    if len(draws) < R:
+        if not all(p.greedy for p in params[len(draws):]):
+            raise ValueError("one draw index per SamplingParams")
+        draws.extend([0] * (R - len(draws)))
     host = np.empty(5 * R, dtype=np.float32)
-    draws = array("q", draw_index)
     flags = native.lib().lsbh_pack_sampling(R, b"".join([p.packed for p in params]), draws.buffer_info()[0],
                                             host.ctypes.data, host.ctypes.data + 16 * R)
     if flags < 0:

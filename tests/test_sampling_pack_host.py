@@ -25,3 +25,25 @@ def test_what_does_not_fit_is_refused():
         _pack([SamplingParams(top_k=2 ** 31)], [0])
     with pytest.raises(ValueError):
         _pack([SamplingParams()], [])
+
+
+def test_greedy_rows_are_not_asked_for_more_than_their_temperature():
+    greedy = SamplingParams(temperature=0.0, top_k=2 ** 40)
+    for draws in ([None, None], [], [2 ** 70, -1], [0.5, 1]):
+        host, all_greedy, penal = _pack([greedy, greedy], draws)
+        assert all_greedy and not penal and host[:8].reshape(2, 4)[:, 0].tolist() == [0.0, 0.0]
+    assert _pack([greedy, SamplingParams(seed=3)], [None, 4])[0][7] == np.float32(uniform(3, 4))
+
+
+@pytest.mark.parametrize("draw", [-1, 2 ** 63 - 1, 2 ** 63, 2 ** 64 + 5, 2 ** 90, np.int64(7)])
+def test_any_whole_number_is_a_draw(draw):
+    host, _, _ = _pack([SamplingParams(seed=11), SamplingParams(seed=12)], [draw, 1, 99])
+    assert host[3] == np.float32(uniform(11, int(draw))) and host[7] == np.float32(uniform(12, 1))
+
+
+def test_what_is_no_whole_number_or_too_large_is_refused():
+    with pytest.raises(TypeError):
+        _pack([SamplingParams()], [0.5])
+    for k in (2 ** 31, 2 ** 63, 2 ** 80):
+        with pytest.raises(OverflowError):
+            _pack([SamplingParams(top_k=k)], [0])
