@@ -247,7 +247,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
         }
     }
     if (greedy) {
-        if (rank == 0 && tid == 0) out[row] = mi;
+        if (rank == 0 && tid == 0) out[row] = mi < vocab ? mi : 0;      // (nothing but -infinities and NaN: the first token)
         cluster.sync();                                       // (a peer may still read this block's part)
         return;
     }

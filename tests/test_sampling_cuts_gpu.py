@@ -60,3 +60,21 @@ def test_cuts_of_rows_that_the_histogram_does_not_spread(kind):
         rows[:, ::1000] = np.float32(3e38) * np.sign(rows[:, ::1000])
         rows = np.clip(rows, -3e38, 60.0)
     check(rows, COMBOS, seed=3)
+
+
+@pytest.mark.parametrize("vocab", [5, 32770, 128256, 377003])
+def test_rows_without_a_value_name_the_first_token(vocab):
+    from llm_singularity_b200 import kernels as ops
+    rows = np.full((6, vocab), -np.inf, dtype=np.float32)
+    rows[1::3] = np.nan
+    rows[2, ::2] = np.nan
+    rows[5, vocab - 2] = -1e30                             # (one value: it is the maximum, whatever surrounds it)
+    rows[5, :vocab - 2:3] = np.nan
+    want = [0, 0, 0, 0, 0, vocab - 2]
+    for t, k, p in [(0.0, 0, 1.0), (0.0, 3, 0.5)] + COMBOS:
+        params = torch.tensor([[t, p, 1.0, 0.3]] * 6, device="cuda")
+        out = torch.full((6,), -1, dtype=torch.int32, device="cuda")
+        ops.sample(torch.from_numpy(rows).cuda(), params, torch.full((6,), k, dtype=torch.int32, device="cuda"), None, None, out)
+        got = out.tolist()
+        # (a NaN counts as the largest value of a top-k cut, which may leave nothing else: any token then)
+        assert got[:5] == want[:5] and (k and t or got[5] == want[5]) and 0 <= got[5] < vocab, (t, k, p, got)
