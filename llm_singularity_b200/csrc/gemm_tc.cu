@@ -1228,10 +1228,6 @@ LSB_API int lsb_gemm_tc_supported(const void* x, const void* w, int M, int N, in
     return M > 0 && N > 0 && K > 0 && K % 8 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0;
 }
 
-// The plan for a product: orientation (swap = weights on the 128-row side), tile width and K
-// splits.  With more than one split the blocks of a tile form a thread-block cluster and sum their
-// partial tiles through distributed shared memory, so there is no scratch in global memory; the
-// portable cluster size limits the splits to 8.
 // The width of a prompt product's tiles, and whether pairs of blocks walk them.  What a 64-deep step of a tile costs is
 // about its (128 + bn) rows of operands; a pair of blocks reads half of w per block, which makes a step 1/16 shorter,
 // against a start and an end across two blocks of some four steps, and an odd number of 128-row tiles is padded to an
@@ -1247,13 +1243,19 @@ static void prompt_tiles(int M, int N, int num_kb, int sms, int* bn, bool* pair)
     for (int c = 256; c >= 128; c -= 64) {
         const long long tn = (N + c - 1) / c;
         const long long one = (tm * tn + sms - 1) / sms * num_kb * (kBM + c) * 16;
-        const long long two = ((tm + 1) / 2 * tn + sms / 2 - 1) / (sms / 2) * num_kb * (kBM + c) * 15 + 4 * (kBM + 256) * 16;
         if (one < least) { least = one; *bn = c; *pair = false; }
+        if (sms < 2) continue;                   // (num_sms() does not know)
+        const long long two = ((tm + 1) / 2 * tn + sms / 2 - 1) / (sms / 2) * num_kb * (kBM + c) * 15 + 4 * (kBM + 256) * 16;
         if (two < least) { least = two; *bn = c; *pair = true; }
     }
 }
 
-LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn, int* splits) {
+// The plan for a product: orientation (swap = weights on the 128-row side), tile width and K
+// splits.  With more than one split the blocks of a tile form a thread-block cluster and sum their
+// partial tiles through distributed shared memory, so there is no scratch in global memory; the
+// portable cluster size limits the splits to 8.
+static void plan(int M, int N, int K, int swiglu, int* swap, int* bn, int* splits, bool* pair) {
+    *pair = false;
     const int num_kb = (K + kBK - 1) / kBK;
     const int sms = num_sms();
     const int most = sms * 13 / 16;              // "nearly every SM has a tile" (120 of 148)
@@ -1275,8 +1277,7 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
         *splits = s;
     } else {
         *swap = 0;
-        bool pair;
-        if (N >= kPersistentMin) prompt_tiles(M, N, num_kb, sms, bn, &pair);
+        if (N >= kPersistentMin) prompt_tiles(M, N, num_kb, sms, bn, pair);
         else *bn = N > 64 ? 128 : 64;
         *splits = 1;
         // A few hundred tokens make too few 128 x 256 tiles for the SMs.  Where the walk through K
@@ -1297,9 +1298,21 @@ LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn
                 *splits = (num_kb + per - 1) / per;
             }
         }
-        if (*splits > 1) *bn = 256;
+        if (*splits > 1) { *bn = 256; *pair = false; }
     }
+}
+
+LSB_API int lsb_gemm_tc_plan(int M, int N, int K, int swiglu, int* swap, int* bn, int* splits) {
+    bool pair;
+    plan(M, N, K, swiglu, swap, bn, splits, &pair);
     return 0;
+}
+// Do pairs of blocks walk the product's tiles?  (A gated one with a 32-bit result goes another way.)
+LSB_API int lsb_gemm_tc_pairs(int M, int N, int K, int swiglu) {
+    int swap, bn, splits;
+    bool pair;
+    plan(M, N, K, swiglu, &swap, &bn, &splits, &pair);
+    return pair;
 }
 
 // out[M, N] = x[M, K] * w[N, K]^T, bf16 inputs, bf16 or float output.
@@ -1318,7 +1331,8 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
     if (swiglu && (N % 2)) return (int)cudaErrorInvalidValue;
     if (!known_act(swiglu) || (plain && !known_plain(plain))) return (int)cudaErrorInvalidValue;
     int swap, bn, splits;
-    lsb_gemm_tc_plan(M, N, K, swiglu, &swap, &bn, &splits);
+    bool pair;
+    plan(M, N, K, swiglu, &swap, &bn, &splits, &pair);
     if (!swap && out_f32 && swiglu && bn > 128) bn = 256;      // (not a persistent product: widths that are compiled)
     const int n_out = swiglu ? N / 2 : N;
     GemmParams prm;
@@ -1350,7 +1364,8 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
         prm.swiglu = swiglu ? 1 : 0;
         prm.static_operand = 2;
         if ((rc = make_map(&mp, x, M, K, kBM))) return rc;
-        if ((rc = make_map(&mq, w, N, K, bn))) return rc;
+        if (out_f32 && swiglu) pair = false;                   // (not a persistent product)
+        if ((rc = make_map(&mq, w, N, K, pair ? bn / 2 : bn))) return rc;
         grid = dim3((M + kBM - 1) / kBM, (N + bn - 1) / bn, 1);
     }
     // Blocks of a split product are co-scheduled as clusters: four stages keep their shared memory
@@ -1363,12 +1378,7 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
     if (!swap && !(out_f32 && swiglu) && bn >= 128) {
         // prompts: persistent blocks, double-buffered accumulator
         const int tm = (M + kBM - 1) / kBM, tn = (N + bn - 1) / bn;
-        bool pair = false;
-        if (N >= kPersistentMin) prompt_tiles(M, N, prm.num_kb, sms, &bn, &pair);
-        if (pair) {
-            if ((rc = make_map(&mq, w, N, K, bn / 2))) return rc;
-            return launch_pair(mp, mq, prm, bn, (tm + 1) / 2, tn, stream);
-        }
+        if (pair) return launch_pair(mp, mq, prm, bn, (tm + 1) / 2, tn, stream);
         return launch_persistent(mp, mq, prm, bn, tm, tn, stream);
     }
     if (splits > 1) {

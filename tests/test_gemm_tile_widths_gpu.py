@@ -39,6 +39,7 @@ def test_pairs_of_blocks(M, N, K, gated, out_dtype):
     from llm_singularity_b200 import kernels as ops
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     x, w = (torch.randn(n, K, device="cuda", generator=g).to(torch.bfloat16) for n in (M, N))
+    assert ops._lib("gemm_tc").lsb_gemm_tc_pairs(M, N, K, int(gated))        # (on the 148 SMs of a B200)
     y = ops.linear(x, w, out_dtype=out_dtype, gated=gated)
     want = x.double() @ w.double().T
     tol = 2.0 ** -25 * K * K ** 0.5            # each 16 products a cut to 2^-23 of sums that stay below 4 sqrt(K)
