@@ -1,4 +1,4 @@
-// out[M, N] = x[M, K] * w[N, K]^T of 32-bit values with 32-bit sums, no bit of an operand dropped.  Three kernels, by the
+// out[M, N] = x[M, K] * w[N, K]^T of 32-bit values with 32-bit sums, no bit of an operand that could show in one dropped.  Three kernels, by the
 // number of rows and K; K a multiple of 4 and 16-byte aligned bases (anything else is csrc/gemm.cu's).  An activation of
 // a gated product (w's rows alternate gate_i, up_i, out is [M, N / 2]) is applied where the sums meet.  The reference
 // hands such products to cublasSgemm (kernels/src/cublas_provider.cpp:36-51) and launches silu(g) * u by itself
@@ -23,9 +23,9 @@
 //   K = 8,192 2.2e-7 and 8.1e-7 (at K of 100 and 256 the two are alike, which is where the line comes from).  The four
 //   products of a layer at 1B sizes, 500 rows (61 GFLOP): 1,491 -> 470 us.  What bounds it is the traffic of
 //   shared memory and the chain of a stage: 0.66 us where its products take 0.4 (both operands in shared
-//   memory: 0.9; one group of eight warps besides: 1.05).  Values that bfloat16 cannot split (infinities, NaN, a row
-//   that lies below 2^-95 as a whole) and sums that leave the range are done over by multiply-adds at the end, so
-//   that they come out as there.
+//   memory: 0.9; one group of eight warps besides: 1.05).  Sums that values which bfloat16 cannot split (infinities, NaN,
+//   numbers below 2^-103) could show in and sums that leave the range are done over by multiply-adds at the end, so that
+//   they come out as there.
 //
 // * More rows, smaller K: multiply-adds on the 32-bit pipes.  Eight warps of 64 x 64 outputs (8 x 16 a thread), arranged
 //   as a tile of 128 x 256, 128 x 128, 64 x 128 or 64 x 64; in the smaller tiles the warps that are left share out each
@@ -446,6 +446,10 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& h, uint32_t& 
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(b), "f"(a));
 }
 
+// (a number's magnitude as an integer, zeros the largest of all)
+__device__ __forceinline__ uint32_t twice_less_one(float v) { return 2u * __float_as_uint(v) - 1u; }
+constexpr uint32_t kTiny = 2u * ((127u - 103u) << 23) - 1u;            // of 2^-103
+
 template <int BN>
 struct SplitLayout {
     static constexpr int kRows = kSM + BN;
@@ -468,15 +472,15 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     unsigned char* ring = (unsigned char*)(((uintptr_t)raw_smem + 1023) & ~(uintptr_t)1023);
     unsigned char* planes = ring + (size_t)R * L::kRaw;
     __shared__ uint64_t raw_full[R], raw_empty[R], split_full[2], split_empty[2], acc_full[2], acc_empty[2], done;
-    __shared__ uint32_t tmem_slot, seen[L::kRows];
-    __shared__ int abort_flag;
+    __shared__ uint32_t tmem_slot, least[L::kRows];
+    __shared__ int abort_flag, any_tiny;
     lsb_pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m0 = (int)blockIdx.y * kSM, n0 = (int)blockIdx.x * BN;
     const int steps = (p.K + kSK - 1) / kSK;
-    if (tid < L::kRows) seen[tid] = 0;
+    if (tid < L::kRows) least[tid] = 0xffffffffu;
     if (tid == 0) {
-        abort_flag = 0;
+        abort_flag = any_tiny = 0;
         for (int s = 0; s < R; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kSGroup / 32); }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&split_full[s], kSGroup / 32);
@@ -573,7 +577,7 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         };
         const int group = warp / (kSGroup / 32), r = tid % kSGroup;     // stages it % 2 == group
         const bool has_row = r < L::kRows;
-        uint32_t bits = 0;
+        uint32_t low = 0xffffffffu;                                     // the least number of the row but zero: twice its bits, less one
         for (int it = group; it < steps && ok; it += 2) {
             const int s = it % R;
             if (!mbar_wait(&raw_full[s], (uint32_t)(it / R) & 1, &abort_flag)) { ok = false; break; }
@@ -589,8 +593,7 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float4 a = *reinterpret_cast<const float4*>(from + (((4 * j + i) ^ (r & 7)) << 4));
-                        bits |= __float_as_uint(a.x) | __float_as_uint(a.y);
-                        bits |= __float_as_uint(a.z) | __float_as_uint(a.w);
+                        low = min(low, min(min(twice_less_one(a.x), twice_less_one(a.y)), min(twice_less_one(a.z), twice_less_one(a.w))));
                         split3(a.x, a.y, h[2 * i], m[2 * i], l[2 * i]);
                         split3(a.z, a.w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1]);
                     }
@@ -629,24 +632,45 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             for (int j = 0; j < kMine; j += 4)
                 *reinterpret_cast<float4*>(row + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
         }
-        if (has_row) atomicOr(&seen[r], bits);
+        if (has_row) atomicMin(&least[r], low);
+        if (low < kTiny) any_tiny = 1;
         tmem_fence_before();
         asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
         if (!abort_flag) {
             const float* tile = reinterpret_cast<const float*>(ring);
-            // A row with nothing from 2^-95 up (but not all zeros) has values whose third part bfloat16 cannot hold.
-            auto faint = [&](int r) { return (seen[r] & 0x70000000u) == 0 && (seen[r] & 0x7fffffffu) != 0; };
+            // A number below 2^-103 loses less than 2^-125 with the parts that bfloat16 has no normal number for (one that
+            // is not below has them all), which is at most K 2^-125 times the largest number of the other operand's row in
+            // a sum.  Sums that this could show in are done over; the largest are looked up only where there is such a number.
+            float* largest = reinterpret_cast<float*>(planes);          // [kRows] (every product has been waited for)
+            if (any_tiny) {
+                for (int r = warp; r < L::kRows; r += kSWorkers / 32) {
+                    const bool of_x = r < kSM;
+                    const long long at = of_x ? m0 + r : n0 + r - kSM;
+                    float big = 0.f;
+                    if (at < (of_x ? p.M : p.N))
+                        for (int k = lane * 4; k < p.K; k += 128) {
+                            const float4 a = *reinterpret_cast<const float4*>((of_x ? p.x : p.w) + at * p.K + k);
+                            big = fmaxf(fmaxf(big, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(a.z), fabsf(a.w)));
+                        }
+                    big = lsb_warp_max(big);
+                    if (lane == 0) largest[r] = big * ((float)p.K * 0x1p-101f);
+                }
+                asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
+            }
             for (int e = tid; e < kSM * BN / 4; e += kSWorkers) {
                 const int row = e / (BN / 4), col = e % (BN / 4) * 4;
                 if (m0 + row >= p.M || n0 + col >= p.N) continue;
                 __align__(16) float v[4];
                 *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(tile + row * L::LDT + col);
-                const bool row_faint = faint(row);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (!(fabsf(v[i]) <= 3.402823466e38f) || row_faint || faint(kSM + col + i))
-                        if (n0 + col + i < p.N)
-                            v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
+                for (int i = 0; i < 4; ++i) {
+                    bool over = !(fabsf(v[i]) <= 3.402823466e38f);
+                    if (any_tiny)
+                        over |= (least[row] < kTiny && fabsf(v[i]) < largest[kSM + col + i]) ||
+                                (least[kSM + col + i] < kTiny && fabsf(v[i]) < largest[row]);
+                    if (over && n0 + col + i < p.N)
+                        v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
+                }
                 store_four(p, m0 + row, n0 + col, *reinterpret_cast<float4*>(v));
             }
         }

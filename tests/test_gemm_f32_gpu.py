@@ -93,3 +93,27 @@ def test_weights_that_the_kernel_in_front_makes(M, N, K):
         assert torch.equal(made, w) and bool(((y.double() - want).abs() <= bound).all())
         made.zero_()                             # (its memory goes to the next turn's weights)
         del made
+
+
+@pytest.mark.parametrize("N", [300, 20000])
+@pytest.mark.parametrize("K", [512, 2052])
+def test_split_products_of_small_values_beside_large_ones(N, K):
+    """Rows with ordinary numbers and ones whose parts bfloat16 has no numbers for, against rows that are zero at the
+    ordinary ones, or so large at the small ones that they count; and products near the smallest normal number."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x, w = (torch.randn(n, K, device="cuda", generator=g) for n in (140, N))
+    x[:, 9] = (1 + torch.rand(140, device="cuda", generator=g)) * 2.0 ** torch.linspace(-126, -80, 140, device="cuda").round()
+    w[:, 3] = (1 + torch.rand(N, device="cuda", generator=g)) * 2.0 ** torch.linspace(-120, -60, N, device="cuda").round()
+    w[5], x[7] = 0.0, 0.0
+    w[5, 9], x[7, 3] = 1.0, 1.0                                      # selections
+    x[11, ::2] *= 2.0 ** -110
+    w[13, ::2], w[13, 1::2] = w[13, ::2] * 1e30, 0.0                 # the small ones of x's row 11 times large ones
+    x[20] *= 2.0 ** -62
+    w[21] *= 2.0 ** -60
+    w[22] *= 2.0 ** -75
+    y, want = ops.linear(x, w), x.double() @ w.double().T
+    bound = 2.0 ** -24 * (x.abs().double() @ w.abs().double().T) * (2 + K ** 0.5) + K * 2.0 ** -149
+    assert bool(((y.double() - want).abs() <= bound).all())
+    for m, n in [(slice(None), 5), (7, slice(None))]:                # a selection is the number itself
+        assert torch.equal(y[m, n], want[m, n].float())
