@@ -117,3 +117,28 @@ def test_split_products_of_small_values_beside_large_ones(N, K):
     assert bool(((y.double() - want).abs() <= bound).all())
     for m, n in [(slice(None), 5), (7, slice(None))]:                # a selection is the number itself
         assert torch.equal(y[m, n], want[m, n].float())
+
+
+@pytest.mark.parametrize("M, N, K", [(17, 64, 512), (130, 2050, 516), (500, 2048, 2048), (129, 66, 8192), (1000, 130, 4100)])
+def test_split_products_keep_24_bits(M, N, K):
+    """The error of whole results, where a part of an operand left out would show (2^-17 of it or more)."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, w = (torch.randn(n, K, device="cuda", generator=g) for n in (M, N))
+    want = x.double() @ w.double().T
+    # (multiply-adds: 1.6e-7 at K = 512, 8e-7 at 8,192)
+    assert ((ops.linear(x, w).double() - want).norm() / want.norm()).item() < 4e-7
+
+
+@pytest.mark.parametrize("M, N, K", [(17, 70, 512), (130, 2050, 1028), (300, 9000, 544)])
+def test_every_part_of_a_split_counts(M, N, K):
+    """One number a row of x, with all 24 bits in use: each result is one product."""
+    from llm_singularity_b200 import kernels as ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    x, at = torch.zeros(M, K, device="cuda"), (37 * torch.arange(M, device="cuda")) % K
+    parts = 1.0 + torch.tensor([2.0 ** -9 + 2.0 ** -18 + 2.0 ** -23, -2.0 ** -9 - 2.0 ** -17 - 2.0 ** -23, 2.0 ** -10 + 2.0 ** -22, 2.0 ** -23], device="cuda")
+    x[torch.arange(M), at] = parts[torch.arange(M, device="cuda") % 4] * 2.0 ** (torch.arange(M, device="cuda") % 9 - 4)
+    want = x.double() @ w.double().T
+    # six of the nine products of parts: what is left out is below 2^-25; the sums of the six are cut to 2^-23, twice
+    assert bool(((ops.linear(x, w).double() - want).abs() <= 2.0 ** -22 * want.abs()).all())
