@@ -13,19 +13,13 @@
 // All three products of a token and the sums over a chunk run on mma.sync (bfloat16 operands, 32-bit sums).
 // What is not a bfloat16 number already goes in as the sum of two (the rounded value and the rounded
 // rest, 16 digits of mantissa): the states, the weighted keys, the weighted scores and, where they were
-// rotated in 32-bit (kSplit), queries and keys, or, where an activation makes them on the way in (kActed),
-// queries, keys and values; so nothing of the recurrence is rounded to bfloat16's 8 digits.
-//
-// kActed reads the projection itself (bfloat16) and applies silu in 32-bit while a tile is laid down, once in the first
-// kernel and once in the third: no pass of its own over memory.  A prompt of 1,500 tokens with
-// fades fixed by head (16 heads of 128 x 128): 83 us (output 50, gain 28, chain 5) where the walk took 528 in three; what bounds the two large ones is
-// the shared memory that mma.sync's operands pass through.
+// rotated in 32-bit (SPLIT), queries and keys; so nothing of the recurrence is rounded to bfloat16's 8 digits.
 // Sums of logarithms are formed in 64-bit and kept as pairs of floats: the difference of two of them is good
 // to 32-bit however far the memory has faded.  Different chunks and heads are different blocks; the sums
 // form in another order than in the walk: equal beyond rounding.
 //
 // rows: bfloat16 [tokens, ld]; a head's q, k and v at q_off, k_off (head h / share) and v_off (head h) with the rests
-// of q and k (kSplit) at q_lo and k_lo.  The state is [slot, head, V, N] 32-bit, N (channels of q and k)
+// of q and k (SPLIT) at q_lo and k_lo.  The state is [slot, head, V, N] 32-bit, N (channels of q and k)
 // contiguous; N and V multiples of 8 up to 128.  Scratch: a row per chunk, chunk j of request r at
 // q_start[r] / 128 + r + j.
 #include "common.cuh"
@@ -40,7 +34,6 @@ constexpr int kThreads = 256;
 struct ChunkArgs {
     const bf16* rows; long long ld;
     int q_off, k_off, v_off, q_lo, k_lo;
-    int q_silu, k_silu, v_silu;          // kActed: which pass silu
     int heads, share, N, V;
     const float *log_keep, *write;       // [tokens, heads] (null: log_fixed, and 1)
     const float* log_fixed;              // [heads]
@@ -77,28 +70,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
     hi = pack2(a, b);
     lo = pack2(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
-}
-
-// How queries, keys and values lie in the rows: as they are; queries and keys with their rests beside them; or as a
-// projection left them, with an activation to be applied (the values' rests matter then too).
-enum Mode : int { kPlain = 0, kSplit = 1, kActed = 2 };
-
-__device__ __forceinline__ float silu(float z) { return z * __fdividef(1.f, 1.f + __expf(-z)); }
-// two bfloat16 numbers through silu in 32-bit, as rounded values and rounded rests
-__device__ __forceinline__ void act2(uint32_t raw, bool act, uint32_t& hi, uint32_t& lo) {
-    const float a = __uint_as_float(raw << 16), b = __uint_as_float(raw & 0xffff0000u);
-    if (act) split2(silu(a), silu(b), hi, lo);
-    else { hi = raw; lo = 0u; }
-}
-__device__ __forceinline__ void act8(const uint4& raw, bool act, uint4& hi, uint4& lo) {
-    act2(raw.x, act, hi.x, lo.x);
-    act2(raw.y, act, hi.y, lo.y);
-    act2(raw.z, act, hi.z, lo.z);
-    act2(raw.w, act, hi.w, lo.w);
-}
-// eight values of a row, or zeros
-__device__ __forceinline__ uint4 row8(const bf16* src, bool real) {
-    return real ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);
 }
 
 // c of every token of the chunk (base-2 logarithm, a pair of floats) and its write factor into shared memory;
@@ -151,14 +122,13 @@ __device__ __forceinline__ Where chunk_of(const ChunkArgs& a) {
     return w;
 }
 
-template <int NP, int VP, int MODE>
+template <int NP, int VP, bool SPLIT>
 __global__ void __launch_bounds__(kThreads) chunk_gain_kernel(ChunkArgs a) {
-    constexpr bool SPLIT = MODE == kSplit, ACTED = MODE == kActed;
     constexpr int KS = NP + 8, VS = VP + 8;                     // row strides: four words past a multiple of 32
     extern __shared__ __align__(16) unsigned char sm[];
     bf16* k_hi = reinterpret_cast<bf16*>(sm);                   // [kL][KS], weighted keys
     bf16* k_lo = k_hi + kL * KS;
-    bf16* vs = k_lo + kL * KS;                                  // [kL][VS], and the rests of ACTED values behind them
+    bf16* vs = k_lo + kL * KS;                                  // [kL][VS]
     __shared__ float2 cum[kL];
     __shared__ float wr[kL];
     lsb_pdl_launch_dependents();
@@ -170,10 +140,7 @@ __global__ void __launch_bounds__(kThreads) chunk_gain_kernel(ChunkArgs a) {
     for (int w = threadIdx.x; w < kL * VG; w += kThreads) {
         const int s = w / VG, c = (w - s * VG) * 8;
         const bool real = s < at.n && c < a.V;
-        const bf16* src = a.rows + (real ? (size_t)(at.t0 + s) * a.ld + a.v_off + h * a.V + c : 0);
-        if (ACTED)
-            act8(row8(src, real), a.v_silu, *reinterpret_cast<uint4*>(vs + s * VS + c), *reinterpret_cast<uint4*>(vs + (kL + s) * VS + c));
-        else copy16(vs + s * VS + c, src, real);
+        copy16(vs + s * VS + c, a.rows + (real ? (size_t)(at.t0 + s) * a.ld + a.v_off + h * a.V + c : 0), real);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (warp == 0) chunk_sums(a, at.t0, at.n, h, cum, wr);
@@ -201,7 +168,6 @@ __global__ void __launch_bounds__(kThreads) chunk_gain_kernel(ChunkArgs a) {
                     x.x += y.x;
                     x.y += y.y;
                 }
-                if (ACTED && a.k_silu) x = make_float2(silu(x.x), silu(x.y));
                 split2(x.x * f, x.y * f, ph[j], pl[j]);
             }
         }
@@ -222,9 +188,8 @@ __global__ void __launch_bounds__(kThreads) chunk_gain_kernel(ChunkArgs a) {
         const uint32_t ka = smem_u32(k_hi + ((i8 & 1) * 8 + l8) * KS + n0 + (i8 >> 1) * 8);
         const int steps = (at.n + 15) >> 4;
         for (int ks = 0; ks < steps; ++ks) {
-            uint32_t fa[4], fl[4];
+            uint32_t fa[4];
             ldsm4_t(fa, va + ks * 16 * VS * 2);
-            if (ACTED) ldsm4_t(fl, va + (kL + ks * 16) * VS * 2);
 #pragma unroll
             for (int j = 0; j < WN / 16; ++j) {
                 uint32_t b[4], c[4];
@@ -235,10 +200,6 @@ __global__ void __launch_bounds__(kThreads) chunk_gain_kernel(ChunkArgs a) {
                 mma16816(e[2 * j + 1], fa, b[2], b[3]);
                 mma16816(e[2 * j], fa, c[0], c[1]);
                 mma16816(e[2 * j + 1], fa, c[2], c[3]);
-                if (ACTED) {
-                    mma16816(e[2 * j], fl, b[0], b[1]);
-                    mma16816(e[2 * j + 1], fl, b[2], b[3]);
-                }
             }
         }
         float* dst = a.gain + (at.row * a.heads + h) * (size_t)a.V * a.N;
@@ -303,16 +264,15 @@ __global__ void __launch_bounds__(kChainThreads) chunk_chain_kernel(ChunkArgs a)
     *reinterpret_cast<float4*>(st) = cur;
 }
 
-template <int NP, int VP, int MODE>
+template <int NP, int VP, bool SPLIT>
 __global__ void __launch_bounds__(kThreads) chunk_output_kernel(ChunkArgs a) {
-    constexpr bool ACTED = MODE == kActed, SPLIT = MODE != kPlain;   // (queries and keys have rests in both)
     constexpr int KS = NP + 8, VS = VP + 8;
     extern __shared__ __align__(16) unsigned char sm[];
     bf16* s_hi = reinterpret_cast<bf16*>(sm);                   // [VP][KS] start state
     bf16* s_lo = s_hi + VP * KS;
     bf16* k_hi = s_lo + VP * KS;                                // [kL][KS]
     bf16* k_lo = k_hi + (SPLIT ? kL * KS : 0);
-    bf16* vs = k_lo + kL * KS;                                  // [kL][VS], and the rests of ACTED values behind them
+    bf16* vs = k_lo + kL * KS;                                  // [kL][VS]
     __shared__ float2 cum[kL];
     __shared__ float wr[kL];
     lsb_pdl_launch_dependents();
@@ -334,21 +294,13 @@ __global__ void __launch_bounds__(kThreads) chunk_output_kernel(ChunkArgs a) {
         const int s = w / NG, c = (w - s * NG) * 8;
         const bool real = s < at.n && c < a.N;
         const bf16* src = a.rows + (real ? (size_t)(at.t0 + s) * a.ld + hk * a.N + c : 0);
-        if (ACTED) {
-            act8(row8(src + (real ? a.k_off : 0), real), a.k_silu, *reinterpret_cast<uint4*>(k_hi + s * KS + c),
-                 *reinterpret_cast<uint4*>(k_lo + s * KS + c));
-        } else {
-            copy16(k_hi + s * KS + c, src + (real ? a.k_off : 0), real);
-            if (SPLIT) copy16(k_lo + s * KS + c, src + (real ? a.k_lo : 0), real);
-        }
+        copy16(k_hi + s * KS + c, src + (real ? a.k_off : 0), real);
+        if (SPLIT) copy16(k_lo + s * KS + c, src + (real ? a.k_lo : 0), real);
     }
     for (int w = threadIdx.x; w < kL * VG; w += kThreads) {
         const int s = w / VG, c = (w - s * VG) * 8;
         const bool real = s < at.n && c < a.V;
-        const bf16* src = a.rows + (real ? (size_t)(at.t0 + s) * a.ld + a.v_off + h * a.V + c : 0);
-        if (ACTED)
-            act8(row8(src, real), a.v_silu, *reinterpret_cast<uint4*>(vs + s * VS + c), *reinterpret_cast<uint4*>(vs + (kL + s) * VS + c));
-        else copy16(vs + s * VS + c, src, real);
+        copy16(vs + s * VS + c, a.rows + (real ? (size_t)(at.t0 + s) * a.ld + a.v_off + h * a.V + c : 0), real);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (warp == 0) chunk_sums(a, at.t0, at.n, h, cum, wr);
@@ -366,10 +318,7 @@ __global__ void __launch_bounds__(kThreads) chunk_output_kernel(ChunkArgs a) {
             q[ks][1] = ok_b && in0 ? *reinterpret_cast<const uint32_t*>(qb + a.q_off + c) : 0u;
             q[ks][2] = ok_a && in1 ? *reinterpret_cast<const uint32_t*>(qa + a.q_off + c + 8) : 0u;
             q[ks][3] = ok_b && in1 ? *reinterpret_cast<const uint32_t*>(qb + a.q_off + c + 8) : 0u;
-            if (ACTED) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) act2(q[ks][i], a.q_silu, q[ks][i], ql[SPLIT ? ks : 0][i]);
-            } else if (SPLIT) {
+            if (SPLIT) {
                 ql[SPLIT ? ks : 0][0] = ok_a && in0 ? *reinterpret_cast<const uint32_t*>(qa + a.q_lo + c) : 0u;
                 ql[SPLIT ? ks : 0][1] = ok_b && in0 ? *reinterpret_cast<const uint32_t*>(qb + a.q_lo + c) : 0u;
                 ql[SPLIT ? ks : 0][2] = ok_a && in1 ? *reinterpret_cast<const uint32_t*>(qa + a.q_lo + c + 8) : 0u;
@@ -483,11 +432,6 @@ __global__ void __launch_bounds__(kThreads) chunk_output_kernel(ChunkArgs a) {
             mma16816(o[2 * j + 1], ph, b[2], b[3]);
             mma16816(o[2 * j], pl, b[0], b[1]);
             mma16816(o[2 * j + 1], pl, b[2], b[3]);
-            if (ACTED) {
-                ldsm4_t(b, va + ((kL + g * 16) * VS + j * 16) * 2);
-                mma16816(o[2 * j], ph, b[0], b[1]);
-                mma16816(o[2 * j + 1], ph, b[2], b[3]);
-            }
         }
     }
     const size_t ldo = (size_t)a.heads * a.V;
@@ -561,41 +505,39 @@ LSB_API int lsb_chunk_tokens() { return kL; }
 
 LSB_API int lsb_chunk_scan_supported(int N, int V) { return N > 0 && V > 0 && N % 8 == 0 && V % 8 == 0 && N <= 128 && V <= 128; }
 
-template <int NP, int VP, int MODE>
+template <int NP, int VP, bool SPLIT>
 static int run_chunks(const ChunkArgs& a, int n_requests, int chunks, cudaStream_t stream) {
     constexpr int KS = NP + 8, VS = VP + 8;
-    constexpr int kValues = MODE == kActed ? 2 : 1;
-    constexpr size_t gain_sm = (size_t)(2 * kL * KS + kValues * kL * VS) * sizeof(bf16);
-    constexpr size_t out_sm = (size_t)(2 * VP * KS + (MODE != kPlain ? 2 : 1) * kL * KS + kValues * kL * VS) * sizeof(bf16);
+    constexpr size_t gain_sm = (size_t)(2 * kL * KS + kL * VS) * sizeof(bf16);
+    constexpr size_t out_sm = (size_t)(2 * VP * KS + (SPLIT ? 2 : 1) * kL * KS + kL * VS) * sizeof(bf16);
     static int configured = -1;
     if (configured < 0) {
-        configured = (int)cudaFuncSetAttribute(chunk_gain_kernel<NP, VP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gain_sm);
+        configured = (int)cudaFuncSetAttribute(chunk_gain_kernel<NP, VP, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gain_sm);
         if (!configured)
-            configured = (int)cudaFuncSetAttribute(chunk_output_kernel<NP, VP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_sm);
+            configured = (int)cudaFuncSetAttribute(chunk_output_kernel<NP, VP, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_sm);
     }
     if (configured) return configured;
     dim3 grid(chunks, a.heads, n_requests);
-    int rc = lsb_launch(chunk_gain_kernel<NP, VP, MODE>, grid, dim3(kThreads), gain_sm, stream, 1, a);
+    int rc = lsb_launch(chunk_gain_kernel<NP, VP, SPLIT>, grid, dim3(kThreads), gain_sm, stream, 1, a);
     if (rc) return rc;
     const int per = a.V * a.N / 4;
     rc = lsb_launch(chunk_chain_kernel, dim3((per + kChainThreads - 1) / kChainThreads, a.heads, n_requests), dim3(kChainThreads), 0,
                     stream, 1, a);
     if (rc) return rc;
-    return lsb_launch(chunk_output_kernel<NP, VP, MODE>, grid, dim3(kThreads), out_sm, stream, 1, a);
+    return lsb_launch(chunk_output_kernel<NP, VP, SPLIT>, grid, dim3(kThreads), out_sm, stream, 1, a);
 }
 
 // log_keep and write [tokens, heads] (both or neither), else log_fixed [heads]; q_lo, k_lo >= 0: queries and keys are split.
-// silu: 1 for queries + 2 for keys + 4 for values that pass it on the way in (and are not split then).
 // gain, starts, fade: scratch of tokens / 128 + requests rows (see above).  q_start and table_rows begin at the
 // first request to be run.
 LSB_API int lsb_chunk_scan(const void* rows, long long ld, int q_off, int k_off, int v_off, int q_lo, int k_lo, int heads,
                            int key_heads, int N, int V, const float* log_keep, const float* write, const float* log_fixed,
-                           float q_scale, int silu, float* state, int n_slots, const int* q_start, const int* table_rows, int n_requests,
+                           float q_scale, float* state, int n_slots, const int* q_start, const int* table_rows, int n_requests,
                            int max_q_len, float* out, float* gain, void* starts, float* fade, cudaStream_t stream) {
     if (n_requests <= 0 || max_q_len <= 0) return 0;
     const bool split = q_lo >= 0;
     if (!lsb_chunk_scan_supported(N, V) || heads <= 0 || key_heads <= 0 || heads % key_heads || heads > 65535 || n_requests > 65535 ||
-        (split != (k_lo >= 0)) || silu < 0 || silu > 7 || (silu && split) || (!log_keep && !log_fixed) || (log_keep && !write) || !gain || !starts || !fade)
+        (split != (k_lo >= 0)) || (!log_keep && !log_fixed) || (log_keep && !write) || !gain || !starts || !fade)
         return (int)cudaErrorInvalidValue;
     if ((uintptr_t)rows % 16 || ld % 8 || q_off % 8 || k_off % 8 || v_off % 8 || (split && (q_lo % 8 || k_lo % 8)) ||
         (uintptr_t)state % 16 || (uintptr_t)gain % 16 || (uintptr_t)starts % 16 || (uintptr_t)out % 8)
@@ -603,7 +545,6 @@ LSB_API int lsb_chunk_scan(const void* rows, long long ld, int q_off, int k_off,
     ChunkArgs a;
     a.rows = (const bf16*)rows; a.ld = ld;
     a.q_off = q_off; a.k_off = k_off; a.v_off = v_off; a.q_lo = q_lo; a.k_lo = k_lo;
-    a.q_silu = silu & 1; a.k_silu = silu & 2; a.v_silu = silu & 4;
     a.heads = heads; a.share = heads / key_heads; a.N = N; a.V = V;
     a.log_keep = log_keep; a.write = write; a.log_fixed = log_fixed; a.q_scale = q_scale;
     a.state = state; a.n_slots = n_slots; a.q_start = q_start; a.table_rows = table_rows;
@@ -611,9 +552,8 @@ LSB_API int lsb_chunk_scan(const void* rows, long long ld, int q_off, int k_off,
     const int chunks = (max_q_len + kL - 1) / kL;
 #define LSB_CHUNKS(NP, VP)                                                           \
     do {                                                                             \
-        if (silu) return run_chunks<NP, VP, kActed>(a, n_requests, chunks, stream);  \
-        if (split) return run_chunks<NP, VP, kSplit>(a, n_requests, chunks, stream); \
-        return run_chunks<NP, VP, kPlain>(a, n_requests, chunks, stream);            \
+        if (split) return run_chunks<NP, VP, true>(a, n_requests, chunks, stream);   \
+        return run_chunks<NP, VP, false>(a, n_requests, chunks, stream);             \
     } while (0)
     if (N <= 64) {
         if (V <= 64) LSB_CHUNKS(64, 64);

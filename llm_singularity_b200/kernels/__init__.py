@@ -1141,13 +1141,16 @@ def chunk_scan(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: in
                log_keep: Optional[torch.Tensor] = None, write: Optional[torch.Tensor] = None,
                log_decay: Optional[torch.Tensor] = None, q_scale: float = 1.0, acts=("none", "none", "none")) -> None:
     """What ``linear_scan`` does for a memory that fades by one number per head and token, for the requests from
-    ``first`` on, in chunks on the tensor cores.  ``rows`` bfloat16: q, k and v at their offsets, with ``q_lo`` / ``k_lo``
-    the rounded rests of q and k.  ``log_keep`` and ``write`` (32-bit [T, heads]): the logarithm of the fade and the
-    factor of a write; or ``log_decay`` [heads], the same for every token, with writes as they are.  ``acts``: what q, k and v
-    pass on the way in ("silu" or "none"; not where they come with rests), in 32-bit."""
+    ``first`` on, in chunks.  ``rows`` bfloat16: q, k and v at their offsets, with ``q_lo`` / ``k_lo`` the rounded rests
+    of q and k.  ``log_keep`` and ``write`` (32-bit [T, heads]): the logarithm of the fade and the factor of a write; or
+    ``log_decay`` [heads], the same for every token, with writes as they are.  ``acts``: what q, k and v pass on the way in
+    ("silu" or "none"; with ``log_decay``, not where they come with rests).
+
+    With ``log_decay`` and no rests everything is held and summed in 32-bit (``csrc/chunk_scan_f32.cu``); otherwise on the
+    tensor cores, as sums of two bfloat16 numbers where it is not bfloat16 already (``csrc/chunk_scan.cu``)."""
     silu = sum(1 << i for i, name in enumerate(acts) if _SCAN_ACTS[name])
-    if silu and q_lo >= 0:
-        raise KernelError("chunk_scan: operands with rests have passed their activations")
+    if silu and (q_lo >= 0 or log_decay is None):
+        raise KernelError("chunk_scan: activations on the way in go with a fixed decay and operands without rests")
     _req(rows, "rows", torch.bfloat16, 2)
     _req(state, "state", torch.float32, 4)
     _req(out, "out", torch.float32, 2)
@@ -1164,15 +1167,22 @@ def chunk_scan(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: in
             if tuple(t.shape) != shape:
                 raise KernelError(f"chunk_scan: {name} must be {list(shape)}")
     n_req = ctx.n_requests - first
+    q_start, table_rows = (ctypes.c_void_p(t.data_ptr() + 4 * first) for t in (ctx.q_start, ctx.table_rows))
+    if log_decay is not None and log_keep is None and q_lo < 0:
+        n = T // int(_lib("chunk_scan_f32").lsb_chunk_f32_tokens()) + n_req
+        gain = torch.empty(n * heads * value_dim * key_dim, dtype=torch.float32, device=rows.device)
+        _call("chunk_scan_f32", "lsb_chunk_scan_f32", _p(rows), _ll(ld), _i(q_off), _i(k_off), _i(v_off), _i(heads), _i(key_heads),
+              _i(key_dim), _i(value_dim), _p(log_decay), _f(q_scale), _i(silu), _p(state), _i(state.shape[0]), q_start, table_rows,
+              _i(n_req), _i(ctx.max_q_len), _p(out), _p(gain), _stream(out))
+        return
     n = T // int(_lib("chunk_scan").lsb_chunk_tokens()) + n_req
     gain = _chunk_scratch("gain", n * heads * value_dim * key_dim, rows.device, torch.float32)
     starts = _chunk_scratch("starts", n * heads * 2 * value_dim * key_dim, rows.device, torch.bfloat16)
     fade = _chunk_scratch("fade", n * heads, rows.device, torch.float32)
     _call("chunk_scan", "lsb_chunk_scan", _p(rows), _ll(ld), _i(q_off), _i(k_off), _i(v_off), _i(q_lo), _i(k_lo), _i(heads),
-          _i(key_heads), _i(key_dim), _i(value_dim), _p(log_keep), _p(write), _p(log_decay), _f(q_scale), _i(silu),
-          _p(state), _i(state.shape[0]), ctypes.c_void_p(ctx.q_start.data_ptr() + 4 * first),
-          ctypes.c_void_p(ctx.table_rows.data_ptr() + 4 * first), _i(n_req), _i(ctx.max_q_len), _p(out), _p(gain), _p(starts),
-          _p(fade), _stream(out))
+          _i(key_heads), _i(key_dim), _i(value_dim), _p(log_keep), _p(write), _p(log_decay), _f(q_scale), _p(state),
+          _i(state.shape[0]), q_start, table_rows, _i(n_req), _i(ctx.max_q_len), _p(out), _p(gain), _p(starts), _p(fade),
+          _stream(out))
 
 
 # ----------------------------------------------------------------- state-space memory

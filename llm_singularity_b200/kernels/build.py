@@ -50,6 +50,7 @@ SOURCES: Dict[str, object] = {          # library -> its source file (or files)
     "output_norm": "output_norm.cu",
     "state_space": "state_space.cu",
     "chunk_scan": "chunk_scan.cu",
+    "chunk_scan_f32": "chunk_scan_f32.cu",
     "attention_prep": "attention_prep.cu",
     "attention_dv": "attention_dv.cu",
     "attention_diff": "attention_diff.cu",

@@ -11,8 +11,9 @@ b = 1 - a; no key, no other scale).  The outputs are RMS-normed (all heads toget
 over the row, or each head by itself with one weight of head size or none), optionally multiplied by
 sigmoid or silu of W_g x, and projected by W_o.  With a fixed decay q and k may be rotated by the tokens'
 positions and k scaled (retention): the projections leave their product in 32-bit, walked tokens are rotated
-there, and queries and keys are rotated into sums of two bfloat16 numbers.  Prompt portions of a memory with a fixed decay
-run in chunks on the tensor cores (``csrc/chunk_scan.cu``), everything else token by token.
+there, and prompt portions run in chunks on the tensor cores (``csrc/chunk_scan.cu``) with rotated queries and
+keys as sums of two bfloat16 numbers.  Prompt portions of a memory with a fixed decay and no rotation run in chunks in
+32-bit (``csrc/chunk_scan_f32.cu``), everything else token by token.
 
 The state starts at zero when a request takes a slot, is 32-bit, and is carried from step to
 step in the slot's row of a ``StateSpec`` cache.  One product makes all projections of a step
@@ -56,7 +57,7 @@ class LinearRecurrence(Part):
         if self.k_scale != 1.0 and s.gate != "fixed_decay":
             raise ValueError("a factor on k goes with a fixed decay")
         if s.gate == "fixed_decay" and rt.dtype == torch.bfloat16:
-            self.kernels = self.kernels + ("chunk_scan",)
+            self.kernels = self.kernels + (("chunk_scan",) if self.position is not None else ("chunk_scan", "chunk_scan_f32"))
         # the output kernel that knows heads without a weight and the silu gate
         self.plain_output = s.out_norm != "unit" and self.gate_act == "sigmoid"
         if not self.plain_output:
@@ -120,7 +121,7 @@ class LinearRecurrence(Part):
         o = self.rt.empty(x.shape[0], self.vv, dtype=torch.float32)
         # [T, q | k or f | v | g]
         proj = ops.linear(x, self.w_in) if self.position is None else ops.linear(x, self.w_in, out_dtype=torch.float32)
-        # prompt portions in chunks on the tensor cores where they can be, the rest walked
+        # prompt portions in chunks where they can be, the rest walked
         first = ops.chunk_scan_first(ctx, self.rt.dtype, s.key_dim, s.value_dim) \
             if self.log_decay is not None and hasattr(ops, "chunk_scan_first") else None
         if self.position is None:
