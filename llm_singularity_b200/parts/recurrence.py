@@ -122,8 +122,7 @@ class LinearRecurrence(Part):
         # [T, q | k or f | v | g]
         proj = ops.linear(x, self.w_in) if self.position is None else ops.linear(x, self.w_in, out_dtype=torch.float32)
         # prompt portions in chunks where they can be, the rest walked
-        first = ops.chunk_scan_first(ctx, self.rt.dtype, s.key_dim, s.value_dim) \
-            if self.log_decay is not None and hasattr(ops, "chunk_scan_first") else None
+        first = ops.chunk_scan_first(ctx, self.rt.dtype, s.key_dim, s.value_dim) if self.log_decay is not None else None
         if self.position is None:
             if first is None or not self.fades:
                 self._walk(proj, ctx, cache, o)
