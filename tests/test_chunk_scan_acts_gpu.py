@@ -29,8 +29,8 @@ def test_against_the_recurrence(acts, q_lens, heads, N, V):
             t += 1
         end[(1, 3, 0)[r]] = S
     log_decay = torch.log(decay.double()).float().cuda()
-    # operands keep 16 digits of mantissa (2^-17 each) and silu is good to 2^-20: three of the one, two of the other
-    # in a term, the terms' errors of either sign
+    # silu is good to 2^-20, up to three of them in a term, the terms' errors of either sign (what 32-bit sums keep is
+    # held far closer where no silu stands in front, tests/test_chunk_scan_f32_gpu.py)
     tol = 3e-5
     for chunked in (False, True):
         state, out = start.cuda(), torch.zeros(T, heads * V, device="cuda")
