@@ -420,10 +420,11 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
     ``into = (residual, norm_weight, eps)``: the product is added to ``residual`` ([M, N] 32-bit, in
     place) and what comes back is a ``NormOut``: what follows the RMS norm with that weight.
 
-    float32 operands lose no bit and have 32-bit sums: on the CUDA cores, or with many rows and K from 512 on the
-    tensor cores as exact splits into bfloat16 parts (``csrc/gemm_f32.cu``).  bfloat16 operands run on the
-    tensor cores (tcgen05, accumulators in TMEM) when K is a multiple of 8, else on the CUDA
-    cores as well.
+    float32 operands lose no bit that could show and have 32-bit sums: on the CUDA cores, or with many rows and K from 512
+    on the tensor cores as exact splits into bfloat16 parts (``csrc/gemm_f32.cu``); which of them, and so the order of a
+    row's sums, depends on M, N and K.  bfloat16 operands run on the tensor cores (tcgen05, accumulators in TMEM) when K
+    is a multiple of 8, else on the CUDA cores as well; there ``w`` is taken for resident, its first rows are read before
+    the kernels in front of this one on the stream have ended (a 32-bit ``w`` may be their result).
 
     ``gated``: the rows of ``w`` alternate gate_i, up_i and the result is [M, N / 2] with
     ``out[m, i] = act(d[m, 2i]) * d[m, 2i + 1]`` (applied in the product's epilogue on the
@@ -812,7 +813,8 @@ def paged_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache, s
 
     bfloat16 with head size 64 or 128 runs on the tensor cores: single decode tokens in the
     split-KV kernel, prompt portions in the tiled kernel.  Everything else (32-bit, other head
-    sizes) runs the generic kernel.  ``decode_rope = (inv_freq, store, rotary_dim)`` says that
+    sizes) runs the generic kernels, whose cut of a single token's keys depends on how many single tokens the step
+    holds and on its longest context (not in a captured step).  ``decode_rope = (inv_freq, store, rotary_dim)`` says that
     single tokens come unrotated and not yet in the cache (see ``rope_store_attention``).  ``only``: "single"
     or "portions" launches just that kernel; ``stream``: a raw stream to launch on instead of the
     current one."""
