@@ -7,9 +7,8 @@
 // * Up to 16 rows (a decode step) the product is weight traffic.  Weight rows are dealt out over one
 //   block per SM, sixteen at most at a time: four to a warp, each row's K in two parts.  A warp copies the weights it
 //   needs into a ring of shared memory itself (asynchronously, some 140 KB in flight an SM, the first of them asked for
-//   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three
-//   others of its part.  The sums of a group meet once, over lanes by halving exchanges and over the two parts in shared
-//   memory, in a fixed order.
+//   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three others of its part.  The sums of a
+//   group meet once, over lanes by halving exchanges and over the two parts in shared memory, in a fixed order.
 //   The four products of a layer at 1B sizes, 8 rows (243 MB): 71 us (3.4 TB/s); as 64 x 64 tiles, 56 of their 64 rows
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
 //   four times the exchanges at the end of a group: 89 us.)
@@ -31,11 +30,10 @@
 // * More rows, smaller K: multiply-adds on the 32-bit pipes.  Eight warps of 64 x 64 outputs (8 x 16 a thread), arranged
 //   as a tile of 128 x 256, 128 x 128, 64 x 128 or 64 x 64; in the smaller tiles the warps that are left share out each
 //   slice of K and their sums meet at the end, so that few tiles still give an SM eight busy warps.  Slices come by
-//   asynchronous copies, three to five in flight.  2,048 x 8,192 x 256: 200 us, 43 TFLOP/s of the 70 that a loop of
-//   nothing but multiply-adds reaches here.  Up to 128 rows go the first way where its blocks have ended before a tile has.
+//   asynchronous copies, three to five in flight.  500 x 16,384 x 2,048: 764 us, 44 TFLOP/s of the 70 that a loop of
+//   nothing but multiply-adds reaches here.
 //
-// A row's sum is taken in an order that K and the kernel fix, the same from run to run; which kernel, and so the last digits,
-// depends on the number of rows beside it.
+// A row's sum is taken in an order that K and the kernel fix, the same from run to run.
 #include "common.cuh"
 #include "gate_act.cuh"
 
@@ -56,12 +54,8 @@ constexpr int kRowThreads = 256;
 constexpr int kRowsMax = 16;                   // rows of x a block takes
 constexpr int kRB = 16;                        // most weight rows of a group: four for each of four warps, twice (two parts of K)
 constexpr int kRW = kRB / 4;
-// Rows that may still go this way, sixteen to a block: where by the counts below the blocks have ended before a tile has
-// (17 x 1,024 x 480: 6.0 us, as tiles of 64 x 64 16.1; 48 x 128 x 320 7.5 and 11.3, 128 x 128 x 320 17.4 and 11.5),
-// and from kSplitK on only times matrices of up to kSmallMatrix numbers, as from the first (96 x 128 x 2,048: 36 us, split 42;
-// 96 x 512 x 512 17 and 13): the split sums of larger ones are the more exact.
-constexpr int kRowsMost = 128;
-constexpr long long kSmallMatrix = 1 << 18;
+constexpr int kRowsSmall = 128;                // rows that still go this way, sixteen to a block, ...
+constexpr long long kSmallMatrix = 1 << 18;    // ... where the matrix is so small that a tile's latency shows
 constexpr int kKS = 512;                       // K of a stage: two steps of 128 for each part
 
 struct RowsParams {
@@ -357,7 +351,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_f32_kernel(const Ti
 
 // ------------------------------------------------------------------ many rows, on the tensor cores
 constexpr int kSplitK = 512;                   // K from which on the split sums are the more exact ones
-constexpr double kSplitFixed = 3.4, kSplitAlong = 0.019;              // us of a tile of 64 columns, about (K = 512: 13.1, 4,096: 81.0)
 constexpr int kSM = 128;                       // rows of x of a tile (tensor memory lanes)
 constexpr int kSK = 32;                        // K of a stage: 128 bytes of a 32-bit row, 64 of a plane's
 constexpr int kSPlanes = 3;
@@ -703,22 +696,6 @@ static int num_sms() {
     return cached[dev];
 }
 
-// Groups of as many weight rows as share a matrix out evenly over the SMs' turns.
-static void share_out(int N, int unit, int sms, int* per, int* groups) {
-    const int turns = (N + sms * kRB - 1) / (sms * kRB);
-    *per = ((N + sms * turns - 1) / (sms * turns) + unit - 1) / unit * unit;
-    *groups = (N + *per - 1) / *per;
-}
-// What gemm_rows_f32_kernel takes, about (us): rounds of its blocks (one an SM) times the groups of each.
-static double rows_time(int M, int N, int K) {
-    const int sms = num_sms();
-    int per, groups;
-    share_out(N, 1, sms, &per, &groups);
-    const int blocks = groups < sms ? groups : sms;
-    const long long rounds = ((long long)blocks * ((M + kRowsMax - 1) / kRowsMax) + sms - 1) / sms;
-    return (double)rounds * ((groups + blocks - 1) / blocks) * (1.9 + 0.035 * per + 0.002 * K);
-}
-
 template <int MT, int ST>
 static int launch_rows(RowsParams p, cudaStream_t stream) {
     static int configured = -1;
@@ -726,8 +703,12 @@ static int launch_rows(RowsParams p, cudaStream_t stream) {
     if (configured < 0)
         configured = (int)cudaFuncSetAttribute(gemm_rows_f32_kernel<MT, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (configured) return configured;
-    const int sms = num_sms();
-    share_out(p.N, p.act ? 2 : 1, sms, &p.per, &p.groups);
+    // groups of as many rows as share the matrix out evenly over the SMs' turns
+    const int unit = p.act ? 2 : 1, sms = num_sms();
+    const int turns = (p.N + sms * kRB - 1) / (sms * kRB);
+    p.per = (p.N + sms * turns - 1) / (sms * turns);
+    p.per = (p.per + unit - 1) / unit * unit;
+    p.groups = (p.N + p.per - 1) / p.per;
     const int blocks = p.groups < sms ? p.groups : sms;
     return lsb_launch(gemm_rows_f32_kernel<MT, ST>, dim3(blocks, (p.M + kRowsMax - 1) / kRowsMax), dim3(kRowThreads), smem, stream, 1, p);
 }
@@ -792,24 +773,7 @@ LSB_API int lsb_gemm_f32_supported(const void* x, const void* w, int M, int N, i
 LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, int act, cudaStream_t stream) {
     if (!lsb_gemm_f32_supported(x, w, M, N, K) || ((uintptr_t)out % 16)) return (int)cudaErrorInvalidValue;
     if (act < 0 || act > LSB_ACT_NONE || (act && (N & 1))) return (int)cudaErrorInvalidValue;
-    const long long sms = num_sms();
-    const TileParams p{x, w, out, M, N, K, act};
-    // The tile that takes the least by this count: rounds over the SMs times what a tile takes, a part of it whatever K and
-    // a part along K (whole slices).  Within 8 % of the fastest of the five on 120 shapes (17 to 2,048 rows, N 128 to
-    // 20,000, K 20 to 480).  128 x 256, 128 x 128, 64 x 128, 64 x 64, us: 2,048 x 2,048 x 64 18 / 19 / 22 / 29;
-    // 2,048 x 8,192 x 256 215 / 200 / 218 / 259; 200 x 4,096 x 128 30 / 16 / 9.6 / 11.7; 500 x 512 x 128 29 / 16 / 9.4 / 6.2.
-    const int bm[4] = {128, 128, 64, 64}, bn[4] = {256, 128, 128, 64}, bk[4] = {32, 32, 32, 64};
-    const double fixed[4] = {3.5, 2.9, 2.5, 2.1}, along[4] = {0.19, 0.098, 0.051, 0.0295};
-    int best = 0;
-    double least = 0.0;
-    for (int c = 0; c < 4; ++c) {
-        const long long tiles = (long long)((M + bm[c] - 1) / bm[c]) * ((N + bn[c] - 1) / bn[c]);
-        const double t = (double)((tiles + sms - 1) / sms) * (fixed[c] + along[c] * ((K + bk[c] - 1) / bk[c] * bk[c]));
-        if (c == 0 || t < least) { least = t; best = c; }
-    }
-    const bool split = K >= kSplitK;
-    if (split) least = kSplitFixed + kSplitAlong * K;           // (a round of tiles of 64 columns)
-    if (M <= kRowsMax || (M <= kRowsMost && (!split || (long long)N * K <= kSmallMatrix) && rows_time(M, N, K) < least)) {
+    if (M <= kRowsMax || (M <= kRowsSmall && (long long)N * K <= kSmallMatrix)) {
         RowsParams p{x, w, out, M, N, K, 0, 0, act};
         if (M == 1) return launch_rows<1, 6>(p, stream);
         if (M == 2) return launch_rows<2, 5>(p, stream);
@@ -817,11 +781,24 @@ LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int 
         if (M <= 8) return launch_rows<8, 4>(p, stream);
         return launch_rows<16, 3>(p, stream);
     }
-    if (split) {
+    // The tile whose rounds over the SMs cover the least area; a smaller one brings more of x and w a
+    // multiply-add and pays its end more often, so it has to win by a few per cent.
+    const TileParams p{x, w, out, M, N, K, act};
+    const long long sms = num_sms();
+    if (K >= kSplitK) {
         // 64 columns a block take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so only where one round
         // does (500 x 3,072 x 2,048: 87.4 and 54.9)
         if ((long long)((M + kSM - 1) / kSM) * ((N + 63) / 64) <= sms) return launch_split<64>(p, stream);
         return launch_split<128>(p, stream);
+    }
+    const int bm[4] = {128, 128, 64, 64}, bn[4] = {256, 128, 128, 64};
+    const double cost[4] = {1.0, 1.0, 1.03, 1.08};
+    int best = 0;
+    double least = 0.0;
+    for (int c = 0; c < 4; ++c) {
+        const long long tiles = (long long)((M + bm[c] - 1) / bm[c]) * ((N + bn[c] - 1) / bn[c]);
+        const double area = (double)((tiles + sms - 1) / sms) * bm[c] * bn[c] * cost[c];
+        if (c == 0 || area < least) { least = area; best = c; }
     }
     switch (best) {
         case 0: return launch_tile<2, 4, 1, 32, 3>(p, stream);

@@ -1,4 +1,4 @@
-"""Products in true 32-bit at the edges of the three kernels' tiles, against 64-bit sums."""
+"""Products in true 32-bit at the edges of the two kernels' tiles, against 64-bit sums."""
 import pytest
 import torch
 
@@ -142,10 +142,3 @@ def test_every_part_of_a_split_counts(M, N, K):
     want = x.double() @ w.double().T
     # six of the nine products of parts: what is left out is below 2^-25; the sums of the six are cut to 2^-23, twice
     assert bool(((ops.linear(x, w).double() - want).abs() <= 2.0 ** -22 * want.abs()).all())
-
-
-@pytest.mark.parametrize("activation", [None, "silu"])
-@pytest.mark.parametrize("M, N, K", [(17, 4096, 480), (32, 2050, 256), (33, 1024, 508), (65, 130, 484), (100, 6, 508), (128, 2, 300)])
-def test_more_rows_than_a_block_takes(M, N, K, activation):
-    """Up to 128 rows a matrix may be shared out over blocks of sixteen rows, several turns each."""
-    _check(M, N, K, activation)
