@@ -593,7 +593,8 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float4 a = *reinterpret_cast<const float4*>(from + (((4 * j + i) ^ (r & 7)) << 4));
-                        low = min(low, min(min(twice_less_one(a.x), twice_less_one(a.y)), min(twice_less_one(a.z), twice_less_one(a.w))));
+                        low = __vimin3_u32(low, twice_less_one(a.x), twice_less_one(a.y));
+                        low = __vimin3_u32(low, twice_less_one(a.z), twice_less_one(a.w));
                         split3(a.x, a.y, h[2 * i], m[2 * i], l[2 * i]);
                         split3(a.z, a.w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1]);
                     }
