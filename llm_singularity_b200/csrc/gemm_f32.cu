@@ -1,5 +1,5 @@
-// out[M, N] = x[M, K] * w[N, K]^T of 32-bit values with 32-bit sums, no bit of an operand that could show in one dropped.  Three kernels, by the
-// number of rows and K; K a multiple of 4 and 16-byte aligned bases (anything else is csrc/gemm.cu's).  An activation of
+// out[M, N] = x[M, K] * w[N, K]^T of 32-bit values with 32-bit sums, no bit of an operand that could show in one dropped.
+// Three kernels, by the number of rows and K; K a multiple of 4 and 16-byte aligned bases (anything else is csrc/gemm.cu's).  An activation of
 // a gated product (w's rows alternate gate_i, up_i, out is [M, N / 2]) is applied where the sums meet.  The reference
 // hands such products to cublasSgemm (kernels/src/cublas_provider.cpp:36-51) and launches silu(g) * u by itself
 // (kernels/src/activations.cu:11-21).
@@ -7,8 +7,9 @@
 // * Up to 16 rows (a decode step) the product is weight traffic.  Weight rows are dealt out over one
 //   block per SM, sixteen at most at a time: four to a warp, each row's K in two parts.  A warp copies the weights it
 //   needs into a ring of shared memory itself (asynchronously, some 140 KB in flight an SM, the first of them asked for
-//   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three others of its part.  The sums of a
-//   group meet once, over lanes by halving exchanges and over the two parts in shared memory, in a fixed order.
+//   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three
+//   others of its part.  The sums of a group meet once, over lanes by halving exchanges and over the two parts in shared
+//   memory, in a fixed order.
 //   The four products of a layer at 1B sizes, 8 rows (243 MB): 71 us (3.4 TB/s); as 64 x 64 tiles, 56 of their 64 rows
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
 //   four times the exchanges at the end of a group: 89 us.)
@@ -30,10 +31,11 @@
 // * More rows, smaller K: multiply-adds on the 32-bit pipes.  Eight warps of 64 x 64 outputs (8 x 16 a thread), arranged
 //   as a tile of 128 x 256, 128 x 128, 64 x 128 or 64 x 64; in the smaller tiles the warps that are left share out each
 //   slice of K and their sums meet at the end, so that few tiles still give an SM eight busy warps.  Slices come by
-//   asynchronous copies, three to five in flight.  500 x 16,384 x 2,048: 764 us, 44 TFLOP/s of the 70 that a loop of
+//   asynchronous copies, three to five in flight.  2,048 x 8,192 x 256: 200 us, 43 TFLOP/s of the 70 that a loop of
 //   nothing but multiply-adds reaches here.
 //
-// A row's sum is taken in an order that K and the kernel fix, the same from run to run.
+// A row's sum is taken in an order that K and the kernel fix, the same from run to run; which kernel, and so the last digits,
+// depends on the number of rows beside it.
 #include "common.cuh"
 #include "gate_act.cuh"
 
@@ -54,8 +56,12 @@ constexpr int kRowThreads = 256;
 constexpr int kRowsMax = 16;                   // rows of x a block takes
 constexpr int kRB = 16;                        // most weight rows of a group: four for each of four warps, twice (two parts of K)
 constexpr int kRW = kRB / 4;
-constexpr int kRowsSmall = 128;                // rows that still go this way, sixteen to a block, ...
-constexpr long long kSmallMatrix = 1 << 18;    // ... where the matrix is so small that a tile's latency shows
+// More rows that still go this way, sixteen to a block, where the matrix is so small that a tile's latency shows: up to some
+// 48 of them are faster so (us, this way and as tiles of 64 x 64: 17 x 640 x 128 4.9 and 5.7, 48 x 128 x 320 7.5 and 11.3), 64 to
+// 128 only along a longer K (64 x 128 x 320 9.7 and 11.5, 128 x 512 x 128 17.0 and 6.1), but the sums are
+// the closer ones throughout: K = 128 7.4e-8 of the norm and 9.7e-8, K = 320 8.2e-8 and 1.3e-7.
+constexpr int kRowsSmall = 128;
+constexpr long long kSmallMatrix = 1 << 18;
 constexpr int kKS = 512;                       // K of a stage: two steps of 128 for each part
 
 struct RowsParams {
@@ -782,8 +788,13 @@ LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int 
         if (M <= 8) return launch_rows<8, 4>(p, stream);
         return launch_rows<16, 3>(p, stream);
     }
-    // The tile whose rounds over the SMs cover the least area; a smaller one brings more of x and w a
-    // multiply-add and pays its end more often, so it has to win by a few per cent.
+    // The tile whose rounds over the SMs cover the least area; a smaller one brings more of x and w a multiply-add and pays
+    // its end more often, so it has to win by a few per cent.  At the K that is left for them (below 512) each is the
+    // fastest somewhere (128 x 256, 128 x 128, 64 x 128, 64 x 64, us: 1,000 x 8,192 x 256 108 / 114 / 109 / 130; 2,048 x 8,192 x 256
+    // 215 / 200 / 218 / 259; 200 x 4,096 x 128 30 / 16 / 9.6 / 11.7; 500 x 512 x 128 29 / 16 / 9.4 / 6.2), and this count finds it within
+    // 10 % on most of 120 shapes; along the shortest K it picks too small a tile (500 x 20,000 x 20: 65 us, 128 x 128 29; 2,048 x
+    // 2,048 x 64: 28, 128 x 256 18), whose sums are the closer ones: more warps share K out (K = 320, from the smallest tile to the
+    // largest: 1.3, 1.7, 2.4 and 3.2e-7 of the norm).
     const TileParams p{x, w, out, M, N, K, act};
     const long long sms = num_sms();
     if (K >= kSplitK) {

@@ -1,4 +1,4 @@
-"""Products in true 32-bit at the edges of the two kernels' tiles, against 64-bit sums."""
+"""Products in true 32-bit at the edges of the three kernels' tiles, against 64-bit sums."""
 import pytest
 import torch
 
