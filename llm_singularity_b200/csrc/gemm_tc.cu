@@ -162,11 +162,12 @@ struct GemmParams {
     // earlier in the stream, so a block reads it only after the wait on that kernel.
     const int* tile_group;
     int group_rows;
-    // persistent form: columns of a tile (a multiple of 16 up to 256) and stages of the ring
-    int bn, stages;
     // Swapped: P stacks the groups' matrices and tile_group[j0 / BN] names the group of a BN-row tile of Q.
     int group_swap;
 };
+// (Kernel parameters are copied at every launch: eight bytes more here, the two numbers that only the persistent kernels take,
+// made a call of `linear` 0.3 us longer on the host, 9.4 -> 9.7.)
+static_assert(sizeof(GemmParams) == 96, "what every launch copies");
 
 template <int BN>
 __device__ __forceinline__ void load_acc(uint32_t tmem_base, int q, int c0, bool have, uint32_t (&r)[32]) {
@@ -688,18 +689,18 @@ static constexpr size_t persistent_smem(int bn, int stages) {
 // pass's width): a warp that is a pass behind would find its rows overwritten otherwise.
 template <bool GATED>
 __device__ __forceinline__ void drain_staged(const GemmParams& prm, unsigned char* epi, uint32_t tmem_acc, int q, int lane,
-                                             int i0, int j0) {
+                                             int i0, int j0, int bn) {
     constexpr int PASS = GATED ? 128 : 64;
     int h = 0;
 #pragma unroll 1
-    for (; h + PASS <= prm.bn; h += PASS) epilogue_staged<PASS, GATED>(prm, epi, tmem_acc + h, q, lane, i0, j0 + h);
-    if (GATED && (prm.bn & 64)) epilogue_staged<64, GATED>(prm, epi + q * 2048, tmem_acc + h, q, lane, i0, j0 + h);
+    for (; h + PASS <= bn; h += PASS) epilogue_staged<PASS, GATED>(prm, epi, tmem_acc + h, q, lane, i0, j0 + h);
+    if (GATED && (bn & 64)) epilogue_staged<64, GATED>(prm, epi + q * 2048, tmem_acc + h, q, lane, i0, j0 + h);
 }
 
+// BN: columns of a tile (a multiple of 16 up to 256); STAGES: of the ring
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
-                          const GemmParams prm, int tiles_m, int tiles_n) {
-    const int BN = prm.bn, STAGES = prm.stages;
+                          const GemmParams prm, int tiles_m, int tiles_n, const int BN, const int STAGES) {
     const uint32_t kPBytes = kBM * kBK * 2, kStageBytes = kPBytes + (uint32_t)BN * (kBK * 2);
     // two accumulators, each a power of two of TMEM columns
     const uint32_t acc_cols = BN <= 16 ? 16 : BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
@@ -844,8 +845,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_p, const __gri
             if (!ok) break;
             const uint32_t tmem_acc = tmem_base + (uint32_t)a * acc_cols;
             if (aligned && j0 + BN <= prm.rows_q) {
-                if (prm.swiglu == 1) drain_staged<true>(prm, epi, tmem_acc, q, lane, i0, j0);
-                else drain_staged<false>(prm, epi, tmem_acc, q, lane, i0, j0);
+                if (prm.swiglu == 1) drain_staged<true>(prm, epi, tmem_acc, q, lane, i0, j0, BN);
+                else drain_staged<false>(prm, epi, tmem_acc, q, lane, i0, j0, BN);
             } else if (aligned32 && j0 + BN <= prm.rows_q) {
 #pragma unroll 1
                 for (int h = 0; h < BN; h += 32)
@@ -928,8 +929,7 @@ static constexpr size_t pair_smem(int bn, int stages) {
 
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
-                    const GemmParams prm, int tiles_m, int tiles_n) {
-    const int BN = prm.bn, STAGES = prm.stages;
+                    const GemmParams prm, int tiles_m, int tiles_n, const int BN, const int STAGES) {
     const uint32_t kPBytes = kBM * kBK * 2, kStageBytes = kPBytes + (uint32_t)(BN / 2) * (kBK * 2);
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);   // (the same offset in both blocks)
@@ -1054,8 +1054,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             if (i0 >= prm.rows_p) {
                 // (the second block's rows lie past the matrix)
             } else if (aligned && j0 + BN <= prm.rows_q) {
-                if (prm.swiglu == 1) drain_staged<true>(prm, epi, tmem_acc, q, lane, i0, j0);
-                else drain_staged<false>(prm, epi, tmem_acc, q, lane, i0, j0);
+                if (prm.swiglu == 1) drain_staged<true>(prm, epi, tmem_acc, q, lane, i0, j0, BN);
+                else drain_staged<false>(prm, epi, tmem_acc, q, lane, i0, j0, BN);
             } else if (aligned32 && j0 + BN <= prm.rows_q) {
 #pragma unroll 1
                 for (int h = 0; h < BN; h += 32)
@@ -1129,7 +1129,7 @@ static int launch(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams
 }
 
 // bn columns a tile; as deep a ring as fits
-static int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, GemmParams prm, int bn, int tiles_m,
+static int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& prm, int bn, int tiles_m,
                              int tiles_n, cudaStream_t stream) {
     static int configured = -1;
     static int sms = 0;
@@ -1141,16 +1141,15 @@ static int launch_persistent(const CUtensorMap& mp, const CUtensorMap& mq, GemmP
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
     if (configured) return configured;
-    prm.bn = bn;
-    prm.stages = kMaxStages;
-    while (persistent_smem(bn, prm.stages) > kPersistentSmem) --prm.stages;
+    int stages = kMaxStages;
+    while (persistent_smem(bn, stages) > kPersistentSmem) --stages;
     const int tiles = tiles_m * tiles_n;
     const int blocks = tiles < sms ? tiles : sms;
-    return lsb_launch(gemm_tc_persistent_kernel, dim3(blocks), dim3(kGemmThreads), persistent_smem(bn, prm.stages), stream, 1,
-                      mp, mq, prm, tiles_m, tiles_n);
+    return lsb_launch(gemm_tc_persistent_kernel, dim3(blocks), dim3(kGemmThreads), persistent_smem(bn, stages), stream, 1,
+                      mp, mq, prm, tiles_m, tiles_n, bn, stages);
 }
 
-static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, GemmParams prm, int bn, int tiles_m, int tiles_n,
+static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& prm, int bn, int tiles_m, int tiles_n,
                        cudaStream_t stream) {
     static int configured = -1;
     static int sms = 0;
@@ -1161,15 +1160,14 @@ static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, GemmParams 
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
     if (configured) return configured;
-    prm.bn = bn;
-    prm.stages = kMaxStages;
-    while (pair_smem(bn, prm.stages) > kPersistentSmem) --prm.stages;
+    int stages = kMaxStages;
+    while (pair_smem(bn, stages) > kPersistentSmem) --stages;
     const int tiles = tiles_m * tiles_n;
     const int pairs = tiles < sms / 2 ? tiles : sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = pair_smem(bn, prm.stages);
+    cfg.dynamicSmemBytes = pair_smem(bn, stages);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
@@ -1183,7 +1181,7 @@ static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, GemmParams 
     attr[n++].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel, mp, mq, prm, tiles_m, tiles_n);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel, mp, mq, prm, tiles_m, tiles_n, bn, stages);
 }
 
 // What happens when a wait runs out, shown without a fault: one block, a barrier that nothing
