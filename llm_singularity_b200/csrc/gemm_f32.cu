@@ -776,6 +776,12 @@ LSB_API int lsb_gemm_f32_supported(const void* x, const void* w, int M, int N, i
     return M > 0 && N > 0 && K > 0 && K % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0 && M <= 32 * 65535;
 }
 
+// Columns of a split product's blocks.  64 take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so only where
+// one round does (500 x 3,072 x 2,048: 87.4 and 54.9).
+LSB_API int lsb_gemm_f32_split_columns(int M, int N) {
+    return (long long)((M + kSM - 1) / kSM) * ((N + 63) / 64) <= num_sms() ? 64 : 128;
+}
+
 // act: 0, or the activation of a gated product (1 silu, 2 gelu in its tanh form, 3 none), N even then.
 LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K, int act, cudaStream_t stream) {
     if (!lsb_gemm_f32_supported(x, w, M, N, K) || ((uintptr_t)out % 16)) return (int)cudaErrorInvalidValue;
@@ -798,10 +804,7 @@ LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int 
     const TileParams p{x, w, out, M, N, K, act};
     const long long sms = num_sms();
     if (K >= kSplitK) {
-        // 64 columns a block take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so only where one round
-        // does (500 x 3,072 x 2,048: 87.4 and 54.9)
-        if ((long long)((M + kSM - 1) / kSM) * ((N + 63) / 64) <= sms) return launch_split<64>(p, stream);
-        return launch_split<128>(p, stream);
+        return lsb_gemm_f32_split_columns(M, N) == 64 ? launch_split<64>(p, stream) : launch_split<128>(p, stream);
     }
     const int bm[4] = {128, 128, 64, 64}, bn[4] = {256, 128, 128, 64};
     const double cost[4] = {1.0, 1.0, 1.03, 1.08};

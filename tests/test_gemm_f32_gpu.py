@@ -52,6 +52,13 @@ def test_split_products(M, N, K, activation):
     _check(M, N, K, activation)
 
 
+def test_split_products_are_made_in_both_widths():
+    """The shapes above take blocks of 64 columns and of 128 (on the 148 SMs of a B200)."""
+    from llm_singularity_b200 import kernels as ops
+    columns = ops._lib("gemm_f32").lsb_gemm_f32_split_columns
+    assert [columns(M, N) for M, N in ((17, 64), (129, 66), (300, 3002), (500, 2048), (257, 9000), (200, 20002))] == [64] * 4 + [128] * 2
+
+
 @pytest.mark.parametrize("N", [700, 20000])
 def test_split_products_out_of_range(N):
     """Values that the parts cannot hold: infinities, NaN, rows near and below the smallest normal number, the largest numbers."""
