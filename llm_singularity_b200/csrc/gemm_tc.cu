@@ -241,7 +241,9 @@ __device__ __forceinline__ void store_chunk(const GemmParams& prm, uint32_t (&r)
     const int ncols = min(n, prm.rows_q - j);              // may be <= 0
     if (prm.swiglu == 2) {
         // rows alternate gate, up: even lanes hold gates, their odd neighbours the matching ups
-        for (int x = 0; x < n; ++x) {
+#pragma unroll
+        for (int x = 0; x < 32; ++x) {
+            if (x >= n) continue;                              // (every lane alike)
             const float v = __uint_as_float(r[x]);
             const float other = __shfl_xor_sync(0xffffffffu, v, 1);
             if (!(lane & 1) && row_ok && x < ncols) {
@@ -271,7 +273,9 @@ __device__ __forceinline__ void store_chunk(const GemmParams& prm, uint32_t (&r)
                 *reinterpret_cast<uint4*>(dst + x / 2) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         } else {
-            for (int x = 0; x + 1 < ncols; x += 2) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 2) {
+                if (x + 1 >= ncols) break;
                 const float v = silu_mul(__uint_as_float(r[x]), __uint_as_float(r[x + 1]));
                 if (prm.out_f32) put<float>(prm.out, o + (x >> 1) * prm.ldc_j, v);
                 else put<bf16>(prm.out, o + (x >> 1) * prm.ldc_j, v);
@@ -288,7 +292,11 @@ __device__ __forceinline__ void store_chunk(const GemmParams& prm, uint32_t (&r)
             for (int x = 0; x < 32; x += 4)
                 *reinterpret_cast<uint4*>(dst + x) = make_uint4(r[x], r[x + 1], r[x + 2], r[x + 3]);
         } else {
-            for (int x = 0; x < ncols; ++x) dst[x * prm.ldc_j] = __uint_as_float(r[x]);
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+                if (x < ncols) *dst = __uint_as_float(r[x]);
+                dst += prm.ldc_j;
+            }
         }
     } else {
         bf16* dst = reinterpret_cast<bf16*>(prm.out) + o;
@@ -304,7 +312,11 @@ __device__ __forceinline__ void store_chunk(const GemmParams& prm, uint32_t (&r)
                 *reinterpret_cast<uint4*>(dst + x) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         } else {
-            for (int x = 0; x < ncols; ++x) dst[x * prm.ldc_j] = __float2bfloat16_rn(__uint_as_float(r[x]));
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+                if (x < ncols) *dst = __float2bfloat16_rn(__uint_as_float(r[x]));
+                dst += prm.ldc_j;
+            }
         }
     }
 }
@@ -456,7 +468,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     using L = SmemLayout<BN, STAGES>;
     constexpr uint32_t kTmemCols = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
     constexpr int kPartSwizzle = BN / 4 >= 8 ? 7 : BN / 4 - 1;     // see the partial tile below
-    static_assert((size_t)kBM * BN * 4 <= (size_t)STAGES * L::kStageBytes, "the partial tile lives in the stage buffers");
+    static_assert((size_t)kBM * BN * (BN <= 128 ? 6 : 4) <= (size_t)STAGES * L::kStageBytes,
+                  "the partial tile lives in the stage buffers, with the sums as they leave (weights on its rows) behind it");
     extern __shared__ unsigned char smem_raw[];
     // stage buffers need 1024-byte alignment (swizzle atom); the dynamic window is only 16-aligned
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -595,7 +608,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t r[32];
                 load_acc<BN>(tmem_base, q, c0, nkb > 0, r);
-                const int n = BN - c0 >= 32 ? 32 : 16;
+                constexpr int n = BN >= 32 ? 32 : 16;          // (known here: an index that is not puts r in local memory)
+#pragma unroll
                 for (int x = 0; x < n; x += 4)
                     part[((c0 + x) / 4) ^ (il & kPartSwizzle)] = make_uint4(r[x], r[x + 1], r[x + 2], r[x + 3]);
             }
@@ -611,8 +625,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             const uint4* part = reinterpret_cast<const uint4*>(stages);
             const int t = (warp - 2) * 32 + lane;
             const bool rows_whole = prm.ldc_j == 1 && (prm.ldc_i & 3) == 0 && (((uintptr_t)prm.out) & 15) == 0;
-            for (int g4 = (int)rank * 128 + t; g4 < kBM * BN / 4; g4 += prm.splits * 128) {
-                const int row = g4 / (BN / 4), c4 = g4 % (BN / 4);
+            // A block's share is every splits-th group of eight rows.  Weights on the tile's rows, bfloat16: eight rows of a
+            // column are 16 bytes of the output, so the sums change places in shared memory behind the partial tile and
+            // every column of a group leaves in one store (64 rows times 5,120 x 3,072: 12.9 us with stores of single values, 2 bytes on a
+            // line each, 11.4 so).  A lane a row in the reads from the peers, so that stores are runs by themselves, is slower
+            // than either (64 x 3,072 x 2,048: 12.5 us, 8.5, 8.0): distributed shared memory wants neighbouring lanes at neighbouring places.
+            const bool turned = prm.ldc_i == 1 && prm.ldc_j != 1 && !prm.out_f32 && (prm.rows_p & 7) == 0 && (prm.ldc_j & 7) == 0 &&
+                                (((uintptr_t)prm.out) & 15) == 0;
+            bf16* turn = reinterpret_cast<bf16*>(stages + (size_t)kBM * BN * 4);           // [group][4][BN / 4][8 rows]
+            const int groups = (kBM / 8 - (int)rank + prm.splits - 1) / prm.splits;
+            for (int e = t; e < groups * 2 * BN; e += 128) {
+                const int group = (int)rank + e / (2 * BN) * prm.splits;
+                const int row = group * 8 + e % (2 * BN) / (BN / 4), c4 = e % (BN / 4);
                 const uint4* src = part + (size_t)row * (BN / 4) + (c4 ^ (row & kPartSwizzle));
                 float4 v[8];                                  // all peers' loads in flight at once
 #pragma unroll
@@ -627,7 +651,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                     acc.z = plain_act(acc.z, prm.plain); acc.w = plain_act(acc.w, prm.plain);
                 }
                 const int i = i0 + row, j = j0 + c4 * 4;
-                if (i < prm.rows_p) {
+                if (turned) {
+                    const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+                        turn[(group * BN + x * (BN / 4) + c4) * 8 + (row & 7)] = __float2bfloat16_rn(vals[x]);
+                } else if (i < prm.rows_p) {
                     const long long o0 = (long long)i * prm.ldc_i + (long long)j * prm.ldc_j;
                     if (rows_whole && j + 3 < prm.rows_q) {
                         if (prm.out_f32) {
@@ -647,6 +676,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                             else put<bf16>(prm.out, o, vals[x]);
                         }
                     }
+                }
+            }
+            if (turned) {
+                asm volatile("bar.sync 2, 128;" ::: "memory");                      // the four epilogue warps
+                for (int e = t; e < groups * BN; e += 128) {
+                    const int group = (int)rank + e / BN * prm.splits, jj = e % BN;
+                    const int i = i0 + group * 8, j = j0 + jj % (BN / 4) * 4 + jj / (BN / 4);
+                    if (i < prm.rows_p && j < prm.rows_q)
+                        *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(prm.out) + i + (long long)j * prm.ldc_j) =
+                            *reinterpret_cast<const uint4*>(turn + (group * BN + jj) * 8);
                 }
             }
         }
@@ -1263,7 +1302,11 @@ static void plan(int M, int N, int K, int swiglu, int* swap, int* bn, int* split
         const int tiles = (N + kBM - 1) / kBM;
         int s = 1;
         if (tiles < most && !swiglu) {           // too few slabs to fill the SMs: split K
-            s = (sms + tiles - 1) / tiles;
+            // as many ways as are sure to fit at once with two blocks an SM (clusters don't straddle the chip's groups of SMs:
+            // 256 blocks do in eights, 288 in sixes don't).  64 rows, us, with as many blocks as SMs / so: 24 slabs of K 2,048
+            // 8.0 / 7.2, 32 of 4,096 12.1 / 11.0, 40 of 3,072 11.4 / 10.7, 32 of 14,336 27.9 / 25.7; 48 of 4,096 with four, five, six
+            // ways 14.4 / 14.0 / 20.7.
+            s = sms * 7 / 4 / tiles;
             if (s > 8) s = 8;
             if (s > num_kb / 4) s = num_kb / 4 > 0 ? num_kb / 4 : 1;   // at least 4 K blocks each
             if (s < 1) s = 1;
@@ -1367,7 +1410,9 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
         grid = dim3((M + kBM - 1) / kBM, (N + bn - 1) / bn, 1);
     }
     // Blocks of a split product are co-scheduled as clusters: four stages keep their shared memory
-    // small enough for two or three blocks per SM, so that every cluster finds room at once.
+    // small enough for two or three blocks per SM, so that every cluster finds room at once.  (Three stages of 128 columns:
+    // with four a block had the SM to itself, and the clusters took two rounds: 100 rows times 3,072 x 2,048 18.5 us then,
+    // 10.0 now, 4,096 x 14,336 48.0 and 28.2.)
     // Unsplit products run one block per SM and want the deeper ring to keep HBM busy.
     if (!swap && splits > 1) {
         grid.z = splits;
@@ -1384,7 +1429,7 @@ LSB_API int lsb_gemm_tc(const void* x, const void* w, void* out, int out_f32, in
             case 16: rc = launch<16, 4>(mp, mq, prm, grid, stream); break;
             case 32: rc = launch<32, 4>(mp, mq, prm, grid, stream); break;
             case 64: rc = launch<64, 4>(mp, mq, prm, grid, stream); break;
-            case 128: rc = launch<128, 4>(mp, mq, prm, grid, stream); break;
+            case 128: rc = launch<128, 3>(mp, mq, prm, grid, stream); break;
             default: return (int)cudaErrorInvalidValue;
         }
     } else if (swap && !swiglu && (int)grid.x >= 2 * sms) {
