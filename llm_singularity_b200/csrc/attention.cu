@@ -25,12 +25,15 @@
 //   walking all of its keys took 1,548 us.
 // * Portions are arithmetic: 64 rows (16 queries of 4 heads that share their keys) against a tile, 4 rows by 2 or 4
 //   keys a thread for the scores and the same 4 rows for the weighted sum, so that a row's maximum, its sum and its
-//   probabilities stay within half a warp; two multiply-adds to an instruction.  500 tokens, the same heads:
-//   88 us (1.0 GFLOP); a warp for each (row, head) took 650 us.
+//   probabilities stay within half a warp; two multiply-adds to an instruction.  The last rows of a portion see the most
+//   keys, and few portions leave SMs idle: the tiles of a block's keys are dealt out over a cluster, whose sums meet
+//   as those of single tokens do.  500 tokens, the same heads: 85 us (1.0 GFLOP), 91 with a block to all of its
+//   keys; 120 tokens after 300 31 and 68, 40 after 300 20 and 50; a warp for each (row, head) took 650 us for the 500.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
 #include <float.h>
+#include <math.h>
 
 namespace cg = cooperative_groups;
 
@@ -58,6 +61,7 @@ struct AttnParams {
     const float* slopes;
     int heads;                                  // query heads of a block
     int head_blocks;                            // blocks of a kv head's group
+    int splits;                                 // (portions) blocks that share out a block's keys
 };
 
 typedef unsigned long long pair32;              // two 32-bit values
@@ -303,16 +307,18 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
     constexpr int CPT = HDC / 64;               // groups of four columns of a thread's sums
     extern __shared__ __align__(16) float sm[];
     __shared__ long long off[2][KT];
+    cg::cluster_group cluster = cg::this_cluster();
     lsb_pdl_launch_dependents();
     lsb_pdl_wait();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, r = blockIdx.z;
+    const int splits = p.splits, split = (int)blockIdx.x % splits;
     const int g = blockIdx.y / p.head_blocks, group = p.nh / p.nkv;
     const int h0 = g * group + (int)(blockIdx.y % p.head_blocks) * p.heads;
     const int H = min(p.heads, (g + 1) * group - h0);
     const int qs0 = p.q_start[r], q_len = p.q_start[r + 1] - qs0;
     const int queries = kRows / p.heads;
-    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * queries;          // the longest rows first
-    if (q_len <= 1 || i0 >= q_len) return;
+    const int i0 = ((int)gridDim.x - 1 - (int)blockIdx.x) / splits * queries;          // the longest rows first
+    if (q_len <= 1 || i0 >= q_len) return;                     // (all blocks of the cluster alike)
     const int hd = p.hd, ldk = hd + 4, ldp = KT + 4;
     float* qs = sm;
     float* ks = qs + kRows * ldk;
@@ -320,7 +326,8 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
     float* ps = vs + KT * hd;
     const int pos0 = p.kv_len[r] - q_len + i0;                 // of the block's first query
     const int pos_last = min(pos0 + queries, p.kv_len[r]) - 1;
-    const int lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+    // this block's tiles: every splits-th
+    const int lo = ((p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0) + split * KT, stride = splits * KT;
     const int* table = p.block_table + (size_t)p.table_rows[r] * p.table_stride;
 
     // row x: query i0 + x / heads, head h0 + x % heads (rows beyond the portion or the group stay zero)
@@ -331,15 +338,13 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
             : 0.f;
     }
     if (tid < KT) off[0][tid] = lo + tid <= pos_last ? key_offset(p, table, g, lo + tid) : -1;
-    int pos[4], row_lo[4];
-    float slope[4], m[4], l[4];
+    int pos[4];
+    float m[4], l[4];
     pair32 acc[4][2 * CPT];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int x = ty * 4 + i;
         pos[i] = min(pos0 + x / p.heads, pos_last);
-        row_lo[i] = p.window > 0 ? pos[i] - p.window + 1 : 0;
-        slope[i] = p.slopes && x % p.heads < H ? p.slopes[h0 + x % p.heads] : 0.f;
         m[i] = -FLT_MAX;
         l[i] = 0.f;
 #pragma unroll
@@ -348,9 +353,9 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
     __syncthreads();
     Tile<T, KT, HDC> tile;
     tile.fetch(p, off[0], tid);
-    for (int base = lo, turn = 0; base <= pos_last; base += KT, turn ^= 1) {
+    for (int base = lo, turn = 0; base <= pos_last; base += stride, turn ^= 1) {
         const bool finite = tile.park(p, ks, vs, ldk, tid);
-        const int next = base + KT;
+        const int next = base + stride;
         if (tid < KT) off[turn ^ 1][tid] = next + tid <= pos_last ? key_offset(p, table, g, next + tid) : -1;
         const bool by_row = __syncthreads_or(!finite);
         if (next <= pos_last) tile.fetch(p, off[turn ^ 1], tid);
@@ -380,13 +385,16 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
         for (int i = 0; i < 4; ++i) {
             float s[KPT], mx = m[i];
             bool seen[KPT];
+            // (worked out again for every tile: registers are short)
+            const int row_lo = p.window > 0 ? pos[i] - p.window + 1 : 0, head = p.slopes ? (ty * 4 + i) % p.heads : H;
+            const float slope = head < H ? p.slopes[h0 + head] : 0.f;
 #pragma unroll
             for (int j = 0; j < KPT; ++j) {
                 const int key = base + tx + 16 * j;
                 float u, v;
                 apart(s2[i][j], u, v);
-                seen[j] = key <= pos[i] && key >= row_lo[i] && off[turn][tx + 16 * j] >= 0;
-                s[j] = seen[j] ? modified(p, u + v, slope[i], pos[i] - key) : -FLT_MAX;
+                seen[j] = key <= pos[i] && key >= row_lo && off[turn][tx + 16 * j] >= 0;
+                s[j] = seen[j] ? modified(p, u + v, slope, pos[i] - key) : -FLT_MAX;
                 mx = fmaxf(mx, s[j]);
             }
 #pragma unroll
@@ -415,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
                 if (off[turn][k] < 0) continue;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    if (base + k > pos[i] || base + k < row_lo[i]) continue;
+                    if (base + k > pos[i] || (p.window > 0 && base + k < pos[i] - p.window + 1)) continue;
                     const pair32 we = twice(ps[(ty * 4 + i) * ldp + k]);
 #pragma unroll
                     for (int c = 0; c < CPT; ++c) {
@@ -453,6 +461,45 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
         }
         __syncthreads();
     }
+    if (splits > 1) {
+        // the blocks' sums meet: each brings its share of the rows together, blocks in order
+        float* os = qs;                                        // [kRows][ldk] (the queries have been used)
+        float* ml = ps;                                        // [kRows] (maximum, sum)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = ty * 4 + i;
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                const int d = tx * 4 + 64 * c;
+                if (d < hd) *reinterpret_cast<ulonglong2*>(os + x * ldk + d) = make_ulonglong2(acc[i][2 * c], acc[i][2 * c + 1]);
+            }
+            if (tx == 0) { ml[2 * x] = m[i]; ml[2 * x + 1] = l[i]; }
+        }
+        cluster.sync();
+        const int rows = (kRows + splits - 1) / splits, x0 = split * rows, x1 = min(kRows, x0 + rows), per = hd >> 2;
+        for (int e = tid; e < (x1 - x0) * per; e += kThreads) {
+            const int x = x0 + e / per, d = e % per * 4, qi = i0 + x / p.heads, h = x % p.heads;
+            if (qi >= q_len || h >= H || x / p.heads >= queries) continue;
+            float top = -FLT_MAX, sum = 0.f, out[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int k = 0; k < splits; ++k) top = fmaxf(top, *cluster.map_shared_rank(ml + 2 * x, k));
+            for (int k = 0; k < splits; ++k) {
+                const float2 of = *reinterpret_cast<const float2*>(cluster.map_shared_rank(ml + 2 * x, k));
+                const float4 o = *reinterpret_cast<const float4*>(cluster.map_shared_rank(os + x * ldk + d, k));
+                const float f = expf(of.x - top);
+                sum += f * of.y;
+                out[0] += f * o.x;
+                out[1] += f * o.y;
+                out[2] += f * o.z;
+                out[3] += f * o.w;
+            }
+            const float inv = sum > 0.f ? 1.f / sum : 0.f;
+            T* to = reinterpret_cast<T*>(p.out) + (size_t)(qs0 + qi) * p.nh * hd + (size_t)(h0 + h) * hd + d;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) to[k] = lsb_from_float<T>(out[k] * inv);
+        }
+        cluster.sync();                                        // (a peer may still read this block's sums)
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int x = ty * 4 + i, qi = i0 + x / p.heads, h = x % p.heads;
@@ -486,6 +533,49 @@ static int num_sms() {
     return cached[dev];
 }
 
+// clusters of consecutive blocks along x
+static int launch_clusters(void (*kernel)(AttnParams), dim3 grid, size_t smem, unsigned cluster, const AttnParams& p, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (lsb_pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
+// Blocks that share out the keys of a portion's rows.  Blocks are taken to run in rounds of `room`, the longest first, the
+// lengths falling evenly from the longest to the shortest (tiles of keys); meeting costs a block as much as 0.3 to 0.6 of a
+// tile.  (32 / 8 heads of 64 in 32-bit, us with 1 / 2 / 4 / 6 blocks: 500 tokens 91 / 85 / 91 / 120, 240 45 / 31 / 36 / 52, 120 after
+// 300 68 / 51 / 31 / 43, 40 after 300 50 / 31 / 26 / 19, 40 12 / 14 / 16 / 19; 16 / 8 of 256 in bfloat16, 300 after 2,000 812 / 793 / 636 / 597.)
+static int portion_splits(long long blocks, long long room, int longest, int shortest) {
+    int best = 1;
+    double least = 0.0;
+    for (int s = 1; s <= kMaxSplits && s <= longest; ++s) {
+        const long long n = blocks * s, rounds = (n + room - 1) / room;
+        if (s > 1 && rounds > 16) break;                       // (the SMs are busy without)
+        double cost = 0.0;
+        for (long long r = 0; r < rounds && r < 64; ++r) {
+            const double tiles = longest - (double)(longest - shortest) * (double)(r * room) / (double)n;
+            cost += ceil(tiles / s) + (s > 1 ? 0.6 : 0.3);
+        }
+        if (rounds > 64) cost *= (double)rounds / 64.0;
+        if (s == 1 || cost < least) { least = cost; best = s; }
+    }
+    return best;
+}
+
 template <typename T, int KT, int HDC>
 static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int max_keys, cudaStream_t stream) {
     static int configured = -1;
@@ -509,33 +599,25 @@ static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int
         if (max_keys > 0 && splits > (max_keys + KT - 1) / KT) splits = (max_keys + KT - 1) / KT;
         splits = splits < 1 ? 1 : splits > kMaxSplits ? kMaxSplits : splits;
         if ((long long)p.nkv * s.head_blocks > 65535) return (int)cudaErrorInvalidValue;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)splits, p.nkv * s.head_blocks, n_requests);
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = single_smem<KT>(p.hd, s.heads);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        int n = 0;
-        if (lsb_pdl_enabled()) {
-            attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[n++].val.programmaticStreamSerializationAllowed = 1;
-        }
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = (unsigned)splits;
-        attr[n].val.clusterDim.y = 1;
-        attr[n++].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = n;
-        const int rc = (int)cudaLaunchKernelEx(&cfg, attention_single_kernel<T, KT, HDC>, s);
+        const int rc = launch_clusters(attention_single_kernel<T, KT, HDC>, dim3((unsigned)splits, p.nkv * s.head_blocks, n_requests),
+                                       single_smem<KT>(p.hd, s.heads), (unsigned)splits, s, stream);
         if (rc) return rc;
     }
     if (max_q_len > 1) {
         p.heads = group < kPortionHeads ? group : kPortionHeads;
         p.head_blocks = (group + p.heads - 1) / p.heads;
-        const int queries = kRows / p.heads;
         if ((long long)p.nkv * p.head_blocks > 65535) return (int)cudaErrorInvalidValue;
-        const dim3 grid((max_q_len + queries - 1) / queries, p.nkv * p.head_blocks, n_requests);
-        return lsb_launch(attention_portion_kernel<T, KT, HDC>, grid, dim3(kThreads), portion_smem<KT>(p.hd), stream, 1, p);
+        const int queries = kRows / p.heads;
+        const long long tiles = (max_q_len + queries - 1) / queries, blocks = tiles * p.nkv * p.head_blocks;
+        // (where the contexts are not known, they are taken for the portions alone)
+        const int keys = max_keys > max_q_len ? max_keys : max_q_len;
+        p.splits = portion_splits(blocks * (n_requests > n_single ? n_requests - n_single : 1), (HDC <= 128 ? 2 : 1) * num_sms(), (keys + KT - 1) / KT,
+                                  (keys - max_q_len) / KT + 1);
+        if (tiles * p.splits > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+        const dim3 grid((unsigned)(tiles * p.splits), p.nkv * p.head_blocks, n_requests);
+        // (a launch in clusters of one was 8 % slower)
+        if (p.splits == 1) return lsb_launch(attention_portion_kernel<T, KT, HDC>, grid, dim3(kThreads), portion_smem<KT>(p.hd), stream, 1, p);
+        return launch_clusters(attention_portion_kernel<T, KT, HDC>, grid, portion_smem<KT>(p.hd), p.splits, p, stream);
     }
     return 0;
 }
@@ -552,7 +634,7 @@ LSB_API int lsb_paged_attention_generic(
     if (hd % 16 || hd <= 0 || hd > kMaxHeadDim || nkv <= 0 || nh % nkv) return (int)cudaErrorInvalidValue;
     if (n_requests > 65535 || nh > 65535) return (int)cudaErrorInvalidValue;
     const AttnParams p{qkv, qkv_stride, k_pages, v_pages, q_start, kv_len, table_rows, block_table, table_stride, out,
-                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0};
+                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0, 1};
     LSB_DISPATCH_DTYPE(dtype, {
         if (hd <= 64) return launch<T, 64, 64>(p, n_requests, max_q_len, n_single, max_keys, stream);
         if (hd <= 128) return launch<T, 32, 128>(p, n_requests, max_q_len, n_single, max_keys, stream);
