@@ -19,10 +19,11 @@
 //   are not.  Blocks of 128 x 128 outputs (x 64 where those fit the SMs at once) take x and w as they are by
 //   TMA; sixteen warps, two groups by turns, split a stage of 32 along K, x's parts into tensor memory, w's into
 //   shared memory.  The tensor core cuts its sums rather than rounding them, so the leading products stay there for
-//   128 of K only and are then added up in registers; the five small ones have their own sums, 2^-8 as large.
-//   Error against 64 bits, 500 x 2,048 x 2,048: 1.5e-7 of the norm, 4.1e-7 by multiply-adds; K = 512 1.3e-7 and 1.6e-7;
-//   K = 8,192 2.2e-7 and 8.1e-7 (at K of 100 and 256 the two are alike, which is where the line comes from).  The four
-//   products of a layer at 1B sizes, 500 rows (61 GFLOP): 1,491 -> 470 us.  What bounds it is the traffic of
+//   128 of K only and are then added up in registers; the five small ones have their own sums, 2^-8 as large.  Where tiles
+//   are too few for the SMs, or leave a last round of them half empty, K is shared out over a cluster, whose sums meet in order.
+//   Error against 64 bits, 500 x 2,048 x 2,048: 1.4e-7 of the norm, 4.1e-7 by multiply-adds; K = 512 1.3e-7 and 1.6e-7;
+//   K = 8,192 1.7e-7 and 8.1e-7 (at K of 100 and 256 the two are alike, which is where the line comes from).  The four
+//   products of a layer at 1B sizes, 500 rows (61 GFLOP): 1,491 us by multiply-adds, 470 with all of K a block, 372 so.  What bounds it is the traffic of
 //   shared memory and the chain of a stage: 0.66 us where its products take 0.4 (both operands in shared
 //   memory: 0.9; one group of eight warps besides: 1.05).  Sums that values which bfloat16 cannot split (infinities, NaN,
 //   numbers below 2^-103) could show in and sums that leave the range are done over by multiply-adds at the end, so that
@@ -39,7 +40,10 @@
 #include "common.cuh"
 #include "gate_act.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda.h>
+
+namespace cg = cooperative_groups;
 
 LSB_DEFINE_STATUS()
 
@@ -217,6 +221,10 @@ struct TileParams {
     const float* w;
     float* out;
     int M, N, K, act;
+    // (split products)
+    int steps;                                 // stages of K a block takes, of a cluster along K
+    int tiles_m, tiles_n, tile0;               // tiles of the matrix, and the first of this launch
+    int rows_first;                            // neighbouring tiles share w
 };
 
 // outputs (m, n .. n + 3), as far as n goes, or what the gated product makes of them (N is even then)
@@ -364,6 +372,7 @@ constexpr int kSGroup = 256;                   // eight warps: a row of x or w e
 constexpr int kSWorkers = 2 * kSGroup;         // ... and as many for the stage after it
 constexpr int kSThreads = kSWorkers + 64;      // ... one warp for the copies, one for the products
 constexpr int kSChunk = 4;                     // stages (K = 128) whose leading products meet in tensor memory
+constexpr int kSSplits = 8;                    // most blocks of a cluster along K (the portable size)
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -478,12 +487,15 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     unsigned char* ring = (unsigned char*)(((uintptr_t)raw_smem + 1023) & ~(uintptr_t)1023);
     unsigned char* planes = ring + (size_t)R * L::kRaw;
     __shared__ uint64_t raw_full[R], raw_empty[R], split_full[2], split_empty[2], acc_full[2], acc_empty[2], done;
-    __shared__ uint32_t tmem_slot, least[L::kRows];
+    __shared__ uint32_t tmem_slot, least[L::kRows], all_least[L::kRows];
     __shared__ int abort_flag, any_tiny;
     lsb_pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m0 = (int)blockIdx.y * kSM, n0 = (int)blockIdx.x * BN;
-    const int steps = (p.K + kSK - 1) / kSK;
+    const int tile_at = p.tile0 + (int)blockIdx.x;
+    const int m0 = (p.rows_first ? tile_at % p.tiles_m : tile_at / p.tiles_n) * kSM, n0 = (p.rows_first ? tile_at / p.tiles_m : tile_at % p.tiles_n) * BN;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int splits = (int)gridDim.z, first = (int)blockIdx.z * p.steps;
+    const int steps = min(p.steps, (p.K + kSK - 1) / kSK - first);      // (at least one)
     if (tid < L::kRows) least[tid] = 0xffffffffu;
     if (tid == 0) {
         abort_flag = any_tiny = 0;
@@ -517,8 +529,8 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 const int s = it % R;
                 if (it >= R && !mbar_wait(&raw_empty[s], (uint32_t)(it / R - 1) & 1, &abort_flag)) break;
                 mbar_expect(&raw_full[s], L::kRaw);
-                tma_rows(base + s * L::kRaw, &map_x, &raw_full[s], it * kSK, m0);
-                tma_rows(base + s * L::kRaw + kSM * kSK * 4, &map_w, &raw_full[s], it * kSK, n0);
+                tma_rows(base + s * L::kRaw, &map_x, &raw_full[s], (first + it) * kSK, m0);
+                tma_rows(base + s * L::kRaw + kSM * kSK * 4, &map_w, &raw_full[s], (first + it) * kSK, n0);
             }
             for (int k = it > R ? it - R : 0; k < it; ++k) {            // (no copy is in flight when the block leaves)
                 int ignore = 0;
@@ -642,48 +654,72 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         if (has_row) atomicMin(&least[r], low);
         if (low < kTiny) any_tiny = 1;
         tmem_fence_before();
-        asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
-        if (!abort_flag) {
-            const float* tile = reinterpret_cast<const float*>(ring);
-            // A number below 2^-103 loses less than 2^-125 with the parts that bfloat16 has no normal number for (one that
-            // is not below has them all), which is at most K 2^-125 times the largest number of the other operand's row in
-            // a sum.  Sums that this could show in are done over; the largest are looked up only where there is such a number.
-            float* largest = reinterpret_cast<float*>(planes);          // [kRows] (every product has been waited for)
-            if (any_tiny) {
-                for (int r = warp; r < L::kRows; r += kSWorkers / 32) {
-                    const bool of_x = r < kSM;
-                    const long long at = of_x ? m0 + r : n0 + r - kSM;
-                    float big = 0.f;
-                    if (at < (of_x ? p.M : p.N))
-                        for (int k = lane * 4; k < p.K; k += 128) {
-                            const float4 a = *reinterpret_cast<const float4*>((of_x ? p.x : p.w) + at * p.K + k);
-                            big = fmaxf(fmaxf(big, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(a.z), fabsf(a.w)));
-                        }
-                    big = lsb_warp_max(big);
-                    if (lane == 0) largest[r] = big * ((float)p.K * 0x1p-101f);
+    }
+    __syncwarp();
+    // the sums of all stretches of K are there, each in its block; a block brings its share of the rows together
+    if (splits > 1) cluster.sync();
+    else __syncthreads();
+    if (warp < kSWorkers / 32 && !abort_flag) {
+        const float* tile = reinterpret_cast<const float*>(ring);
+        const int share = kSM / splits, row0 = (int)blockIdx.z * share, rows = (int)blockIdx.z == splits - 1 ? kSM - row0 : share;
+        // A number below 2^-103 loses less than 2^-125 with the parts that bfloat16 has no normal number for (one that
+        // is not below has them all), which is at most K 2^-125 times the largest number of the other operand's row in
+        // a sum.  Sums that this could show in are done over; the largest are looked up only where there is such a number.
+        float* largest = reinterpret_cast<float*>(planes);              // [kRows] (every product has been waited for)
+        bool tiny = any_tiny;
+        for (int k = 0; k < splits && splits > 1; ++k) tiny |= *cluster.map_shared_rank(&any_tiny, k) != 0;
+        if (tiny) {
+            for (int r = warp; r < L::kRows; r += kSWorkers / 32) {
+                const bool of_x = r < kSM;
+                if (of_x && (r < row0 || r >= row0 + rows)) continue;
+                const long long at = of_x ? m0 + r : n0 + r - kSM;
+                float big = 0.f;
+                if (at < (of_x ? p.M : p.N))
+                    for (int k = lane * 4; k < p.K; k += 128) {
+                        const float4 a = *reinterpret_cast<const float4*>((of_x ? p.x : p.w) + at * p.K + k);
+                        big = fmaxf(fmaxf(big, fmaxf(fabsf(a.x), fabsf(a.y))), fmaxf(fabsf(a.z), fabsf(a.w)));
+                    }
+                big = lsb_warp_max(big);
+                if (lane == 0) {
+                    largest[r] = big * ((float)p.K * 0x1p-101f);
+                    uint32_t least_of = least[r];
+                    for (int k = 0; k < splits && splits > 1; ++k) least_of = min(least_of, *cluster.map_shared_rank(&least[r], k));
+                    all_least[r] = least_of;
                 }
-                asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
             }
-            for (int e = tid; e < kSM * BN / 4; e += kSWorkers) {
-                const int row = e / (BN / 4), col = e % (BN / 4) * 4;
-                if (m0 + row >= p.M || n0 + col >= p.N) continue;
-                __align__(16) float v[4];
-                *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(tile + row * L::LDT + col);
+            asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
+        }
+        for (int e = tid; e < rows * (BN / 4); e += kSWorkers) {
+            const int row = row0 + e / (BN / 4), col = e % (BN / 4) * 4;
+            if (m0 + row >= p.M || n0 + col >= p.N) continue;
+            __align__(16) float v[4];
+            const float* at = tile + row * L::LDT + col;
+            if (splits > 1) {
+                float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                for (int k = 0; k < splits; ++k) {                      // (in order)
+                    const float4 a = *reinterpret_cast<const float4*>(cluster.map_shared_rank(at, k));
+                    sum.x += a.x; sum.y += a.y; sum.z += a.z; sum.w += a.w;
+                }
+                *reinterpret_cast<float4*>(v) = sum;
+            } else {
+                *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(at);
+            }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    bool over = !(fabsf(v[i]) <= 3.402823466e38f);
-                    if (any_tiny)
-                        over |= (least[row] < kTiny && fabsf(v[i]) < largest[kSM + col + i]) ||
-                                (least[kSM + col + i] < kTiny && fabsf(v[i]) < largest[row]);
-                    if (over && n0 + col + i < p.N)
-                        v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
-                }
-                store_four(p, m0 + row, n0 + col, *reinterpret_cast<float4*>(v));
+            for (int i = 0; i < 4; ++i) {
+                bool over = !(fabsf(v[i]) <= 3.402823466e38f);
+                if (tiny)
+                    over |= (all_least[row] < kTiny && fabsf(v[i]) < largest[kSM + col + i]) ||
+                            (all_least[kSM + col + i] < kTiny && fabsf(v[i]) < largest[row]);
+                if (over && n0 + col + i < p.N)
+                    v[i] = plain_dot(p.x + (long long)(m0 + row) * p.K, p.w + (long long)(n0 + col + i) * p.K, p.K);
             }
+            store_four(p, m0 + row, n0 + col, *reinterpret_cast<float4*>(v));
         }
     }
     __syncwarp();
-    __syncthreads();
+    if (splits > 1) cluster.sync();                                     // (a peer may still read this block's sums)
+    else __syncthreads();
     if (warp == kSWorkers / 32) {
         tmem_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kColumns));
@@ -756,30 +792,106 @@ static int map_rows(CUtensorMap* map, const float* ptr, int rows, int K, int box
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
+// Blocks of gemm_split_f32_kernel<BN> that run at once in clusters of `splits`.
 template <int BN>
-static int launch_split(const TileParams& p, cudaStream_t stream) {
+static int split_room(int splits) {
+    using L = SplitLayout<BN>;
+    static int cached[64][kSSplits + 1] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    int& room = cached[dev][splits];
+    if (room == 0) {
+        int clusters = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, splits);
+        cfg.blockDim = dim3(kSThreads);
+        cfg.dynamicSmemBytes = L::kTotal;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = splits;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (splits == 1 || cudaFuncSetAttribute(gemm_split_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, gemm_split_f32_kernel<BN>, &cfg) != cudaSuccess || clusters <= 0) {
+            cudaGetLastError();
+            clusters = num_sms() / splits;
+        }
+        room = clusters * splits < 1 ? 1 : clusters * splits;
+    }
+    return room;
+}
+
+template <int BN>
+static int launch_split(TileParams p, int tile0, int tiles, int splits, cudaStream_t stream) {
     using L = SplitLayout<BN>;
     static int configured = -1;
     if (configured < 0)
         configured = (int)cudaFuncSetAttribute(gemm_split_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
     if (configured) return configured;
-    const dim3 grid((p.N + BN - 1) / BN, (p.M + kSM - 1) / kSM);
-    if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+    // whole chunks of leading products a block; the last one may have fewer
+    const int chunks = (p.K + kSK * kSChunk - 1) / (kSK * kSChunk), per = (chunks + splits - 1) / splits;
+    p.steps = per * kSChunk;
+    p.tiles_m = (p.M + kSM - 1) / kSM;
+    p.tiles_n = (p.N + BN - 1) / BN;
+    p.tile0 = tile0;
+    p.rows_first = p.M <= p.N;
+    const dim3 grid(tiles, 1, (chunks + per - 1) / per);
     CUtensorMap mx, mw;
     int rc;
     if ((rc = map_rows(&mx, p.x, p.M, p.K, kSM))) return rc;
     if ((rc = map_rows(&mw, p.w, p.N, p.K, BN))) return rc;
-    return lsb_launch(gemm_split_f32_kernel<BN>, grid, dim3(kSThreads), L::kTotal, stream, 1, mx, mw, p);
+    return lsb_launch(gemm_split_f32_kernel<BN>, grid, dim3(kSThreads), L::kTotal, stream, (int)grid.z, mx, mw, p);
 }
 
 LSB_API int lsb_gemm_f32_supported(const void* x, const void* w, int M, int N, int K) {
     return M > 0 && N > 0 && K > 0 && K % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0 && M <= 32 * 65535;
 }
 
-// Columns of a split product's blocks.  64 take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so only where
-// one round does (500 x 3,072 x 2,048: 87.4 and 54.9).
+// Columns of a split product's blocks that take all of K.  64 take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so
+// only where one round does (500 x 3,072 x 2,048: 87.4 and 54.9).
 LSB_API int lsb_gemm_f32_split_columns(int M, int N) {
     return (long long)((M + kSM - 1) / kSM) * ((N + 63) / 64) <= num_sms() ? 64 : 128;
+}
+
+// How a split product's tiles go to the SMs: `columns` wide, a block for all of K of the first `whole` of them, a cluster of `splits`
+// blocks along K for each of the rest.  A block takes about its fixed part and its stages (fitted to 20 shapes), a cluster some
+// 2.5 us more to meet; blocks run in rounds.  500 rows, us, whole and so: 2,048 x 2,048 44 / 31 (two parts), 2,048 x 8,192 161 / 95,
+// 16,384 x 2,048 gated 220 / 195 (three whole rounds, the rest in two parts), 3,072 x 2,048 52 / 52 (whole: 96 tiles); 40 rows
+// times 2,048 x 8,192 159 / 38 (eight parts); 300 times 16,384 x 2,048 160 / 159 (whole).
+struct SplitPlan { int columns, splits; long long whole, tiles; };
+static SplitPlan split_plan(int M, int N, int K) {
+    const int chunks = (K + kSK * kSChunk - 1) / (kSK * kSChunk);
+    SplitPlan best{};
+    double least = 0.0;
+    for (int bn = 64; bn <= 128; bn += 64) {
+        const double stage = bn == 64 ? 0.62 : 0.70, fixed = bn == 64 ? 4.8 : 7.0, meet = 2.5;
+        const long long tiles = (long long)((M + kSM - 1) / kSM) * ((N + bn - 1) / bn), room = bn == 64 ? split_room<64>(1) : split_room<128>(1);
+        const double round = fixed + chunks * kSChunk * stage;
+        auto offer = [&](long long whole, int splits, double us) {
+            if (splits > 1) us *= 1.03;                        // (in doubt whole)
+            if (best.columns == 0 || us < least) { least = us; best = SplitPlan{bn, splits, whole, tiles}; }
+        };
+        offer(tiles, 1, round * (double)((tiles + room - 1) / room));
+        const long long full = tiles / room;
+        for (int s = 2; s <= kSSplits && s <= chunks; ++s) {
+            const long long at_once = bn == 64 ? split_room<64>(s) : split_room<128>(s);
+            const double part = fixed + meet + (chunks + s - 1) / s * kSChunk * stage;
+            offer(0, s, part * (double)((tiles * s + at_once - 1) / at_once));
+            if (full > 0 && tiles > full * room)
+                offer(full * room, s, round * (double)full + part * (double)(((tiles - full * room) * s + at_once - 1) / at_once));
+        }
+    }
+    return best;
+}
+template <int BN>
+static int run_split(const TileParams& p, const SplitPlan& plan, cudaStream_t stream) {
+    if (plan.tiles > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+    if (plan.whole) {
+        const int rc = launch_split<BN>(p, 0, (int)plan.whole, 1, stream);
+        if (rc || plan.whole == plan.tiles) return rc;
+    }
+    return launch_split<BN>(p, (int)plan.whole, (int)(plan.tiles - plan.whole), plan.splits, stream);
 }
 
 // act: 0, or the activation of a gated product (1 silu, 2 gelu in its tanh form, 3 none), N even then.
@@ -801,10 +913,11 @@ LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int 
     // 10 % on most of 120 shapes; along the shortest K it picks too small a tile (500 x 20,000 x 20: 65 us, 128 x 128 29; 2,048 x
     // 2,048 x 64: 28, 128 x 256 18), whose sums are the closer ones: more warps share K out (K = 320, from the smallest tile to the
     // largest: 1.3, 1.7, 2.4 and 3.2e-7 of the norm).
-    const TileParams p{x, w, out, M, N, K, act};
+    const TileParams p{x, w, out, M, N, K, act, 0, 0, 0, 0, 0};
     const long long sms = num_sms();
     if (K >= kSplitK) {
-        return lsb_gemm_f32_split_columns(M, N) == 64 ? launch_split<64>(p, stream) : launch_split<128>(p, stream);
+        const SplitPlan plan = split_plan(M, N, K);
+        return plan.columns == 64 ? run_split<64>(p, plan, stream) : run_split<128>(p, plan, stream);
     }
     const int bm[4] = {128, 128, 64, 64}, bn[4] = {256, 128, 128, 64};
     const double cost[4] = {1.0, 1.0, 1.03, 1.08};
