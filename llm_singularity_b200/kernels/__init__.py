@@ -2292,8 +2292,8 @@ def sample(logits: torch.Tensor, params: torch.Tensor, top_k: torch.Tensor,
            out: torch.Tensor, work: Optional[torch.Tensor] = None) -> None:
     """One token per row of ``logits``.  ``params[r] = (temperature, top_p, repetition_penalty,
     u)``; ``top_k[r]`` (0 = off); ``prev_tokens[prev_start[r]:prev_start[r+1]]`` are the tokens the
-    repetition penalty applies to; ``work`` is scratch shaped like ``logits`` (used only where a row's
-    slices do not fit the blocks' shared memory)."""
+    repetition penalty applies to; ``work`` is scratch shaped like ``logits`` (used only where there are such tokens
+    and a row's slices do not fit the blocks' shared memory)."""
     _req(logits, "logits", torch.float32, 2)
     R, V = logits.shape
     _req(params, "params", torch.float32, 2)
@@ -2304,7 +2304,7 @@ def sample(logits: torch.Tensor, params: torch.Tensor, top_k: torch.Tensor,
     if prev_start is not None:
         _req(prev_start, "prev_start", torch.int32, 1)
         _req(prev_tokens, "prev_tokens", torch.int32, 1)
-    if work is None and _lib("sampling").lsb_sample_needs_work(_i(V)):
+    if work is None and prev_start is not None and _lib("sampling").lsb_sample_needs_work(_i(V)):
         work = torch.empty_like(logits)
     if work is not None:
         _req(work, "work", torch.float32, 2)
