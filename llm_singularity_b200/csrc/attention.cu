@@ -22,7 +22,9 @@
 // * Single tokens are cache traffic: a block takes a kv head's group of query heads over one of up to eight
 //   stretches of the request's keys, and the stretches' sums meet through distributed shared memory.  8 requests
 //   of 300 to 1,500 tokens, 32 / 8 heads of 64 in 32-bit (29 MB): 24 us; one warp for each (request, head)
-//   walking all of its keys took 1,548 us.
+//   walking all of its keys took 1,548 us.  The kernel can rotate the token's queries and key and store the key and value by
+//   itself (every block takes them from the projection, one writes the page), which saves a kernel of 4 us in the chain of
+//   a decode step, and asks for its first keys while the projection is computed: a layer at 1B sizes, 8 requests, 110 -> 100 us.
 // * Portions are arithmetic: 64 rows (16 queries of 4 heads that share their keys) against a tile, 4 rows by 2 or 4
 //   keys a thread for the scores and the same 4 rows for the weighted sum, so that a row's maximum, its sum and its
 //   probabilities stay within half a warp; two multiply-adds to an instruction.  The last rows of a portion see the most
@@ -62,6 +64,10 @@ struct AttnParams {
     int heads;                                  // query heads of a block
     int head_blocks;                            // blocks of a kv head's group
     int splits;                                 // (portions) blocks that share out a block's keys
+    // (single tokens, null: done already) the projection comes unrotated: dims i and i + rotary_dim / 2 turn by p * inv_freq[i], and
+    // the new key and value go to their page if `store`
+    const float* inv_freq;
+    int rotary_dim, store;
 };
 
 typedef unsigned long long pair32;              // two 32-bit values
@@ -117,16 +123,22 @@ struct Tile {
             }
         }
     }
-    // (returns whether every value of this thread's is a number and finite)
-    __device__ __forceinline__ bool park(const AttnParams& p, float* ks, float* vs, int ldk, int tid) const {
+    // (returns whether every value of this thread's is a number and finite)  own: the row of a token's own key, which is at
+    // `fresh`, its value behind it (-1: none)
+    __device__ __forceinline__ bool park(const AttnParams& p, float* ks, float* vs, int ldk, int tid, int own = -1,
+                                         const float* fresh = nullptr) const {
         const int per = p.hd >> 2;
         float zero = 0.f;                                      // times a number 0, times anything else NaN
 #pragma unroll
         for (int j = 0; j < kPieces; ++j) {
             const int idx = j * kThreads + tid, row = idx / per, d = (idx - row * per) * 4;
             if (row < KT) {
-                *reinterpret_cast<float4*>(ks + row * ldk + d) = widen(k[j]);
-                const float4 w = widen(v[j]);
+                float4 u = widen(k[j]), w = widen(v[j]);
+                if (row == own) {
+                    u = *reinterpret_cast<const float4*>(fresh + d);
+                    w = *reinterpret_cast<const float4*>(fresh + p.hd + d);
+                }
+                *reinterpret_cast<float4*>(ks + row * ldk + d) = u;
                 *reinterpret_cast<float4*>(vs + row * p.hd + d) = w;
                 zero = fmaf(w.x, zero, fmaf(w.y, zero, fmaf(w.z, zero, w.w * zero)));
             }
@@ -157,16 +169,18 @@ constexpr int kAccs = 4;
 
 template <int KT>
 static size_t single_smem(int hd, int heads) {
-    return ((size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)heads * hd * 2 + (size_t)heads * (KT + 4) + heads * 4) * 4;
+    return ((size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)heads * hd * 2 + (size_t)heads * (KT + 4) + heads * 4 + 2 * (size_t)hd) * 4;
 }
 
 template <typename T, int KT, int HDC>
 __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const AttnParams p) {
     extern __shared__ __align__(16) float sm[];
     __shared__ long long off[2][KT];
+    __shared__ float cs[2][kMaxHeadDim / 2];                   // cosines and sines of the token's position
     cg::cluster_group cluster = cg::this_cluster();
     lsb_pdl_launch_dependents();
-    lsb_pdl_wait();
+    // The step's metadata and tables are there before its first kernel, so all that follows from them is had before the wait
+    // for the projection, the first keys and values among it.
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int splits = (int)gridDim.x, split = (int)blockIdx.x, r = blockIdx.z;
     const int g = blockIdx.y / p.head_blocks, group = p.nh / p.nkv;
@@ -181,6 +195,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const Att
     float* os = qs + p.heads * hd;                             // [heads][hd], the stretch's sums
     float* ps = os + p.heads * hd;                             // [heads][KT + 4]
     float* ml = ps + p.heads * lds;                            // running maximum, sum, factor of the last tile; m and l stay
+    float* fresh = ml + p.heads * 4;                           // the token's own key and value
     const int pos = p.kv_len[r] - 1;
     const int lo = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
     // this block's stretch: whole sixteens of keys
@@ -188,8 +203,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const Att
     const int first = lo + split * per, last = min(pos + 1, first + per);     // [first, last), maybe empty
     const int* table = p.block_table + (size_t)p.table_rows[r] * p.table_stride;
 
-    const T* q = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.qkv_stride + (size_t)h0 * hd;
-    for (int i = tid; i < H * hd; i += kThreads) qs[i] = lsb_to_float(q[i]) * p.scale;
+    const bool rotates = p.inv_freq != nullptr, stores = rotates && p.store;
+    const int half = rotates ? p.rotary_dim >> 1 : 0;
+    for (int i = tid; i < half; i += kThreads) sincosf((float)pos * p.inv_freq[i], &cs[1][i], &cs[0][i]);
     if (tid < H) { ml[4 * tid] = -FLT_MAX; ml[4 * tid + 1] = 0.f; }
     if (tid < KT) off[0][tid] = first + tid < last ? key_offset(p, table, g, first + tid) : -1;
     float acc[kAccs];
@@ -197,9 +213,36 @@ __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const Att
     for (int a = 0; a < kAccs; ++a) acc[a] = 0.f;
     __syncthreads();
     Tile<T, KT, HDC> tile;
-    tile.fetch(p, off[0], tid);
+    // (what its page holds of a key that comes with the projection is not used; one that another layer's kernel writes in this
+    // step is waited for)
+    const bool early = stores || pos < first || pos >= first + KT;
+    if (early) tile.fetch(p, off[0], tid);
+    lsb_pdl_wait();
+    if (!early) tile.fetch(p, off[0], tid);
+    const T* token = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.qkv_stride;
+    // element d of a head at x, rotated, as the projection's type holds it
+    auto turned = [&](const T* x, int d) -> float {
+        if (d >= 2 * half) return lsb_to_float(x[d]);
+        const int i = d < half ? d : d - half;
+        const float x0 = lsb_to_float(x[i]), x1 = lsb_to_float(x[i + half]);
+        return lsb_to_float(lsb_from_float<T>(d < half ? x0 * cs[0][i] - x1 * cs[1][i] : x0 * cs[1][i] + x1 * cs[0][i]));
+    };
+    for (int i = tid; i < H * hd; i += kThreads) qs[i] = turned(token + (size_t)(h0 + i / hd) * hd, i % hd) * p.scale;
+    if (stores && pos >= first && pos < last) {
+        const long long to = blockIdx.y % p.head_blocks == 0 ? key_offset(p, table, g, pos) : -1;       // (one block writes)
+        for (int d = tid; d < hd; d += kThreads) {
+            const float u = turned(token + (size_t)(p.nh + g) * hd, d), w = lsb_to_float(token[(size_t)(p.nh + p.nkv + g) * hd + d]);
+            fresh[d] = u;
+            fresh[hd + d] = w;
+            if (to >= 0) {
+                reinterpret_cast<T*>(const_cast<void*>(p.k_pages))[to + d] = lsb_from_float<T>(u);
+                reinterpret_cast<T*>(const_cast<void*>(p.v_pages))[to + d] = lsb_from_float<T>(w);
+            }
+        }
+    }
+    __syncthreads();
     for (int base = first, turn = 0; base < last; base += KT, turn ^= 1) {
-        tile.park(p, ks, vs, ldk, tid);
+        tile.park(p, ks, vs, ldk, tid, stores && pos < last ? pos - base : -1, fresh);
         const int next = base + KT;
         if (tid < KT) off[turn ^ 1][tid] = next + tid < last ? key_offset(p, table, g, next + tid) : -1;
         __syncthreads();
@@ -624,17 +667,20 @@ static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int
 
 // qkv: [tokens, qkv_stride] with the nh*hd query values first in each row.  softcap: 0 for none; slopes: float [nh] or
 // null.  n_single: requests that bring one token; max_keys: the longest context (0: not known, the launch is captured).
+// inv_freq: null, or the rotation of single tokens (float [rotary_dim / 2]), which come unrotated then, keys and values behind the
+// queries in their rows; `store`: and not yet in their pages.
 LSB_API int lsb_paged_attention_generic(
     const void* qkv, int qkv_stride, const void* k_pages, const void* v_pages,
     const int* q_start, const int* kv_len, const int* table_rows, const int* block_table,
     int table_stride, void* out, int dtype, int n_requests, int max_q_len, int n_single, int max_keys,
     int nh, int nkv, int hd, int page_size, int num_pages, float scale, int window,
-    float softcap, const float* slopes, cudaStream_t stream) {
+    float softcap, const float* slopes, const float* inv_freq, int rotary_dim, int store, cudaStream_t stream) {
     if (n_requests <= 0 || max_q_len <= 0) return 0;
     if (hd % 16 || hd <= 0 || hd > kMaxHeadDim || nkv <= 0 || nh % nkv) return (int)cudaErrorInvalidValue;
     if (n_requests > 65535 || nh > 65535) return (int)cudaErrorInvalidValue;
+    if (inv_freq && (rotary_dim < 0 || rotary_dim > hd || rotary_dim % 2 || qkv_stride < (nh + 2 * nkv) * hd)) return (int)cudaErrorInvalidValue;
     const AttnParams p{qkv, qkv_stride, k_pages, v_pages, q_start, kv_len, table_rows, block_table, table_stride, out,
-                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0, 1};
+                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0, 1, inv_freq, rotary_dim, store};
     LSB_DISPATCH_DTYPE(dtype, {
         if (hd <= 64) return launch<T, 64, 64>(p, n_requests, max_q_len, n_single, max_keys, stream);
         if (hd <= 128) return launch<T, 32, 128>(p, n_requests, max_q_len, n_single, max_keys, stream);

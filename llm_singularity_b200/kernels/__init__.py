@@ -615,12 +615,8 @@ def _check_cache(cache, nkv: int, hd: int, dtype) -> None:
     _req(cache.block_table, "block_table", torch.int32, 2)
 
 
-def rope_kv_store(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache,
-                  inv_freq: Optional[torch.Tensor], rotary_dim: int, store: bool = True,
-                  skip_single: bool = False) -> None:
-    """Rotate queries and keys of the fused projection in place and write keys and values
-    of this step's tokens into their cache pages.  ``skip_single`` leaves the tokens of requests
-    that bring one token alone (their attention kernel does the same work itself)."""
+def _check_rope(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, inv_freq: Optional[torch.Tensor], rotary_dim: int) -> int:
+    """Refuses what no kernel rotates; the number of tokens."""
     _req(qkv, "qkv", dim=2)
     T = qkv.shape[0]
     if qkv.shape[1] != (nh + 2 * nkv) * hd:
@@ -632,9 +628,19 @@ def rope_kv_store(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache,
         _req(inv_freq, "inv_freq", torch.float32, 1)
         if inv_freq.shape[0] != rotary_dim // 2:
             raise KernelError("inv_freq must have rotary_dim / 2 entries")
-    _check_cache(cache, nkv, hd, qkv.dtype)
     if ctx.n_tokens != T:
         raise KernelError(f"qkv has {T} rows, the step has {ctx.n_tokens} tokens")
+    return T
+
+
+def rope_kv_store(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache,
+                  inv_freq: Optional[torch.Tensor], rotary_dim: int, store: bool = True,
+                  skip_single: bool = False) -> None:
+    """Rotate queries and keys of the fused projection in place and write keys and values
+    of this step's tokens into their cache pages.  ``skip_single`` leaves the tokens of requests
+    that bring one token alone (their attention kernel does the same work itself)."""
+    T = _check_rope(qkv, nh, nkv, hd, ctx, inv_freq, rotary_dim)
+    _check_cache(cache, nkv, hd, qkv.dtype)
     _call("rope_cache", "lsb_rope_kv_store", _p(qkv), _i(_dt(qkv)), _i(T), _i(nh), _i(nkv), _i(hd),
           _p(ctx.positions), _p(ctx.token_req), _p(ctx.table_rows), _p(cache.block_table),
           _i(cache.block_table.shape[1]), _p(inv_freq if rotary_dim else None), _i(rotary_dim),
@@ -762,23 +768,23 @@ def rope_store_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cac
                          inv_freq: Optional[torch.Tensor], rotary_dim: int, store: bool,
                          scale: float, window: int, out: torch.Tensor, softcap: float = 0.0,
                          slopes: Optional[torch.Tensor] = None) -> None:
-    """``rope_kv_store`` followed by ``paged_attention``, as one operation.  Where the decode
-    kernel can do the rotation and the cache write of single tokens itself (tensor-core path,
-    the rotated part of the head a multiple of 16 wide, no score modifier), the separate kernel
+    """``rope_kv_store`` followed by ``paged_attention``, as one operation.  Where the kernel of single
+    tokens can do the rotation and the cache write itself (on the tensor cores with the rotated part
+    of the head a multiple of 16 wide, the generic one with any; no score modifier), the separate kernel
     runs only for the tokens of prompt portions, or not at all."""
     if softcap or slopes is not None:
         rope_kv_store(qkv, nh, nkv, hd, ctx, cache, inv_freq, rotary_dim, store)
         paged_attention(qkv, nh, nkv, hd, ctx, cache, scale, window, out, softcap=softcap, slopes=slopes)
         return
-    fuse = (FUSE_DECODE_ROPE and 0 < rotary_dim <= hd and rotary_dim % 16 == 0 and inv_freq is not None
-            and tensor_core_attention_ok(qkv.dtype, hd, nh, nkv))
+    on_tc = tensor_core_attention_ok(qkv.dtype, hd, nh, nkv)
+    fuse = FUSE_DECODE_ROPE and 0 < rotary_dim <= hd and inv_freq is not None and (rotary_dim % 16 == 0 or not on_tc)
     n_decode = _batch_shape(ctx)[0] if fuse else 0
     if not n_decode:
         rope_kv_store(qkv, nh, nkv, hd, ctx, cache, inv_freq, rotary_dim, store)
         paged_attention(qkv, nh, nkv, hd, ctx, cache, scale, window, out)
         return
     if n_decode < ctx.n_requests:
-        if OVERLAP_ATTENTION and not getattr(ctx, "fixed_launch", False):
+        if on_tc and OVERLAP_ATTENTION and not getattr(ctx, "fixed_launch", False):
             # Single tokens and prompt portions are different requests with different pages: the
             # decode kernel (memory-bound) runs on a second stream beside the rotation and the
             # attention of the portions (compute-bound), and the step's stream waits for both.
@@ -793,6 +799,8 @@ def rope_store_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cac
             _stream_op(lambda: main.wait_event(join))
             return
         rope_kv_store(qkv, nh, nkv, hd, ctx, cache, inv_freq, rotary_dim, store, skip_single=True)
+    elif not on_tc:
+        _check_rope(qkv, nh, nkv, hd, ctx, inv_freq, rotary_dim)
     else:
         _req(inv_freq, "inv_freq", torch.float32, 1)
         if inv_freq.shape[0] != rotary_dim // 2 or qkv.shape[1] != (nh + 2 * nkv) * hd:
@@ -844,12 +852,14 @@ def paged_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache, s
     if softcap < 0:
         raise KernelError("attention: the soft cap must be positive (0: none)")
     if modified or not tensor_core_attention_ok(qkv.dtype, hd, nh, nkv):
-        if decode_rope is not None:
-            raise KernelError("attention: only the tensor-core decode kernel rotates by itself")
+        if decode_rope is not None and modified:
+            raise KernelError("attention: scores are modified where queries and keys come rotated")
+        rotation = (None, False, 0) if decode_rope is None else decode_rope
         # (a captured launch has to serve contexts of any length)
         longest = 0 if getattr(ctx, "fixed_launch", False) else ctx.max_kv_len
         _call("attention", "lsb_paged_attention_generic", *common, _i(_dt(qkv)), _i(ctx.n_requests), _i(ctx.max_q_len),
-              _i(_batch_shape(ctx)[0]), _i(longest), *tail, _f(softcap), _p(slopes), _stream(out))
+              _i(_batch_shape(ctx)[0]), _i(longest), *tail, _f(softcap), _p(slopes),
+              _p(rotation[0]), _i(rotation[2]), _i(1 if rotation[1] else 0), _stream(out))
         return
     R = ctx.n_requests
     n_decode, first, last = _batch_shape(ctx)
