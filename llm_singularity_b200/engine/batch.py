@@ -52,6 +52,10 @@ class StepContext:
     max_kv_len: int
 
 
+def _address(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]
+
+
 class ContextBuilder:
     """Packs step metadata into one pinned buffer and copies it to the device once."""
 
@@ -73,6 +77,7 @@ class ContextBuilder:
         self._turn = 0
         self._offsets = np.zeros(8, dtype=np.int64)
         self._summary = np.zeros(4, dtype=np.int64)
+        self._offsets_ptr, self._summary_ptr = _address(self._offsets), _address(self._summary)
 
     def _grow(self, n: int) -> None:
         cap = max(n, 2 * self._cap)
@@ -119,44 +124,41 @@ class ContextBuilder:
         host = self._host_np[i]
         # one pass in the host library writes tokens, positions, each token's entry, where each
         # entry starts, its length after the step, its block-table row and the wanted rows
-        o = native.lib().lsbh_pack_step(R, q_len.ctypes.data, starts_a.ctypes.data, rows_a.ctypes.data,
-                                        flat.ctypes.data, want_count.ctypes.data, wants_a.ctypes.data,
-                                        host.ctypes.data, self._cap, self._offsets.ctypes.data,
-                                        self._summary.ctypes.data)
+        o = native.lib().lsbh_pack_step(R, _address(q_len), _address(starts_a), _address(rows_a),
+                                        _address(flat), _address(want_count), _address(wants_a),
+                                        _address(host), self._cap, self._offsets_ptr,
+                                        self._summary_ptr)
         if o < 0:
             r = -o - 2
             if o == -1 or q_len[r] <= 0:
                 raise ValueError("a step needs at least one entry, and every entry at least one token")
             bad = next(w for w in wants[r] if not 0 <= w < q_len[r])
             raise ValueError(f"entry {r}: wanted place {bad} outside its {q_len[r]} tokens")
-        s_tok, s_pos, s_req, s_qs, s_kv, s_rows, s_want, end = (int(x) for x in self._offsets)
-        s_extra = []
+        places = self._offsets.tolist()
+        s_qs, s_kv, s_rows = places[3:6]
         for e in extra:
             host[o:o + len(e)] = e
-            s_extra.append((o, o + len(e)))
             o += len(e)
 
         dev = self._dev[i] if static is None else static
         if dev.numel() < o:
             raise ValueError(f"static metadata buffer holds {dev.numel()} ints, step needs {o}")
-        dev[:o].copy_(self._host[i][:o], non_blocking=True)
+        used = dev[:o]
+        used.copy_(self._host[i][:o], non_blocking=True)
         if self._cuda:
             if self._events[i] is None:
                 self._events[i] = torch.cuda.Event()
             self._events[i].record()
 
         ctx = StepContext()
-        ctx.token_ids = dev[s_tok:s_pos]
-        ctx.positions = dev[s_pos:s_req]
-        ctx.token_req = dev[s_req:s_qs]
-        ctx.q_start = dev[s_qs:s_kv]
-        ctx.kv_len = dev[s_kv:s_rows]
-        ctx.table_rows = dev[s_rows:s_want]
-        ctx.want_rows = dev[s_want:end]
+        # one split makes all the views (9 us of a step's 66 were spent on a slice for each)
+        sizes = [b - a for a, b in zip(places, places[1:])] + [len(e) for e in extra]
+        (ctx.token_ids, ctx.positions, ctx.token_req, ctx.q_start, ctx.kv_len, ctx.table_rows,
+         ctx.want_rows, *on_device) = used.split_with_sizes(sizes)
         ctx.n_tokens, ctx.n_requests, ctx.n_wanted = T, R, W
         ctx.h_q_len = q_len
         ctx.h_q_start = host[s_qs:s_kv].copy()
         ctx.h_kv_len = host[s_kv:s_rows].copy()
         ctx.h_table_rows = rows_a
-        ctx.max_q_len, ctx.max_kv_len = int(self._summary[2]), int(self._summary[3])
-        return ctx, [dev[a:b] for a, b in s_extra]
+        ctx.max_q_len, ctx.max_kv_len = self._summary[2:].tolist()
+        return ctx, on_device

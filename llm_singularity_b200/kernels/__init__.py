@@ -10,6 +10,7 @@ wrongly.
 from __future__ import annotations
 
 import ctypes
+import operator
 import weakref
 from typing import Dict, Iterable, Optional
 
@@ -164,6 +165,9 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _req(t: torch.Tensor, name: str, dtype=None, dim: Optional[int] = None, contiguous=True):
+    if isinstance(t, torch.Tensor) and t.is_cuda and (dtype is None or t.dtype is dtype) and (dim is None or t.ndim == dim) \
+            and (not contiguous or t.is_contiguous()):
+        return t
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor (there is no CPU path)")
     if dtype is not None and t.dtype != dtype:
@@ -185,10 +189,10 @@ _raw_stream = torch._C._cuda_getCurrentRawStream      # (device index) -> cudaSt
 
 
 def _stream(t: torch.Tensor):
-    return ctypes.c_void_p(_raw_stream(t.device.index))
+    return ctypes.c_void_p(_raw_stream(t.get_device()))
 
 
-_i = ctypes.c_int
+_i = operator.index             # (a whole number goes over as a C int as it is; an object of its own for each is 5 us a layer)
 _ll = ctypes.c_longlong
 _f = ctypes.c_float
 
@@ -532,12 +536,12 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
         return out
     _chain_ends()
     if x.dtype == torch.bfloat16 and tensor_core_gemm_ok(x, w):
-        out = torch.empty((M, N // 2 if gated else N), dtype=out_dtype, device=x.device)
+        out = x.new_empty((M, N // 2 if gated else N), dtype=out_dtype)
         _call("gemm_tc", "lsb_gemm_tc", _p(x), _p(w), _p(out), _i(1 if out_dtype == torch.float32 else 0),
               _i(M), _i(N), _i(K), _i(act), _f(0.0), _stream(out))
         return out
-    if x.dtype == torch.float32 and _lib("gemm_f32").lsb_gemm_f32_supported(_p(x), _p(w), _i(M), _i(N), _i(K)):
-        out = torch.empty((M, N // 2 if gated else N), dtype=out_dtype, device=x.device)
+    if x.dtype == torch.float32 and _f32_gemm_ok(x, w):
+        out = x.new_empty((M, N // 2 if gated else N))
         _call("gemm_f32", "lsb_gemm_f32", _p(x), _p(w), _p(out), _i(M), _i(N), _i(K), _i(act if gated else 0), _stream(out))
         if plain_act is not None:
             plain_activation(out, out, plain_act)
@@ -580,6 +584,13 @@ def small_gemm_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     if M > 16 or K % 64 or per_sm > 32 or (per_sm + 16) * K * 2 > 180 * 1024:
         return False                                  # cheap refusals first; the library has the last word
     return bool(_lib("gemm_small").lsb_gemm_small_supported(_p(x), _p(w), _i(M), _i(N), _i(K)))
+
+
+def _f32_gemm_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """What lsb_gemm_f32_supported says, without asking: rows that are read 16 bytes at a time, grids within their limits."""
+    M, K = x.shape
+    return (K % 4 == 0 and K > 0 and 0 < M <= 32 * 65535 and w.shape[0] > 0 and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0)
 
 
 def tensor_core_gemm_ok(x: torch.Tensor, w: torch.Tensor) -> bool:

@@ -28,6 +28,7 @@ Block           ``forward(residual, pending, ctx, cache, writes_cache) -> pendin
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import cached_property
 from typing import Any, Callable, Dict, Optional, Tuple
 
 import torch
@@ -256,7 +257,17 @@ class Runtime:
         return self._ops
 
     def empty(self, *shape, dtype=None) -> torch.Tensor:
-        return torch.empty(shape, dtype=dtype or self.dtype, device=self.device)
+        if self.device.type == "cuda" and self.device.index is None:      # (whichever device is current)
+            return torch.empty(shape, dtype=dtype or self.dtype, device=self.device)
+        if dtype is None or dtype is self.dtype:
+            return self._pattern.new_empty(shape)
+        return self._pattern.new_empty(shape, dtype=dtype)
+
+    @cached_property
+    def _pattern(self) -> torch.Tensor:
+        """A tensor without elements of the device and the compute dtype (asking it for another takes the host half of what
+        naming both does)."""
+        return torch.empty(0, dtype=self.dtype, device=self.device)
 
 
 class Part:
