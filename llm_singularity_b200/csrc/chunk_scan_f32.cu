@@ -180,8 +180,11 @@ __global__ void __launch_bounds__(kChainThreads) chunk_chain_f32_kernel(ScanArgs
     float4 cur = known ? *reinterpret_cast<const float4*>(st) : make_float4(0.f, 0.f, 0.f, 0.f);
     float* at = a.gain + ((size_t)(q0 / kL + r) * a.heads + h) * per + i;
     const size_t step = (size_t)a.heads * per;
-    constexpr int kAhead = 8;
-    for (int s0 = 0; s0 < chunks; s0 += kAhead) {               // eight chunks' loads in flight at once
+    // 24 chunks' loads in flight at once: a thread's chain is bound by their latency, not by what an SM can hold (all three
+    // kernels, 16 heads of 128 x 128, us, with 8 / 16 / 24: 400 tokens 54.8 / 53.5 / 53.3, 1,000 74.5 / 70.4 / 70.0, 1,500
+    // 87.0 / 82.5 / 80.0, 4,000 231 / 212 / 209; a ring of 16, each loaded again as it is used, 52.7 / 69.8 / 81.7 / 213)
+    constexpr int kAhead = 24;
+    for (int s0 = 0; s0 < chunks; s0 += kAhead) {
         float4 e[kAhead];
 #pragma unroll
         for (int k = 0; k < kAhead; ++k) e[k] = *reinterpret_cast<const float4*>(at + min(s0 + k, chunks - 1) * step);
