@@ -114,11 +114,10 @@ template <int HD> __device__ __forceinline__ bf16* tile_ptr(bf16* base, int row,
 #ifndef LSB_DEC_CHUNK
 #define LSB_DEC_CHUNK 16
 #endif
-#ifndef LSB_DEC_STAGES
-#define LSB_DEC_STAGES 2
-#endif
 constexpr int kChunk = LSB_DEC_CHUNK;           // keys a warp handles per step
-constexpr int kDecStages = LSB_DEC_STAGES;        // chunks in flight per warp
+constexpr int kDecStages = 2;         // a warp's ring of chunks ...
+// ... and the deeper one, with which an SM holds one block fewer
+template <int HD> constexpr int kDeepStages = HD == 64 ? 4 : 3;
 constexpr int kBtCache = 1024;       // block-table entries kept in shared memory per block
 
 __device__ __forceinline__ int div_page(int key, int page_size, int page_shift) {
@@ -132,7 +131,7 @@ __device__ __forceinline__ int div_page(int key, int page_size, int page_shift) 
 #ifndef LSB_DEC_MINBLOCKS
 #define LSB_DEC_MINBLOCKS 4
 #endif
-template <int HD, bool LOW8>
+template <int HD, bool LOW8, int STAGES>
 __global__ void __launch_bounds__(kThreads, HD == 64 ? LSB_DEC_MINBLOCKS : 3)
 decode_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
                         bf16* k_pages, bf16* v_pages,
@@ -141,13 +140,13 @@ decode_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
                         int table_stride, bf16* __restrict__ out, float* __restrict__ part_o,
                         float* __restrict__ part_ml, int nh, int nkv, int page_size, int num_pages,
                         float scale, int window, int splits, int cluster_merge,
-                        const float* __restrict__ inv_freq, int rotary_dim, int store_kv) {
+                        const float* __restrict__ inv_freq, int rotary_dim, int store_kv, int longest_first) {
     constexpr int CPR = HD / 8, KS = HD / 16;
     constexpr int kStageElems = 2 * kChunk * HD;             // K rows then V rows
     extern __shared__ __align__(128) unsigned char smem_raw[];
     bf16* sQ = reinterpret_cast<bf16*>(smem_raw);            // [16][HD]
     bf16* sKV = sQ + 16 * HD;                                // [4 warps][stages][K|V][16][HD]
-    int* sBT = reinterpret_cast<int*>(sKV + 4 * kDecStages * kStageElems);
+    int* sBT = reinterpret_cast<int*>(sKV + 4 * STAGES * kStageElems);
     float* sCS = reinterpret_cast<float*>(sBT + kBtCache);   // [cos HD/2][sin HD/2] of the position
     lsb_pdl_launch_dependents();
 
@@ -158,15 +157,48 @@ decode_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
     // the first keys and values of every warp can be had while the projection is still being
     // computed.  Only the chunk that holds the token's own position must wait: its last row is
     // written during this step (by this kernel, the rotary kernel or another layer's).
-    const int split = blockIdx.x, g = blockIdx.y, r = blockIdx.z;
-    const int qs = q_start[r];
-    const bool single = q_start[r + 1] - qs == 1;
+    const int split = blockIdx.x, g = blockIdx.y;
+    int r = blockIdx.z, qs, kv_len, row;
+    bool single;
+    // Where blocks run in two rounds, requests longest first: those that begin last end soon (64 requests of 150 - 2,100 tokens,
+    // head size 128: 50.4 -> 42.9 us with the rest alike).  Every block finds the one of its rank, at most one a thread; some 0.4
+    // us of a block's start, which is why three rounds and more stay in order (128 requests of 200 - 300 tokens 34.1 -> 36.5).
+    if (longest_first) {
+        __shared__ __align__(16) uint32_t keys[kThreads];
+        __shared__ int4 chosen;
+        const int t = threadIdx.x, n = gridDim.z;
+        int4 own = make_int4(t, 0, 0, 0);
+        if (t < n) {
+            const int s0 = q_start[t], s1 = q_start[t + 1], len = kv_len_arr[t];
+            own = make_int4(t, s0, s1 - s0 == 1 ? len : 0, table_rows[t]);
+        }
+        const uint32_t key = t < n ? (uint32_t)own.z << 7 | (127 - t) : 0u;      // no two alike; equal lengths in their order
+        keys[t] = key;
+        __syncthreads();
+        int before = 0;
+#pragma unroll 4
+        for (int j = 0; j < n; j += 4) {
+            const uint4 k = *reinterpret_cast<const uint4*>(keys + j);
+            before += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
+        }
+        if (t < n && before == r) chosen = own;
+        __syncthreads();
+        own = chosen;
+        r = own.x; qs = own.y; kv_len = own.z; row = own.w;
+        single = kv_len > 0;
+        kv_len = max(kv_len, 1);
+    } else {
+        qs = q_start[r];
+        single = q_start[r + 1] - qs == 1;
+        kv_len = kv_len_arr[r];
+        row = table_rows[r];
+    }
+
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = nh / nkv;
-    const int kv_len = kv_len_arr[r];
     const int p = kv_len - 1;
     const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
-    const int* bt = block_table + (size_t)table_rows[r] * table_stride;
+    const int* bt = block_table + (size_t)row * table_stride;
     const int page_shift = (page_size & (page_size - 1)) == 0 ? __ffs(page_size) - 1 : -1;
 
     const int first_chunk = lo / kChunk;
@@ -189,12 +221,12 @@ decode_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
             sBT[idx] = (page0 + idx < table_stride) ? __ldcg(bt + page0 + idx) : -1;
     __syncthreads();
 
-    bf16* ring = sKV + (size_t)warp * kDecStages * kStageElems;
+    bf16* ring = sKV + (size_t)warp * STAGES * kStageElems;
     const int n_mine = (c1 - c0 - warp + 3) / 4;             // chunks c0 + warp, c0 + warp + 4, ...
     auto issue = [&](int i) {
         if (i < n_mine) {
             const int chunk = c0 + warp + 4 * i;
-            bf16* dK = ring + (size_t)(i % kDecStages) * kStageElems;
+            bf16* dK = ring + (size_t)(i % STAGES) * kStageElems;
             bf16* dV = dK + kChunk * HD;
             if (page_shift >= 0 && page_size >= kChunk) {
                 // the chunk lies inside one page: one table entry, then a contiguous run of rows
@@ -241,10 +273,10 @@ decode_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
     };
 
     // the warp's first chunks are on their way before the wait if none of them is the last one
-    const bool early = single && cached && c0 + warp + 4 * (kDecStages - 2) < p / kChunk;
+    const bool early = single && cached && c0 + warp + 4 * (STAGES - 2) < p / kChunk;
     if (early) {
 #pragma unroll
-        for (int i = 0; i < kDecStages - 1; ++i) issue(i);
+        for (int i = 0; i < STAGES - 1; ++i) issue(i);
     }
 
     lsb_pdl_wait();
@@ -330,15 +362,15 @@ decode_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
 
     if (!early) {
 #pragma unroll
-        for (int i = 0; i < kDecStages - 1; ++i) issue(i);
+        for (int i = 0; i < STAGES - 1; ++i) issue(i);
     }
 
     for (int i = 0; i < n_mine; ++i) {
-        issue(i + kDecStages - 1);
-        cp_async_wait<kDecStages - 1>();
+        issue(i + STAGES - 1);
+        cp_async_wait<STAGES - 1>();
         __syncwarp();
         const int chunk = c0 + warp + 4 * i;
-        bf16* tK = ring + (size_t)(i % kDecStages) * kStageElems;
+        bf16* tK = ring + (size_t)(i % STAGES) * kStageElems;
         bf16* tV = tK + kChunk * HD;
 
         constexpr int NT = kChunk / 8;                         // 8-key score tiles per chunk
@@ -756,22 +788,26 @@ prefill_attention_kernel(const bf16* __restrict__ qkv, int qkv_stride,
 }
 
 // ------------------------------------------------------------------ host side
-template <int HD> constexpr size_t decode_smem() {
-    return (16 * HD + 4 * kDecStages * 2 * kChunk * HD) * sizeof(bf16) + kBtCache * sizeof(int) +
+template <int HD, int STAGES = kDecStages> constexpr size_t decode_smem() {
+    return (16 * HD + 4 * STAGES * 2 * kChunk * HD) * sizeof(bf16) + kBtCache * sizeof(int) +
            HD * sizeof(float);
 }
 template <int HD> constexpr size_t prefill_smem() {
     return (kPfRows * HD + 2 * kPfStages * kTile * HD) * sizeof(bf16) + kBtCache * sizeof(int);
 }
 
+template <int HD, bool LOW8, int STAGES> static cudaError_t allow_decode_smem() {
+    return cudaFuncSetAttribute(decode_attention_kernel<HD, LOW8, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)decode_smem<HD, STAGES>());
+}
+
 template <int HD> static int configure_once() {
     static int done = -1;
     if (done >= 0) return done;
-    cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel<HD, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem<HD>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(decode_attention_kernel<HD, false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem<HD>());
+    cudaError_t e = allow_decode_smem<HD, true, kDecStages>();
+    if (e == cudaSuccess) e = allow_decode_smem<HD, false, kDecStages>();
+    if (e == cudaSuccess) e = allow_decode_smem<HD, true, kDeepStages<HD>>();
+    if (e == cudaSuccess) e = allow_decode_smem<HD, false, kDeepStages<HD>>();
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(prefill_attention_kernel<HD>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_smem<HD>());
@@ -788,7 +824,7 @@ template <int HD> static int max_cluster() {
     if (configure_once<HD>()) return value;
     bool ok = true;
     for (int low8 = 0; low8 < 2 && ok; ++low8) {
-        auto kernel = low8 ? decode_attention_kernel<HD, true> : decode_attention_kernel<HD, false>;
+        auto kernel = low8 ? decode_attention_kernel<HD, true, kDecStages> : decode_attention_kernel<HD, false, kDecStages>;
         ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         if (!ok) break;
         cudaLaunchConfig_t cfg = {};
@@ -807,21 +843,59 @@ template <int HD> static int max_cluster() {
     return value;
 }
 
+template <int HD, int STAGES> static int decode_fits(int group) {
+    if (configure_once<HD>()) return 1;
+    int n = 0;
+    const cudaError_t e =
+        group <= 8 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attention_kernel<HD, true, STAGES>, kThreads, decode_smem<HD, STAGES>())
+                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attention_kernel<HD, false, STAGES>, kThreads, decode_smem<HD, STAGES>());
+    if (e != cudaSuccess) { (void)cudaGetLastError(); return 1; }
+    return n < 1 ? 1 : n;
+}
+
 // Blocks of the decode kernel that fit an SM at once (registers and shared memory), for query groups
 // of `group` heads: what the number of key splits is sized by.
 LSB_API int lsb_decode_blocks_per_sm(int hd, int group) {
     if ((hd != 64 && hd != 128) || group < 1) return 1;
-    if ((hd == 64 ? configure_once<64>() : configure_once<128>())) return 1;
-    int n = 0;
-    cudaError_t e;
-    if (hd == 64)
-        e = group <= 8 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attention_kernel<64, true>, kThreads, decode_smem<64>())
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attention_kernel<64, false>, kThreads, decode_smem<64>());
-    else
-        e = group <= 8 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attention_kernel<128, true>, kThreads, decode_smem<128>())
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decode_attention_kernel<128, false>, kThreads, decode_smem<128>());
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return 1; }
-    return n < 1 ? 1 : n;
+    return hd == 64 ? decode_fits<64, kDecStages>(group) : decode_fits<128, kDecStages>(group);
+}
+
+static int num_sms() {
+    static int cached[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    if (cached[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
+        cached[dev] = n;
+    }
+    return cached[dev];
+}
+// How a batch's blocks are to run.  A block of the shallow ring has 32 KB of keys and values under way at head size 128 (16 at 64),
+// so that a last round of few blocks waits for one answer after the other: 512 on 148 x 3 places took 60 us where the bytes take
+// 44, 800 took 72 where they take 68.  The deeper ring has two chunks under way (three at 64) on one block fewer an SM.  It serves
+// unsplit keys where its places hold the blocks at once, or in two rounds where the shallow ring needs two as well.  us, shallow /
+// deep, 8 kv heads, all requests of some 1,100 tokens: head size 128, 37 requests 30.6 / 29.0, 55 (not taken) 41 / 47, 58 57 / 47, 64
+// 60 / 50, 72 62 / 55, 76 (not taken) 62 / 69; of 4,000, 30 requests 78.7 / 79.0, 64 193 / 155; head size 64, 40 requests 19.0 / 17.0,
+// 55 22.7 / 21.6, 64 (not taken) 25 / 34, 76 38 / 35, 100 44 / 39, 111 45 / 43, 116 (not taken) 46 / 51.  Of 150 - 2,100 tokens, both dealt out
+// longest first: head size 128, 64 requests 50 / 44, head size 64, 100 requests 40.6 / 41.4.  Not `beside` a prompt's attention on a
+// second stream, whose blocks then find less room (31 tokens and a portion of 512, 3B sizes: a layer 1.4 % longer).
+struct DecodeShape {
+    bool deep, longest_first;
+};
+template <int HD> static DecodeShape decode_shape(int n_requests, int nkv, int group, int splits, bool beside) {
+    static int fits[2][2] = {};                              // [groups of at most 8 heads][deep]
+    int* f = fits[group <= 8];
+    if (!f[0]) {
+        f[1] = decode_fits<HD, kDeepStages<HD>>(group);
+        f[0] = decode_fits<HD, kDecStages>(group);
+    }
+    const long long blocks = (long long)n_requests * nkv, shallow = (long long)f[0] * num_sms(), deep = (long long)f[1] * num_sms();
+    DecodeShape s;
+    s.deep = splits == 1 && !beside && (blocks <= deep || (blocks > shallow && blocks <= 2 * deep));
+    const long long room = s.deep ? deep : shallow;
+    s.longest_first = splits == 1 && n_requests <= kThreads && blocks > room && blocks <= 2 * room;
+    return s;
 }
 
 LSB_API int lsb_decode_max_cluster(int hd) { return hd == 64 ? max_cluster<64>() : hd == 128 ? max_cluster<128>() : 8; }
@@ -838,7 +912,7 @@ static int decode_launch(const void* qkv, int qkv_stride, void* k_pages, void* v
                          const int* block_table, int table_stride, void* out, float* scratch,
                          int n_requests, int nh, int nkv, int hd, int page_size, int num_pages,
                          float scale, int window, int splits, const float* inv_freq, int rotary_dim,
-                         int store_kv, int max_cluster_size, cudaStream_t stream) {
+                         int store_kv, int max_cluster_size, bool beside, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (nkv <= 0 || nh % nkv || nh / nkv > 16 || splits < 1 || n_requests > 65535 || nkv > 65535)
         return (int)cudaErrorInvalidValue;
@@ -853,14 +927,18 @@ static int decode_launch(const void* qkv, int qkv_stride, void* k_pages, void* v
     do {                                                                                           \
         int rc = configure_once<HD>();                                                             \
         if (rc) return rc;                                                                         \
-        rc = lsb_launch(nh / nkv <= 8 ? decode_attention_kernel<HD, true>                          \
-                                      : decode_attention_kernel<HD, false>,                        \
-            grid, dim3(kThreads), decode_smem<HD>(), stream,                                       \
+        const DecodeShape shape = decode_shape<HD>(n_requests, nkv, nh / nkv, splits, beside);     \
+        const bool low8 = nh / nkv <= 8;                                                           \
+        rc = lsb_launch(shape.deep ? low8 ? decode_attention_kernel<HD, true, kDeepStages<HD>>     \
+                                          : decode_attention_kernel<HD, false, kDeepStages<HD>>    \
+                                   : low8 ? decode_attention_kernel<HD, true, kDecStages>          \
+                                          : decode_attention_kernel<HD, false, kDecStages>,        \
+            grid, dim3(kThreads), shape.deep ? decode_smem<HD, kDeepStages<HD>>() : decode_smem<HD>(), stream, \
             in_cluster ? splits : 1,                                                               \
             (const bf16*)qkv, qkv_stride, (bf16*)k_pages, (bf16*)v_pages, q_start,                \
             kv_len, table_rows, block_table, table_stride, (bf16*)out, part_o, part_ml, nh, nkv,  \
             page_size, num_pages, scale, window, splits, in_cluster ? 1 : 0, inv_freq, rotary_dim,  \
-            store_kv);                                                                             \
+            store_kv, shape.longest_first ? 1 : 0);                                                \
         if (rc) return rc;                                                                         \
         if (splits > 1 && !in_cluster)                                                             \
             rc = lsb_launch(decode_merge_kernel<HD>, dim3(nh, n_requests), dim3(64), 0, stream, 1, \
@@ -881,26 +959,26 @@ LSB_API int lsb_decode_attention(const void* qkv, int qkv_stride, const void* k_
                                  float scale, int window, int splits, cudaStream_t stream) {
     return decode_launch(qkv, qkv_stride, const_cast<void*>(k_pages), const_cast<void*>(v_pages), q_start,
                          kv_len, table_rows, block_table, table_stride, out, scratch, n_requests, nh, nkv,
-                         hd, page_size, num_pages, scale, window, splits, nullptr, 0, 0, 0, stream);
+                         hd, page_size, num_pages, scale, window, splits, nullptr, 0, 0, 0, false, stream);
 }
 
 // The same over a projection that has not been rotated yet: the kernel rotates the queries and the
 // new key by `inv_freq` (rotary_dim / 2 entries; rotary_dim a multiple of 16, at most hd: the dims
 // from there on pass through) at position kv_len - 1 and, if `store_kv`, writes the new key and
 // value into their page.  Replaces the separate rotary kernel
-// for single decode tokens.
+// for single decode tokens.  `beside`: a prompt's attention runs on another stream meanwhile.
 LSB_API int lsb_decode_attention_rope(const void* qkv, int qkv_stride, void* k_pages, void* v_pages,
                                       const int* q_start, const int* kv_len, const int* table_rows,
                                       const int* block_table, int table_stride, void* out, float* scratch,
                                       int n_requests, int nh, int nkv, int hd, int page_size,
                                       int num_pages, float scale, int window, int splits,
-                                      const float* inv_freq, int rotary_dim, int store_kv,
+                                      const float* inv_freq, int rotary_dim, int store_kv, int beside,
                                       cudaStream_t stream) {
     if (!inv_freq || rotary_dim < 16 || rotary_dim % 16 || rotary_dim > hd)
         return (int)cudaErrorInvalidValue;
     return decode_launch(qkv, qkv_stride, k_pages, v_pages, q_start, kv_len, table_rows, block_table,
                          table_stride, out, scratch, n_requests, nh, nkv, hd, page_size, num_pages,
-                         scale, window, splits, inv_freq, rotary_dim, store_kv, 0, stream);
+                         scale, window, splits, inv_freq, rotary_dim, store_kv, 0, beside != 0, stream);
 }
 
 // Prompt portions (and, unless skip_single, single tokens too).  bf16, hd 64 or 128.
@@ -985,5 +1063,5 @@ LSB_API int lsb_decode_attention_noalloc(const void* qkv, int qkv_stride, const 
     return decode_launch(qkv, qkv_stride, const_cast<void*>(k_pages), const_cast<void*>(v_pages), q_start,
                          kv_len, table_rows, block_table, table_stride, out, scratch, n_requests, nh, nkv,
                          hd, page_size, num_pages, scale, window, splits, nullptr, 0, 0, kNoAllocCluster,
-                         stream);
+                         false, stream);
 }

@@ -682,8 +682,8 @@ _decode_occupancy: Dict[tuple, int] = {}
 
 def decode_splits(n_decode: int, nkv: int, device=None, hd: int = 64, group: int = 4) -> int:
     """How many ways each request's keys are split among thread blocks in the decode kernel: as many
-    as fill four fifths of the blocks the SMs hold at once (four an SM at head size 64, two at 128,
-    where a block has twice the registers and shared memory), never a second round of blocks.
+    as fill four fifths of the blocks the SMs hold at once (four an SM at head size 64, three at 128,
+    where a block has more registers and twice the shared memory), never a second round of blocks.
     Measured inside decode steps at context 4096: head size 64, 8 requests: 7 splits (6: 1 % slower,
     9: 10 %); 32 requests: 2 (1: 14 % slower, 3: 10 %); head size 128, 8 requests: 4 or 5 splits 27 -
     28 us a layer, 7 splits (a second round for four blocks) 42 us; 32 requests: 1 split 84 us, 2
@@ -898,7 +898,8 @@ def paged_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache, s
                   _i(splits), on)
         else:
             _call("attention_tc", "lsb_decode_attention_rope", *common, _p(scratch), _i(R), *tail,
-                  _i(splits), _p(decode_rope[0]), _i(decode_rope[2]), _i(1 if decode_rope[1] else 0), on)
+                  _i(splits), _p(decode_rope[0]), _i(decode_rope[2]), _i(1 if decode_rope[1] else 0),
+                  _i(0 if stream is None else 1), on)
     if n_decode < R and only != "single":
         # prompt portions: tcgen05 kernel for long ones (128-row tiles), mma.sync kernel otherwise
         # The grid has a slab of blocks per request, and blocks that find a single token leave at
