@@ -10,7 +10,7 @@
 //   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three
 //   others of its part.  The sums of a group meet once, over lanes by halving exchanges and over the two parts in shared
 //   memory, in a fixed order.
-//   The four products of a layer at 1B sizes, 8 rows (243 MB): 71 us (3.4 TB/s); as 64 x 64 tiles, 56 of their 64 rows
+//   The four products of a layer at 1B sizes, 8 rows (243 MB): 57 us (4.3 TB/s); as 64 x 64 tiles, 56 of their 64 rows
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
 //   four times the exchanges at the end of a group: 89 us.)
 //
@@ -51,6 +51,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast
 // 16 bytes from global to shared memory, zeros where `have` is false (nothing is read then)
 __device__ __forceinline__ void copy16(uint32_t dst, const float* src, bool have) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(have ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy16(uint32_t dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -96,21 +99,46 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
     const int at = kg * 128 + lane * 4;        // this thread's place in a step of 256
     const uint32_t base = smem_u32(ring) + (uint32_t)at * 4u;
 
-    auto copy_w = [&](int it) {
-        const int g = (int)blockIdx.x + (it / chunks) * (int)gridDim.x, k0 = it % chunks * kKS + at;
-        const int n0 = g * p.per, rows = min(p.per, p.N - n0);
-        const uint32_t st = base + (uint32_t)(it % ST) * (kRB + MT) * kKS * 4u;
+    constexpr uint32_t kStage = (kRB + MT) * kKS * 4u;
+    // The copies' place, carried along: group, chunk of K and bytes into the ring.  (Found anew for each stage by dividing, and every
+    // copy guarded, 16,384 x 2,048 gated took 26.4 us where it takes 21.3 with four rows, 32.0 and 26.6 with eight, 46.2 and 39.6 with
+    // sixteen: two warps a scheduler are bound by their own instructions.)
+    int to_g = (int)blockIdx.x, to_chunk = 0;
+    uint32_t to = 0;
+    auto copy_stage = [&]() {
+        const int k0 = to_chunk * kKS + at, n0 = to_g * p.per, rows = min(p.per, p.N - n0);
+        const float* src = p.w + (size_t)(n0 + rg * kRW) * p.K + k0;
+        const float* xs = x + (size_t)rg * p.K + k0;
+        const uint32_t st = base + to + (uint32_t)(rg * kRW) * kKS * 4u, sx = base + to + (uint32_t)(kRB + rg) * kKS * 4u;
+        if (to_chunk * kKS + kKS <= p.K && rg * kRW + kRW <= rows && M == MT) {
 #pragma unroll
-        for (int i = 0; i < kRW; ++i) {
-            const int r = rg * kRW + i;
-            if (r >= rows) break;
-            const float* src = p.w + (size_t)(n0 + r) * p.K;
+            for (int i = 0; i < kRW; ++i, src += p.K) {
+                copy16(st + (uint32_t)i * kKS * 4u, src);
+                copy16(st + (uint32_t)(i * kKS + 256) * 4u, src + 256);
+            }
+#pragma unroll
+            for (int m = 0; m < MT; m += 4, xs += 4 * (size_t)p.K) {
+                if (MT < 4 && rg >= MT) break;
+                copy16(sx + (uint32_t)m * kKS * 4u, xs);
+                copy16(sx + (uint32_t)(m * kKS + 256) * 4u, xs + 256);
+            }
+        } else {
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int k = k0 + 256 * j;
-                copy16(st + (uint32_t)(r * kKS + 256 * j) * 4u, k < p.K ? src + k : p.w, k < p.K);
+                const bool in = k0 + 256 * j < p.K;
+#pragma unroll
+                for (int i = 0; i < kRW; ++i)
+                    if (rg * kRW + i < rows) copy16(st + (uint32_t)(i * kKS + 256 * j) * 4u, in ? src + (size_t)i * p.K + 256 * j : p.w, in);
+#pragma unroll
+                for (int m = 0; m < MT; m += 4) {
+                    if (rg + m >= MT) break;
+                    const bool have = in && rg + m < M;
+                    copy16(sx + (uint32_t)(m * kKS + 256 * j) * 4u, have ? xs + (size_t)m * p.K + 256 * j : p.x, have);
+                }
             }
         }
+        to = to + kStage == ST * kStage ? 0 : to + kStage;
+        if (++to_chunk == chunks) { to_chunk = 0; to_g += (int)gridDim.x; }
     };
     auto warm_w = [&](int it) {                // (a lane's 16 bytes are an eighth of a line)
         const int g = (int)blockIdx.x + (it / chunks) * (int)gridDim.x, k0 = it % chunks * kKS + at;
@@ -120,46 +148,32 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
             for (int k = k0; k < min(p.K, k0 + kKS); k += 256)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (size_t)(n0 + r) * p.K + k));
     };
-    auto copy_x = [&](int it) {
-        const int k0 = it % chunks * kKS + at;
-        const uint32_t st = base + ((uint32_t)(it % ST) * (kRB + MT) + kRB) * kKS * 4u;
-#pragma unroll
-        for (int m = rg; m < MT; m += 4)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int k = k0 + 256 * j;
-                const bool have = m < M && k < p.K;
-                copy16(st + (uint32_t)(m * kKS + 256 * j) * 4u, have ? x + (size_t)m * p.K + k : p.x, have);
-            }
-    };
     // w may be what the kernel before has yet to write: ahead of the wait its first lines are only asked for (L2, where
     // writes go too), and read behind it
     for (int it = 0; it < ST - 1 && it < total; ++it) warm_w(it);
     lsb_pdl_wait();
     for (int it = 0; it < ST - 1; ++it) {
-        if (it < total) { copy_w(it); copy_x(it); }
+        if (it < total) copy_stage();
         copies_commit();
     }
     float acc[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[v] = 0.f;
     int chunk = 0, done = 0;
+    const float* st = ring + at;
     for (int it = 0; it < total; ++it) {
         copies_wait<ST - 2>();
         // the four warps of this part of K share the rows of x; past this point none still reads the stage before
         asm volatile("bar.sync %0, 128;" ::"r"(1 + kg) : "memory");
-        if (it + ST - 1 < total) { copy_w(it + ST - 1); copy_x(it + ST - 1); }
+        if (it + ST - 1 < total) copy_stage();
         copies_commit();
-        const int n0 = ((int)blockIdx.x + done * (int)gridDim.x) * p.per, rows = min(p.per, p.N - n0);
-        const float* st = ring + (size_t)(it % ST) * (kRB + MT) * kKS + at;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             if (chunk * kKS + kg * 128 + 256 * j >= p.K) break;       // (the warp's whole step lies past K)
             float4 wv[kRW];
 #pragma unroll
-            for (int i = 0; i < kRW; ++i)
-                wv[i] = rg * kRW + i < rows ? *reinterpret_cast<const float4*>(st + (rg * kRW + i) * kKS + 256 * j)
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i = 0; i < kRW; ++i)           // (what stands in rows the group does not have goes into sums of their own)
+                wv[i] = *reinterpret_cast<const float4*>(st + (rg * kRW + i) * kKS + 256 * j);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const float4 xv = *reinterpret_cast<const float4*>(st + (kRB + m) * kKS + 256 * j);
@@ -172,7 +186,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
                 }
             }
         }
+        st = st + kStage / 4 == ring + at + ST * (kStage / 4) ? ring + at : st + kStage / 4;
         if (++chunk < chunks) continue;
+        const int n0 = ((int)blockIdx.x + done * (int)gridDim.x) * p.per, rows = min(p.per, p.N - n0);
         // the group's sums: lanes exchange halves until each holds V / 32 of them (or one, by several lanes) ...
         int n = V, first = 0;
 #pragma unroll
