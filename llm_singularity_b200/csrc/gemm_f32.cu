@@ -10,7 +10,7 @@
 //   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three
 //   others of its part.  The sums of a group meet once, over lanes by halving exchanges and over the two parts in shared
 //   memory, in a fixed order.
-//   The four products of a layer at 1B sizes, 8 rows (243 MB): 57 us (4.3 TB/s); as 64 x 64 tiles, 56 of their 64 rows
+//   The four products of a layer at 1B sizes, 8 rows (243 MB): 71 us (3.4 TB/s); as 64 x 64 tiles, 56 of their 64 rows
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
 //   four times the exchanges at the end of a group: 89 us.)
 //
@@ -101,8 +101,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
 
     constexpr uint32_t kStage = (kRB + MT) * kKS * 4u;
     // The copies' place, carried along: group, chunk of K and bytes into the ring.  (Found anew for each stage by dividing, and every
-    // copy guarded, 16,384 x 2,048 gated took 26.4 us where it takes 21.3 with four rows, 32.0 and 26.6 with eight, 46.2 and 39.6 with
-    // sixteen: two warps a scheduler are bound by their own instructions.)
+    // copy guarded, PLACEOLD.)
     int to_g = (int)blockIdx.x, to_chunk = 0;
     uint32_t to = 0;
     auto copy_stage = [&]() {
@@ -110,12 +109,25 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
         const float* src = p.w + (size_t)(n0 + rg * kRW) * p.K + k0;
         const float* xs = x + (size_t)rg * p.K + k0;
         const uint32_t st = base + to + (uint32_t)(rg * kRW) * kKS * 4u, sx = base + to + (uint32_t)(kRB + rg) * kKS * 4u;
-        if (to_chunk * kKS + kKS <= p.K && rg * kRW + kRW <= rows && M == MT) {
+        const bool whole = to_chunk * kKS + kKS <= p.K;
+        if (whole && rg * kRW + kRW <= rows) {
 #pragma unroll
             for (int i = 0; i < kRW; ++i, src += p.K) {
                 copy16(st + (uint32_t)i * kKS * 4u, src);
                 copy16(st + (uint32_t)(i * kKS + 256) * 4u, src + 256);
             }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kRW; ++i, src += p.K) {
+                if (rg * kRW + i >= rows) break;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const bool in = k0 + 256 * j < p.K;
+                    copy16(st + (uint32_t)(i * kKS + 256 * j) * 4u, in ? src + 256 * j : p.w, in);
+                }
+            }
+        }
+        if (whole && M == MT) {
 #pragma unroll
             for (int m = 0; m < MT; m += 4, xs += 4 * (size_t)p.K) {
                 if (MT < 4 && rg >= MT) break;
@@ -124,16 +136,12 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const bool in = k0 + 256 * j < p.K;
+            for (int m = 0; m < MT; m += 4, xs += 4 * (size_t)p.K) {
+                if (MT < 4 && rg >= MT) break;
 #pragma unroll
-                for (int i = 0; i < kRW; ++i)
-                    if (rg * kRW + i < rows) copy16(st + (uint32_t)(i * kKS + 256 * j) * 4u, in ? src + (size_t)i * p.K + 256 * j : p.w, in);
-#pragma unroll
-                for (int m = 0; m < MT; m += 4) {
-                    if (rg + m >= MT) break;
-                    const bool have = in && rg + m < M;
-                    copy16(sx + (uint32_t)(m * kKS + 256 * j) * 4u, have ? xs + (size_t)m * p.K + 256 * j : p.x, have);
+                for (int j = 0; j < 2; ++j) {
+                    const bool have = rg + m < M && k0 + 256 * j < p.K;
+                    copy16(sx + (uint32_t)(m * kKS + 256 * j) * 4u, have ? xs + 256 * j : p.x, have);
                 }
             }
         }
