@@ -24,18 +24,20 @@
 //   of 300 to 1,500 tokens, 32 / 8 heads of 64 in 32-bit (29 MB): 24 us; one warp for each (request, head)
 //   walking all of its keys took 1,548 us.  The kernel can rotate the token's queries and key and store the key and value by
 //   itself (every block takes them from the projection, one writes the page), which saves a kernel of 4 us in the chain of
-//   a decode step, and asks for its first keys while the projection is computed: a layer at 1B sizes, 8 requests, 110 -> 100 us.
+//   a step of single tokens whose blocks the SMs hold at once, and asks for its first keys while the projection is computed: a layer at 1B sizes, 8 requests, 110 -> 100 us.
 // * Portions are arithmetic: 64 rows (16 queries of 4 heads that share their keys) against a tile, 4 rows by 2 or 4
 //   keys a thread for the scores and the same 4 rows for the weighted sum, so that a row's maximum, its sum and its
 //   probabilities stay within half a warp; two multiply-adds to an instruction.  The last rows of a portion see the most
 //   keys, and few portions leave SMs idle: the tiles of a block's keys are dealt out over a cluster, whose sums meet
-//   as those of single tokens do.  500 tokens, the same heads: 85 us (1.0 GFLOP), 91 with a block to all of its
-//   keys; 120 tokens after 300 31 and 68, 40 after 300 20 and 50; a warp for each (row, head) took 650 us for the 500.
+//   as those of single tokens do.  500 tokens, the same heads: 83 us (1.0 GFLOP), 91 with a block to all of its
+//   keys; 120 tokens after 300 31 and 68, 40 after 300 19 and 50; a warp for each (row, head) took 650 us for the 500.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
 #include <float.h>
 #include <math.h>
+
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -63,9 +65,15 @@ struct AttnParams {
     const float* slopes;
     int heads;                                  // query heads of a block
     int head_blocks;                            // blocks of a kv head's group
-    int splits;                                 // (portions) blocks that share out a block's keys
-    // (single tokens, null: done already) the projection comes unrotated: dims i and i + rotary_dim / 2 turn by p * inv_freq[i], and
-    // the new key and value go to their page if `store`
+};
+// What only some kernels take is no parameter of the others: with it behind theirs the compiler makes them 2 - 5 % slower (64 tokens at
+// 500 keys, 8 kv heads of 128: 117.2 -> 122.8 us).
+struct SplitParams : AttnParams {
+    int splits;                                 // blocks that share out a portion's keys
+};
+// Single tokens whose projection comes unrotated: dims i and i + rotary_dim / 2 turn by position * inv_freq[i], and the new key and
+// value go to their page if `store`.
+struct RotatingParams : AttnParams {
     const float* inv_freq;
     int rotary_dim, store;
 };
@@ -123,22 +131,16 @@ struct Tile {
             }
         }
     }
-    // (returns whether every value of this thread's is a number and finite)  own: the row of a token's own key, which is at
-    // `fresh`, its value behind it (-1: none)
-    __device__ __forceinline__ bool park(const AttnParams& p, float* ks, float* vs, int ldk, int tid, int own = -1,
-                                         const float* fresh = nullptr) const {
+    // (returns whether every value of this thread's is a number and finite)
+    __device__ __forceinline__ bool park(const AttnParams& p, float* ks, float* vs, int ldk, int tid) const {
         const int per = p.hd >> 2;
         float zero = 0.f;                                      // times a number 0, times anything else NaN
 #pragma unroll
         for (int j = 0; j < kPieces; ++j) {
             const int idx = j * kThreads + tid, row = idx / per, d = (idx - row * per) * 4;
             if (row < KT) {
-                float4 u = widen(k[j]), w = widen(v[j]);
-                if (row == own) {
-                    u = *reinterpret_cast<const float4*>(fresh + d);
-                    w = *reinterpret_cast<const float4*>(fresh + p.hd + d);
-                }
-                *reinterpret_cast<float4*>(ks + row * ldk + d) = u;
+                *reinterpret_cast<float4*>(ks + row * ldk + d) = widen(k[j]);
+                const float4 w = widen(v[j]);
                 *reinterpret_cast<float4*>(vs + row * p.hd + d) = w;
                 zero = fmaf(w.x, zero, fmaf(w.y, zero, fmaf(w.z, zero, w.w * zero)));
             }
@@ -168,19 +170,22 @@ __device__ __forceinline__ float modified(const AttnParams& p, float s, float sl
 constexpr int kAccs = 4;
 
 template <int KT>
-static size_t single_smem(int hd, int heads) {
-    return ((size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)heads * hd * 2 + (size_t)heads * (KT + 4) + heads * 4 + 2 * (size_t)hd) * 4;
+static size_t single_smem(int hd, int heads, bool rotates) {
+    return ((size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)heads * hd * 2 + (size_t)heads * (KT + 4) + heads * 4 + (rotates ? 2 * (size_t)hd : 0)) * 4;
 }
 
-template <typename T, int KT, int HDC>
-__global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const AttnParams p) {
+// P: AttnParams, or RotatingParams to rotate and store.
+template <typename T, int KT, int HDC, typename P>
+__global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const P p) {
+    constexpr bool ROTATES = std::is_same<P, RotatingParams>::value;
     extern __shared__ __align__(16) float sm[];
     __shared__ long long off[2][KT];
-    __shared__ float cs[2][kMaxHeadDim / 2];                   // cosines and sines of the token's position
+    __shared__ float cs[2][ROTATES ? kMaxHeadDim / 2 : 1];     // cosines and sines of the token's position
     cg::cluster_group cluster = cg::this_cluster();
     lsb_pdl_launch_dependents();
-    // The step's metadata and tables are there before its first kernel, so all that follows from them is had before the wait
-    // for the projection, the first keys and values among it.
+    // The step's metadata and tables are there before its first kernel, so with a rotation all that follows from them is had before
+    // the wait for the projection, the first keys and values among it.
+    if constexpr (!ROTATES) lsb_pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int splits = (int)gridDim.x, split = (int)blockIdx.x, r = blockIdx.z;
     const int g = blockIdx.y / p.head_blocks, group = p.nh / p.nkv;
@@ -203,9 +208,16 @@ __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const Att
     const int first = lo + split * per, last = min(pos + 1, first + per);     // [first, last), maybe empty
     const int* table = p.block_table + (size_t)p.table_rows[r] * p.table_stride;
 
-    const bool rotates = p.inv_freq != nullptr, stores = rotates && p.store;
-    const int half = rotates ? p.rotary_dim >> 1 : 0;
-    for (int i = tid; i < half; i += kThreads) sincosf((float)pos * p.inv_freq[i], &cs[1][i], &cs[0][i]);
+    const T* token = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.qkv_stride;
+    bool stores = false;
+    int half = 0;
+    if constexpr (ROTATES) {
+        stores = p.store;
+        half = p.rotary_dim >> 1;
+        for (int i = tid; i < half; i += kThreads) sincosf((float)pos * p.inv_freq[i], &cs[1][i], &cs[0][i]);
+    } else {
+        for (int i = tid; i < H * hd; i += kThreads) qs[i] = lsb_to_float(token[(size_t)h0 * hd + i]) * p.scale;
+    }
     if (tid < H) { ml[4 * tid] = -FLT_MAX; ml[4 * tid + 1] = 0.f; }
     if (tid < KT) off[0][tid] = first + tid < last ? key_offset(p, table, g, first + tid) : -1;
     float acc[kAccs];
@@ -213,36 +225,47 @@ __global__ void __launch_bounds__(kThreads, 2) attention_single_kernel(const Att
     for (int a = 0; a < kAccs; ++a) acc[a] = 0.f;
     __syncthreads();
     Tile<T, KT, HDC> tile;
-    // (what its page holds of a key that comes with the projection is not used; one that another layer's kernel writes in this
-    // step is waited for)
-    const bool early = stores || pos < first || pos >= first + KT;
-    if (early) tile.fetch(p, off[0], tid);
-    lsb_pdl_wait();
-    if (!early) tile.fetch(p, off[0], tid);
-    const T* token = reinterpret_cast<const T*>(p.qkv) + (size_t)t * p.qkv_stride;
-    // element d of a head at x, rotated, as the projection's type holds it
-    auto turned = [&](const T* x, int d) -> float {
-        if (d >= 2 * half) return lsb_to_float(x[d]);
-        const int i = d < half ? d : d - half;
-        const float x0 = lsb_to_float(x[i]), x1 = lsb_to_float(x[i + half]);
-        return lsb_to_float(lsb_from_float<T>(d < half ? x0 * cs[0][i] - x1 * cs[1][i] : x0 * cs[1][i] + x1 * cs[0][i]));
-    };
-    for (int i = tid; i < H * hd; i += kThreads) qs[i] = turned(token + (size_t)(h0 + i / hd) * hd, i % hd) * p.scale;
-    if (stores && pos >= first && pos < last) {
-        const long long to = blockIdx.y % p.head_blocks == 0 ? key_offset(p, table, g, pos) : -1;       // (one block writes)
-        for (int d = tid; d < hd; d += kThreads) {
-            const float u = turned(token + (size_t)(p.nh + g) * hd, d), w = lsb_to_float(token[(size_t)(p.nh + p.nkv + g) * hd + d]);
-            fresh[d] = u;
-            fresh[hd + d] = w;
-            if (to >= 0) {
-                reinterpret_cast<T*>(const_cast<void*>(p.k_pages))[to + d] = lsb_from_float<T>(u);
-                reinterpret_cast<T*>(const_cast<void*>(p.v_pages))[to + d] = lsb_from_float<T>(w);
+    if constexpr (!ROTATES) {
+        tile.fetch(p, off[0], tid);
+    } else {
+        // (what its page holds of a key that comes with the projection is not used; one that another layer's kernel writes in this
+        // step is waited for)
+        const bool early = stores || pos < first || pos >= first + KT;
+        if (early) tile.fetch(p, off[0], tid);
+        lsb_pdl_wait();
+        if (!early) tile.fetch(p, off[0], tid);
+        // element d of a head at x, rotated, as the projection's type holds it
+        auto turned = [&](const T* x, int d) -> float {
+            if (d >= 2 * half) return lsb_to_float(x[d]);
+            const int i = d < half ? d : d - half;
+            const float x0 = lsb_to_float(x[i]), x1 = lsb_to_float(x[i + half]);
+            return lsb_to_float(lsb_from_float<T>(d < half ? x0 * cs[0][i] - x1 * cs[1][i] : x0 * cs[1][i] + x1 * cs[0][i]));
+        };
+        for (int i = tid; i < H * hd; i += kThreads) qs[i] = turned(token + (size_t)(h0 + i / hd) * hd, i % hd) * p.scale;
+        if (stores && pos >= first && pos < last) {
+            const long long to = blockIdx.y % p.head_blocks == 0 ? key_offset(p, table, g, pos) : -1;       // (one block writes)
+            for (int d = tid; d < hd; d += kThreads) {
+                const float u = turned(token + (size_t)(p.nh + g) * hd, d), w = lsb_to_float(token[(size_t)(p.nh + p.nkv + g) * hd + d]);
+                fresh[d] = u;
+                fresh[hd + d] = w;
+                if (to >= 0) {
+                    reinterpret_cast<T*>(const_cast<void*>(p.k_pages))[to + d] = lsb_from_float<T>(u);
+                    reinterpret_cast<T*>(const_cast<void*>(p.v_pages))[to + d] = lsb_from_float<T>(w);
+                }
             }
         }
+        __syncthreads();
     }
-    __syncthreads();
     for (int base = first, turn = 0; base < last; base += KT, turn ^= 1) {
-        tile.park(p, ks, vs, ldk, tid, stores && pos < last ? pos - base : -1, fresh);
+        tile.park(p, ks, vs, ldk, tid);
+        if (stores && pos < last && pos - base < KT) {
+            // the token's own key and value over what their page held, by the threads that have just put it there
+            const int row = pos - base, pieces = hd >> 2, piece = (tid + kThreads - row * pieces % kThreads) % kThreads;
+            if (piece < pieces) {
+                *reinterpret_cast<float4*>(ks + row * ldk + piece * 4) = *reinterpret_cast<const float4*>(fresh + piece * 4);
+                *reinterpret_cast<float4*>(vs + row * hd + piece * 4) = *reinterpret_cast<const float4*>(fresh + hd + piece * 4);
+            }
+        }
         const int next = base + KT;
         if (tid < KT) off[turn ^ 1][tid] = next + tid < last ? key_offset(p, table, g, next + tid) : -1;
         __syncthreads();
@@ -344,17 +367,22 @@ static size_t portion_smem(int hd) {
     return ((size_t)kRows * (hd + 4) + (size_t)KT * (hd + 4) + (size_t)KT * hd + (size_t)kRows * (KT + 4)) * 4;
 }
 
-template <typename T, int KT, int HDC>
-__global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portion_kernel(const AttnParams p) {
+// P: AttnParams, or SplitParams where a cluster of p.splits blocks shares out the keys of its rows.  (One kernel for both: 500
+// tokens at 4,000 keys, 32 / 8 heads of 64 in 32-bit, whole, 746 us where it takes 691.)
+template <typename T, int KT, int HDC, typename P>
+__global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portion_kernel(const P p) {
+    constexpr bool SPLIT = std::is_same<P, SplitParams>::value;
     constexpr int KPT = KT / 16;                // keys of a thread's scores
     constexpr int CPT = HDC / 64;               // groups of four columns of a thread's sums
     extern __shared__ __align__(16) float sm[];
     __shared__ long long off[2][KT];
-    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ float slopes[kRows];             // of the rows' heads
     lsb_pdl_launch_dependents();
     lsb_pdl_wait();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, r = blockIdx.z;
-    const int splits = p.splits, split = (int)blockIdx.x % splits;
+    int splits = 1;
+    if constexpr (SPLIT) splits = p.splits;
+    const int split = SPLIT ? (int)blockIdx.x % splits : 0;
     const int g = blockIdx.y / p.head_blocks, group = p.nh / p.nkv;
     const int h0 = g * group + (int)(blockIdx.y % p.head_blocks) * p.heads;
     const int H = min(p.heads, (g + 1) * group - h0);
@@ -370,7 +398,7 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
     const int pos0 = p.kv_len[r] - q_len + i0;                 // of the block's first query
     const int pos_last = min(pos0 + queries, p.kv_len[r]) - 1;
     // this block's tiles: every splits-th
-    const int lo = ((p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0) + split * KT, stride = splits * KT;
+    const int lo = ((p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0) + split * KT, stride = SPLIT ? splits * KT : KT;
     const int* table = p.block_table + (size_t)p.table_rows[r] * p.table_stride;
 
     // row x: query i0 + x / heads, head h0 + x % heads (rows beyond the portion or the group stay zero)
@@ -381,6 +409,9 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
             : 0.f;
     }
     if (tid < KT) off[0][tid] = lo + tid <= pos_last ? key_offset(p, table, g, lo + tid) : -1;
+    if (p.slopes && tid < kRows) slopes[tid] = tid % p.heads < H ? p.slopes[h0 + tid % p.heads] : 0.f;
+    // (a row sees the keys whose distance is below this: one unsigned comparison for both of its ends)
+    const unsigned reach = p.window > 0 ? (unsigned)p.window : 0x7fffffffu;
     int pos[4];
     float m[4], l[4];
     pair32 acc[4][2 * CPT];
@@ -428,15 +459,13 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
         for (int i = 0; i < 4; ++i) {
             float s[KPT], mx = m[i];
             bool seen[KPT];
-            // (worked out again for every tile: registers are short)
-            const int row_lo = p.window > 0 ? pos[i] - p.window + 1 : 0, head = p.slopes ? (ty * 4 + i) % p.heads : H;
-            const float slope = head < H ? p.slopes[h0 + head] : 0.f;
+            const float slope = p.slopes ? slopes[ty * 4 + i] : 0.f;
 #pragma unroll
             for (int j = 0; j < KPT; ++j) {
                 const int key = base + tx + 16 * j;
                 float u, v;
                 apart(s2[i][j], u, v);
-                seen[j] = key <= pos[i] && key >= row_lo && off[turn][tx + 16 * j] >= 0;
+                seen[j] = (unsigned)(pos[i] - key) < reach && off[turn][tx + 16 * j] >= 0;
                 s[j] = seen[j] ? modified(p, u + v, slope, pos[i] - key) : -FLT_MAX;
                 mx = fmaxf(mx, s[j]);
             }
@@ -466,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
                 if (off[turn][k] < 0) continue;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    if (base + k > pos[i] || (p.window > 0 && base + k < pos[i] - p.window + 1)) continue;
+                    if ((unsigned)(pos[i] - (base + k)) >= reach) continue;
                     const pair32 we = twice(ps[(ty * 4 + i) * ldp + k]);
 #pragma unroll
                     for (int c = 0; c < CPT; ++c) {
@@ -504,7 +533,8 @@ __global__ void __launch_bounds__(kThreads, HDC <= 128 ? 2 : 1) attention_portio
         }
         __syncthreads();
     }
-    if (splits > 1) {
+    if constexpr (SPLIT) {
+        cg::cluster_group cluster = cg::this_cluster();
         // the blocks' sums meet: each brings its share of the rows together, blocks in order
         float* os = qs;                                        // [kRows][ldk] (the queries have been used)
         float* ml = ps;                                        // [kRows] (maximum, sum)
@@ -577,7 +607,8 @@ static int num_sms() {
 }
 
 // clusters of consecutive blocks along x
-static int launch_clusters(void (*kernel)(AttnParams), dim3 grid, size_t smem, unsigned cluster, const AttnParams& p, cudaStream_t stream) {
+template <typename P>
+static int launch_clusters(void (*kernel)(P), dim3 grid, size_t smem, unsigned cluster, const P& p, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreads);
@@ -619,15 +650,19 @@ static int portion_splits(long long blocks, long long room, int longest, int sho
     return best;
 }
 
+// rot: null, or the rotation of single tokens
 template <typename T, int KT, int HDC>
-static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int max_keys, cudaStream_t stream) {
+static int launch(AttnParams p, const RotatingParams* rot, int n_requests, int max_q_len, int n_single, int max_keys, cudaStream_t stream) {
     static int configured = -1;
     const int group = p.nh / p.nkv;
     if (configured < 0) {
-        // (the largest either kernel asks for: heads of HDC, as many as a block takes of the smallest, 16)
-        configured = (int)cudaFuncSetAttribute(attention_single_kernel<T, KT, HDC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (!configured)
-            configured = (int)cudaFuncSetAttribute(attention_portion_kernel<T, KT, HDC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        // (the largest any of them asks for: heads of HDC, as many as a block takes of the smallest, 16)
+        const auto allow = [](auto kernel) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); };
+        int rc = allow(attention_single_kernel<T, KT, HDC, AttnParams>);
+        if (!rc) rc = allow(attention_single_kernel<T, KT, HDC, RotatingParams>);
+        if (!rc) rc = allow(attention_portion_kernel<T, KT, HDC, AttnParams>);
+        if (!rc) rc = allow(attention_portion_kernel<T, KT, HDC, SplitParams>);
+        configured = rc;
     }
     if (configured) return configured;
     if (n_single > 0) {
@@ -642,8 +677,16 @@ static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int
         if (max_keys > 0 && splits > (max_keys + KT - 1) / KT) splits = (max_keys + KT - 1) / KT;
         splits = splits < 1 ? 1 : splits > kMaxSplits ? kMaxSplits : splits;
         if ((long long)p.nkv * s.head_blocks > 65535) return (int)cudaErrorInvalidValue;
-        const int rc = launch_clusters(attention_single_kernel<T, KT, HDC>, dim3((unsigned)splits, p.nkv * s.head_blocks, n_requests),
-                                       single_smem<KT>(p.hd, s.heads), (unsigned)splits, s, stream);
+        const dim3 grid((unsigned)splits, p.nkv * s.head_blocks, n_requests);
+        const size_t smem = single_smem<KT>(p.hd, s.heads, rot != nullptr);
+        int rc;
+        if (rot) {
+            RotatingParams turned = *rot;
+            static_cast<AttnParams&>(turned) = s;
+            rc = launch_clusters(attention_single_kernel<T, KT, HDC, RotatingParams>, grid, smem, (unsigned)splits, turned, stream);
+        } else {
+            rc = launch_clusters(attention_single_kernel<T, KT, HDC, AttnParams>, grid, smem, (unsigned)splits, s, stream);
+        }
         if (rc) return rc;
     }
     if (max_q_len > 1) {
@@ -651,16 +694,19 @@ static int launch(AttnParams p, int n_requests, int max_q_len, int n_single, int
         p.head_blocks = (group + p.heads - 1) / p.heads;
         if ((long long)p.nkv * p.head_blocks > 65535) return (int)cudaErrorInvalidValue;
         const int queries = kRows / p.heads;
-        const long long tiles = (max_q_len + queries - 1) / queries, blocks = tiles * p.nkv * p.head_blocks;
+        const long long tiles = (max_q_len + queries - 1) / queries;
+        const long long blocks = tiles * p.nkv * p.head_blocks;
         // (where the contexts are not known, they are taken for the portions alone)
         const int keys = max_keys > max_q_len ? max_keys : max_q_len;
-        p.splits = portion_splits(blocks * (n_requests > n_single ? n_requests - n_single : 1), (HDC <= 128 ? 2 : 1) * num_sms(), (keys + KT - 1) / KT,
-                                  (keys - max_q_len) / KT + 1);
-        if (tiles * p.splits > 0x7fffffffll) return (int)cudaErrorInvalidValue;
-        const dim3 grid((unsigned)(tiles * p.splits), p.nkv * p.head_blocks, n_requests);
-        // (a launch in clusters of one was 8 % slower)
-        if (p.splits == 1) return lsb_launch(attention_portion_kernel<T, KT, HDC>, grid, dim3(kThreads), portion_smem<KT>(p.hd), stream, 1, p);
-        return launch_clusters(attention_portion_kernel<T, KT, HDC>, grid, portion_smem<KT>(p.hd), p.splits, p, stream);
+        const int splits = portion_splits(blocks * (n_requests > n_single ? n_requests - n_single : 1), (HDC <= 128 ? 2 : 1) * num_sms(), (keys + KT - 1) / KT,
+                                          (keys - max_q_len) / KT + 1);
+        if (tiles * splits > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+        const dim3 grid((unsigned)(tiles * splits), p.nkv * p.head_blocks, n_requests);
+        if (splits == 1) return lsb_launch(attention_portion_kernel<T, KT, HDC, AttnParams>, grid, dim3(kThreads), portion_smem<KT>(p.hd), stream, 1, p);
+        SplitParams parts;
+        static_cast<AttnParams&>(parts) = p;
+        parts.splits = splits;
+        return launch_clusters(attention_portion_kernel<T, KT, HDC, SplitParams>, grid, portion_smem<KT>(p.hd), (unsigned)splits, parts, stream);
     }
     return 0;
 }
@@ -680,11 +726,16 @@ LSB_API int lsb_paged_attention_generic(
     if (n_requests > 65535 || nh > 65535) return (int)cudaErrorInvalidValue;
     if (inv_freq && (rotary_dim < 0 || rotary_dim > hd || rotary_dim % 2 || qkv_stride < (nh + 2 * nkv) * hd)) return (int)cudaErrorInvalidValue;
     const AttnParams p{qkv, qkv_stride, k_pages, v_pages, q_start, kv_len, table_rows, block_table, table_stride, out,
-                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0, 1, inv_freq, rotary_dim, store};
+                       nh, nkv, hd, page_size, num_pages, scale, window, softcap, slopes, 0, 0};
+    RotatingParams rot;
+    rot.inv_freq = inv_freq;
+    rot.rotary_dim = rotary_dim;
+    rot.store = store;
+    const RotatingParams* rotation = inv_freq ? &rot : nullptr;
     LSB_DISPATCH_DTYPE(dtype, {
-        if (hd <= 64) return launch<T, 64, 64>(p, n_requests, max_q_len, n_single, max_keys, stream);
-        if (hd <= 128) return launch<T, 32, 128>(p, n_requests, max_q_len, n_single, max_keys, stream);
-        return launch<T, 32, 256>(p, n_requests, max_q_len, n_single, max_keys, stream);
+        if (hd <= 64) return launch<T, 64, 64>(p, rotation, n_requests, max_q_len, n_single, max_keys, stream);
+        if (hd <= 128) return launch<T, 32, 128>(p, rotation, n_requests, max_q_len, n_single, max_keys, stream);
+        return launch<T, 32, 256>(p, rotation, n_requests, max_q_len, n_single, max_keys, stream);
     });
     return 0;
 }

@@ -775,6 +775,18 @@ def _batch_shape(ctx):
     return shape
 
 
+def _single_tokens_rotate(ctx, nh: int, nkv: int, hd: int, device) -> bool:
+    """Where the generic kernel rotates by itself: in a step of single tokens alone (beside a portion the rotary kernel runs all the
+    same: 8 tokens at 2,000 keys and a portion of 40, head size 64, 66.5 us with and 70.3 without it) whose blocks the
+    SMs hold at once (64 tokens at 500 keys, 8 kv heads of 128: 117 us with the rotary kernel, 119 without; 8 at 1,000 52 and
+    49)."""
+    n_decode = _batch_shape(ctx)[0]
+    if n_decode != ctx.n_requests or nkv <= 0 or hd <= 0:     # (what no kernel takes is refused further on)
+        return False
+    heads = max(1, 1024 // hd)                                # most query heads of a block
+    return n_decode * nkv * -(-(nh // nkv) // heads) <= 2 * num_sms(device)
+
+
 def rope_store_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache,
                          inv_freq: Optional[torch.Tensor], rotary_dim: int, store: bool,
                          scale: float, window: int, out: torch.Tensor, softcap: float = 0.0,
@@ -788,14 +800,15 @@ def rope_store_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cac
         paged_attention(qkv, nh, nkv, hd, ctx, cache, scale, window, out, softcap=softcap, slopes=slopes)
         return
     on_tc = tensor_core_attention_ok(qkv.dtype, hd, nh, nkv)
-    fuse = FUSE_DECODE_ROPE and 0 < rotary_dim <= hd and inv_freq is not None and (rotary_dim % 16 == 0 or not on_tc)
+    fuse = FUSE_DECODE_ROPE and 0 < rotary_dim <= hd and inv_freq is not None and (
+        rotary_dim % 16 == 0 if on_tc else _single_tokens_rotate(ctx, nh, nkv, hd, qkv.device))
     n_decode = _batch_shape(ctx)[0] if fuse else 0
     if not n_decode:
         rope_kv_store(qkv, nh, nkv, hd, ctx, cache, inv_freq, rotary_dim, store)
         paged_attention(qkv, nh, nkv, hd, ctx, cache, scale, window, out)
         return
     if n_decode < ctx.n_requests:
-        if on_tc and OVERLAP_ATTENTION and not getattr(ctx, "fixed_launch", False):
+        if OVERLAP_ATTENTION and not getattr(ctx, "fixed_launch", False):
             # Single tokens and prompt portions are different requests with different pages: the
             # decode kernel (memory-bound) runs on a second stream beside the rotation and the
             # attention of the portions (compute-bound), and the step's stream waits for both.
