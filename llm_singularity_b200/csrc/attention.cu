@@ -629,30 +629,85 @@ static int launch_clusters(void (*kernel)(P), dim3 grid, size_t smem, unsigned c
     return (int)cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-// Blocks that share out the keys of a portion's rows.  Blocks are taken to run in rounds of `room`, the longest first, the
-// lengths falling evenly from the longest to the shortest (tiles of keys); meeting costs a block as much as 0.3 to 0.6 of a
-// tile.  (32 / 8 heads of 64 in 32-bit, us with 1 / 2 / 4 / 6 blocks: 500 tokens 91 / 85 / 91 / 120, 240 45 / 31 / 36 / 52, 120 after
-// 300 68 / 51 / 31 / 43, 40 after 300 50 / 31 / 26 / 19, 40 12 / 14 / 16 / 19; 16 / 8 of 256 in bfloat16, 300 after 2,000 812 / 793 / 636 / 597.)
-static int portion_splits(long long blocks, long long room, int longest, int shortest) {
+// Blocks that share out the keys of a portion's rows.  Blocks are taken to run in rounds of `room(s)`, the longest first, the
+// lengths falling evenly from the longest to the shortest (tiles of keys).  A block's set-up and end cost it as much as 0.6 of a
+// tile, 0.8 where a cluster meets, and clusters have to promise 5 % (all fitted to 57 shapes in one to eight parts: no choice is slower
+// than whole blocks there, the geometric mean is 1.3 % above the best).  32 / 8 heads of 64 in 32-bit, us with 1 / 2 / 4 / 8 blocks, the
+// choice in front: 500 tokens (2) 97 / 88 / 94 / 142, 240 (2) 53 / 35 / 40 / 71, 40 (1) 15.6 / 20.5 / 16.6 / 21.1, 40 after 300 (6: 22) 59 / 43 / 32 /
+// 22, 40 after 3,960 (8) 510 / 261 / 189 / 102, 500 after 3,500 (1) 691 / 701 / 702 / 740, with a window of 1,000 (1) 185 / 200 / 211 / 239;
+// 16 / 8 of 256 in bfloat16, 300 after 2,000 (3: 578) 829 / 793 / 640 / 698.
+template <typename Room>
+static int portion_splits(long long blocks, Room room, int longest, int shortest) {
     int best = 1;
     double least = 0.0;
     for (int s = 1; s <= kMaxSplits && s <= longest; ++s) {
-        const long long n = blocks * s, rounds = (n + room - 1) / room;
+        const long long n = blocks * s, at_once = room(s), rounds = (n + at_once - 1) / at_once;
         if (s > 1 && rounds > 16) break;                       // (the SMs are busy without)
-        double cost = 0.0;
-        for (long long r = 0; r < rounds && r < 64; ++r) {
-            const double tiles = longest - (double)(longest - shortest) * (double)(r * room) / (double)n;
-            cost += ceil(tiles / s) + (s > 1 ? 0.6 : 0.3);
+        double cost = ceil((double)longest / s) + (s > 1 ? 0.8 : 0.6);
+        for (long long r = 1; r < rounds && r < 64; ++r) {
+            const double tiles = (longest - (double)(longest - shortest) * (double)(r * at_once) / (double)n) / s + 0.25;
+            cost += (tiles < 1.0 ? 1.0 : tiles) + (s > 1 ? 0.8 : 0.6);
         }
         if (rounds > 64) cost *= (double)rounds / 64.0;
+        if (s == 1) cost *= 0.95;
         if (s == 1 || cost < least) { least = cost; best = s; }
     }
     return best;
 }
+// Blocks of a portion kernel that run at once in clusters of `splits`: fewer than the SMs hold where clusters don't fill a group of SMs.
+template <typename T, int KT, int HDC>
+static long long portion_room(int hd, int splits) {
+    const long long whole = (HDC <= 128 ? 2ll : 1ll) * num_sms();
+    static int cached[64][kMaxHeadDim / 16 + 1][kMaxSplits + 1] = {};
+    int dev = 0;
+    if (splits == 1 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return whole;
+    int& clusters = cached[dev][hd / 16][splits];
+    if (clusters == 0) {
+        int n = 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(splits);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = portion_smem<KT>(hd);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = splits;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(attention_portion_kernel<T, KT, HDC, SplitParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, attention_portion_kernel<T, KT, HDC, SplitParams>, &cfg) != cudaSuccess || n <= 0) {
+            (void)cudaGetLastError();
+            n = (int)(whole / splits);
+        }
+        clusters = n < 1 ? 1 : n;
+    }
+    return (long long)clusters * splits;
+}
+// The blocks from the sizes of a step: `portions` requests of up to max_q_len tokens whose longest context is `keys`, 0 where it is
+// not known (a captured launch).  A window bounds what a block walks, whatever the context; without either, the portions
+// are taken to be all of their contexts (captured portions of 500: 88 us as a prompt where whole blocks take 97, 701 after 3,500 where
+// they take 691; all with the rotary kernel in front).
+template <typename T, int KT, int HDC>
+static int splits_of_portions(int hd, int nh, int nkv, long long portions, int max_q_len, int keys, int window) {
+    const int group = nh / nkv, heads = group < kPortionHeads ? group : kPortionHeads, queries = kRows / heads;
+    const long long tiles = (max_q_len + queries - 1) / queries, blocks = tiles * nkv * ((group + heads - 1) / heads) * portions;
+    const long long seen = window > 0 ? (long long)window + queries - 1 : 0x7fffffffll;       // most keys of a block
+    long long most = keys > max_q_len ? keys : max_q_len, least = most - max_q_len + 1;
+    if (window > 0 && keys <= 0) most = least = seen;
+    most = most < seen ? most : seen;
+    least = least < most ? least : most;
+    return portion_splits(blocks, [&](int s) { return portion_room<T, KT, HDC>(hd, s); }, (int)((most + KT - 1) / KT), (int)((least + KT - 1) / KT));
+}
+LSB_API int lsb_portion_splits(int hd, int nh, int nkv, int portions, int max_q_len, int keys, int window) {
+    return hd <= 64    ? splits_of_portions<float, 64, 64>(hd, nh, nkv, portions, max_q_len, keys, window)
+           : hd <= 128 ? splits_of_portions<float, 32, 128>(hd, nh, nkv, portions, max_q_len, keys, window)
+                       : splits_of_portions<float, 32, 256>(hd, nh, nkv, portions, max_q_len, keys, window);
+}
 
 // rot: null, or the rotation of single tokens
 template <typename T, int KT, int HDC>
-static int launch(AttnParams p, const RotatingParams* rot, int n_requests, int max_q_len, int n_single, int max_keys, cudaStream_t stream) {
+static int launch(AttnParams p, const RotatingParams* rot, int n_requests, int max_q_len, int n_single, int max_keys, int portion_keys,
+                  cudaStream_t stream) {
     static int configured = -1;
     const int group = p.nh / p.nkv;
     if (configured < 0) {
@@ -695,11 +750,7 @@ static int launch(AttnParams p, const RotatingParams* rot, int n_requests, int m
         if ((long long)p.nkv * p.head_blocks > 65535) return (int)cudaErrorInvalidValue;
         const int queries = kRows / p.heads;
         const long long tiles = (max_q_len + queries - 1) / queries;
-        const long long blocks = tiles * p.nkv * p.head_blocks;
-        // (where the contexts are not known, they are taken for the portions alone)
-        const int keys = max_keys > max_q_len ? max_keys : max_q_len;
-        const int splits = portion_splits(blocks * (n_requests > n_single ? n_requests - n_single : 1), (HDC <= 128 ? 2 : 1) * num_sms(), (keys + KT - 1) / KT,
-                                          (keys - max_q_len) / KT + 1);
+        const int splits = splits_of_portions<T, KT, HDC>(p.hd, p.nh, p.nkv, n_requests > n_single ? n_requests - n_single : 1, max_q_len, portion_keys, p.window);
         if (tiles * splits > 0x7fffffffll) return (int)cudaErrorInvalidValue;
         const dim3 grid((unsigned)(tiles * splits), p.nkv * p.head_blocks, n_requests);
         if (splits == 1) return lsb_launch(attention_portion_kernel<T, KT, HDC, AttnParams>, grid, dim3(kThreads), portion_smem<KT>(p.hd), stream, 1, p);
@@ -712,13 +763,14 @@ static int launch(AttnParams p, const RotatingParams* rot, int n_requests, int m
 }
 
 // qkv: [tokens, qkv_stride] with the nh*hd query values first in each row.  softcap: 0 for none; slopes: float [nh] or
-// null.  n_single: requests that bring one token; max_keys: the longest context (0: not known, the launch is captured).
+// null.  n_single: requests that bring one token; max_keys, portion_keys: the longest context, and of those with more tokens (0: not known,
+// the launch is captured).
 // inv_freq: null, or the rotation of single tokens (float [rotary_dim / 2]), which come unrotated then, keys and values behind the
 // queries in their rows; `store`: and not yet in their pages.
 LSB_API int lsb_paged_attention_generic(
     const void* qkv, int qkv_stride, const void* k_pages, const void* v_pages,
     const int* q_start, const int* kv_len, const int* table_rows, const int* block_table,
-    int table_stride, void* out, int dtype, int n_requests, int max_q_len, int n_single, int max_keys,
+    int table_stride, void* out, int dtype, int n_requests, int max_q_len, int n_single, int max_keys, int portion_keys,
     int nh, int nkv, int hd, int page_size, int num_pages, float scale, int window,
     float softcap, const float* slopes, const float* inv_freq, int rotary_dim, int store, cudaStream_t stream) {
     if (n_requests <= 0 || max_q_len <= 0) return 0;
@@ -733,9 +785,9 @@ LSB_API int lsb_paged_attention_generic(
     rot.store = store;
     const RotatingParams* rotation = inv_freq ? &rot : nullptr;
     LSB_DISPATCH_DTYPE(dtype, {
-        if (hd <= 64) return launch<T, 64, 64>(p, rotation, n_requests, max_q_len, n_single, max_keys, stream);
-        if (hd <= 128) return launch<T, 32, 128>(p, rotation, n_requests, max_q_len, n_single, max_keys, stream);
-        return launch<T, 32, 256>(p, rotation, n_requests, max_q_len, n_single, max_keys, stream);
+        if (hd <= 64) return launch<T, 64, 64>(p, rotation, n_requests, max_q_len, n_single, max_keys, portion_keys, stream);
+        if (hd <= 128) return launch<T, 32, 128>(p, rotation, n_requests, max_q_len, n_single, max_keys, portion_keys, stream);
+        return launch<T, 32, 256>(p, rotation, n_requests, max_q_len, n_single, max_keys, portion_keys, stream);
     });
     return 0;
 }

@@ -775,6 +775,15 @@ def _batch_shape(ctx):
     return shape
 
 
+def _portion_keys(ctx) -> int:
+    """The longest context of the requests that bring more than one token (0: there are none); kept like the above."""
+    longest = getattr(ctx, "_portion_keys", None)
+    if longest is None:
+        longest = int(ctx.h_kv_len.max(where=ctx.h_q_len != 1, initial=0))
+        ctx._portion_keys = longest
+    return longest
+
+
 def _single_tokens_rotate(ctx, nh: int, nkv: int, hd: int, device) -> bool:
     """Where the generic kernel rotates by itself: in a step of single tokens alone (beside a portion the rotary kernel runs all the
     same: 8 tokens at 2,000 keys and a portion of 40, head size 64, 66.5 us with and 70.3 without it) whose blocks the
@@ -846,7 +855,8 @@ def paged_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache, s
     bfloat16 with head size 64 or 128 runs on the tensor cores: single decode tokens in the
     split-KV kernel, prompt portions in the tiled kernel.  Everything else (32-bit, other head
     sizes) runs the generic kernels, whose cut of a single token's keys depends on how many single tokens the step
-    holds and on its longest context (not in a captured step).  ``decode_rope = (inv_freq, store, rotary_dim)`` says that
+    holds and on its longest context, and that of a portion's on how many portions there are, their most tokens and
+    their longest context (a captured step's on its numbers of requests and tokens alone).  ``decode_rope = (inv_freq, store, rotary_dim)`` says that
     single tokens come unrotated and not yet in the cache (see ``rope_store_attention``).  ``only``: "single"
     or "portions" launches just that kernel; ``stream``: a raw stream to launch on instead of the
     current one."""
@@ -880,9 +890,9 @@ def paged_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache, s
             raise KernelError("attention: scores are modified where queries and keys come rotated")
         rotation = (None, False, 0) if decode_rope is None else decode_rope
         # (a captured launch has to serve contexts of any length)
-        longest = 0 if getattr(ctx, "fixed_launch", False) else ctx.max_kv_len
+        longest, of_portions = (0, 0) if getattr(ctx, "fixed_launch", False) else (ctx.max_kv_len, _portion_keys(ctx))
         _call("attention", "lsb_paged_attention_generic", *common, _i(_dt(qkv)), _i(ctx.n_requests), _i(ctx.max_q_len),
-              _i(_batch_shape(ctx)[0]), _i(longest), *tail, _f(softcap), _p(slopes),
+              _i(_batch_shape(ctx)[0]), _i(longest), _i(of_portions), *tail, _f(softcap), _p(slopes),
               _p(rotation[0]), _i(rotation[2]), _i(1 if rotation[1] else 0), _stream(out))
         return
     R = ctx.n_requests
