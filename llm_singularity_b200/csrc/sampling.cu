@@ -17,9 +17,9 @@
 // k, for the largest few lanes' maxima of each stretch: the k-th largest of those is a value that at least k values
 // reach, and seldom many more.  Those few are collected, and one block makes both cuts and the draw among them.  A cut
 // by mass alone takes a histogram over the values near the maximum, linear in the distance to it, that the blocks
-// add up through distributed shared memory: a value adds its part of the bucket's upper end, as a count and a 32-bit
-// remainder (64-bit additions in shared memory are loops of compare and swap: 183 us for 128 rows that made them for
-// all values), and the values of the one bucket the cut falls into are picked among by counting.
+// add up through distributed shared memory: a value adds its part of the bucket's upper end, as a count and a whole
+// number of its exponential's last places, in 32-bit (64-bit additions in shared memory are loops of compare and swap: 183 us for 128
+// rows that made them for all values), and the values of the one bucket the cut falls into are picked among by counting.
 // A larger k takes a histogram of counts over the whole row first; a bucket with more than kList values (rows
 // whose values are all but equal, or with outliers that stretch the range) is bisected instead, on the order-preserving
 // integer image of the floats, as many as 32 walks.  Few rows leave their values, divided, in shared memory for the walks
@@ -60,6 +60,9 @@ constexpr int kFewK = 128;                    // a k whose values the stretches'
 constexpr int kTops = 8;                      // most of a stretch's lanes' maxima that are looked at
 constexpr int kPool = 2 * kFewK + kMaxStretches;              // ... of all stretches together
 constexpr float kNear = 10.f;                 // how far below the maximum the histogram of masses goes at first
+constexpr float kStep = kNear / (kBuckets - 1);               // ... a bucket's
+constexpr float kRestScale = 16777216.f;      // 2^24, places of what a value lacks to the upper end of its bucket
+constexpr double kMostRest = 0.01;            // ... more than any lacks (1 - e^(-kNear / 1023))
 constexpr int kSliceBytes = 176 * 1024;       // most shared memory for a slice
 
 __device__ __forceinline__ unsigned int ordered(float f) {
@@ -92,7 +95,7 @@ struct Shared {
     unsigned int cnt[kBuckets];               // this block's histogram
     union {
         u64 mass[kBuckets];
-        unsigned int rest[kBuckets];          // what the counted values' masses lack to the upper end of their bucket
+        unsigned int rest[2 * kBuckets];      // what the counted values' masses lack to the upper end of their bucket (behind those: odd lanes')
         u64 list_mass[kList];
     };
     unsigned int tot_cnt[kBuckets];           // the row's, the same in every block
@@ -181,19 +184,13 @@ __device__ __forceinline__ int find_bucket(Shared<THREADS>& s, u64& before, Val 
     return s.found;
 }
 
-// e^(-b step), the exponent formed in 64-bit, the power good to 32-bit like every weight
-__device__ __forceinline__ double upper_end(int b, float step) {
-    const double e = -(double)b * ((double)step * 1.4426950408889634), whole = rint(e);
-    return (double)ldexpf(exp2f((float)(e - whole)), (int)whole);
-}
-
 // params per row: {temperature, top_p, repetition_penalty, u}.  stretch: values of a stretch; slice: of a block, whole stretches.
 // PARKED: the first walk leaves the row's values, penalties applied, in shared memory (`work` where a slice does not fit) for
 // the walks behind it; otherwise they are read, and divided by the temperature, again.
 template <int THREADS, bool PARKED, int PER_SM>
 __global__ void __launch_bounds__(THREADS, PER_SM)
 sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vocab, int stretch, int slice, int slice_in_smem,
-              float mass_scale, float rest_scale, const float* __restrict__ params, const int* __restrict__ top_ks,
+              float mass_scale, int near, const float* __restrict__ params, const int* __restrict__ top_ks,
               const int* __restrict__ prev_start, const int* __restrict__ prev_tokens, int* __restrict__ out) {
     constexpr int kWarps = THREADS / 32;
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -588,14 +585,18 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
             cluster.sync();
         };
         // The same for the values down to kNear below the maximum, in one walk with the mass of those that are kept further down,
-        // which is returned.  Within a bucket a mass is its upper end's, e^(-b step), times 1 - r with r below 1 %: r is added up as
-        // a 32-bit integer (rest_scale leaves room for a slice of them; its last place is no more than that of the
-        // exponential).
+        // which is returned.  Within a bucket a mass is its upper end's, e^(-b step), times 1 - r with r below 1 %: 1 - r is an
+        // exponential of 24 bits, so r is a whole number of 2^-24, which 32-bit integers add up without a loss (a value that is a
+        // rounding above the upper end lacks nothing).  `near`: how many of them a bucket takes, by odd and even lanes, so that a
+        // slice's values fit.
         auto near_histogram = [&]() -> u64 {
-            const float step = kNear / (kBuckets - 1);
-            for (int b = tid; b < kBuckets; b += THREADS) { s.cnt[b] = 0u; s.rest[b] = 0u; }
+            for (int b = tid; b < kBuckets; b += THREADS) {
+                s.cnt[b] = s.rest[b] = 0u;
+                if (near > 1) s.rest[kBuckets + b] = 0u;
+            }
             __syncthreads();
             u64 beyond = 0ull;
+            const int half = near > 1 ? (lane & 1) * kBuckets : 0;
             for (int st = warp; st < stretches; st += kWarps) {
                 float part = 0.f;
                 walk(st, [&](int, const float (&v)[4], int m) {
@@ -604,13 +605,14 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
                         const float x = divided(v[e]);
                         if (e < m && ordered(x) >= thr) {
                             const float d = mx - x;
-                            if (d <= span) {
-                                const int b = bucket(x);
+                            const int b = bucket(x);
+                            const float w = expf(b < kBuckets ? fmaf((float)b, kStep, -d) : -d);      // (one exponential for both)
+                            if (b < kBuckets) {
                                 atomicAdd(&s.cnt[b], 1u);
-                                const unsigned int r = __float2uint_rn((1.f - expf(fmaf((float)b, step, -d))) * rest_scale);
-                                if (r) atomicAdd(&s.rest[b], r);
+                                const unsigned int r = __float2uint_rn((1.f - w) * kRestScale);
+                                if (r) atomicAdd(&s.rest[half + b], r);
                             } else {
-                                part += weight_of(x);
+                                part += w > 0.f ? w : 0.f;
                             }
                         }
                     }
@@ -619,18 +621,27 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
             }
             beyond = block_sum(lane == 0 ? beyond : 0ull, s);
             if (tid == 0) s.tail = beyond;
-            cluster.sync();
+            auto arrival = cluster.barrier_arrive();
+            const int share = kBuckets / blocks;
+            double ends[kBuckets / THREADS];
+#pragma unroll
+            for (int i = 0; i < kBuckets / THREADS; ++i) {
+                const int j = tid + i * THREADS;
+                ends[i] = j < share ? exp(-(double)(rank * share + j) * (double)kStep) * (double)mass_scale : 0.0;
+            }
+            cluster.barrier_wait(std::move(arrival));
             u64 all = 0ull;
             of_blocks(&s.tail, [&](u64 x) { all += x; });
-            const int share = kBuckets / blocks;
-            for (int j = tid; j < share; j += THREADS) {
-                const int b = rank * share + j;
+#pragma unroll
+            for (int i = 0; i < kBuckets / THREADS; ++i) {
+                const int j = tid + i * THREADS, b = rank * share + j;
+                if (j >= share) continue;
                 unsigned int c = 0u;
-                u64 rest = 0ull;
+                u64 lack = 0ull;
                 of_blocks(&s.cnt[b], [&](unsigned int x) { c += x; });
-                of_blocks(&s.rest[b], [&](unsigned int x) { rest += x; });
-                const u64 m = c ? __double2ull_rn(upper_end(b, step) * ((double)c - (double)rest / (double)rest_scale) * (double)mass_scale)
-                                : 0ull;
+                of_blocks(&s.rest[b], [&](unsigned int x) { lack += x; });
+                if (near > 1) of_blocks(&s.rest[kBuckets + b], [&](unsigned int x) { lack += x; });
+                const u64 m = __double2ull_rn(ends[i] * ((double)c - (double)lack * (1.0 / (double)kRestScale)));
                 for (int r = 0; r < blocks; ++r) {
                     *cluster.map_shared_rank(&s.tot_cnt[b], r) = c;
                     *cluster.map_shared_rank(&s.tot_mass[b], r) = m;
@@ -716,13 +727,12 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
             // the smallest v with mass(x > v) <= top_p * (mass kept so far); everything >= v is kept.  Most of the mass lies
             // near the maximum and most of the values do not: the histogram goes kNear down (e^-10 of the maximum's weight)
             // first, all the way if the cut lies further.
-            const bool near = rest_scale > 0.f;
             double tot = 0.0, most = 0.0;
             span = kNear;
             inv = (float)(kBuckets - 1) / kNear;
             ranged = false;
             u64 before = 0ull, beyond = 0ull;
-            if (near) beyond = near_histogram();
+            if (near > 0) beyond = near_histogram();
             else {
                 tot = row_mass([&](float x) { return ordered(x) >= thr ? weight_of(x) : 0.f; });
                 most = (double)top_p * tot;
@@ -731,7 +741,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int vo
             auto find = [&](bool first) {
                 return find_bucket(s, before, [&](int i) { return s.tot_mass[i]; },
                                    [&](u64 sum) {
-                                       if (!near || !first) return;
+                                       if (near == 0 || !first) return;
                                        tot = (double)(sum + beyond);
                                        most = (double)top_p * tot;
                                    },
@@ -935,9 +945,9 @@ LSB_API int lsb_sample(const float* logits, float* work, int rows, int vocab, co
     int log2 = 0;
     while (log2 < 31 && (1ll << log2) < vocab) ++log2;
     const float mass_scale = (float)(1ull << (63 - log2 < 44 ? 63 - log2 : 44));
-    // what a bucket's masses lack is less than 1 % each: places of 2^-23 have to fit a slice
     const Plan p = plan(vocab);
-    const float rest_scale = (double)p.slice * 0.01 * 8388608.0 < 4294967296.0 ? 8388608.f : 0.f;
+    const double rest = p.slice * kMostRest * kRestScale;    // most that a bucket of a block lacks (half of it is even lanes')
+    const int near = rest < 4294967296.0 ? 1 : rest < 2 * 4294967296.0 ? 2 : 0;
     // Two blocks with their slices in shared memory fit an SM, four without.  Rows, us with and without (and with a histogram
     // for each cut): 128,256 logits, 8 blocks a row: 8 27 / 44 (28), 32 31 / 48 (34), 64 50 / 53 (60), 101 67 / 65 (83), 127 82 / 77 (99),
     // 256 156 / 134 (208); 32,000, 4 blocks: 8 19 / 30 (18), 64 22 / 32 (23), 101 29 / 33 (33), 127 34 / 32 (38); 50,257, 8 blocks: 64 40 / 35
@@ -954,9 +964,9 @@ LSB_API int lsb_sample(const float* logits, float* work, int rows, int vocab, co
         if (configured) return configured;
         if (!smem && !work) return (int)cudaErrorInvalidValue;
         return lsb_launch(blocks <= num_sms() ? sample_kernel<512, true, 1> : sample_kernel<512, true, 2>, dim3(rows, 1, p.blocks), dim3(512), smem,
-                          stream, p.blocks, logits, work, vocab, p.stretch, p.slice, smem ? 1 : 0, mass_scale, rest_scale, params, top_k,
+                          stream, p.blocks, logits, work, vocab, p.stretch, p.slice, smem ? 1 : 0, mass_scale, near, params, top_k,
                           prev_start, prev_tokens, out);
     }
     return lsb_launch(sample_kernel<256, false, 4>, dim3(rows, 1, p.blocks), dim3(256), 0, stream, p.blocks, logits, work, vocab,
-                      p.stretch, p.slice, 0, mass_scale, rest_scale, params, top_k, prev_start, prev_tokens, out);
+                      p.stretch, p.slice, 0, mass_scale, near, params, top_k, prev_start, prev_tokens, out);
 }
