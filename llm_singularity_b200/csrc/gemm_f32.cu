@@ -43,6 +43,8 @@
 #include <cooperative_groups.h>
 #include <cuda.h>
 
+#include <type_traits>
+
 namespace cg = cooperative_groups;
 
 LSB_DEFINE_STATUS()
@@ -245,10 +247,6 @@ struct TileParams {
     const float* w;
     float* out;
     int M, N, K, act;
-    // (split products)
-    int steps;                                 // stages of K a block takes, of a cluster along K
-    int tiles_m, tiles_n, tile0;               // tiles of the matrix, and the first of this launch
-    int rows_first;                            // neighbouring tiles share w
 };
 
 // outputs (m, n .. n + 3), as far as n goes, or what the gated product makes of them (N is even then)
@@ -502,24 +500,45 @@ struct SplitLayout {
     static_assert(kSM * LDT * 4 <= kRing * kRaw, "the sums leave through the ring");
 };
 
+// A launch of clusters along K, or of some of a matrix's tiles.
+struct PartParams : TileParams {
+    int steps;                                 // stages of K a block takes
+    int tiles_m, tiles_n, tile0;               // tiles of the matrix, and the first of this launch
+};
+// Tiles that run side by side share w (rows of tiles first), which is the larger operand then; else x.
 template <int BN>
+__host__ __device__ __forceinline__ bool rows_first(int M, int N) { return M <= N && (N + BN - 1) / BN <= 65535; }
+
+// P: TileParams (a block for all of K of every tile) or PartParams.  (As one kernel, whole products of a short K took 0.6 us
+// a round more: 640 x 2,048 x 512 17.7 -> 18.4 us, 2,000 x 2,048 x 512 34.4 -> 35.9.)
+template <int BN, typename P>
 __global__ void __launch_bounds__(kSThreads, 1)
-gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const TileParams p) {
+gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const P p) {
+    constexpr bool PARTS = std::is_same<P, PartParams>::value;
     using L = SplitLayout<BN>;
     constexpr int R = L::kRing;
     extern __shared__ unsigned char raw_smem[];
     unsigned char* ring = (unsigned char*)(((uintptr_t)raw_smem + 1023) & ~(uintptr_t)1023);
     unsigned char* planes = ring + (size_t)R * L::kRaw;
     __shared__ uint64_t raw_full[R], raw_empty[R], split_full[2], split_empty[2], acc_full[2], acc_empty[2], done;
-    __shared__ uint32_t tmem_slot, least[L::kRows], all_least[L::kRows];
+    __shared__ uint32_t tmem_slot, least[L::kRows], least_parts[PARTS ? L::kRows : 1];
     __shared__ int abort_flag, any_tiny;
     lsb_pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tile_at = p.tile0 + (int)blockIdx.x;
-    const int m0 = (p.rows_first ? tile_at % p.tiles_m : tile_at / p.tiles_n) * kSM, n0 = (p.rows_first ? tile_at / p.tiles_m : tile_at % p.tiles_n) * BN;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int splits = (int)gridDim.z, first = (int)blockIdx.z * p.steps;
-    const int steps = min(p.steps, (p.K + kSK - 1) / kSK - first);      // (at least one)
+    int m0, n0, splits = 1, first = 0, steps = (p.K + kSK - 1) / kSK;
+    if constexpr (PARTS) {
+        const int at = p.tile0 + (int)blockIdx.x;
+        m0 = rows_first<BN>(p.M, p.N) ? at % p.tiles_m : at / p.tiles_n;
+        n0 = rows_first<BN>(p.M, p.N) ? at / p.tiles_m : at % p.tiles_n;
+        splits = (int)gridDim.z;
+        first = (int)blockIdx.z * p.steps;
+        steps = min(p.steps, steps - first);                            // (at least one)
+    } else {
+        m0 = rows_first<BN>(p.M, p.N) ? blockIdx.x : blockIdx.y;
+        n0 = rows_first<BN>(p.M, p.N) ? blockIdx.y : blockIdx.x;
+    }
+    m0 *= kSM;
+    n0 *= BN;
     if (tid < L::kRows) least[tid] = 0xffffffffu;
     if (tid == 0) {
         abort_flag = any_tiny = 0;
@@ -681,21 +700,28 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     }
     __syncwarp();
     // the sums of all stretches of K are there, each in its block; a block brings its share of the rows together
-    if (splits > 1) cluster.sync();
+    cg::cluster_group cluster = cg::this_cluster();
+    if (PARTS && splits > 1) cluster.sync();
     else __syncthreads();
     if (warp < kSWorkers / 32 && !abort_flag) {
         const float* tile = reinterpret_cast<const float*>(ring);
-        const int share = kSM / splits, row0 = (int)blockIdx.z * share, rows = (int)blockIdx.z == splits - 1 ? kSM - row0 : share;
+        int row0 = 0, rows = kSM;
+        if constexpr (PARTS) {
+            row0 = (int)blockIdx.z * (kSM / splits);
+            rows = (int)blockIdx.z == splits - 1 ? kSM - row0 : kSM / splits;
+        }
+        uint32_t* all_least = PARTS ? least_parts : least;
         // A number below 2^-103 loses less than 2^-125 with the parts that bfloat16 has no normal number for (one that
         // is not below has them all), which is at most K 2^-125 times the largest number of the other operand's row in
         // a sum.  Sums that this could show in are done over; the largest are looked up only where there is such a number.
         float* largest = reinterpret_cast<float*>(planes);              // [kRows] (every product has been waited for)
         bool tiny = any_tiny;
-        for (int k = 0; k < splits && splits > 1; ++k) tiny |= *cluster.map_shared_rank(&any_tiny, k) != 0;
+        if constexpr (PARTS)
+            for (int k = 0; k < splits && splits > 1; ++k) tiny |= *cluster.map_shared_rank(&any_tiny, k) != 0;
         if (tiny) {
             for (int r = warp; r < L::kRows; r += kSWorkers / 32) {
                 const bool of_x = r < kSM;
-                if (of_x && (r < row0 || r >= row0 + rows)) continue;
+                if (PARTS && of_x && (r < row0 || r >= row0 + rows)) continue;
                 const long long at = of_x ? m0 + r : n0 + r - kSM;
                 float big = 0.f;
                 if (at < (of_x ? p.M : p.N))
@@ -706,9 +732,11 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 big = lsb_warp_max(big);
                 if (lane == 0) {
                     largest[r] = big * ((float)p.K * 0x1p-101f);
-                    uint32_t least_of = least[r];
-                    for (int k = 0; k < splits && splits > 1; ++k) least_of = min(least_of, *cluster.map_shared_rank(&least[r], k));
-                    all_least[r] = least_of;
+                    if constexpr (PARTS) {
+                        uint32_t least_of = least[r];
+                        for (int k = 0; k < splits && splits > 1; ++k) least_of = min(least_of, *cluster.map_shared_rank(&least[r], k));
+                        all_least[r] = least_of;
+                    }
                 }
             }
             asm volatile("bar.sync 1, %0;" ::"n"(kSWorkers) : "memory");
@@ -718,7 +746,7 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             if (m0 + row >= p.M || n0 + col >= p.N) continue;
             __align__(16) float v[4];
             const float* at = tile + row * L::LDT + col;
-            if (splits > 1) {
+            if (PARTS && splits > 1) {
                 float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
                 for (int k = 0; k < splits; ++k) {                      // (in order)
@@ -742,7 +770,7 @@ gemm_split_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         }
     }
     __syncwarp();
-    if (splits > 1) cluster.sync();                                     // (a peer may still read this block's sums)
+    if (PARTS && splits > 1) cluster.sync();                            // (a peer may still read this block's sums)
     else __syncthreads();
     if (warp == kSWorkers / 32) {
         tmem_fence_after();
@@ -836,8 +864,8 @@ static int split_room(int splits) {
         attr[0].val.clusterDim.z = splits;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (splits == 1 || cudaFuncSetAttribute(gemm_split_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&clusters, gemm_split_f32_kernel<BN>, &cfg) != cudaSuccess || clusters <= 0) {
+        if (splits == 1 || cudaFuncSetAttribute(gemm_split_f32_kernel<BN, PartParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, gemm_split_f32_kernel<BN, PartParams>, &cfg) != cudaSuccess || clusters <= 0) {
             cudaGetLastError();
             clusters = num_sms() / splits;
         }
@@ -847,25 +875,42 @@ static int split_room(int splits) {
 }
 
 template <int BN>
-static int launch_split(TileParams p, int tile0, int tiles, int splits, cudaStream_t stream) {
-    using L = SplitLayout<BN>;
+static int split_maps(const TileParams& p, CUtensorMap* mx, CUtensorMap* mw) {
     static int configured = -1;
-    if (configured < 0)
-        configured = (int)cudaFuncSetAttribute(gemm_split_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
+    if (configured < 0) {
+        configured = (int)cudaFuncSetAttribute(gemm_split_f32_kernel<BN, TileParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SplitLayout<BN>::kTotal);
+        if (!configured)
+            configured = (int)cudaFuncSetAttribute(gemm_split_f32_kernel<BN, PartParams>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SplitLayout<BN>::kTotal);
+    }
     if (configured) return configured;
+    const int rc = map_rows(mx, p.x, p.M, p.K, kSM);
+    return rc ? rc : map_rows(mw, p.w, p.N, p.K, BN);
+}
+template <int BN>
+static int launch_whole(const TileParams& p, cudaStream_t stream) {
+    CUtensorMap mx, mw;
+    const int rc = split_maps<BN>(p, &mx, &mw);
+    if (rc) return rc;
+    const unsigned tiles_m = (p.M + kSM - 1) / kSM, tiles_n = (p.N + BN - 1) / BN;
+    if (!rows_first<BN>(p.M, p.N) && tiles_m > 65535) return (int)cudaErrorInvalidValue;
+    const dim3 grid = rows_first<BN>(p.M, p.N) ? dim3(tiles_m, tiles_n) : dim3(tiles_n, tiles_m);
+    return lsb_launch(gemm_split_f32_kernel<BN, TileParams>, grid, dim3(kSThreads), SplitLayout<BN>::kTotal, stream, 1, mx, mw, p);
+}
+template <int BN>
+static int launch_parts(const TileParams& tile, int tile0, int tiles, int splits, cudaStream_t stream) {
+    CUtensorMap mx, mw;
+    const int rc = split_maps<BN>(tile, &mx, &mw);
+    if (rc) return rc;
+    PartParams p;
+    static_cast<TileParams&>(p) = tile;
     // whole chunks of leading products a block; the last one may have fewer
     const int chunks = (p.K + kSK * kSChunk - 1) / (kSK * kSChunk), per = (chunks + splits - 1) / splits;
     p.steps = per * kSChunk;
     p.tiles_m = (p.M + kSM - 1) / kSM;
     p.tiles_n = (p.N + BN - 1) / BN;
     p.tile0 = tile0;
-    p.rows_first = p.M <= p.N;
     const dim3 grid(tiles, 1, (chunks + per - 1) / per);
-    CUtensorMap mx, mw;
-    int rc;
-    if ((rc = map_rows(&mx, p.x, p.M, p.K, kSM))) return rc;
-    if ((rc = map_rows(&mw, p.w, p.N, p.K, BN))) return rc;
-    return lsb_launch(gemm_split_f32_kernel<BN>, grid, dim3(kSThreads), L::kTotal, stream, (int)grid.z, mx, mw, p);
+    return lsb_launch(gemm_split_f32_kernel<BN, PartParams>, grid, dim3(kSThreads), SplitLayout<BN>::kTotal, stream, (int)grid.z, mx, mw, p);
 }
 
 LSB_API int lsb_gemm_f32_supported(const void* x, const void* w, int M, int N, int K) {
@@ -911,11 +956,12 @@ static SplitPlan split_plan(int M, int N, int K) {
 template <int BN>
 static int run_split(const TileParams& p, const SplitPlan& plan, cudaStream_t stream) {
     if (plan.tiles > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+    if (plan.splits == 1) return launch_whole<BN>(p, stream);
     if (plan.whole) {
-        const int rc = launch_split<BN>(p, 0, (int)plan.whole, 1, stream);
-        if (rc || plan.whole == plan.tiles) return rc;
+        const int rc = launch_parts<BN>(p, 0, (int)plan.whole, 1, stream);
+        if (rc) return rc;
     }
-    return launch_split<BN>(p, (int)plan.whole, (int)(plan.tiles - plan.whole), plan.splits, stream);
+    return launch_parts<BN>(p, (int)plan.whole, (int)(plan.tiles - plan.whole), plan.splits, stream);
 }
 
 // act: 0, or the activation of a gated product (1 silu, 2 gelu in its tanh form, 3 none), N even then.
@@ -937,7 +983,7 @@ LSB_API int lsb_gemm_f32(const float* x, const float* w, float* out, int M, int 
     // 10 % on most of 120 shapes; along the shortest K it picks too small a tile (500 x 20,000 x 20: 65 us, 128 x 128 29; 2,048 x
     // 2,048 x 64: 28, 128 x 256 18), whose sums are the closer ones: more warps share K out (K = 320, from the smallest tile to the
     // largest: 1.3, 1.7, 2.4 and 3.2e-7 of the norm).
-    const TileParams p{x, w, out, M, N, K, act, 0, 0, 0, 0, 0};
+    const TileParams p{x, w, out, M, N, K, act};
     const long long sms = num_sms();
     if (K >= kSplitK) {
         const SplitPlan plan = split_plan(M, N, K);
