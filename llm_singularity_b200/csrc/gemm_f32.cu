@@ -10,13 +10,13 @@
 //   in L2 before the wait on the kernel before, which may be the one that makes w) and shares the rows of x with the three
 //   others of its part.  The sums of a group meet once, over lanes by halving exchanges and over the two parts in shared
 //   memory, in a fixed order.
-//   The four products of a layer at 1B sizes, 8 rows (243 MB): 71 us (3.4 TB/s); as 64 x 64 tiles, 56 of their 64 rows
+//   The four products of a layer at 1B sizes, 8 rows (243 MB): 58 us (4.2 TB/s); as 64 x 64 tiles, 56 of their 64 rows
 //   empty and as few as 32 of them: 1,202 us.  (A thread's places of K for all sixteen rows, with no sharing at all, cost
 //   four times the exchanges at the end of a group: 89 us.)
 //
 // * More rows (a prompt), K from 512: the tensor cores.  A 32-bit value is exactly the sum of three bfloat16 values (8
 //   bits each of its 24), so a product is nine products of parts; the six that reach 2^-23 of it are taken, the other three
-//   are not.  Blocks of 128 x 128 outputs (x 64 where those fit the SMs at once) take x and w as they are by
+//   are not.  Blocks of 128 x 128 outputs, or 128 x 64 (split_plan, below, has the choice), take x and w as they are by
 //   TMA; sixteen warps, two groups by turns, split a stage of 32 along K, x's parts into tensor memory, w's into
 //   shared memory.  The tensor core cuts its sums rather than rounding them, so the leading products stay there for
 //   128 of K only and are then added up in registers; the five small ones have their own sums, 2^-8 as large.  Where tiles
@@ -35,8 +35,9 @@
 //   asynchronous copies, three to five in flight.  2,048 x 8,192 x 256: 200 us, 43 TFLOP/s of the 70 that a loop of
 //   nothing but multiply-adds reaches here.
 //
-// A row's sum is taken in an order that K and the kernel fix, the same from run to run; which kernel, and so the last digits,
-// depends on the number of rows beside it.
+// A row's sum is taken in an order that is the same from run to run.  M, N and K fix it: which kernel, into how many parts K is cut
+// for which of the tiles; so the last digits depend on the number of rows beside a row and, where whole tiles and shared-out
+// ones make up one product, on where in it a sum lies.
 #include "common.cuh"
 #include "gate_act.cuh"
 
@@ -103,7 +104,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) gemm_rows_f32_kernel(const Row
 
     constexpr uint32_t kStage = (kRB + MT) * kKS * 4u;
     // The copies' place, carried along: group, chunk of K and bytes into the ring.  (Found anew for each stage by dividing, and every
-    // copy guarded, PLACEOLD.)
+    // copy guarded, 16,384 x 2,048 gated took 28.0 us where it takes 23.0 with four rows, 33.7 and 28.3 with eight, 48.9 and 42.2 with
+    // twelve; 512 x 2,048 of twelve rows, whose x is copied guarded all the same, 6.9 and 7.0.)
     int to_g = (int)blockIdx.x, to_chunk = 0;
     uint32_t to = 0;
     auto copy_stage = [&]() {
@@ -917,17 +919,11 @@ LSB_API int lsb_gemm_f32_supported(const void* x, const void* w, int M, int N, i
     return M > 0 && N > 0 && K > 0 && K % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0 && M <= 32 * 65535;
 }
 
-// Columns of a split product's blocks that take all of K.  64 take 0.9 of the time of 128 (500 x 2,048 x 2,048: 46.3 and 52.0 us), so
-// only where one round does (500 x 3,072 x 2,048: 87.4 and 54.9).
-LSB_API int lsb_gemm_f32_split_columns(int M, int N) {
-    return (long long)((M + kSM - 1) / kSM) * ((N + 63) / 64) <= num_sms() ? 64 : 128;
-}
-
 // How a split product's tiles go to the SMs: `columns` wide, a block for all of K of the first `whole` of them, a cluster of `splits`
 // blocks along K for each of the rest.  A block takes about its fixed part and its stages (fitted to 20 shapes), a cluster some
 // 2.5 us more to meet; blocks run in rounds.  500 rows, us, whole and so: 2,048 x 2,048 44 / 31 (two parts), 2,048 x 8,192 161 / 95,
 // 16,384 x 2,048 gated 220 / 195 (three whole rounds, the rest in two parts), 3,072 x 2,048 52 / 52 (whole: 96 tiles); 40 rows
-// times 2,048 x 8,192 159 / 38 (eight parts); 300 times 16,384 x 2,048 160 / 159 (whole).
+// times 2,048 x 8,192 159 / 38 (six parts); 300 times 16,384 x 2,048 160 / 159 (whole).
 struct SplitPlan { int columns, splits; long long whole, tiles; };
 static SplitPlan split_plan(int M, int N, int K) {
     const int chunks = (K + kSK * kSChunk - 1) / (kSK * kSChunk);
@@ -952,6 +948,14 @@ static SplitPlan split_plan(int M, int N, int K) {
         }
     }
     return best;
+}
+// The plan as the product makes it, for its tests: columns, blocks along K of the tiles behind `whole`, `whole`, tiles.
+LSB_API void lsb_gemm_f32_split_plan(int M, int N, int K, long long* plan) {
+    const SplitPlan p = split_plan(M, N, K);
+    plan[0] = p.columns;
+    plan[1] = p.splits;
+    plan[2] = p.whole;
+    plan[3] = p.tiles;
 }
 template <int BN>
 static int run_split(const TileParams& p, const SplitPlan& plan, cudaStream_t stream) {

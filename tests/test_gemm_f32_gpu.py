@@ -52,11 +52,20 @@ def test_split_products(M, N, K, activation):
     _check(M, N, K, activation)
 
 
-def test_split_products_are_made_in_both_widths():
-    """The shapes above take blocks of 64 columns and of 128 (on the 148 SMs of a B200)."""
+def split_plan(M, N, K):
+    """(columns, parts of K, tiles whose blocks take all of K, tiles) as the product makes them."""
+    import ctypes
     from llm_singularity_b200 import kernels as ops
-    columns = ops._lib("gemm_f32").lsb_gemm_f32_split_columns
-    assert [columns(M, N) for M, N in ((17, 64), (129, 66), (300, 3002), (500, 2048), (257, 9000), (200, 20002))] == [64] * 4 + [128] * 2
+    plan = (ctypes.c_longlong * 4)()
+    ops._lib("gemm_f32").lsb_gemm_f32_split_plan(M, N, K, plan)
+    return tuple(plan)
+
+
+def test_split_products_are_made_in_both_widths():
+    """The shapes above take blocks of 64 columns and of 128, whole and shared out (on the 148 SMs of a B200)."""
+    kinds = {(columns, parts > 1, whole > 0) for columns, parts, whole, _ in
+             (split_plan(*s) for s in ((17, 64, 4100), (129, 66, 4096), (300, 3002, 540), (500, 2048, 2052), (257, 9000, 512), (200, 20002, 544)))}
+    assert {(64, True, False), (64, False, True), (128, True, False), (128, True, True)} <= kinds
 
 
 @pytest.mark.parametrize("N", [700, 20000])

@@ -3,13 +3,24 @@ numbers that only one part of K knows to be small."""
 import pytest
 import torch
 
-from test_gemm_f32_gpu import _check
+from test_gemm_f32_gpu import _check, split_plan
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M, N, K", [(17, 64, 4100), (17, 130, 640), (40, 2048, 8192), (129, 2050, 1156), (150, 2048, 2048), (300, 3074, 2052),
-                                     (500, 2048, 1540), (500, 9600, 1024), (640, 4098, 772)])
+SHAPES = [(17, 64, 4100), (17, 130, 640), (40, 2048, 8192), (129, 2050, 1156), (150, 2048, 2048), (300, 3074, 2052), (500, 2048, 1540),
+          (500, 9600, 1024), (640, 4098, 772), (129, 66, 4096)]
+
+
+def test_the_shapes_take_what_they_are_for():
+    plans = [split_plan(*s) for s in SHAPES]
+    parts = {p for _, p, _, _ in plans}
+    assert {2, 4, 5, 6, 7, 8} <= parts
+    assert any(p > 1 and 0 < whole < tiles for _, p, whole, tiles in plans)                  # whole tiles and shared-out ones
+    assert any(-(-K // 128) % p for (_, _, K), (_, p, _, _) in zip(SHAPES, plans))           # a last part that is short
+
+
+@pytest.mark.parametrize("M, N, K", SHAPES)
 @pytest.mark.parametrize("activation", [None, "silu"])
 def test_parts_of_k(M, N, K, activation):
     _check(M, N, K, activation)
