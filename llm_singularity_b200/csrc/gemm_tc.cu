@@ -241,16 +241,22 @@ __device__ __forceinline__ void store_chunk(const GemmParams& prm, uint32_t (&r)
     const int ncols = min(n, prm.rows_q - j);              // may be <= 0
     if (prm.swiglu == 2) {
         // rows alternate gate, up: even lanes hold gates, their odd neighbours the matching ups
+        // (eight at a time, the rest moved down: 32 of them in a row are more code than the instruction cache likes, an
+        // index that is not known puts r in local memory)
+#pragma unroll 1
+        for (int x0 = 0; x0 < n; x0 += 8) {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) {
-            if (x >= n) continue;                              // (every lane alike)
-            const float v = __uint_as_float(r[x]);
-            const float other = __shfl_xor_sync(0xffffffffu, v, 1);
-            if (!(lane & 1) && row_ok && x < ncols) {
-                const long long o = (long long)(i >> 1) * prm.ldc_i + (long long)(j + x) * prm.ldc_j;
-                if (prm.out_f32) put<float>(prm.out, o, silu_mul(v, other));
-                else put<bf16>(prm.out, o, silu_mul(v, other));
+            for (int x = 0; x < 8; ++x) {
+                const float v = __uint_as_float(r[x]);
+                const float other = __shfl_xor_sync(0xffffffffu, v, 1);
+                if (!(lane & 1) && row_ok && x0 + x < ncols) {
+                    const long long o = (long long)(i >> 1) * prm.ldc_i + (long long)(j + x0 + x) * prm.ldc_j;
+                    if (prm.out_f32) put<float>(prm.out, o, silu_mul(v, other));
+                    else put<bf16>(prm.out, o, silu_mul(v, other));
+                }
             }
+#pragma unroll
+            for (int x = 0; x < 24; ++x) r[x] = r[x + 8];
         }
         return;
     }
@@ -462,7 +468,8 @@ struct SmemLayout {
 };
 
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(kGemmThreads)
+// (Without the 1 the compiler takes 56 registers, and spills, for more blocks an SM than there is shared memory for.)
+__global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                const GemmParams prm) {
     using L = SmemLayout<BN, STAGES>;
@@ -627,16 +634,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             const bool rows_whole = prm.ldc_j == 1 && (prm.ldc_i & 3) == 0 && (((uintptr_t)prm.out) & 15) == 0;
             // A block's share is every splits-th group of eight rows.  Weights on the tile's rows, bfloat16: eight rows of a
             // column are 16 bytes of the output, so the sums change places in shared memory behind the partial tile and
-            // every column of a group leaves in one store (64 rows times 5,120 x 3,072: 12.9 us with stores of single values, 2 bytes on a
-            // line each, 11.4 so).  A lane a row in the reads from the peers, so that stores are runs by themselves, is slower
+            // every column of a group leaves in one store (64 rows times 8,192 x 4,096: 16.6 us with stores of single values, 2 bytes on a
+            // line each, 15.9 so; 128 times 5,120 x 2,048 18.9 and 12.1).  A lane a row in the reads from the peers, so that stores are runs by themselves, is slower
             // than either (64 x 3,072 x 2,048: 12.5 us, 8.5, 8.0): distributed shared memory wants neighbouring lanes at neighbouring places.
-            const bool turned = prm.ldc_i == 1 && prm.ldc_j != 1 && !prm.out_f32 && (prm.rows_p & 7) == 0 && (prm.ldc_j & 7) == 0 &&
+            // With fewer than 64 columns to a block's 128 threads the second pass costs more than it saves (32 rows times 2,048 x 2,048 in
+            // eight parts 5.4 us so, 5.2 without; 8,192 x 2,048 in four 9.0 and 9.5).
+            const bool turned = kBM / 8 * BN > 64 * prm.splits && prm.ldc_i == 1 && prm.ldc_j != 1 && !prm.out_f32 && (prm.rows_p & 7) == 0 && (prm.ldc_j & 7) == 0 &&
                                 (((uintptr_t)prm.out) & 15) == 0;
             bf16* turn = reinterpret_cast<bf16*>(stages + (size_t)kBM * BN * 4);           // [group][4][BN / 4][8 rows]
-            const int groups = (kBM / 8 - (int)rank + prm.splits - 1) / prm.splits;
-            for (int e = t; e < groups * 2 * BN; e += 128) {
-                const int group = (int)rank + e / (2 * BN) * prm.splits;
-                const int row = group * 8 + e % (2 * BN) / (BN / 4), c4 = e % (BN / 4);
+            auto summed = [&](int row, int c4) -> float4 {
                 const uint4* src = part + (size_t)row * (BN / 4) + (c4 ^ (row & kPartSwizzle));
                 float4 v[8];                                  // all peers' loads in flight at once
 #pragma unroll
@@ -650,35 +656,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                     acc.x = plain_act(acc.x, prm.plain); acc.y = plain_act(acc.y, prm.plain);
                     acc.z = plain_act(acc.z, prm.plain); acc.w = plain_act(acc.w, prm.plain);
                 }
-                const int i = i0 + row, j = j0 + c4 * 4;
-                if (turned) {
+                return acc;
+            };
+            if (turned) {
+                const int groups = (kBM / 8 - (int)rank + prm.splits - 1) / prm.splits;
+                for (int e = t; e < groups * 2 * BN; e += 128) {
+                    const int group = (int)rank + e / (2 * BN) * prm.splits;
+                    const int row = group * 8 + e % (2 * BN) / (BN / 4), c4 = e % (BN / 4);
+                    const float4 acc = summed(row, c4);
                     const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
                     for (int x = 0; x < 4; ++x)
                         turn[(group * BN + x * (BN / 4) + c4) * 8 + (row & 7)] = __float2bfloat16_rn(vals[x]);
-                } else if (i < prm.rows_p) {
-                    const long long o0 = (long long)i * prm.ldc_i + (long long)j * prm.ldc_j;
-                    if (rows_whole && j + 3 < prm.rows_q) {
-                        if (prm.out_f32) {
-                            *reinterpret_cast<float4*>(reinterpret_cast<float*>(prm.out) + o0) = acc;
-                        } else {
-                            const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y);
-                            const __nv_bfloat162 hi = __floats2bfloat162_rn(acc.z, acc.w);
-                            *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(prm.out) + o0) =
-                                make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-                        }
-                    } else {
-                        const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
-                        for (int x = 0; x < 4; ++x) {
-                            if (j + x >= prm.rows_q) break;
-                            const long long o = o0 + (long long)x * prm.ldc_j;
-                            if (prm.out_f32) put<float>(prm.out, o, vals[x]);
-                            else put<bf16>(prm.out, o, vals[x]);
-                        }
-                    }
                 }
-            }
-            if (turned) {
                 asm volatile("bar.sync 2, 128;" ::: "memory");                      // the four epilogue warps
                 for (int e = t; e < groups * BN; e += 128) {
                     const int group = (int)rank + e / BN * prm.splits, jj = e % BN;
@@ -686,6 +676,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                     if (i < prm.rows_p && j < prm.rows_q)
                         *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(prm.out) + i + (long long)j * prm.ldc_j) =
                             *reinterpret_cast<const uint4*>(turn + (group * BN + jj) * 8);
+                }
+            } else {
+                for (int g4 = (int)rank * 128 + t; g4 < kBM * BN / 4; g4 += prm.splits * 128) {
+                    const int row = g4 / (BN / 4), c4 = g4 % (BN / 4);
+                    const float4 acc = summed(row, c4);
+                    const int i = i0 + row, j = j0 + c4 * 4;
+                    if (i < prm.rows_p) {
+                        const long long o0 = (long long)i * prm.ldc_i + (long long)j * prm.ldc_j;
+                        if (rows_whole && j + 3 < prm.rows_q) {
+                            if (prm.out_f32) {
+                                *reinterpret_cast<float4*>(reinterpret_cast<float*>(prm.out) + o0) = acc;
+                            } else {
+                                const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y);
+                                const __nv_bfloat162 hi = __floats2bfloat162_rn(acc.z, acc.w);
+                                *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(prm.out) + o0) =
+                                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                            }
+                        } else {
+                            const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
+                            for (int x = 0; x < 4; ++x) {
+                                if (j + x >= prm.rows_q) break;
+                                const long long o = o0 + (long long)x * prm.ldc_j;
+                                if (prm.out_f32) put<float>(prm.out, o, vals[x]);
+                                else put<bf16>(prm.out, o, vals[x]);
+                            }
+                        }
+                    }
                 }
             }
         }
