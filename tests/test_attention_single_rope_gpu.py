@@ -44,7 +44,14 @@ def _both(dtype, nh, nkv, hd, rotary, q_lens, kv_lens, window, store, captured):
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
     if store:
         assert torch.equal(va, vb) and bool(((ka - kb).abs() <= 4 * eps * (1 + ka.abs())).all())
-    assert bool(((a.double() - b.double()).abs() <= 40 * eps * (1 + a.double().abs())).all())
+    a, b = a.double().view(T, nh, hd), b.double().view(T, nh, hd)
+    if dtype == torch.bfloat16:
+        # results are rounded once (2^-9 of each); a rotated element that is rounded the other way is 2^-8 of it off, which moves a
+        # score of size 1 and the outputs of its head by no more than that; few are, so that all outputs together agree better still
+        rms = a.square().mean(-1, keepdim=True).sqrt()
+        assert bool(((a - b).abs() <= 2 * eps * (a.abs() + rms)).all()) and (a - b).norm().item() <= eps * a.norm().item()
+    else:
+        assert bool(((a - b).abs() <= 40 * eps * (1 + a.abs())).all())
     assert not b.isnan().any()
 
 
