@@ -159,6 +159,11 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) chunk_gain_f32_kernel(
 
 constexpr int kChainThreads = 128;
 
+// AHEAD: chunks whose loads are in flight at once.  A thread's chain is bound by their latency, so 24 where the longest request has more
+// than 8 chunks; for fewer 24 loads would be of the last one again, in registers that other blocks then lack (all three kernels, 16
+// heads of 128 x 128, us, with 8 / 24: 65 tokens 42.3 / 44.1, 16 requests of 40 68.5 / 81.5, 500 tokens 49.8 / 51.1, 520 52.3 /
+// 51.4, 1,000 70.5 / 65.7, 1,500 84.5 / 77.5, 4,000 226 / 202; a ring of 16, each loaded again as it is used, 1,500 81.7).
+template <int AHEAD>
 __global__ void __launch_bounds__(kChainThreads) chunk_chain_f32_kernel(ScanArgs a) {
     __shared__ float fade[2];                                   // over a whole chunk, and over the request's last
     lsb_pdl_launch_dependents();
@@ -180,16 +185,12 @@ __global__ void __launch_bounds__(kChainThreads) chunk_chain_f32_kernel(ScanArgs
     float4 cur = known ? *reinterpret_cast<const float4*>(st) : make_float4(0.f, 0.f, 0.f, 0.f);
     float* at = a.gain + ((size_t)(q0 / kL + r) * a.heads + h) * per + i;
     const size_t step = (size_t)a.heads * per;
-    // 24 chunks' loads in flight at once: a thread's chain is bound by their latency, not by what an SM can hold (all three
-    // kernels, 16 heads of 128 x 128, us, with 8 / 16 / 24: 400 tokens 54.8 / 53.5 / 53.3, 1,000 74.5 / 70.4 / 70.0, 1,500
-    // 87.0 / 82.5 / 80.0, 4,000 231 / 212 / 209; a ring of 16, each loaded again as it is used, 52.7 / 69.8 / 81.7 / 213)
-    constexpr int kAhead = 24;
-    for (int s0 = 0; s0 < chunks; s0 += kAhead) {
-        float4 e[kAhead];
+    for (int s0 = 0; s0 < chunks; s0 += AHEAD) {
+        float4 e[AHEAD];
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) e[k] = *reinterpret_cast<const float4*>(at + min(s0 + k, chunks - 1) * step);
+        for (int k = 0; k < AHEAD; ++k) e[k] = *reinterpret_cast<const float4*>(at + min(s0 + k, chunks - 1) * step);
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) {
+        for (int k = 0; k < AHEAD; ++k) {
             if (s0 + k < chunks) {
                 *reinterpret_cast<float4*>(at + (s0 + k) * step) = cur;
                 const float f = fade[s0 + k == chunks - 1];
@@ -425,8 +426,8 @@ static int run(ScanArgs a, int n_requests, int chunks, cudaStream_t stream) {
     int rc = lsb_launch(chunk_gain_f32_kernel<NP, VP, GAIN>, grid, dim3(GAIN), gain_sm, stream, 1, a);
     if (rc) return rc;
     const int per = a.V * a.N / 4;
-    rc = lsb_launch(chunk_chain_f32_kernel, dim3((per + kChainThreads - 1) / kChainThreads, a.heads, n_requests), dim3(kChainThreads), 0,
-                    stream, 1, a);
+    rc = lsb_launch(chunks > 8 ? chunk_chain_f32_kernel<24> : chunk_chain_f32_kernel<8>,
+                    dim3((per + kChainThreads - 1) / kChainThreads, a.heads, n_requests), dim3(kChainThreads), 0, stream, 1, a);
     if (rc) return rc;
     return lsb_launch(chunk_output_f32_kernel<NP, VP, kOutThreads>, grid, dim3(kOutThreads), out_sm, stream, 1, a);
 }

@@ -1,4 +1,4 @@
-"""The chain through a portion's chunks takes 24 at a time: lengths around one and two such batches, beside a short request,
+"""The chain through a portion's chunks takes 8 or 24 at a time: lengths around one and two such batches, beside a short request,
 against the token-by-token recurrence in float64."""
 import pytest
 import torch
@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("tokens", [24 * 64 - 1, 24 * 64, 24 * 64 + 1, 25 * 64, 48 * 64 + 1])
+@pytest.mark.parametrize("tokens", [8 * 64, 8 * 64 + 1, 24 * 64 - 1, 24 * 64, 24 * 64 + 1, 25 * 64, 48 * 64 + 1])
 def test_chunks_in_batches(tokens):
     from llm_singularity_b200 import kernels as K
     from llm_singularity_b200.engine.batch import ContextBuilder
