@@ -789,11 +789,15 @@ def _single_tokens_rotate(ctx, nh: int, nkv: int, hd: int, device) -> bool:
     same: 8 tokens at 2,000 keys and a portion of 40, head size 64, 66.5 us with and 70.3 without it) whose blocks the
     SMs hold at once (64 tokens at 500 keys, 8 kv heads of 128: 117 us with the rotary kernel, 119 without; 8 at 1,000 52 and
     49)."""
-    n_decode = _batch_shape(ctx)[0]
-    if n_decode != ctx.n_requests or nkv <= 0 or hd <= 0:     # (what no kernel takes is refused further on)
-        return False
-    heads = max(1, 1024 // hd)                                # most query heads of a block
-    return n_decode * nkv * -(-(nh // nkv) // heads) <= 2 * num_sms(device)
+    kept = getattr(ctx, "_rotation", None)                    # (worked out once per step and kind of layer)
+    if kept is not None and kept[0] == (nh, nkv, hd):
+        return kept[1]
+    n_decode, rotates = _batch_shape(ctx)[0], False
+    if n_decode == ctx.n_requests and nkv > 0 and hd > 0:     # (what no kernel takes is refused further on)
+        heads = max(1, 1024 // hd)                            # most query heads of a block
+        rotates = n_decode * nkv * -(-(nh // nkv) // heads) <= 2 * num_sms(device)
+    ctx._rotation = ((nh, nkv, hd), rotates)
+    return rotates
 
 
 def rope_store_attention(qkv: torch.Tensor, nh: int, nkv: int, hd: int, ctx, cache,
